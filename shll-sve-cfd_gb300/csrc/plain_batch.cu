@@ -69,6 +69,7 @@ PlainBatch* plain_batch_create(const shll_params* p, int count, cudaStream_t s, 
         it.g.DT_ON_DY = dt / dy;
         it.g.alpha = q.mc_alpha;
         it.g.limiter = q.limiter;
+        finish_gas(it.g);
         b->items.push_back(it);
         off += (long)it.nx * it.ny;
     }

@@ -15,18 +15,56 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
+#include "exact_math.cuh"
 #include "shll_internal.h"
 
 namespace SHLL_PLAIN_NS {
 
 #define D(x) ((double)(x))
 
+// A multiplication by a grid constant (DT_ON_DX and the like): by a power of two 2^k (the reference's
+// 0.25 / (R + 1)) it moves the exponent, which costs no FP64 instruction.
+template <typename REAL>
+struct Factor {
+    REAL v;
+    int k;
+    bool pow2;
+};
+template <typename REAL>
+__host__ Factor<REAL> make_factor(REAL v) {
+    Factor<REAL> f;
+    int ex = 0;
+    f.v = v;
+    f.pow2 = std::frexp((double)v, &ex) == 0.5 && ex > -500 && ex < 500;
+    f.k = ex - 1;
+    return f;
+}
+
 template <typename REAL>
 struct Gas {
     REAL R, GAMMA, CV, DT_ON_DX, DT_ON_DY, alpha;
     int limiter;
+    // derived (finish_gas)
+    bool R_one;                                        // R == 1: products with it are skipped
+    REAL gR;                                           // GAMMA * R
+    REAL rCV;                                          // about 1 / CV (float arithmetic)
+    exact_math::Divisor cv;                            // CV as a divisor (FP64 arithmetic)
+    Factor<REAL> lx, ly, hlx, hly;                     // DT_ON_DX, DT_ON_DY and 0.5 times them
 };
+
+template <typename REAL>
+__host__ void finish_gas(Gas<REAL>& g) {
+    g.R_one = g.R == (REAL)1;
+    g.gR = g.GAMMA * g.R;
+    g.rCV = (REAL)1 / g.CV;
+    g.cv = exact_math::divisor((double)g.CV);
+    g.lx = make_factor<REAL>(g.DT_ON_DX);
+    g.ly = make_factor<REAL>(g.DT_ON_DY);
+    g.hlx = make_factor<REAL>((REAL)0.5 * g.DT_ON_DX);
+    g.hly = make_factor<REAL>((REAL)0.5 * g.DT_ON_DY);
+}
 
 template <typename REAL>
 __host__ Gas<REAL> make_gas(const PlainArgs& a) {
@@ -34,50 +72,118 @@ __host__ Gas<REAL> make_gas(const PlainArgs& a) {
     g.R = (REAL)a.R; g.GAMMA = (REAL)a.GAMMA; g.CV = (REAL)a.CV;
     g.DT_ON_DX = (REAL)a.DT_ON_DX; g.DT_ON_DY = (REAL)a.DT_ON_DY;
     g.alpha = (REAL)a.mc_alpha; g.limiter = a.limiter;
+    finish_gas(g);
     return g;
 }
 
+// ---- the reference's expressions, FP64 ----
+// FP64 instructions are the scarce resource of these kernels (19 clocks per warp instruction per
+// SM), so divisions, square roots, comparisons and power-of-two scalings run on the integer pipes
+// (exact_math.cuh) with the same results; the float arithmetic does without FP64.  Measured: one
+// 2D step of 256 x 256 cells in FP64 40.3 -> 25.9 us, of 301 x 277 in float (second order) 29.5 ->
+// 13.4 us, one 1D step of 3001 cells (FP64, second order) 20.5 -> 16.4 us.
+__device__ __forceinline__ double half_of(double x) { return exact_math::scale_pow2(x, -1, 0.5); }
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+// 0.5 * (x + c) (the scaling is exact: one fused operation rounds like the sum)
+__device__ __forceinline__ double half_sum(double x, double c) { return __fma_rn(0.5, x, 0.5 * c); }
+__device__ __forceinline__ float half_sum(float x, float c) { return __fmul_rn(0.5f, __fadd_rn(x, c)); }
+__device__ __forceinline__ bool positive(double x) {
+    const long long b = __double_as_longlong(x);
+    return b > 0 && b <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool positive(float x) { return x > 0.f; }
+// u - f * x
+__device__ __forceinline__ double sub_scaled(double u, const Factor<double>& f, double x) {
+    return f.pow2 ? u - exact_math::scale_pow2(x, f.k, f.v) : u - f.v * x;
+}
+__device__ __forceinline__ float sub_scaled(float u, const Factor<float>& f, float x) { return u - f.v * x; }
+// (REAL)(D(u) - 0.5 * D(lambda) * D(x)), f = 0.5 * lambda
+__device__ __forceinline__ double sub_half_scaled(double u, const Factor<double>& f, double x) {
+    return sub_scaled(u, f, x);
+}
+__device__ __forceinline__ float sub_half_scaled(float u, const Factor<float>& f, float x) {
+    return exact_math::sub_product_ref(u, f.v, x);
+}
+// a divisor used for several quotients
+template <typename REAL>
+struct Den;
+template <>
+struct Den<double> {
+    exact_math::Divisor d;
+    __device__ __forceinline__ explicit Den(double b) : d(exact_math::divisor(b)) {}
+    __device__ __forceinline__ double divide(double a) const { return exact_math::divide(a, d); }
+};
+template <>
+struct Den<float> {
+    float b;
+    __device__ __forceinline__ explicit Den(float x) : b(x) {}
+    __device__ __forceinline__ float divide(float a) const { return a / b; }
+};
 // sqrt of a REAL argument as the reference evaluates it: sqrt(double) rounded to REAL.  For
 // float this equals the correctly rounded sqrtf (53 >= 2*24+2, so the double rounding is exact).
 __device__ __forceinline__ float sqrt_ref(float x) { return sqrtf(x); }
-__device__ __forceinline__ double sqrt_ref(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrt_ref(double x) { return exact_math::square_root(x); }
+// the Z2 of a split flux, (REAL)(0.5 * D(a) * (1.0 - D(M * M)))
+__device__ __forceinline__ double z2(double a, double M) { return half_of(a) * (1.0 - M * M); }
+__device__ __forceinline__ float z2(float a, float M) { return exact_math::z2_ref(a, M * M); }
+// temperature from the specific energy e, (REAL)((D(e) - 0.5 * kinetic) / D(CV)): 1D kinetic =
+// D(p1) * D(p1) (0.5 * D(p1) taken first), 2D the REAL p1 * p1 + p2 * p2
+__device__ __forceinline__ double temp1(const Gas<double>& g, double e, double p1) {
+    return exact_math::divide(e - half_of(p1) * p1, g.cv);
+}
+__device__ __forceinline__ float temp1(const Gas<float>& g, float e, float p1) {
+    const float kh = __fmul_rn(p1, p1);
+    return exact_math::temperature_ref(e, 0.5f * kh, 0.5f * __fmaf_rn(p1, p1, -kh), g.CV, g.rCV);
+}
+__device__ __forceinline__ double temp2(const Gas<double>& g, double e, double p1, double p2) {
+    return exact_math::divide(e - half_of(p1 * p1 + p2 * p2), g.cv);
+}
+__device__ __forceinline__ float temp2(const Gas<float>& g, float e, float p1, float p2) {
+    return exact_math::temperature_ref(e, 0.5f * (p1 * p1 + p2 * p2), 0.f, g.CV, g.rCV);
+}
+template <typename REAL>
+__device__ __forceinline__ REAL times_R(const Gas<REAL>& g, REAL x) { return g.R_one ? x : x * g.R; }
 
 // ---------------- 1D ----------------
 // P from U (base_shll.c:171-176); returns p1 (velocity), p2 (temperature), a (sound speed)
 template <typename REAL>
 __device__ __forceinline__ void prim1(const Gas<REAL>& g, REAL u0, REAL u1, REAL u2, REAL& p1, REAL& p2, REAL& a) {
-    p1 = u1 / u0;
-    p2 = (REAL)((D(u2 / u0) - 0.5 * D(p1) * D(p1)) / D(g.CV));
-    a = sqrt_ref(g.GAMMA * g.R * p2);
+    const Den<REAL> rho(u0);
+    p1 = rho.divide(u1);
+    p2 = temp1(g, rho.divide(u2), p1);
+    a = sqrt_ref(g.gR * p2);
 }
 
 // split fluxes (base_shll.c:134-158) from P (p0 = u0) and U
 template <typename REAL>
 __device__ __forceinline__ void flux1(const Gas<REAL>& g, REAL u0, REAL u1, REAL u2, REAL p1, REAL p2, REAL a,
                                       REAL fp[3], REAL fm[3]) {
-    REAL M = p1 / a;
-    REAL Z1 = (REAL)(0.5 * (D(M) + 1.0));
-    REAL Z2 = (REAL)(0.5 * D(a) * (1.0 - D(M * M)));
-    REAL Z3 = (REAL)(0.5 * (D(M) - 1.0));
-    REAL P = u0 * g.R * p2;
+    REAL M = Den<REAL>(a).divide(p1);
+    REAL Z1 = half_sum(M, (REAL)1);
+    REAL Z2 = z2(a, M);
+    REAL Z3 = half_sum(M, (REAL)-1);
+    REAL P = times_R(g, u0) * p2;
     REAL f0 = u1, f1 = u1 * p1 + P, f2 = p1 * (u2 + P);
     fp[0] = f0 * Z1 + u0 * Z2; fp[1] = f1 * Z1 + u1 * Z2; fp[2] = f2 * Z1 + u2 * Z2;
     fm[0] = -f0 * Z3 - u0 * Z2; fm[1] = -f1 * Z3 - u1 * Z2; fm[2] = -f2 * Z3 - u2 * Z2;
 }
 
 // minmod (2nd_order_base_shll.c:191-201)
-template <typename REAL>
-__device__ __forceinline__ REAL minmod(REAL l, REAL r) {
-    if (l * r < 0.0) return (REAL)0.0;
-    return (fabs(D(l)) < fabs(D(r))) ? l : r;
+__device__ __forceinline__ double minmod(double l, double r) {
+    if (exact_math::product_negative(l, r)) return 0.0;
+    return exact_math::magnitude_less(l, r) ? l : r;
+}
+__device__ __forceinline__ float minmod(float l, float r) {
+    if (__fmul_rn(l, r) < 0.f) return 0.f;
+    return fabsf(l) < fabsf(r) ? l : r;
 }
 // slope of a split flux at an interior cell: minmod, or the MC limiter of
 // base-omp/2nd_order_base_shll.c:316-325
 template <typename REAL>
 __device__ __forceinline__ REAL slope(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr) {
     if (g.limiter == 1)
-        return minmod<REAL>((REAL)(0.5 * D(fr - fl)), g.alpha * minmod<REAL>(fc - fl, fr - fc));
-    return minmod<REAL>(fc - fl, fr - fc);
+        return minmod(half_of(fr - fl), g.alpha * minmod(fc - fl, fr - fc));
+    return minmod(fc - fl, fr - fc);
 }
 
 constexpr int T1 = 256;  // cells per block (1D)
@@ -101,7 +207,7 @@ __device__ __forceinline__ void step1_block(const REAL* __restrict__ Uin, REAL* 
             REAL u0 = Uin[c], u1 = Uin[stride + c], u2 = Uin[2 * stride + c], p1, p2, a;
             prim1(g, u0, u1, u2, p1, p2, a);
             flux1(g, u0, u1, u2, p1, p2, a, fp, fm);
-            bad |= !(u0 > (REAL)0) || !(p2 > (REAL)0);
+            bad |= !positive(u0) || !positive(p2);
         }
 #pragma unroll
         for (int k = 0; k < 3; k++) { sfp[k][t] = fp[k]; sfm[k][t] = fm[k]; }
@@ -134,15 +240,15 @@ __device__ __forceinline__ void step1_block(const REAL* __restrict__ Uin, REAL* 
             if (i == 0) { L = sg * fm; Rr = sfm[k][s + 1]; }
             else if (i == n - 1) { L = sfp[k][s - 1]; Rr = sg * fp; }
             else { L = sfp[k][s - 1]; Rr = sfm[k][s + 1]; }
-            u = u - g.DT_ON_DX * (fp - fm + Rr - L);
+            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
         } else {
             const int d = threadIdx.x + 1;  // slope index of cell i
             REAL Ldf, Rdf;
             if (i == 0) { L = fp; Rr = sfm[k][s + 1]; Ldf = 0; Rdf = sdm[k][d + 1]; }
             else if (i == n - 1) { L = sfp[k][s - 1]; Rr = fm; Ldf = sdp[k][d - 1]; Rdf = 0; }
             else { L = sfp[k][s - 1]; Rr = sfm[k][s + 1]; Ldf = sdp[k][d - 1]; Rdf = sdm[k][d + 1]; }
-            u = u - g.DT_ON_DX * (fp - fm + Rr - L);
-            u = (REAL)(D(u) - 0.5 * D(g.DT_ON_DX) * D(sdp[k][d] + sdm[k][d] - Rdf - Ldf));
+            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
+            u = sub_half_scaled(u, g.hlx, sdp[k][d] + sdm[k][d] - Rdf - Ldf);
         }
         Uout[k * stride + i] = u;
     }
@@ -158,28 +264,30 @@ __global__ void __launch_bounds__(T1) k_step1(const REAL* __restrict__ Uin, REAL
 template <typename REAL>
 __device__ __forceinline__ void prim2(const Gas<REAL>& g, REAL u0, REAL u1, REAL u2, REAL u3, REAL& p1, REAL& p2,
                                       REAL& p3, REAL& a) {
-    p1 = u1 / u0;
-    p2 = u2 / u0;
-    p3 = (REAL)((D(u3 / u0) - 0.5 * D(p1 * p1 + p2 * p2)) / D(g.CV));
-    a = sqrt_ref(g.GAMMA * g.R * p3);
+    const Den<REAL> rho(u0);
+    p1 = rho.divide(u1);
+    p2 = rho.divide(u2);
+    p3 = temp2(g, rho.divide(u3), p1, p2);
+    a = sqrt_ref(g.gR * p3);
 }
 
 // x and y split fluxes (base_shll_2d.c:243-299)
 template <typename REAL>
 __device__ __forceinline__ void flux2(const Gas<REAL>& g, const REAL u[4], REAL p1, REAL p2, REAL p3, REAL a,
                                       REAL fp[4], REAL fm[4], REAL hp[4], REAL hm[4]) {
-    REAL P = u[0] * g.R * p3;
-    REAL M = p1 / a;
-    REAL Z1 = (REAL)(0.5 * (D(M) + 1.0));
-    REAL Z2 = (REAL)(0.5 * D(a) * (1.0 - D(M * M)));
-    REAL Z3 = (REAL)(0.5 * (D(M) - 1.0));
+    REAL P = times_R(g, u[0]) * p3;
+    const Den<REAL> da(a);
+    REAL M = da.divide(p1);
+    REAL Z1 = half_sum(M, (REAL)1);
+    REAL Z2 = z2(a, M);
+    REAL Z3 = half_sum(M, (REAL)-1);
     REAL f[4] = {u[1], u[1] * p1 + P, u[1] * p2, p1 * (u[3] + P)};
 #pragma unroll
     for (int k = 0; k < 4; k++) { fp[k] = f[k] * Z1 + u[k] * Z2; fm[k] = -f[k] * Z3 - u[k] * Z2; }
-    M = p2 / a;
-    Z1 = (REAL)(0.5 * (D(M) + 1.0));
-    Z2 = (REAL)(0.5 * D(a) * (1.0 - D(M * M)));
-    Z3 = (REAL)(0.5 * (D(M) - 1.0));
+    M = da.divide(p2);
+    Z1 = half_sum(M, (REAL)1);
+    Z2 = z2(a, M);
+    Z3 = half_sum(M, (REAL)-1);
     REAL h[4] = {u[2], u[2] * p1, u[2] * p2 + P, p2 * (u[3] + P)};
 #pragma unroll
     for (int k = 0; k < 4; k++) { hp[k] = h[k] * Z1 + u[k] * Z2; hm[k] = -h[k] * Z3 - u[k] * Z2; }
@@ -227,7 +335,7 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             REAL u[4] = {Uin[c], Uin[n + c], Uin[2 * n + c], Uin[3 * n + c]}, p1, p2, p3, a;
             prim2(g, u[0], u[1], u[2], u[3], p1, p2, p3, a);
             flux2(g, u, p1, p2, p3, a, fp, fm, hp, hm);
-            bad |= !(u[0] > (REAL)0) || !(p3 > (REAL)0);
+            bad |= !positive(u[0]) || !positive(p3);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -286,8 +394,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = sy * hm; Tt = F(3, k, li, lj + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = sy * hp; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); }
-            u = u - g.DT_ON_DX * (fp - fm + Rr - L);
-            u = u - g.DT_ON_DY * (hp - hm + Tt - B);
+            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
+            u = sub_scaled(u, g.ly, hp - hm + Tt - B);
         } else {
             // outflow walls, slopes zero on edge cells (2nd_order_base_shll.c:210-458)
             auto DX_ = [&](int q, int r) -> REAL { return sd[(q * 4 + k) * NXS + r * TJ + threadIdx.x]; };
@@ -302,10 +410,10 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = hp; Tt = F(3, k, li, lj + 1); Bdf = 0; Tdf = DY_(1, cc + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = hm; Bdf = DY_(0, cc - 1); Tdf = 0; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); Bdf = DY_(0, cc - 1); Tdf = DY_(1, cc + 1); }
-            u = u - g.DT_ON_DX * (fp - fm + Rr - L);
-            u = (REAL)(D(u) - 0.5 * D(g.DT_ON_DX) * D(DX_(0, r) + DX_(1, r) - Rdf - Ldf));
-            u = u - g.DT_ON_DY * (hp - hm + Tt - B);
-            u = (REAL)(D(u) - 0.5 * D(g.DT_ON_DY) * D(DY_(0, cc) + DY_(1, cc) - Tdf - Bdf));
+            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
+            u = sub_half_scaled(u, g.hlx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
+            u = sub_scaled(u, g.ly, hp - hm + Tt - B);
+            u = sub_half_scaled(u, g.hly, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
         }
         Uout[k * n + c] = u;
     }
@@ -344,12 +452,12 @@ __global__ void k_p_from_u(const REAL* __restrict__ U, REAL* __restrict__ P, lon
             REAL u0 = U[c], p1, p2, a;
             prim1(g, u0, U[n + c], U[2 * n + c], p1, p2, a);
             P[c] = u0; P[n + c] = p1; P[2 * n + c] = p2; P[3 * n + c] = a;
-            bad |= !(u0 > (REAL)0) || !(p2 > (REAL)0);
+            bad |= !positive(u0) || !positive(p2);
         } else {
             REAL u0 = U[c], p1, p2, p3, a;
             prim2(g, u0, U[n + c], U[2 * n + c], U[3 * n + c], p1, p2, p3, a);
             P[c] = u0; P[n + c] = p1; P[2 * n + c] = p2; P[3 * n + c] = p3; P[4 * n + c] = a;
-            bad |= !(u0 > (REAL)0) || !(p3 > (REAL)0);
+            bad |= !positive(u0) || !positive(p3);
         }
     }
     if (bad) atomicOr(flag, SHLL_FLAG_NONPOSITIVE);
@@ -394,7 +502,7 @@ __global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ f
                 if (i == 0) { L = sx * Fm[c]; Rr = Fm[c + sx_]; }
                 else if (i == nx - 1) { L = Fp[c - sx_]; Rr = sx * Fp[c]; }
                 else { L = Fp[c - sx_]; Rr = Fm[c + sx_]; }
-                u = u - g.DT_ON_DX * (Fp[c] - Fm[c] + Rr - L);
+                u = sub_scaled(u, g.lx, Fp[c] - Fm[c] + Rr - L);
                 if (dim == 2) {
                     const REAL* Hp = hp + k * n; const REAL* Hm = hm + k * n;
                     const REAL sy = (k == 2) ? (REAL)1 : (REAL)-1;
@@ -402,7 +510,7 @@ __global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ f
                     if (j == 0) { B = sy * Hm[c]; Tt = Hm[c + 1]; }
                     else if (j == ny - 1) { B = Hp[c - 1]; Tt = sy * Hp[c]; }
                     else { B = Hp[c - 1]; Tt = Hm[c + 1]; }
-                    u = u - g.DT_ON_DY * (Hp[c] - Hm[c] + Tt - B);
+                    u = sub_scaled(u, g.ly, Hp[c] - Hm[c] + Tt - B);
                 }
             } else {
                 auto sl = [&](const REAL* f, long cc, int ii, int st, int nn) -> REAL {
@@ -416,8 +524,8 @@ __global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ f
                     L = Fp[c - sx_]; Rr = Fm[c + sx_];
                     Ldf = sl(Fp, c - sx_, i - 1, sx_, nx); Rdf = sl(Fm, c + sx_, i + 1, sx_, nx);
                 }
-                u = u - g.DT_ON_DX * (Fp[c] - Fm[c] + Rr - L);
-                u = (REAL)(D(u) - 0.5 * D(g.DT_ON_DX) * D(sl(Fp, c, i, sx_, nx) + sl(Fm, c, i, sx_, nx) - Rdf - Ldf));
+                u = sub_scaled(u, g.lx, Fp[c] - Fm[c] + Rr - L);
+                u = sub_half_scaled(u, g.hlx, sl(Fp, c, i, sx_, nx) + sl(Fm, c, i, sx_, nx) - Rdf - Ldf);
                 if (dim == 2) {
                     const REAL* Hp = hp + k * n; const REAL* Hm = hm + k * n;
                     REAL B, Tt, Bdf, Tdf;
@@ -427,8 +535,8 @@ __global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ f
                         B = Hp[c - 1]; Tt = Hm[c + 1];
                         Bdf = sl(Hp, c - 1, j - 1, 1, ny); Tdf = sl(Hm, c + 1, j + 1, 1, ny);
                     }
-                    u = u - g.DT_ON_DY * (Hp[c] - Hm[c] + Tt - B);
-                    u = (REAL)(D(u) - 0.5 * D(g.DT_ON_DY) * D(sl(Hp, c, j, 1, ny) + sl(Hm, c, j, 1, ny) - Tdf - Bdf));
+                    u = sub_scaled(u, g.ly, Hp[c] - Hm[c] + Tt - B);
+                    u = sub_half_scaled(u, g.hly, sl(Hp, c, j, 1, ny) + sl(Hm, c, j, 1, ny) - Tdf - Bdf);
                 }
             }
             U[k * n + c] = u;
