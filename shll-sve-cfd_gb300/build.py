@@ -29,7 +29,7 @@ UNITS = {
     "plain_batch_exact.cu": ["-fmad=false"],
     "refglobals.cu": [],
 }
-HEADERS = ["shll_internal.h", "shll_plain.cuh", "exact_math.cuh", "mixed.h", "mixed_common.cuh", "plain_batch.h",
+HEADERS = ["shll_internal.h", "shll_plain.cuh", "plain_resident.cuh", "exact_math.cuh", "mixed.h", "mixed_common.cuh", "plain_batch.h",
            "plain_batch_kernels.cuh"]
 
 

@@ -31,6 +31,7 @@ struct shll_ctx {
     void* P = nullptr;
     void* F[4] = {nullptr, nullptr, nullptr, nullptr};  // fp, fm, hp, hm (staged; lazily allocated)
     bool fluxes_valid = false;
+    unsigned* prog = nullptr;      // progress counters of 1D runs (allocated by the first one)
     // device checkpoint of the plain state
     void* ckU = nullptr;
     void* ckP = nullptr;
@@ -294,6 +295,7 @@ extern "C" void shll_destroy(shll_ctx* c) {
     cudaFree(c->U[0]); cudaFree(c->U[1]); cudaFree(c->P); cudaFree(c->ckU); cudaFree(c->ckP);
     for (int k = 0; k < 4; k++) cudaFree(c->F[k]);
     cudaFree(c->d_flag);
+    cudaFree(c->prog);
     if (c->mixed) mixed_destroy(c->mixed);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -470,7 +472,20 @@ extern "C" int shll_step(shll_ctx* c, long nsteps) {
         c->steps_taken += nsteps;
         return check_flag(c);
     }
-    for (long s = 0; s < nsteps; s++) {
+    // 1D: several steps per launch (plain_resident.cuh), except that a single step has nothing to share
+    if (c->p.dim == 1 && nsteps > 1) {
+        if (!c->prog && cudaMalloc(&c->prog, sizeof(unsigned) * kPlainProgStride * kPlainProgChunks) != cudaSuccess) {
+            cudaGetLastError();   // (then one launch per sweep, which needs none)
+            c->prog = nullptr;
+        }
+        PlainArgs a = plain_args(c);
+        a.Uin = c->U[c->cur];
+        a.Uout = c->U[c->cur ^ 1];
+        int swaps = 0;
+        CUDA_TRY(c, c->p.precision == SHLL_PREC_F64 ? plain_fast::run(a, nsteps, c->prog, shll_stall_chunk(), &swaps)
+                                                    : plain_exact::run(a, nsteps, c->prog, shll_stall_chunk(), &swaps));
+        c->cur ^= swaps;
+    } else for (long s = 0; s < nsteps; s++) {
         PlainArgs a = plain_args(c);
         a.Uin = c->U[c->cur];
         a.Uout = c->U[c->cur ^ 1];

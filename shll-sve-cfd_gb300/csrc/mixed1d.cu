@@ -1784,6 +1784,7 @@ static std::atomic<int> g_resident{1};
 extern "C" void shll_set_resident(int on) { g_resident = on ? 1 : 0; }
 static std::atomic<int> g_stall{-1};
 extern "C" void shll_debug_stall_chunk(int chunk) { g_stall = chunk; }
+int shll_stall_chunk() { return g_stall.load(); }
 static std::atomic<int> g_pair_flux{1};
 extern "C" void shll_set_pair_flux(int on) { g_pair_flux = on == 2 ? 2 : (on ? 1 : 0); }
 

@@ -2,10 +2,13 @@
 // rounded separately (this file is compiled with -fmad=false), IEEE division and square root:
 // bit-identical to the reference's gcc builds (which contain no fused multiply-add on x86-64).
 #define SHLL_PLAIN_NS plain_exact
-#include "shll_plain.cuh"
+#include "plain_resident.cuh"
 
 namespace plain_exact {
 cudaError_t step(const PlainArgs& a) { return a.real_bits == 32 ? step_t<float>(a) : step_t<double>(a); }
+cudaError_t run(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps) {
+    return a.real_bits == 32 ? run_t<float>(a, steps, prog, stall, swaps) : run_t<double>(a, steps, prog, stall, swaps);
+}
 cudaError_t stage(const PlainArgs& a, int which) {
     return a.real_bits == 32 ? stage_t<float>(a, which) : stage_t<double>(a, which);
 }

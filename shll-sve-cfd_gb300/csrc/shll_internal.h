@@ -20,6 +20,9 @@ void shll_ref_set_step(double dt, double dtdx, double dtdy);
 // kernel launches issued by the library (shll_kernel_launches)
 void shll_count_launches(long n);
 
+// the chunk that shll_debug_stall_chunk keeps from publishing its progress (-1: none)
+int shll_stall_chunk();
+
 enum { STAGE_U_FROM_P = 0, STAGE_P_FROM_U = 1, STAGE_F_FROM_P = 2, STAGE_UPDATE = 3 };
 
 // Arguments of the plain (reference-arithmetic) kernels.  The constants are the reference's
@@ -36,11 +39,17 @@ struct PlainArgs {
     cudaStream_t stream;
 };
 
+// 1D runs of several steps (plain_resident.cuh): progress counters one 128-byte line apart, for at
+// most kPlainProgChunks chunks
+constexpr int kPlainProgStride = 32, kPlainProgChunks = 512;
+
 namespace plain_fast {
 cudaError_t step(const PlainArgs& a);
+cudaError_t run(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps);
 cudaError_t stage(const PlainArgs& a, int which);
 }
 namespace plain_exact {
 cudaError_t step(const PlainArgs& a);
+cudaError_t run(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps);
 cudaError_t stage(const PlainArgs& a, int which);
 }
