@@ -60,68 +60,75 @@ EM_FN uint32_t em_seed(float x) {
 }
 
 // A divisor b: its significand mb in [2^52, 2^53), a 32-bit reciprocal r <= 2^84 / mb (relative
-// error below 2^-30), its biased exponent (0 or 2047 for a zero, subnormal or non-finite b, whose
-// quotients take the hardware division) and its bits.
+// error below 2^-29), its bits.
 struct Divisor {
     uint64_t mb, bits;
     uint32_t r;
-    int e;
 };
+
+EM_FN uint64_t em_significand(uint64_t bits) { return (bits & (kOne52 - 1)) | kOne52; }
+EM_FN int em_exponent(uint64_t bits) { return (int)(bits >> 52) & 0x7ff; }
 
 EM_FN Divisor divisor(double b) {
     Divisor d;
     d.bits = em_dbits(b);
-    d.e = (int)(d.bits >> 52) & 0x7ff;
-    d.mb = (d.bits & (kOne52 - 1)) | kOne52;
+    d.mb = em_significand(d.bits);
     // seed: 1 / beta, beta = mb / 2^52 cut to 24 bits, as a 24-bit fixed-point number R0 / 2^24
     const float bf = em_bitsf(0x3f800000u | ((uint32_t)(d.mb >> 29) & 0x7fffffu));
     const uint32_t R0 = em_seed(em_rcp(bf));
-    // 1 - beta R0 / 2^24 = E / 2^76 with |E| < 2^56: its low 64 bits are all of it
-    const int64_t E = -(int64_t)(d.mb * R0);
-    const int32_t Eh = (int32_t)(E >> 24);
-    // one Newton step, scaled to 2^32 and lowered by 2 so that it never reaches 1 / beta
-    const int64_t t = (int64_t)(int32_t)R0 * Eh;         // R0 E / 2^24
-    d.r = (R0 << 8) + (uint32_t)(int32_t)(t >> 44) - 2u;
+    // 1 - beta R0 / 2^24 = -D / 2^76 with |D| < 2^56: the low 64 bits of mb R0 are all of it
+    const int32_t Dh = (int32_t)((int64_t)(d.mb * R0) >> 24);
+    // one Newton step, scaled to 2^32 and lowered so that it never reaches 1 / beta
+    d.r = (R0 << 8) - (uint32_t)((int32_t)(((int64_t)(int32_t)R0 * Dh) >> 32) >> 12) - 3u;
     return d;
+}
+
+// a / b, correctly rounded, for normal a and b whose quotient is normal (the exponents of both, and
+// their difference, well inside the range; anything else gives a meaningless value and no fault)
+EM_FN double divide_plain(double a, const Divisor& d) {
+    const uint64_t ab = em_dbits(a);
+    const uint64_t ma = em_significand(ab);
+    const bool less = ma < d.mb;
+    const uint64_t N = less ? ma + ma : ma;              // N / mb in [1, 2)
+    // first 30 fraction bits, too small by a few units
+    const uint32_t q1 = em_mulhi((uint32_t)(N >> 22), d.r);
+    const int64_t rem1 = (int64_t)((N << 30) - (uint64_t)q1 * d.mb);
+    // the next 22 bits, rounded: rem1 2^22 / mb = rem1 r / 2^62
+    const int32_t q2 = (int32_t)(((int64_t)(int32_t)(rem1 >> 25) * (int32_t)(d.r >> 1)) >> 32);
+    const int32_t r = (q2 + 8) >> 4;
+    const int64_t rem2 = 2 * (int64_t)(((uint64_t)rem1 << 22) - (uint64_t)((int64_t)r * (int64_t)d.mb));
+    uint64_t Q = ((uint64_t)q1 << 22) + (int64_t)r;
+    // the quotient of two 53-bit numbers is never half way between two 53-bit numbers
+    if (rem2 > (int64_t)d.mb) Q++;
+    if (rem2 < -(int64_t)d.mb) Q--;
+    // (Q's bit 52 adds one to the exponent field)
+    const uint32_t hi = (uint32_t)(Q >> 32) + (uint32_t)((ab >> 32) & 0xfff00000u) - (uint32_t)((d.bits >> 32) & 0xfff00000u) +
+                        ((less ? 1021u : 1022u) << 20);
+    return em_bitsd(((uint64_t)hi << 32) | (uint32_t)Q);
 }
 
 // a / b, correctly rounded (round to nearest even); every special case as the hardware's
 EM_FN double divide(double a, const Divisor& d) {
     const uint64_t ab = em_dbits(a);
-    const int ea = (int)(ab >> 52) & 0x7ff;
-    const uint64_t ma = (ab & (kOne52 - 1)) | kOne52;
-    const uint64_t sign = (ab ^ d.bits) & (1ull << 63);
-    const bool less = ma < d.mb;
-    const uint64_t N = less ? ma << 1 : ma;              // N / mb in [1, 2)
-    const int e = ea - d.e + 1023 - (less ? 1 : 0);      // biased exponent of the quotient
-    // first 30 fraction bits, never too large by more than the reciprocal allows
-    const uint32_t q1 = em_mulhi((uint32_t)(N >> 22), d.r);
-    const int64_t rem1 = (int64_t)((N << 30) - (uint64_t)q1 * d.mb);
-    // the next 22 bits, rounded: rem1 2^22 / mb = rem1 r / 2^62
-    const int64_t q2 = (int64_t)(int32_t)(rem1 >> 25) * (int32_t)(d.r >> 1);
-    const int32_t r = ((int32_t)(q2 >> 35) + 1) >> 1;
-    uint64_t Q = ((uint64_t)q1 << 22) + (int64_t)r;
-    const int64_t rem = (int64_t)(((uint64_t)rem1 << 22) - (uint64_t)((int64_t)r * (int64_t)d.mb));
-    // the quotient of two 53-bit numbers is never half way between two 53-bit numbers
-    if (2 * rem > (int64_t)d.mb) Q++;
-    if (2 * rem < -(int64_t)d.mb) Q--;
-    double q = em_bitsd(sign | (((uint64_t)(uint32_t)e << 52) + (Q - kOne52)));
-    // exponents 1..2045 of the quotient and normal operands; a zero dividend is common (gas at rest)
-    const bool plain = (unsigned)(e - 1) < 2045u && (unsigned)(ea - 1) < 2046u && (unsigned)(d.e - 1) < 2046u;
-    if (!plain) {
-        if ((ab << 1) == 0 && (unsigned)(d.e - 1) < 2046u) q = em_bitsd(sign);
-        else q = em_hwdiv(a, em_bitsd(d.bits));
+    const int ea = em_exponent(ab), eb = em_exponent(d.bits);
+    // (the plain division takes the divisor's sign for 0: flipped in below)
+    if ((unsigned)(ea - 1) < 2046u && (unsigned)(eb - 1) < 2046u && (unsigned)(ea - eb + 1021) < 2043u) {
+        Divisor p = d;
+        p.bits &= ~(1ull << 63);
+        return em_bitsd(em_dbits(divide_plain(a, p)) ^ (d.bits & (1ull << 63)));
     }
-    return q;
+    // a zero dividend is common (gas at rest)
+    if ((ab << 1) == 0 && (unsigned)(eb - 1) < 2046u) return em_bitsd((ab ^ d.bits) & (1ull << 63));
+    return em_hwdiv(a, em_bitsd(d.bits));
 }
 
-// sqrt(a), correctly rounded
-EM_FN double square_root(double a) {
+// sqrt(a), correctly rounded, for a normal positive a; *root: it as a divisor (its reciprocal is a
+// by-product)
+EM_FN double square_root_plain(double a, Divisor* root) {
     const uint64_t ab = em_dbits(a);
-    const int ea = (int)(ab >> 52);                      // (with the sign: negative a is not plain)
-    if ((unsigned)(ea - 1) >= 2046u) return em_hwsqrt(a);
+    const int ea = (int)(ab >> 52);
     const int odd = (ea & 1) ^ 1;                        // unbiased exponent odd
-    const uint64_t M = ((ab & (kOne52 - 1)) | kOne52) << odd;   // X = M / 2^52 in [1, 4)
+    const uint64_t M = em_significand(ab) << odd;        // X = M / 2^52 in [1, 4)
     const uint32_t Mh = (uint32_t)(M >> 22);             // X 2^30
     // seed 1 / sqrt(X), one Newton step: y <- y + y (1 - X y^2) / 2, to about 2^-30
     const float xf = em_bitsf(0x3f800000u + ((uint32_t)odd << 23) + ((uint32_t)((ab & (kOne52 - 1)) >> 29)));
@@ -129,18 +136,28 @@ EM_FN double square_root(double a) {
     const uint32_t T = (uint32_t)(((uint64_t)Y0 * Y0) >> 16);   // y^2 2^32
     const int64_t e0 = (int64_t)((1ull << 62) - (uint64_t)T * Mh);   // (1 - X y^2) 2^62, |.| < 2^43
     const int64_t t = (int64_t)(int32_t)Y0 * (int32_t)(e0 >> 20);    // y e0 2^(24 + 42)
-    const uint32_t y = (Y0 << 8) + (uint32_t)(int32_t)(t >> 35) - 4u;   // y (1 + e0 / 2) 2^32
+    const uint32_t y = (Y0 << 8) + (uint32_t)((int32_t)(t >> 32) >> 3) - 4u;   // y (1 + e0 / 2) 2^32
     // first 30 fraction bits, then 22 more from the exact remainder
     const uint32_t s1 = em_mulhi(Mh, y);
     const int64_t rem1 = (int64_t)((M << 8) - (uint64_t)s1 * s1);
     const int64_t s2 = (int64_t)(int32_t)(rem1 >> 6) * (int32_t)(y >> 1);   // rem1 y 2^25
-    const int32_t r = ((int32_t)(s2 >> 33) + 1) >> 1;    // rem1 2^22 / (2 s1) = rem1 y / 2^41, y = y' / 2^32
+    const int32_t r = ((int32_t)(s2 >> 32) + 2) >> 2;    // rem1 2^22 / (2 s1) = rem1 y / 2^41, y = y' / 2^32
     uint64_t S = ((uint64_t)s1 << 22) + (int64_t)r;
     const int64_t rem = (int64_t)((M << 52) - S * S);
     if (rem > (int64_t)S) S++;
     if (rem <= -(int64_t)S) S--;
     const int e = ((ea - odd - 1023) >> 1) + 1023;
-    return em_bitsd(((uint64_t)(uint32_t)e << 52) + (S - kOne52));
+    root->mb = S;
+    root->r = y;
+    root->bits = ((uint64_t)(uint32_t)(e - 1) << 52) + S;
+    return em_bitsd(root->bits);
+}
+
+// sqrt(a), correctly rounded; every special case as the hardware's
+EM_FN double square_root(double a) {
+    Divisor root;
+    if ((unsigned)((int)(em_dbits(a) >> 52) - 1) < 2046u) return square_root_plain(a, &root);
+    return em_hwsqrt(a);
 }
 
 // x 2^k for a power of two the reference multiplies by (k small): the exponent field moves; zeros
@@ -152,13 +169,14 @@ EM_FN double scale_pow2(double x, int k, double pow2k) {
     return (b << 1) == 0 ? x : em_mul(x, pow2k);
 }
 
-// l * r < 0.0 as the FP64 product decides it (a product that underflows to zero is not negative)
-EM_FN bool product_negative(double l, double r) {
+// l * r < 0.0 as the FP64 product decides it (a product that underflows to zero is not negative),
+// for l and r given as `scale` (1 or 2) times themselves
+EM_FN bool product_negative(double l, double r, double inv_scale) {
     const uint64_t lb = em_dbits(l), rb = em_dbits(r);
     const int el = (int)(lb >> 52) & 0x7ff, er = (int)(rb >> 52) & 0x7ff;
     if ((unsigned)(el - 1) < 2046u && (unsigned)(er - 1) < 2046u && el + er >= 1000) return ((lb ^ rb) >> 63) != 0;
     if ((lb << 1) == 0 || (rb << 1) == 0) return false;
-    return em_mul(l, r) < 0.0;
+    return em_mul(em_mul(l, inv_scale), em_mul(r, inv_scale)) < 0.0;
 }
 
 // fabs(l) < fabs(r); false when either is a NaN
@@ -174,6 +192,21 @@ EM_FN bool magnitude_less(double l, double r) {
 // clear of the half-way points the rounded double expression can only be R, otherwise (a chance of
 // about 2^-17) the double expression itself decides.
 
+// the double expressions themselves, out of line so that none of their FP64 instructions is issued
+// ahead of the branch that needs them
+#ifdef __CUDACC__
+#define EM_SLOW __host__ __device__ __noinline__
+#else
+#define EM_SLOW inline
+#endif
+static EM_SLOW float temperature_slow(float e, float kh, float kl, float c) {
+    return (float)em_hwdiv(em_add((double)e, -((double)kh + (double)kl)), (double)c);
+}
+static EM_SLOW float z2_slow(float a, float t) { return (float)em_mul(0.5 * (double)a, em_add(1.0, -(double)t)); }
+static EM_SLOW float sub_product_slow(float u, float c, float s) {
+    return (float)em_add((double)u, -em_mul((double)c, (double)s));
+}
+
 // true when R + rem (exact to 2^-18 half units) certainly rounds to R, R in the middle of the range
 EM_FN bool rounds_to(float R, float rem) {
     const uint32_t b = em_fbits(R), e = b & 0x7f800000u;
@@ -188,6 +221,24 @@ EM_FN float two_sum(float a, float b, float& e) {
     return s;
 }
 
+// FP32 quotients and square roots, correctly rounded, for operands and results well inside the range
+// (a zero dividend included): a residual step with a refined reciprocal (Markstein, IBM J. Res. Dev. 34
+// (1990) 111), without the range branches of the general forms.
+// y: 1 / b, refined
+EM_FN float reciprocal_plain(float b, float y) { return em_fma(em_fma(-b, y, 1.0f), y, y); }
+EM_FN float divide_plain(float a, float b, float y) {
+    const float q = em_mul(a, y);
+    return em_fma(em_fma(-q, b, a), y, q);
+}
+// *y: about 1 / sqrt(x)
+EM_FN float square_root_plain(float x, float* y) {
+    float r = em_rsqrt(x);
+    r = em_fma(em_mul(0.5f, r), em_fma(-em_mul(x, r), r, 1.0f), r);
+    const float s = em_mul(x, r);
+    *y = r;
+    return em_fma(em_fma(-s, s, x), em_mul(0.5f, r), s);
+}
+
 // (float)((D(e) - k) / D(c)) with k = kh + kl the exact subtrahend (D(k) a double of at most 48
 // bits) and rc an approximation of 1 / c
 EM_FN float temperature_ref(float e, float kh, float kl, float c, float rc) {
@@ -200,7 +251,7 @@ EM_FN float temperature_ref(float e, float kh, float kl, float c, float rc) {
     const float rem = em_add(ql, -em_add(R, -qh));
     // (no large cancellation, which would magnify the rounding of sl)
     if (rounds_to(R, rem) && fabsf(kh) < 16.0f * fabsf(sh)) return R;
-    return (float)em_hwdiv(em_add((double)e, -((double)kh + (double)kl)), (double)c);
+    return temperature_slow(e, kh, kl, c);
 }
 
 // (float)(0.5 * D(a) * (1.0 - D(t)))
@@ -211,8 +262,7 @@ EM_FN float z2_ref(float a, float t) {
     const float pl = em_fma(a, wl, em_fma(a, wh, -ph));
     const float R = em_add(ph, pl);
     const float rem = em_add(pl, -em_add(R, -ph));
-    if (rounds_to(R, rem)) return em_mul(0.5f, R);
-    return (float)em_mul(0.5 * (double)a, em_add(1.0, -(double)t));
+    return rounds_to(R, rem) ? em_mul(0.5f, R) : z2_slow(a, t);
 }
 
 // (float)(D(u) - D(c) * D(s)) for a float c (the product is exact in double)
@@ -226,7 +276,7 @@ EM_FN float sub_product_ref(float u, float c, float s) {
     const float R = em_add(sh, sl);
     const float rem = em_add(sl, -em_add(R, -sh));
     if (rounds_to(R, rem) && fabsf(ph) < 16.0f * fabsf(sh)) return R;
-    return (float)em_add((double)u, -em_mul((double)c, (double)s));
+    return sub_product_slow(u, c, s);
 }
 
 }  // namespace exact_math

@@ -4,6 +4,7 @@
 // (shll_plain.cuh): the reference's FP64 arithmetic with fused multiply-add allowed (the kernels
 // of this unit), or without it, bit-identical to the FP64 reference build (plain_batch_exact.cu).
 #define SHLL_PLAIN_NS plain_batch_ns
+#define SHLL_PLAIN_FMA 1   // products and sums may be fused
 #include "plain_batch_kernels.cuh"
 
 #include <algorithm>

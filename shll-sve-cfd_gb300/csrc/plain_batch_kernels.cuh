@@ -19,7 +19,7 @@ template <int ORDER>
 __global__ void __launch_bounds__(T1) k_batch1(const PItem* __restrict__ items, const PBlk* __restrict__ blks,
                                                double* U0, double* U1, long plane, int step, int* flags) {
     const PBlk bk = blks[blockIdx.x];
-    const PItem it = items[bk.item];
+    const PItem& it = items[bk.item];
     if (step >= it.steps) return;
     const int inb = (it.par + step) & 1;
     const double* Uin = (inb ? U1 : U0) + it.base;
@@ -31,7 +31,7 @@ template <int ORDER>
 __global__ void __launch_bounds__(TI * TJ) k_batch2(const PItem* __restrict__ items, const PBlk* __restrict__ blks,
                                                     double* U0, double* U1, long plane, int step, int* flags) {
     const PBlk bk = blks[blockIdx.x];
-    const PItem it = items[bk.item];
+    const PItem& it = items[bk.item];
     if (step >= it.steps) return;
     const int inb = (it.par + step) & 1;
     const double* Uin = (inb ? U1 : U0) + it.base;

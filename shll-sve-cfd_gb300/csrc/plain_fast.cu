@@ -1,6 +1,7 @@
 // SHLL_PREC_F64: reference arithmetic in FP64 with fused multiply-add allowed (compiled with
 // the default -fmad=true).
 #define SHLL_PLAIN_NS plain_fast
+#define SHLL_PLAIN_FMA 1   // products and sums may be fused
 #include "plain_resident.cuh"
 
 namespace plain_fast {

@@ -96,10 +96,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
             REAL* F = flux + par * 6 * T;
             REAL fp[3], fm[3];
             if (valid) {
-                REAL p1, p2, snd;
-                prim1(g, u[0], u[1], u[2], p1, p2, snd);
-                flux1(g, u[0], u[1], u[2], p1, p2, snd, fp, fm);
-                bad |= !positive(u[0]) || !positive(p2);
+                bad |= cell1(g, u, fp, fm);
 #pragma unroll
                 for (int q = 0; q < 3; q++) { F[q * T + tid] = fp[q]; F[(3 + q) * T + tid] = fm[q]; }
             }
@@ -112,7 +109,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
                         const REAL sg = (q == 1) ? (REAL)1 : (REAL)-1;
                         const REAL L = i == 0 ? sg * fm[q] : F[q * T + tid - 1];
                         const REAL Rr = i == n - 1 && i != 0 ? sg * fp[q] : F[(3 + q) * T + tid + 1];
-                        u[q] = sub_scaled(u[q], g.lx, fp[q] - fm[q] + Rr - L);
+                        u[q] = sub_scaled(u[q], g.sx, fp[q] - fm[q] + Rr - L);
                     }
                 }
             } else {
@@ -136,8 +133,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
                         const REAL L = wl ? fp[q] : F[q * T + tid - 1], Ldf = wl ? (REAL)0 : slp[q * T + tid - 1];
                         const REAL Rr = wr ? fm[q] : F[(3 + q) * T + tid + 1];
                         const REAL Rdf = wr ? (REAL)0 : slp[(3 + q) * T + tid + 1];
-                        u[q] = sub_scaled(u[q], g.lx, fp[q] - fm[q] + Rr - L);
-                        u[q] = sub_half_scaled(u[q], g.hlx, dp[q] + dm[q] - Rdf - Ldf);
+                        u[q] = sub_scaled(u[q], g.sx, fp[q] - fm[q] + Rr - L);
+                        u[q] = sub_half_scaled(u[q], g.hsx, dp[q] + dm[q] - Rdf - Ldf);
                     }
                 }
             }

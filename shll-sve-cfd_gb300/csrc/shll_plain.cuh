@@ -24,12 +24,11 @@ namespace SHLL_PLAIN_NS {
 
 #define D(x) ((double)(x))
 
-// A multiplication by a grid constant (DT_ON_DX and the like): by a power of two 2^k (the reference's
-// 0.25 / (R + 1)) it moves the exponent, which costs no FP64 instruction.
+// A grid constant (DT_ON_DX and the like), and whether it is a power of two (the reference's
+// 0.25 / (R + 1)), so that products with it are exact.
 template <typename REAL>
 struct Factor {
     REAL v;
-    int k;
     bool pow2;
 };
 template <typename REAL>
@@ -38,7 +37,6 @@ __host__ Factor<REAL> make_factor(REAL v) {
     int ex = 0;
     f.v = v;
     f.pow2 = std::frexp((double)v, &ex) == 0.5 && ex > -500 && ex < 500;
-    f.k = ex - 1;
     return f;
 }
 
@@ -51,8 +49,15 @@ struct Gas {
     REAL gR;                                           // GAMMA * R
     REAL rCV;                                          // about 1 / CV (float arithmetic)
     exact_math::Divisor cv;                            // CV as a divisor (FP64 arithmetic)
+    bool plain;                                        // the constants suit the cells' main path
     Factor<REAL> lx, ly, hlx, hly;                     // DT_ON_DX, DT_ON_DY and 0.5 times them
+    Factor<REAL> sx, sy, hsx, hsy;                     // the same for fluxes as cell1 and cell2 scale them
 };
+
+// The split fluxes of cell1 and cell2 are kFluxScale times the reference's: in FP64 twice (the factors
+// 0.5 of Z1, Z2 and Z3 are left out, and half the grid constants make up for it, all exactly).
+template <typename REAL>
+constexpr REAL kFluxScale = sizeof(REAL) == 8 ? (REAL)2 : (REAL)1;
 
 template <typename REAL>
 __host__ void finish_gas(Gas<REAL>& g) {
@@ -64,6 +69,13 @@ __host__ void finish_gas(Gas<REAL>& g) {
     g.ly = make_factor<REAL>(g.DT_ON_DY);
     g.hlx = make_factor<REAL>((REAL)0.5 * g.DT_ON_DX);
     g.hly = make_factor<REAL>((REAL)0.5 * g.DT_ON_DY);
+    g.sx = make_factor<REAL>(g.DT_ON_DX / kFluxScale<REAL>);
+    g.sy = make_factor<REAL>(g.DT_ON_DY / kFluxScale<REAL>);
+    g.hsx = make_factor<REAL>((REAL)0.5 * g.DT_ON_DX / kFluxScale<REAL>);
+    g.hsy = make_factor<REAL>((REAL)0.5 * g.DT_ON_DY / kFluxScale<REAL>);
+    const double c[3] = {(double)g.CV, (double)g.R, (double)g.gR};
+    g.plain = true;
+    for (double v : c) g.plain = g.plain && v > 1e-9 && v < 1e9;
 }
 
 template <typename REAL>
@@ -92,9 +104,18 @@ __device__ __forceinline__ bool positive(double x) {
     return b > 0 && b <= 0x7ff0000000000000ll;
 }
 __device__ __forceinline__ bool positive(float x) { return x > 0.f; }
-// u - f * x
+// u - f * x.  With f a power of two f * x is exact unless it is subnormal, so that one fused operation
+// rounds like the product and the difference.
 __device__ __forceinline__ double sub_scaled(double u, const Factor<double>& f, double x) {
-    return f.pow2 ? u - exact_math::scale_pow2(x, f.k, f.v) : u - f.v * x;
+#if SHLL_PLAIN_FMA
+    return __fma_rn(-f.v, x, u);
+#else
+    if (!f.pow2) return u - f.v * x;
+    const double r = __fma_rn(-f.v, x, u);
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    if (h < (600u << 20) && (h | (unsigned)__double2loint(x)) != 0u) return u - f.v * x;
+    return r;
+#endif
 }
 __device__ __forceinline__ float sub_scaled(float u, const Factor<float>& f, float x) { return u - f.v * x; }
 // (REAL)(D(u) - 0.5 * D(lambda) * D(x)), f = 0.5 * lambda
@@ -168,22 +189,107 @@ __device__ __forceinline__ void flux1(const Gas<REAL>& g, REAL u0, REAL u1, REAL
     fm[0] = -f0 * Z3 - u0 * Z2; fm[1] = -f1 * Z3 - u1 * Z2; fm[2] = -f2 * Z3 - u2 * Z2;
 }
 
+// ---- a cell of the fused kernels, 1D ----
+// Split fluxes (kFluxScale times) of a cell with conserved state u; returns whether its density or
+// temperature is not positive.  The main path is free of branches and special cases: it holds for
+// states and constants whose exponents are well inside the range (a momentum may be zero); any other
+// cell takes the general functions.
+// (a value, not through pointers, which would keep the main path's fluxes in local memory)
+template <typename REAL, int NF>
+struct CellFlux {
+    REAL f[NF];
+    int bad;
+};
+template <typename REAL>
+__device__ __noinline__ CellFlux<REAL, 6> cell1_general(const Gas<REAL>& g, REAL u0, REAL u1, REAL u2) {
+    CellFlux<REAL, 6> c;
+    REAL p1, p2, a;
+    prim1(g, u0, u1, u2, p1, p2, a);
+    flux1(g, u0, u1, u2, p1, p2, a, c.f, c.f + 3);
+    for (int k = 0; k < 6; k++) c.f[k] *= kFluxScale<REAL>;
+    c.bad = !positive(u0) || !positive(p2);
+    return c;
+}
+__device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)__double2hiint(x); }
+__device__ __forceinline__ bool is_zero(double x) { return ((hi_word(x) << 1) | (unsigned)__double2loint(x)) == 0u; }
+// exponent (biased) in [lo, lo + n) and positive
+__device__ __forceinline__ bool in_range(double x, unsigned lo, unsigned n) { return (hi_word(x) >> 20) - lo < n; }
+__device__ __forceinline__ bool in_range(float x, unsigned lo, unsigned n) { return (__float_as_uint(x) >> 23) - lo < n; }
+// momentum: zero, or of a magnitude whose quotients and products stay normal
+__device__ __forceinline__ bool momentum_plain(double x) {
+    return ((hi_word(x) & 0x7fffffffu) >> 20) - 323u < 800u || is_zero(x);
+}
+__device__ __forceinline__ bool momentum_plain(float x) {
+    return ((__float_as_uint(x) & 0x7fffffffu) >> 23) - 67u < 120u || x == 0.f;
+}
+__device__ __forceinline__ bool all_ones(float x) { return (__float_as_uint(x) & 0x7fffffu) == 0x7fffffu; }
+__device__ __forceinline__ double divide_or_zero(double a, const exact_math::Divisor& d) {
+    const double q = exact_math::divide_plain(a, d);
+    return is_zero(a) ? a : q;
+}
+
+__device__ __forceinline__ int cell1(const Gas<double>& g, const double u[3], double fp[3], double fm[3]) {
+    const exact_math::Divisor rho = exact_math::divisor(u[0]);
+    const double p1 = divide_or_zero(u[1], rho);
+    const double e = exact_math::divide_plain(u[2], rho);
+    // e - 0.5 * p1 * p1 (the scaling is exact beside a normal e)
+    const double t = __fma_rn(-0.5, __dmul_rn(p1, p1), e);
+    const double p2 = exact_math::divide_plain(t, g.cv);
+    exact_math::Divisor snd;
+    const double a = exact_math::square_root_plain(g.gR * p2, &snd);
+    const double M = divide_or_zero(p1, snd);
+    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * (1.0 - M * M);   // twice the reference's
+    const double P = times_R(g, u[0]) * p2;
+    const double F[3] = {u[1], u[1] * p1 + P, p1 * (u[2] + P)};
+#pragma unroll
+    for (int k = 0; k < 3; k++) { fp[k] = F[k] * Z1 + u[k] * Z2; fm[k] = -F[k] * Z3 - u[k] * Z2; }
+    if (g.plain && in_range(u[0], 923, 200) && in_range(u[2], 923, 200) && momentum_plain(u[1]) && in_range(t, 900, 250))
+        return 0;
+    const auto c = cell1_general(g, u[0], u[1], u[2]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) { fp[k] = c.f[k]; fm[k] = c.f[3 + k]; }
+    return c.bad;
+}
+__device__ __forceinline__ int cell1(const Gas<float>& g, const float u[3], float fp[3], float fm[3]) {
+    const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
+    const float p1 = exact_math::divide_plain(u[1], u[0], y), e = exact_math::divide_plain(u[2], u[0], y);
+    const float p2 = temp1(g, e, p1), x = g.gR * p2;
+    float ya;
+    const float a = exact_math::square_root_plain(x, &ya);
+    const float M = exact_math::divide_plain(p1, a, exact_math::reciprocal_plain(a, ya));
+    const float Z1 = half_sum(M, 1.f), Z3 = half_sum(M, -1.f), Z2 = z2(a, M);
+    const float P = times_R(g, u[0]) * p2;
+    const float F[3] = {u[1], u[1] * p1 + P, p1 * (u[2] + P)};
+#pragma unroll
+    for (int k = 0; k < 3; k++) { fp[k] = F[k] * Z1 + u[k] * Z2; fm[k] = -F[k] * Z3 - u[k] * Z2; }
+    // (a divisor of all-ones significand is the exception of the residual step)
+    if (g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[2], 87, 80) && momentum_plain(u[1]) &&
+        in_range(x, 87, 80) && !all_ones(a))
+        return 0;
+    const auto c = cell1_general(g, u[0], u[1], u[2]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) { fp[k] = c.f[k]; fm[k] = c.f[3 + k]; }
+    return c.bad;
+}
+
 // minmod (2nd_order_base_shll.c:191-201)
-__device__ __forceinline__ double minmod(double l, double r) {
-    if (exact_math::product_negative(l, r)) return 0.0;
+// (inv_scale: 1 / the scale of the arguments, for the sign of their product where it underflows)
+__device__ __forceinline__ double minmod(double l, double r, double inv_scale) {
+    if (exact_math::product_negative(l, r, inv_scale)) return 0.0;
     return exact_math::magnitude_less(l, r) ? l : r;
 }
-__device__ __forceinline__ float minmod(float l, float r) {
+__device__ __forceinline__ float minmod(float l, float r, float) {
     if (__fmul_rn(l, r) < 0.f) return 0.f;
     return fabsf(l) < fabsf(r) ? l : r;
 }
 // slope of a split flux at an interior cell: minmod, or the MC limiter of
 // base-omp/2nd_order_base_shll.c:316-325
 template <typename REAL>
-__device__ __forceinline__ REAL slope(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr) {
+__device__ __forceinline__ REAL slope(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr,
+                                      REAL inv_scale = (REAL)1 / kFluxScale<REAL>) {
     if (g.limiter == 1)
-        return minmod(half_of(fr - fl), g.alpha * minmod(fc - fl, fr - fc));
-    return minmod(fc - fl, fr - fc);
+        return minmod(half_of(fr - fl), g.alpha * minmod(fc - fl, fr - fc, inv_scale), inv_scale);
+    return minmod(fc - fl, fr - fc, inv_scale);
 }
 
 constexpr int T1 = 256;  // cells per block (1D)
@@ -204,10 +310,8 @@ __device__ __forceinline__ void step1_block(const REAL* __restrict__ Uin, REAL* 
         int c = b0 - H + t;
         REAL fp[3] = {0, 0, 0}, fm[3] = {0, 0, 0};
         if (c >= 0 && c < n) {
-            REAL u0 = Uin[c], u1 = Uin[stride + c], u2 = Uin[2 * stride + c], p1, p2, a;
-            prim1(g, u0, u1, u2, p1, p2, a);
-            flux1(g, u0, u1, u2, p1, p2, a, fp, fm);
-            bad |= !positive(u0) || !positive(p2);
+            const REAL u[3] = {Uin[c], Uin[stride + c], Uin[2 * stride + c]};
+            bad |= cell1(g, u, fp, fm);
         }
 #pragma unroll
         for (int k = 0; k < 3; k++) { sfp[k][t] = fp[k]; sfm[k][t] = fm[k]; }
@@ -240,15 +344,15 @@ __device__ __forceinline__ void step1_block(const REAL* __restrict__ Uin, REAL* 
             if (i == 0) { L = sg * fm; Rr = sfm[k][s + 1]; }
             else if (i == n - 1) { L = sfp[k][s - 1]; Rr = sg * fp; }
             else { L = sfp[k][s - 1]; Rr = sfm[k][s + 1]; }
-            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
+            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
         } else {
             const int d = threadIdx.x + 1;  // slope index of cell i
             REAL Ldf, Rdf;
             if (i == 0) { L = fp; Rr = sfm[k][s + 1]; Ldf = 0; Rdf = sdm[k][d + 1]; }
             else if (i == n - 1) { L = sfp[k][s - 1]; Rr = fm; Ldf = sdp[k][d - 1]; Rdf = 0; }
             else { L = sfp[k][s - 1]; Rr = sfm[k][s + 1]; Ldf = sdp[k][d - 1]; Rdf = sdm[k][d + 1]; }
-            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
-            u = sub_half_scaled(u, g.hlx, sdp[k][d] + sdm[k][d] - Rdf - Ldf);
+            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
+            u = sub_half_scaled(u, g.hsx, sdp[k][d] + sdm[k][d] - Rdf - Ldf);
         }
         Uout[k * stride + i] = u;
     }
@@ -293,6 +397,69 @@ __device__ __forceinline__ void flux2(const Gas<REAL>& g, const REAL u[4], REAL 
     for (int k = 0; k < 4; k++) { hp[k] = h[k] * Z1 + u[k] * Z2; hm[k] = -h[k] * Z3 - u[k] * Z2; }
 }
 
+// a cell of the fused kernels, 2D (see cell1)
+template <typename REAL>
+__device__ __noinline__ CellFlux<REAL, 16> cell2_general(const Gas<REAL>& g, REAL u0, REAL u1, REAL u2, REAL u3) {
+    const REAL u[4] = {u0, u1, u2, u3};
+    CellFlux<REAL, 16> c;
+    REAL p1, p2, p3, a;
+    prim2(g, u0, u1, u2, u3, p1, p2, p3, a);
+    flux2(g, u, p1, p2, p3, a, c.f, c.f + 4, c.f + 8, c.f + 12);
+    for (int k = 0; k < 16; k++) c.f[k] *= kFluxScale<REAL>;
+    c.bad = !positive(u0) || !positive(p3);
+    return c;
+}
+template <typename REAL>
+__device__ __forceinline__ void split2d(const REAL u[4], REAL p1, REAL p2, REAL P, REAL Z1x, REAL Z2x, REAL Z3x, REAL Z1y,
+                                        REAL Z2y, REAL Z3y, REAL fp[4], REAL fm[4], REAL hp[4], REAL hm[4]) {
+    const REAL f[4] = {u[1], u[1] * p1 + P, u[1] * p2, p1 * (u[3] + P)};
+    const REAL h[4] = {u[2], u[2] * p1, u[2] * p2 + P, p2 * (u[3] + P)};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        fp[k] = f[k] * Z1x + u[k] * Z2x; fm[k] = -f[k] * Z3x - u[k] * Z2x;
+        hp[k] = h[k] * Z1y + u[k] * Z2y; hm[k] = -h[k] * Z3y - u[k] * Z2y;
+    }
+}
+__device__ __forceinline__ int cell2(const Gas<double>& g, const double u[4], double fp[4], double fm[4], double hp[4],
+                                     double hm[4]) {
+    const exact_math::Divisor rho = exact_math::divisor(u[0]);
+    const double p1 = divide_or_zero(u[1], rho), p2 = divide_or_zero(u[2], rho);
+    const double e = exact_math::divide_plain(u[3], rho);
+    const double t = __fma_rn(-0.5, p1 * p1 + p2 * p2, e);
+    const double p3 = exact_math::divide_plain(t, g.cv);
+    exact_math::Divisor snd;
+    const double a = exact_math::square_root_plain(g.gR * p3, &snd);
+    const double Mx = divide_or_zero(p1, snd), My = divide_or_zero(p2, snd);
+    split2d<double>(u, p1, p2, times_R(g, u[0]) * p3, Mx + 1.0, a * (1.0 - Mx * Mx), Mx - 1.0, My + 1.0,
+                    a * (1.0 - My * My), My - 1.0, fp, fm, hp, hm);
+    if (g.plain && in_range(u[0], 923, 200) && in_range(u[3], 923, 200) && momentum_plain(u[1]) && momentum_plain(u[2]) &&
+        in_range(t, 900, 250))
+        return 0;
+    const auto c = cell2_general(g, u[0], u[1], u[2], u[3]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) { fp[k] = c.f[k]; fm[k] = c.f[4 + k]; hp[k] = c.f[8 + k]; hm[k] = c.f[12 + k]; }
+    return c.bad;
+}
+__device__ __forceinline__ int cell2(const Gas<float>& g, const float u[4], float fp[4], float fm[4], float hp[4],
+                                     float hm[4]) {
+    const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
+    const float p1 = exact_math::divide_plain(u[1], u[0], y), p2 = exact_math::divide_plain(u[2], u[0], y);
+    const float p3 = temp2(g, exact_math::divide_plain(u[3], u[0], y), p1, p2), x = g.gR * p3;
+    float ya;
+    const float a = exact_math::square_root_plain(x, &ya);
+    ya = exact_math::reciprocal_plain(a, ya);
+    const float Mx = exact_math::divide_plain(p1, a, ya), My = exact_math::divide_plain(p2, a, ya);
+    split2d<float>(u, p1, p2, times_R(g, u[0]) * p3, half_sum(Mx, 1.f), z2(a, Mx), half_sum(Mx, -1.f), half_sum(My, 1.f),
+                   z2(a, My), half_sum(My, -1.f), fp, fm, hp, hm);
+    if (g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[3], 87, 80) && momentum_plain(u[1]) &&
+        momentum_plain(u[2]) && in_range(x, 87, 80) && !all_ones(a))
+        return 0;
+    const auto c = cell2_general(g, u[0], u[1], u[2], u[3]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) { fp[k] = c.f[k]; fm[k] = c.f[4 + k]; hp[k] = c.f[8 + k]; hm[k] = c.f[12 + k]; }
+    return c.bad;
+}
+
 constexpr int TJ = 32;  // tile extent along j (contiguous, threadIdx.x)
 constexpr int TI = 8;   // tile extent along i (threadIdx.y)
 
@@ -332,10 +499,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
         REAL fp[4] = {0, 0, 0, 0}, fm[4] = {0, 0, 0, 0}, hp[4] = {0, 0, 0, 0}, hm[4] = {0, 0, 0, 0};
         if (i >= 0 && i < nx && j >= 0 && j < ny) {
             int c = i * ny + j;
-            REAL u[4] = {Uin[c], Uin[n + c], Uin[2 * n + c], Uin[3 * n + c]}, p1, p2, p3, a;
-            prim2(g, u[0], u[1], u[2], u[3], p1, p2, p3, a);
-            flux2(g, u, p1, p2, p3, a, fp, fm, hp, hm);
-            bad |= !positive(u[0]) || !positive(p3);
+            const REAL u[4] = {Uin[c], Uin[n + c], Uin[2 * n + c], Uin[3 * n + c]};
+            bad |= cell2(g, u, fp, fm, hp, hm);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -394,8 +559,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = sy * hm; Tt = F(3, k, li, lj + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = sy * hp; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); }
-            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
-            u = sub_scaled(u, g.ly, hp - hm + Tt - B);
+            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
+            u = sub_scaled(u, g.sy, hp - hm + Tt - B);
         } else {
             // outflow walls, slopes zero on edge cells (2nd_order_base_shll.c:210-458)
             auto DX_ = [&](int q, int r) -> REAL { return sd[(q * 4 + k) * NXS + r * TJ + threadIdx.x]; };
@@ -410,10 +575,10 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = hp; Tt = F(3, k, li, lj + 1); Bdf = 0; Tdf = DY_(1, cc + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = hm; Bdf = DY_(0, cc - 1); Tdf = 0; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); Bdf = DY_(0, cc - 1); Tdf = DY_(1, cc + 1); }
-            u = sub_scaled(u, g.lx, fp - fm + Rr - L);
-            u = sub_half_scaled(u, g.hlx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
-            u = sub_scaled(u, g.ly, hp - hm + Tt - B);
-            u = sub_half_scaled(u, g.hly, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
+            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
+            u = sub_half_scaled(u, g.hsx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
+            u = sub_scaled(u, g.sy, hp - hm + Tt - B);
+            u = sub_half_scaled(u, g.hsy, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
         }
         Uout[k * n + c] = u;
     }
@@ -515,7 +680,7 @@ __global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ f
             } else {
                 auto sl = [&](const REAL* f, long cc, int ii, int st, int nn) -> REAL {
                     if (ii <= 0 || ii >= nn - 1) return (REAL)0;
-                    return slope(g, f[cc - st], f[cc], f[cc + st]);
+                    return slope(g, f[cc - st], f[cc], f[cc + st], (REAL)1);
                 };
                 REAL L, Rr, Ldf, Rdf;
                 if (i == 0) { L = Fp[c]; Rr = Fm[c + sx_]; Ldf = 0; Rdf = sl(Fm, c + sx_, i + 1, sx_, nx); }
