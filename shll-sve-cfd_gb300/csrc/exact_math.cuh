@@ -169,20 +169,22 @@ EM_FN double scale_pow2(double x, int k, double pow2k) {
     return (b << 1) == 0 ? x : em_mul(x, pow2k);
 }
 
-// l * r < 0.0 as the FP64 product decides it (a product that underflows to zero is not negative),
-// for l and r given as `scale` (1 or 2) times themselves
-EM_FN bool product_negative(double l, double r, double inv_scale) {
+// minmod(l, r): 0 when l * r < 0.0, else the one of smaller magnitude (r on a tie, or when l or r
+// is a NaN), without FP64 instructions.  Sets *special where the sign of the FP64 product must be
+// asked (non-finite operands, or a product that may underflow to zero): minmod_general.
+EM_FN double minmod_plain(double l, double r, bool* special) {
     const uint64_t lb = em_dbits(l), rb = em_dbits(r);
-    const int el = (int)(lb >> 52) & 0x7ff, er = (int)(rb >> 52) & 0x7ff;
-    if ((unsigned)(el - 1) < 2046u && (unsigned)(er - 1) < 2046u && el + er >= 1000) return ((lb ^ rb) >> 63) != 0;
-    if ((lb << 1) == 0 || (rb << 1) == 0) return false;
-    return em_mul(em_mul(l, inv_scale), em_mul(r, inv_scale)) < 0.0;
+    const uint64_t la = lb << 1, ra = rb << 1;
+    const int el = (int)(la >> 53), er = (int)(ra >> 53);
+    *special = *special || (el + er < 1000 && la != 0 && ra != 0) || el == 2047 || er == 2047;
+    const bool negative = (int32_t)((lb ^ rb) >> 32) < 0 && la != 0 && ra != 0;
+    const uint64_t m = la < ra ? lb : rb;
+    return em_bitsd(negative ? 0 : m);
 }
-
-// fabs(l) < fabs(r); false when either is a NaN
-EM_FN bool magnitude_less(double l, double r) {
-    const uint64_t lb = em_dbits(l) << 1, rb = em_dbits(r) << 1;
-    return lb < rb && rb <= (0x7ffull << 53);
+// (inv_scale: 1 / the scale of l and r, for the product)
+EM_FN double minmod_general(double l, double r, double inv_scale) {
+    if (em_mul(em_mul(l, inv_scale), em_mul(r, inv_scale)) < 0.0) return 0.0;
+    return fabs(l) < fabs(r) ? l : r;
 }
 
 // ---- the published arithmetic's double expressions of float values, in FP32 -----------------

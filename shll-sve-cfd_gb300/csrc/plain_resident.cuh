@@ -103,23 +103,36 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
             __syncthreads();
             if constexpr (ORDER == 1) {
                 if (next) {
+                    REAL x[3], v[3];
+                    bool special = false;
 #pragma unroll
                     for (int q = 0; q < 3; q++) {
                         // reflective walls (base_shll.c:93-110)
                         const REAL sg = (q == 1) ? (REAL)1 : (REAL)-1;
                         const REAL L = i == 0 ? sg * fm[q] : F[q * T + tid - 1];
                         const REAL Rr = i == n - 1 && i != 0 ? sg * fp[q] : F[(3 + q) * T + tid + 1];
-                        u[q] = sub_scaled(u[q], g.sx, fp[q] - fm[q] + Rr - L);
+                        x[q] = fp[q] - fm[q] + Rr - L;
+                        v[q] = sub_scaled_plain(u[q], g.sx, x[q], &special);
                     }
+#pragma unroll
+                    for (int q = 0; q < 3; q++) u[q] = special ? sub_scaled(u[q], g.sx, x[q]) : v[q];
                 }
             } else {
                 REAL dp[3] = {0, 0, 0}, dm[3] = {0, 0, 0};
                 if (valid && i >= max(lo + 1, 0) && i < min(hi - 1, n)) {
                     if (i > 0 && i < n - 1) {
+                        bool special = false;
 #pragma unroll
                         for (int q = 0; q < 3; q++) {
-                            dp[q] = slope(g, F[q * T + tid - 1], fp[q], F[q * T + tid + 1]);
-                            dm[q] = slope(g, F[(3 + q) * T + tid - 1], fm[q], F[(3 + q) * T + tid + 1]);
+                            dp[q] = slope_plain(g, F[q * T + tid - 1], fp[q], F[q * T + tid + 1], &special);
+                            dm[q] = slope_plain(g, F[(3 + q) * T + tid - 1], fm[q], F[(3 + q) * T + tid + 1], &special);
+                        }
+                        if (special) {
+#pragma unroll
+                            for (int q = 0; q < 3; q++) {
+                                dp[q] = slope(g, F[q * T + tid - 1], fp[q], F[q * T + tid + 1]);
+                                dm[q] = slope(g, F[(3 + q) * T + tid - 1], fm[q], F[(3 + q) * T + tid + 1]);
+                            }
                         }
                     }
 #pragma unroll
@@ -127,15 +140,21 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
                 }
                 __syncthreads();
                 if (next) {   // outflow walls (2nd_order_base_shll.c:210-262)
+                    REAL x[3], y[3], v[3];
+                    bool special = false;
 #pragma unroll
                     for (int q = 0; q < 3; q++) {
                         const bool wl = i == 0, wr = i == n - 1 && i != 0;
                         const REAL L = wl ? fp[q] : F[q * T + tid - 1], Ldf = wl ? (REAL)0 : slp[q * T + tid - 1];
                         const REAL Rr = wr ? fm[q] : F[(3 + q) * T + tid + 1];
                         const REAL Rdf = wr ? (REAL)0 : slp[(3 + q) * T + tid + 1];
-                        u[q] = sub_scaled(u[q], g.sx, fp[q] - fm[q] + Rr - L);
-                        u[q] = sub_half_scaled(u[q], g.hsx, dp[q] + dm[q] - Rdf - Ldf);
+                        x[q] = fp[q] - fm[q] + Rr - L;
+                        y[q] = dp[q] + dm[q] - Rdf - Ldf;
+                        v[q] = sub_half_scaled_plain(sub_scaled_plain(u[q], g.sx, x[q], &special), g.hsx, y[q], &special);
                     }
+#pragma unroll
+                    for (int q = 0; q < 3; q++)
+                        u[q] = special ? sub_half_scaled(sub_scaled(u[q], g.sx, x[q]), g.hsx, y[q]) : v[q];
                 }
             }
         }

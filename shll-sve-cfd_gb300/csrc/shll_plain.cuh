@@ -105,20 +105,31 @@ __device__ __forceinline__ bool positive(double x) {
 }
 __device__ __forceinline__ bool positive(float x) { return x > 0.f; }
 // u - f * x.  With f a power of two f * x is exact unless it is subnormal, so that one fused operation
-// rounds like the product and the difference.
-__device__ __forceinline__ double sub_scaled(double u, const Factor<double>& f, double x) {
+// rounds like the product and the difference; *special where it may be subnormal (then sub_scaled).
+__device__ __forceinline__ double sub_scaled_plain(double u, const Factor<double>& f, double x, bool* special) {
 #if SHLL_PLAIN_FMA
     return __fma_rn(-f.v, x, u);
 #else
     if (!f.pow2) return u - f.v * x;
-    const double r = __fma_rn(-f.v, x, u);
     const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    if (h < (600u << 20) && (h | (unsigned)__double2loint(x)) != 0u) return u - f.v * x;
-    return r;
+    *special = *special || (h < (600u << 20) && (h | (unsigned)__double2loint(x)) != 0u);
+    return __fma_rn(-f.v, x, u);
 #endif
 }
+__device__ __forceinline__ double sub_scaled(double u, const Factor<double>& f, double x) {
+    bool special = false;
+    const double r = sub_scaled_plain(u, f, x, &special);
+    return special ? u - f.v * x : r;
+}
+__device__ __forceinline__ float sub_scaled_plain(float u, const Factor<float>& f, float x, bool*) { return u - f.v * x; }
 __device__ __forceinline__ float sub_scaled(float u, const Factor<float>& f, float x) { return u - f.v * x; }
 // (REAL)(D(u) - 0.5 * D(lambda) * D(x)), f = 0.5 * lambda
+__device__ __forceinline__ double sub_half_scaled_plain(double u, const Factor<double>& f, double x, bool* special) {
+    return sub_scaled_plain(u, f, x, special);
+}
+__device__ __forceinline__ float sub_half_scaled_plain(float u, const Factor<float>& f, float x, bool*) {
+    return exact_math::sub_product_ref(u, f.v, x);
+}
 __device__ __forceinline__ double sub_half_scaled(double u, const Factor<double>& f, double x) {
     return sub_scaled(u, f, x);
 }
@@ -273,23 +284,35 @@ __device__ __forceinline__ int cell1(const Gas<float>& g, const float u[3], floa
 }
 
 // minmod (2nd_order_base_shll.c:191-201)
-// (inv_scale: 1 / the scale of the arguments, for the sign of their product where it underflows)
-__device__ __forceinline__ double minmod(double l, double r, double inv_scale) {
-    if (exact_math::product_negative(l, r, inv_scale)) return 0.0;
-    return exact_math::magnitude_less(l, r) ? l : r;
+__device__ __forceinline__ double minmod(double l, double r, bool* special) {
+    return exact_math::minmod_plain(l, r, special);
 }
-__device__ __forceinline__ float minmod(float l, float r, float) {
+__device__ __forceinline__ float minmod(float l, float r, bool*) {
     if (__fmul_rn(l, r) < 0.f) return 0.f;
     return fabsf(l) < fabsf(r) ? l : r;
 }
-// slope of a split flux at an interior cell: minmod, or the MC limiter of
-// base-omp/2nd_order_base_shll.c:316-325
+// slope of a split flux at an interior cell from the differences l = fc - fl and r = fr - fc (and
+// c = fr - fl): minmod, or the MC limiter of base-omp/2nd_order_base_shll.c:316-325.  Where *special
+// comes back set, slope_general decides.
+template <typename REAL>
+__device__ __forceinline__ REAL slope_plain(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr, bool* special) {
+    const REAL m = minmod(fc - fl, fr - fc, special);
+    return g.limiter == 1 ? minmod(half_of(fr - fl), g.alpha * m, special) : m;
+}
+template <typename REAL>
+__device__ __noinline__ REAL slope_general(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr, REAL inv_scale) {
+    if constexpr (sizeof(REAL) == 4) return slope_plain(g, fl, fc, fr, nullptr);
+    else {
+        const REAL m = exact_math::minmod_general(fc - fl, fr - fc, inv_scale);
+        return g.limiter == 1 ? exact_math::minmod_general(half_of(fr - fl), g.alpha * m, inv_scale) : m;
+    }
+}
 template <typename REAL>
 __device__ __forceinline__ REAL slope(const Gas<REAL>& g, REAL fl, REAL fc, REAL fr,
                                       REAL inv_scale = (REAL)1 / kFluxScale<REAL>) {
-    if (g.limiter == 1)
-        return minmod(half_of(fr - fl), g.alpha * minmod(fc - fl, fr - fc, inv_scale), inv_scale);
-    return minmod(fc - fl, fr - fc, inv_scale);
+    bool special = false;
+    const REAL s = slope_plain(g, fl, fc, fr, &special);
+    return special ? slope_general(g, fl, fc, fr, inv_scale) : s;
 }
 
 constexpr int T1 = 256;  // cells per block (1D)
