@@ -489,6 +489,7 @@ extern "C" int shll_step(shll_ctx* c, long nsteps) {
         PlainArgs a = plain_args(c);
         a.Uin = c->U[c->cur];
         a.Uout = c->U[c->cur ^ 1];
+        a.chained = s > 0;
         CUDA_TRY(c, plain_step(c, a));
         c->cur ^= 1;
     }

@@ -148,7 +148,7 @@ int plain_batch_run(PlainBatch* b, char* err, size_t len) {
         if (b->dim == 1) {
             for (int a = 0; a < it.nx; a += T1) v.push_back({t, a, 0});
         } else {
-            for (int a = 0; a < it.nx; a += TI)
+            for (int a = 0; a < it.nx; a += kBatchTI)
                 for (int c = 0; c < it.ny; c += TJ) v.push_back({t, a, c});
         }
     }

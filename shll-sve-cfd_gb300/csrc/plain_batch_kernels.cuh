@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(T1) k_batch1(const PItem* __restrict__ items, 
 }
 
 template <int ORDER>
-__global__ void __launch_bounds__(TI * TJ) k_batch2(const PItem* __restrict__ items, const PBlk* __restrict__ blks,
+__global__ void __launch_bounds__(tile_threads(kBatchTI, ORDER)) k_batch2(const PItem* __restrict__ items, const PBlk* __restrict__ blks,
                                                     double* U0, double* U1, long plane, int step, int* flags) {
     const PBlk bk = blks[blockIdx.x];
     const PItem& it = items[bk.item];
@@ -36,7 +36,8 @@ __global__ void __launch_bounds__(TI * TJ) k_batch2(const PItem* __restrict__ it
     const int inb = (it.par + step) & 1;
     const double* Uin = (inb ? U1 : U0) + it.base;
     double* Uout = (inb ? U0 : U1) + it.base;
-    step2_tile<double, ORDER>(Uin, Uout, it.nx, it.ny, plane, it.g, flags + bk.item, bk.a, bk.b);
+    step2_tile<double, ORDER>(Uin, Uout, it.nx, it.ny, plane, it.g, flags + bk.item, bk.a, bk.b,
+                              kBatchTI);
 }
 
 // one time step of the nb active blocks of one order (dim 1: k_batch1, dim 2: k_batch2)
@@ -50,13 +51,14 @@ static cudaError_t batch_launch(int dim, int order, int nb, cudaStream_t s, cons
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev < 64 && !(attr_set & (1ull << dev))) {
-            cudaFuncSetAttribute(k_batch2<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<double, 1>());
-            cudaFuncSetAttribute(k_batch2<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<double, 2>());
+            cudaFuncSetAttribute(k_batch2<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<double>(kBatchTI, 1));
+            cudaFuncSetAttribute(k_batch2<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<double>(kBatchTI, 2));
             attr_set |= 1ull << dev;
         }
-        dim3 blk(TJ, TI);
-        if (order == 1) k_batch2<1><<<nb, blk, smem2<double, 1>(), s>>>(items, blks, U0, U1, plane, step, flags);
-        else k_batch2<2><<<nb, blk, smem2<double, 2>(), s>>>(items, blks, U0, U1, plane, step, flags);
+        const int threads = tile_threads(kBatchTI, order);
+        const size_t smem = smem2<double>(kBatchTI, order);
+        if (order == 1) k_batch2<1><<<nb, threads, smem, s>>>(items, blks, U0, U1, plane, step, flags);
+        else k_batch2<2><<<nb, threads, smem, s>>>(items, blks, U0, U1, plane, step, flags);
     }
     return cudaGetLastError();
 }

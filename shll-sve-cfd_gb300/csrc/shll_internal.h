@@ -37,6 +37,7 @@ struct PlainArgs {
     double R, GAMMA, CV, DT_ON_DX, DT_ON_DY, mc_alpha;
     int* flag;
     cudaStream_t stream;
+    bool chained;   // a step that follows another of the same run directly (2D: programmatic launch)
 };
 
 // 1D runs of several steps (plain_resident.cuh): progress counters one 128-byte line apart, for at

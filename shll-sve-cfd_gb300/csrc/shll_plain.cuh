@@ -432,72 +432,102 @@ __device__ __noinline__ CellFlux<REAL, 16> cell2_general(const Gas<REAL>& g, REA
     c.bad = !positive(u0) || !positive(p3);
     return c;
 }
+// What both directions' split fluxes of a cell need; plain: the main path holds for this cell.
 template <typename REAL>
-__device__ __forceinline__ void split2d(const REAL u[4], REAL p1, REAL p2, REAL P, REAL Z1x, REAL Z2x, REAL Z3x, REAL Z1y,
-                                        REAL Z2y, REAL Z3y, REAL fp[4], REAL fm[4], REAL hp[4], REAL hm[4]) {
-    const REAL f[4] = {u[1], u[1] * p1 + P, u[1] * p2, p1 * (u[3] + P)};
-    const REAL h[4] = {u[2], u[2] * p1, u[2] * p2 + P, p2 * (u[3] + P)};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        fp[k] = f[k] * Z1x + u[k] * Z2x; fm[k] = -f[k] * Z3x - u[k] * Z2x;
-        hp[k] = h[k] * Z1y + u[k] * Z2y; hm[k] = -h[k] * Z3y - u[k] * Z2y;
-    }
-}
-__device__ __forceinline__ int cell2(const Gas<double>& g, const double u[4], double fp[4], double fm[4], double hp[4],
-                                     double hm[4]) {
-    const exact_math::Divisor rho = exact_math::divisor(u[0]);
-    const double p1 = divide_or_zero(u[1], rho), p2 = divide_or_zero(u[2], rho);
-    const double e = exact_math::divide_plain(u[3], rho);
-    const double t = __fma_rn(-0.5, p1 * p1 + p2 * p2, e);
-    const double p3 = exact_math::divide_plain(t, g.cv);
+struct Cell2;
+template <>
+struct Cell2<double> {
+    double p[2], P, a;
     exact_math::Divisor snd;
-    const double a = exact_math::square_root_plain(g.gR * p3, &snd);
-    const double Mx = divide_or_zero(p1, snd), My = divide_or_zero(p2, snd);
-    split2d<double>(u, p1, p2, times_R(g, u[0]) * p3, Mx + 1.0, a * (1.0 - Mx * Mx), Mx - 1.0, My + 1.0,
-                    a * (1.0 - My * My), My - 1.0, fp, fm, hp, hm);
-    if (g.plain && in_range(u[0], 923, 200) && in_range(u[3], 923, 200) && momentum_plain(u[1]) && momentum_plain(u[2]) &&
-        in_range(t, 900, 250))
-        return 0;
-    const auto c = cell2_general(g, u[0], u[1], u[2], u[3]);
-#pragma unroll
-    for (int k = 0; k < 4; k++) { fp[k] = c.f[k]; fm[k] = c.f[4 + k]; hp[k] = c.f[8 + k]; hm[k] = c.f[12 + k]; }
-    return c.bad;
-}
-__device__ __forceinline__ int cell2(const Gas<float>& g, const float u[4], float fp[4], float fm[4], float hp[4],
-                                     float hm[4]) {
-    const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
-    const float p1 = exact_math::divide_plain(u[1], u[0], y), p2 = exact_math::divide_plain(u[2], u[0], y);
-    const float p3 = temp2(g, exact_math::divide_plain(u[3], u[0], y), p1, p2), x = g.gR * p3;
-    float ya;
-    const float a = exact_math::square_root_plain(x, &ya);
-    ya = exact_math::reciprocal_plain(a, ya);
-    const float Mx = exact_math::divide_plain(p1, a, ya), My = exact_math::divide_plain(p2, a, ya);
-    split2d<float>(u, p1, p2, times_R(g, u[0]) * p3, half_sum(Mx, 1.f), z2(a, Mx), half_sum(Mx, -1.f), half_sum(My, 1.f),
-                   z2(a, My), half_sum(My, -1.f), fp, fm, hp, hm);
-    if (g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[3], 87, 80) && momentum_plain(u[1]) &&
-        momentum_plain(u[2]) && in_range(x, 87, 80) && !all_ones(a))
-        return 0;
-    const auto c = cell2_general(g, u[0], u[1], u[2], u[3]);
-#pragma unroll
-    for (int k = 0; k < 4; k++) { fp[k] = c.f[k]; fm[k] = c.f[4 + k]; hp[k] = c.f[8 + k]; hm[k] = c.f[12 + k]; }
-    return c.bad;
-}
-
-constexpr int TJ = 32;  // tile extent along j (contiguous, threadIdx.x)
-constexpr int TI = 8;   // tile extent along i (threadIdx.y)
-
-template <int ORDER>
-struct Tile2 {
-    static constexpr int H = ORDER;
-    static constexpr int WI = TI + 2 * H, WJ = TJ + 2 * H, CELLS = WI * WJ;
+    bool plain;
+    __device__ __forceinline__ Cell2(const Gas<double>& g, const double u[4]) {
+        const exact_math::Divisor rho = exact_math::divisor(u[0]);
+        p[0] = divide_or_zero(u[1], rho);
+        p[1] = divide_or_zero(u[2], rho);
+        const double e = exact_math::divide_plain(u[3], rho);
+        // (symmetric in the two velocities, so that a cell's y flux is the x flux of its mirror image)
+        const double t = __fma_rn(-0.5, __dadd_rn(__dmul_rn(p[0], p[0]), __dmul_rn(p[1], p[1])), e);
+        const double p3 = exact_math::divide_plain(t, g.cv);
+        a = exact_math::square_root_plain(g.gR * p3, &snd);
+        P = times_R(g, u[0]) * p3;
+        plain = g.plain && in_range(u[0], 923, 200) && in_range(u[3], 923, 200) && momentum_plain(u[1]) &&
+                momentum_plain(u[2]) && in_range(t, 900, 250);
+    }
+    __device__ __forceinline__ double mach(double pn) const { return divide_or_zero(pn, snd); }
 };
+template <>
+struct Cell2<float> {
+    float p[2], P, a, ya;
+    bool plain;
+    __device__ __forceinline__ Cell2(const Gas<float>& g, const float u[4]) {
+        const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
+        p[0] = exact_math::divide_plain(u[1], u[0], y);
+        p[1] = exact_math::divide_plain(u[2], u[0], y);
+        const float p3 = temp2(g, exact_math::divide_plain(u[3], u[0], y), p[0], p[1]), x = g.gR * p3;
+        a = exact_math::square_root_plain(x, &ya);
+        ya = exact_math::reciprocal_plain(a, ya);
+        P = times_R(g, u[0]) * p3;
+        plain = g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[3], 87, 80) && momentum_plain(u[1]) &&
+                momentum_plain(u[2]) && in_range(x, 87, 80) && !all_ones(a);
+    }
+    __device__ __forceinline__ float mach(float pn) const { return exact_math::divide_plain(pn, a, ya); }
+};
+__device__ __forceinline__ void z123(double a, double M, double& Z1, double& Z2, double& Z3) {   // twice the reference's
+    Z1 = M + 1.0;
+    Z2 = a * (1.0 - M * M);
+    Z3 = M - 1.0;
+}
+__device__ __forceinline__ void z123(float a, float M, float& Z1, float& Z2, float& Z3) {
+    Z1 = half_sum(M, 1.f);
+    Z2 = z2(a, M);
+    Z3 = half_sum(M, -1.f);
+}
+// The split fluxes of a cell in the directions d0..d1 (0 x, 1 y), stored to out[(8 d + 4 pm + k) *
+// stride], pm 0 plus and 1 minus.  A loop over the directions and not two copies of its body: the
+// cells of a tile's halo need one direction only, and the code stays half as long.
+template <typename REAL>
+__device__ __forceinline__ int cell2(const Gas<REAL>& g, const REAL u[4], int d0, int d1, REAL* out, int stride) {
+    const Cell2<REAL> c(g, u);
+    if (c.plain) {
+#pragma unroll 1
+        for (int d = d0; d <= d1; d++) {
+            const REAL un = d ? u[2] : u[1], ut = d ? u[1] : u[2];     // momentum along d and across
+            const REAL pn = d ? c.p[1] : c.p[0], pt = d ? c.p[0] : c.p[1];
+            REAL Z1, Z2, Z3;
+            z123(c.a, c.mach(pn), Z1, Z2, Z3);
+            const REAL f[4] = {un, un * pn + c.P, un * pt, pn * (u[3] + c.P)};
+            const REAL v[4] = {u[0], un, ut, u[3]};
+            REAL* o = out + 8 * d * stride;
+            const int at[4] = {0, (1 + d) * stride, (2 - d) * stride, 3 * stride};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                o[at[k]] = f[k] * Z1 + v[k] * Z2;
+                o[at[k] + 4 * stride] = -f[k] * Z3 - v[k] * Z2;
+            }
+        }
+        return 0;
+    }
+    const auto q = cell2_general(g, u[0], u[1], u[2], u[3]);
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+        if (k / 8 >= d0 && k / 8 <= d1) out[k * stride] = q.f[k];
+    return q.bad;
+}
 
-template <typename REAL, int ORDER>
-constexpr size_t smem2() {
-    using TL = Tile2<ORDER>;
-    size_t flux = (size_t)16 * TL::CELLS * sizeof(REAL);
-    size_t slopes = ORDER == 2 ? (size_t)8 * ((TI + 2) * TJ + TI * (TJ + 2)) * sizeof(REAL) : 0;
-    return flux + slopes;
+// ---- one 2D step of a TI x 32 tile ----
+// Window: the tile and ORDER cells on each side, without the corners.  Threads: one per tile cell (both
+// directions' fluxes), then one per cell of the halo rows (x flux only) and of the halo columns (y only).
+constexpr int TJ = 32;           // tile extent along j (contiguous)
+constexpr int kBatchTI = 8;      // tile extent along i of the batches
+constexpr int kTileThreads = 768;
+
+__host__ __device__ constexpr int tile_threads(int TI, int H) { return (TI * TJ + 2 * H * TJ + TI * 2 * H + 31) / 32 * 32; }
+
+template <typename REAL>
+constexpr size_t smem2(int TI, int H) {
+    const size_t flux = (size_t)16 * (TI + 2 * H) * (TJ + 2 * H);
+    const size_t slopes = H == 2 ? (size_t)8 * ((TI + 2) * TJ + TI * (TJ + 2)) : 0;
+    return (flux + slopes) * sizeof(REAL);
 }
 
 // One fused 2D time step on a TI x TJ tile.  Shared memory holds fp, fm, hp, hm (4 components
@@ -506,36 +536,38 @@ constexpr size_t smem2() {
 // U[k*stride + i*ny + j].
 template <typename REAL, int ORDER>
 __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* __restrict__ Uout, int nx, int ny,
-                                           long stride, const Gas<REAL>& g, int* __restrict__ flag, int i0, int j0) {
-    using TL = Tile2<ORDER>;
-    constexpr int H = TL::H, WJ = TL::WJ, CELLS = TL::CELLS;
+                                           long stride, const Gas<REAL>& g, int* __restrict__ flag, int i0, int j0,
+                                           const int TI) {
+    constexpr int H = ORDER, WJ = TJ + 2 * H;
+    const int CELLS = (TI + 2 * H) * WJ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     REAL* sf = reinterpret_cast<REAL*>(smem_raw);      // [16][CELLS]: fp0..3 fm0..3 hp0..3 hm0..3
     REAL* sd = sf + 16 * CELLS;                          // order 2 slopes
-    constexpr int NXS = (TI + 2) * TJ, NYS = TI * (TJ + 2);
+    const int NXS = (TI + 2) * TJ, NYS = TI * (TJ + 2);
     const long n = stride;
-    const int tid = threadIdx.y * TJ + threadIdx.x;
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    const int ty = tid / TJ, tx = tid % TJ;
     int bad = 0;
-    for (int t = tid; t < CELLS; t += TI * TJ) {
-        int li = t / WJ, lj = t % WJ;
-        int i = i0 - H + li, j = j0 - H + lj;
-        REAL fp[4] = {0, 0, 0, 0}, fm[4] = {0, 0, 0, 0}, hp[4] = {0, 0, 0, 0}, hm[4] = {0, 0, 0, 0};
-        if (i >= 0 && i < nx && j >= 0 && j < ny) {
-            int c = i * ny + j;
-            const REAL u[4] = {Uin[c], Uin[n + c], Uin[2 * n + c], Uin[3 * n + c]};
-            bad |= cell2(g, u, fp, fm, hp, hm);
-        }
+    REAL u[4] = {1, 0, 0, 1};
+    {
+        int li, lj, d0 = 0, d1 = 1;
+        const int h = tid - TI * TJ;                     // index among the halo cells
+        if (h < 0) { li = ty + H; lj = tx + H; }
+        else if (h < 2 * H * TJ) { li = h / TJ; li += li < H ? 0 : TI; lj = tx + H; d1 = 0; }
+        else { const int q = h - 2 * H * TJ, m = q % (2 * H); li = q / (2 * H) + H; lj = m < H ? m : TJ + m; d0 = 1; }
+        const int i = i0 - H + li, j = j0 - H + lj;
+        if (li < TI + 2 * H && (d0 == 0 || li < TI + H) && i >= 0 && i < nx && j >= 0 && j < ny) {
+            const long c = (long)i * ny + j;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            sf[k * CELLS + t] = fp[k]; sf[(4 + k) * CELLS + t] = fm[k];
-            sf[(8 + k) * CELLS + t] = hp[k]; sf[(12 + k) * CELLS + t] = hm[k];
+            for (int k = 0; k < 4; k++) u[k] = Uin[k * n + c];
+            bad = cell2(g, u, d0, d1, sf + li * WJ + lj, CELLS);
         }
     }
     __syncthreads();
     auto F = [&](int q, int k, int li, int lj) -> REAL { return sf[(q * 4 + k) * CELLS + li * WJ + lj]; };
     if (ORDER == 2) {
         // x slopes for local rows -1..TI (cells i0-1..i0+TI), cols 0..TJ-1
-        for (int t = tid; t < NXS; t += TI * TJ) {
+        for (int t = tid; t < NXS; t += nthreads) {
             int r = t / TJ, lj = t % TJ;
             int i = i0 - 1 + r, j = j0 + lj, li = r - 1 + H, ljj = lj + H;
 #pragma unroll
@@ -549,7 +581,7 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             }
         }
         // y slopes for rows 0..TI-1, cols -1..TJ
-        for (int t = tid; t < NYS; t += TI * TJ) {
+        for (int t = tid; t < NYS; t += nthreads) {
             int r = t / (TJ + 2), c2 = t % (TJ + 2);
             int i = i0 + r, j = j0 - 1 + c2, li = r + H, lj = c2 - 1 + H;
 #pragma unroll
@@ -565,12 +597,13 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
         __syncthreads();
     }
     if (bad) atomicOr(flag, SHLL_FLAG_NONPOSITIVE);
-    const int i = i0 + threadIdx.y, j = j0 + threadIdx.x;
-    if (i >= nx || j >= ny) return;
-    const int c = i * ny + j, li = threadIdx.y + H, lj = threadIdx.x + H;
+    const int i = i0 + ty, j = j0 + tx;
+    if (ty >= TI || i >= nx || j >= ny) return;
+    const long c = (long)i * ny + j;
+    const int li = ty + H, lj = tx + H;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        REAL u = Uin[k * n + c];
+        REAL v = u[k];
         REAL fp = F(0, k, li, lj), fm = F(1, k, li, lj), hp = F(2, k, li, lj), hm = F(3, k, li, lj);
         if (ORDER == 1) {
             // reflective walls: x flips components 0,2,3; y flips 0,1,3 (base_shll_2d.c:150-216)
@@ -582,15 +615,15 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = sy * hm; Tt = F(3, k, li, lj + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = sy * hp; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); }
-            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
-            u = sub_scaled(u, g.sy, hp - hm + Tt - B);
+            v = sub_scaled(v, g.sx, fp - fm + Rr - L);
+            v = sub_scaled(v, g.sy, hp - hm + Tt - B);
         } else {
             // outflow walls, slopes zero on edge cells (2nd_order_base_shll.c:210-458)
-            auto DX_ = [&](int q, int r) -> REAL { return sd[(q * 4 + k) * NXS + r * TJ + threadIdx.x]; };
+            auto DX_ = [&](int q, int r) -> REAL { return sd[(q * 4 + k) * NXS + r * TJ + tx]; };
             auto DY_ = [&](int q, int cc) -> REAL {
-                return sd[8 * NXS + (q * 4 + k) * NYS + threadIdx.y * (TJ + 2) + cc];
+                return sd[8 * NXS + (q * 4 + k) * NYS + ty * (TJ + 2) + cc];
             };
-            const int r = threadIdx.y + 1, cc = threadIdx.x + 1;
+            const int r = ty + 1, cc = tx + 1;
             REAL L, Rr, Ldf, Rdf, B, Tt, Bdf, Tdf;
             if (i == 0) { L = fp; Rr = F(1, k, li + 1, lj); Ldf = 0; Rdf = DX_(1, r + 1); }
             else if (i == nx - 1) { L = F(0, k, li - 1, lj); Rr = fm; Ldf = DX_(0, r - 1); Rdf = 0; }
@@ -598,19 +631,38 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = hp; Tt = F(3, k, li, lj + 1); Bdf = 0; Tdf = DY_(1, cc + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = hm; Bdf = DY_(0, cc - 1); Tdf = 0; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); Bdf = DY_(0, cc - 1); Tdf = DY_(1, cc + 1); }
-            u = sub_scaled(u, g.sx, fp - fm + Rr - L);
-            u = sub_half_scaled(u, g.hsx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
-            u = sub_scaled(u, g.sy, hp - hm + Tt - B);
-            u = sub_half_scaled(u, g.hsy, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
+            v = sub_scaled(v, g.sx, fp - fm + Rr - L);
+            v = sub_half_scaled(v, g.hsx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
+            v = sub_scaled(v, g.sy, hp - hm + Tt - B);
+            v = sub_half_scaled(v, g.hsy, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
         }
-        Uout[k * n + c] = u;
+        Uout[k * n + c] = v;
     }
 }
 
+// Consecutive steps are chained by programmatic dependent launch: the next step's blocks are resident
+// and past their launch when this grid completes (griddepcontrol.wait).
 template <typename REAL, int ORDER>
-__global__ void __launch_bounds__(TI * TJ) k_step2(const REAL* __restrict__ Uin, REAL* __restrict__ Uout, int nx,
-                                                   int ny, Gas<REAL> g, int* __restrict__ flag) {
-    step2_tile<REAL, ORDER>(Uin, Uout, nx, ny, (long)nx * ny, g, flag, blockIdx.y * TI, blockIdx.x * TJ);
+__global__ void __launch_bounds__(kTileThreads) k_step2(const REAL* __restrict__ Uin, REAL* __restrict__ Uout, int nx,
+                                                        int ny, const __grid_constant__ Gas<REAL> g,
+                                                        int* __restrict__ flag, int TI) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    step2_tile<REAL, ORDER>(Uin, Uout, nx, ny, (long)nx * ny, g, flag, blockIdx.y * TI, blockIdx.x * TJ, TI);
+}
+
+// Tile height of a domain: the one with the least work on the busiest SM, counting a halo cell as 0.6
+// of a tile cell (one direction of two) and two rows' worth of fixed cost per tile.  (256 x 256 cells
+// on 152 SMs: 14 rows, one tile per SM, where 8 rows put 256 tiles on them.)
+static int tile_rows(int nx, int ny, int H, int sms) {
+    int best = kBatchTI;
+    double best_t = 1e30;
+    for (int TI = 4; tile_threads(TI, H) <= kTileThreads && TI <= 20; TI++) {
+        const long tiles = (long)((nx + TI - 1) / TI) * ((ny + TJ - 1) / TJ);
+        const double t = (double)((tiles + sms - 1) / sms) * (TI + 0.6 * 2 * H + 0.6 * 2 * H * TI / TJ + 2.0);
+        if (t < best_t) { best_t = t; best = TI; }
+    }
+    return best;
 }
 
 // ---------------- staged kernels (the reference's separate stages) ----------------
@@ -746,16 +798,25 @@ static cudaError_t step_t(const PlainArgs& a) {
         if (a.order == 1) k_step1<REAL, 1><<<grid, T1, 0, a.stream>>>(Uin, Uout, a.nx, g, a.flag);
         else k_step1<REAL, 2><<<grid, T1, 0, a.stream>>>(Uin, Uout, a.nx, g, a.flag);
     } else {
-        dim3 grid((a.ny + TJ - 1) / TJ, (a.nx + TI - 1) / TI), block(TJ, TI);
-        if (a.order == 1) {
-            constexpr size_t sm = smem2<REAL, 1>();
-            cudaFuncSetAttribute(k_step2<REAL, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_step2<REAL, 1><<<grid, block, sm, a.stream>>>(Uin, Uout, a.nx, a.ny, g, a.flag);
-        } else {
-            constexpr size_t sm = smem2<REAL, 2>();
-            cudaFuncSetAttribute(k_step2<REAL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_step2<REAL, 2><<<grid, block, sm, a.stream>>>(Uin, Uout, a.nx, a.ny, g, a.flag);
-        }
+        int dev = 0, sms = 152;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int TI = tile_rows(a.nx, a.ny, a.order, sms);
+        auto* kern = a.order == 1 ? k_step2<REAL, 1> : k_step2<REAL, 2>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)((a.ny + TJ - 1) / TJ), (unsigned)((a.nx + TI - 1) / TI));
+        cfg.blockDim = dim3((unsigned)tile_threads(TI, a.order));
+        cfg.dynamicSmemBytes = smem2<REAL>(TI, a.order);
+        cfg.stream = a.stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = a.chained ? 1 : 0;
+        if (e == cudaSuccess && !a.chained)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<REAL>(20, a.order));
+        if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, Uin, Uout, a.nx, a.ny, g, a.flag, TI);
+        if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
