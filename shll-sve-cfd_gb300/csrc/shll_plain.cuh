@@ -651,18 +651,23 @@ __global__ void __launch_bounds__(kTileThreads) k_step2(const REAL* __restrict__
     step2_tile<REAL, ORDER>(Uin, Uout, nx, ny, (long)nx * ny, g, flag, blockIdx.y * TI, blockIdx.x * TJ, TI);
 }
 
-// Tile height of a domain: the one with the least work on the busiest SM, counting a halo cell as 0.6
-// of a tile cell (one direction of two) and two rows' worth of fixed cost per tile.  (256 x 256 cells
-// on 152 SMs: 14 rows, one tile per SM, where 8 rows put 256 tiles on them.)
-static int tile_rows(int nx, int ny, int H, int sms) {
+// Tile height of a domain.  FP64: the one with the least work on the busiest SM, counting a halo cell
+// as 0.6 of a tile cell (one direction of two) and two rows' worth of fixed cost per tile (256 x 256
+// cells on 152 SMs: 14 rows, one tile per SM, 13.7 us a step, where 8 rows take 15.7 and 12 rows
+// 22.5).  Float steps are bound by latency, which several small tiles on an SM hide from each
+// other: 6 rows (256 x 256, first order: 4.3 us against 5.0 with 14), second order 8 rows (301 x 277:
+// 7.6 us against 8.7 with 10) unless one tile per SM will do (256 x 256: 6.2 us against 7.2 with 8).
+static int tile_rows(int nx, int ny, int H, int sms, bool wide) {
     int best = kBatchTI;
+    long best_tiles = 0;
     double best_t = 1e30;
     for (int TI = 4; tile_threads(TI, H) <= kTileThreads && TI <= 20; TI++) {
         const long tiles = (long)((nx + TI - 1) / TI) * ((ny + TJ - 1) / TJ);
         const double t = (double)((tiles + sms - 1) / sms) * (TI + 0.6 * 2 * H + 0.6 * 2 * H * TI / TJ + 2.0);
-        if (t < best_t) { best_t = t; best = TI; }
+        if (t < best_t) { best_t = t; best = TI; best_tiles = tiles; }
     }
-    return best;
+    if (wide) return best;
+    return H == 1 ? 6 : best_tiles <= sms ? best : 8;
 }
 
 // ---------------- staged kernels (the reference's separate stages) ----------------
@@ -801,7 +806,7 @@ static cudaError_t step_t(const PlainArgs& a) {
         int dev = 0, sms = 152;
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int TI = tile_rows(a.nx, a.ny, a.order, sms);
+        const int TI = tile_rows(a.nx, a.ny, a.order, sms, sizeof(REAL) == 8);
         auto* kern = a.order == 1 ? k_step2<REAL, 1> : k_step2<REAL, 2>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((a.ny + TJ - 1) / TJ), (unsigned)((a.nx + TI - 1) / TI));
