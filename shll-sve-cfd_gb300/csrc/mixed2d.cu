@@ -645,34 +645,127 @@ struct Smem22 {
     float dn[4][4][2];
     float dnd[4][4][2];
     Coef2D cf;
-    float recx[2][TJ][4][2];   // applied x fluxes summed over the steps: [west edge, east edge][column][comp]
-    float recy[2][TI][4][2];   // applied y fluxes: [south edge, north edge][row][comp]
+    float2 rowc[2][TJ + 4][4];   // edge corrections of the window's cells on the lines i0, i0 + TI
+    float2 colc[2][WR2][4];      // and on the lines j0, j0 + TJ (as FP32 pairs, per component)
 };
-static_assert(sizeof(TileC2) == offsetof(Smem22, recx), "the tile constants are copied word for word");
+static_assert(sizeof(TileC2) == offsetof(Smem22, rowc), "the tile constants are copied word for word");
 
-template <bool KAHAN, bool LAM_POW2, bool VEC>
-__global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
-    __shared__ Smem22 S;
-    extern __shared__ __align__(16) float2 g_flux2[];   // [step][16][WR2][WP]
-    const TileD tile = A.tiles[blockIdx.x];
-    const Dom2 D = A.doms[tile.dom];
-    const int ns = min(2, D.steps - A.step);             // steps this domain takes in the launch
-    if (ns <= 0) return;
+// one component of the correction owed to cell (i, j) (edge_correction), as an FP32 pair
+__device__ __forceinline__ float2 edge_correction1(const Args2& A, const Dom2& D, int i, int j, int pp, int k) {
+    float ch = 0.f, cl = 0.f;
+    auto add = [&](const Edge* e) {
+        const float2 w = *reinterpret_cast<const float2*>(&e->r[0][k][0]), o = *reinterpret_cast<const float2*>(&e->r[1][k][0]);
+        two_sum_acc(ch, cl, w.x);
+        two_sum_acc(ch, cl, -o.x);
+        cl = __fadd_rn(cl, __fadd_rn(w.y, -o.y));
+    };
+    if (i > 0 && i % TI == 0) add(&A.ex[pp][D.ex_base + (i / TI - 1) * D.ny + j]);
+    if (j > 0 && j % TJ == 0) add(&A.ey[pp][D.ey_base + (j / TJ - 1) * D.nx + i]);
+    return make_float2(ch, cl);
+}
+
+// The corrections of the window's cells on tile edge lines (those rows and columns of the window, which
+// starts at row i0 - 2 and column j0 - 2), one thread per cell and component: a pair of cells that
+// gathered them for itself made every warp run that code for the few lanes on a line.
+template <class SM>
+__device__ __forceinline__ void load_corrections(const Args2& A, const Dom2& D, int i0, int j0, int pp, SM& S) {
+    constexpr int NR = 2 * (TJ + 4) * 4, NC = 2 * WR2 * 4;
+    for (int t = threadIdx.x; t < NR + NC; t += NT2) {
+        const int k = t & 3;
+        if (t < NR) {
+            const int c = (t >> 2) % (TJ + 4), line = (t >> 2) / (TJ + 4);
+            const int i = i0 + line * TI, j = j0 - 2 + c;
+            if (i > 0 && i < D.nx && j >= 0 && j < D.ny) S.rowc[line][c][k] = edge_correction1(A, D, i, j, pp, k);
+        } else {
+            const int q = (t - NR) >> 2, r = q % WR2, line = q / WR2;
+            const int i = i0 - 2 + r, j = j0 + line * TJ;
+            if (j > 0 && j < D.ny && i >= 0 && i < D.nx) S.colc[line][r][k] = edge_correction1(A, D, i, j, pp, k);
+        }
+    }
+}
+// adds them to the increment pairs of the pair at window row wr, pair column wc (cells (i, jx), (i, jx + 1))
+template <class SM>
+__device__ __forceinline__ void add_corrections(const SM& S, int wr, int wc, int i, int jx, const bool ex[2], float2 h[4],
+                                                float2 l[4]) {
+    auto add = [&](const float2* c, int q) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {   // the pending edge correction joins the increment pair
+            float hh = lane(h[k], q), ll = lane(l[k], q);
+            const float2 v = c[k];
+            two_sum_acc(hh, ll, v.x);
+            ll = __fadd_rn(ll, v.y);
+            set_lane(h[k], q, hh);
+            set_lane(l[k], q, ll);
+        }
+    };
+    if ((wr == 2 || wr == 2 + TI) && i > 0) {
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (ex[q]) add(S.rowc[wr == 2 ? 0 : 1][2 * wc + q], q);
+    } else if ((wc == 1 || wc == 1 + TJ / 2) && jx > 0 && ex[0]) {
+        add(S.colc[wc == 1 ? 0 : 1][wr], 0);
+    }
+}
+
+// A thread's edge record: tasks 0..255 are the tile's west and east edges (128 each: a column and a
+// component), 256..383 its south and north edges (a row and a component).  x_a and x_b: where the two
+// fluxes that meet at the interface lie in a flux buffer (floats [16][WR2][2 * WP]); the applied terms
+// lam (x_a + x_b) of the launch's steps are summed by this thread as the cells apply them.
+struct EdgeTask {
+    bool valid;
+    int xa, xb, dir, k;
+    float* out;       // the record's pair of this tile's side
+    __device__ __forceinline__ EdgeTask(const Dom2& D, int i0, int j0, int hi_i, int hi_j, Edge* exo, Edge* eyo) {
+        const int t = threadIdx.x;
+        k = t & 3;
+        auto at = [](int q, int r, int c) { return (q * WR2 + r) * 2 * WP + c; };
+        if (t < 2 * TJ * 4) {
+            const int col = (t >> 2) % TJ, east = (t >> 2) / TJ, c = 2 + col;
+            const int i = east ? i0 + hi_i : i0;      // the cell east of the interface
+            dir = 0;
+            valid = col < hi_j && (east ? i < D.nx : i > 0);
+            xa = at(k, i - i0 + 1, c);                // fp of the western cell
+            xb = at(4 + k, i - i0 + 2, c);            // fm of the eastern cell
+            out = valid ? exo[D.ex_base + (i / TI - 1) * D.ny + j0 + col].r[east ? 0 : 1][k] : nullptr;
+        } else {
+            const int q = (t - 2 * TJ * 4) >> 2, row = q % TI, north = q / TI;
+            const int j = north ? j0 + hi_j : j0;
+            dir = 1;
+            valid = row < hi_i && (north ? j < D.ny : j > 0);
+            xa = at(8 + k, row + 2, j - j0 + 1);
+            xb = at(12 + k, row + 2, j - j0 + 2);
+            out = valid ? eyo[D.ey_base + (j / TJ - 1) * D.nx + i0 + row].r[north ? 0 : 1][k] : nullptr;
+        }
+    }
+    // the term applied at the interface, lam (x_a + x_b), as an FP32 pair
+    template <bool LAM_POW2>
+    __device__ __forceinline__ void term(const Dom2& D, const float* f, float& th, float& tl) const {
+        const float x = __fadd_rn(f[xa], f[xb]), lh = dir ? D.lyh : D.lxh, ll = dir ? D.lyl : D.lxl;
+        th = __fmul_rn(lh, x);
+        // (fused as the assembler fuses the packed form that the cells apply)
+        tl = LAM_POW2 ? 0.f : __fmaf_rn(ll, x, __fmaf_rn(lh, x, -th));
+    }
+    // the full flux applied: steps times lam Fref, plus the terms
+    __device__ __forceinline__ void store(const float lf[2][4][2], float steps, float rh, float rl) const {
+        float oh, ol;
+        ff_add(__fmul_rn(steps, lf[dir][k][0]), __fmul_rn(steps, lf[dir][k][1]), rh, rl, oh, ol);
+        *reinterpret_cast<float2*>(out) = make_float2(oh, ol);
+    }
+};
+static_assert(2 * TJ * 4 + 2 * TI * 4 == NT2, "one edge task per thread");
+
+// INNER: the whole window lies inside the domain (no walls, no cut tile): no bounds, masks or selects;
+// the values that the outermost window cells take after the first step are read by no own cell.
+template <bool KAHAN, bool LAM_POW2, bool VEC, bool INNER>
+__device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, const int i0, const int j0, const int ns,
+                                             Smem22& S, float2* g_flux2) {
     const int tid = threadIdx.x;
     const int kw = A.step - A.s0;                         // step within the fold window
-    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
-    const int hi_i = min(TI, D.nx - i0), hi_j = min(TJ, D.ny - j0);
+    const int hi_i = INNER ? TI : min(TI, D.nx - i0), hi_j = INNER ? TJ : min(TJ, D.ny - j0);
     const int P = A.plane;
-    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
     const float* phi = A.Ph[kw % 3];                      // increments so far (kw = 0: none)
     const float* pli = A.Pl[kw % 3];
-    float* pho = A.Ph[(kw + ns) % 3];
-    float* plo = A.Pl[(kw + ns) % 3];
     const int pp = (A.step + 2) % 3;                      // edge buffers of the previous launch
-    Edge* exo = A.ex[(A.step + ns - 1) % 3];
-    Edge* eyo = A.ey[(A.step + ns - 1) % 3];
-    if (tid < kTileC2Words)
-        reinterpret_cast<float*>(&S.wc)[tid] = reinterpret_cast<const float*>(&A.tc[tb])[tid];
     auto flux = [&](int b, int q, int r, int c) -> float2& { return g_flux2[((b * 16 + q) * WR2 + r) * WP + c]; };
 
     // ---- this thread's window pair: row wr (cell row i), pair column wc (cells jx, jx + 1) ----
@@ -681,7 +774,7 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
     const int i = i0 - 2 + wr, jx = j0 - 2 + 2 * wc;
     bool ex[2];
 #pragma unroll
-    for (int q = 0; q < 2; q++) ex[q] = pt && i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny;
+    for (int q = 0; q < 2; q++) ex[q] = INNER || (pt && i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny);
     // owner tile of the pair relative to this one (rows i0-2, i0-1 west, i0+16.. east; pair 0 south,
     // pair 17 north); -1: this tile
     const int di = wr < 2 ? -1 : (wr >= 2 + TI ? 1 : 0), dj = wc == 0 ? -1 : (wc == WP - 1 ? 1 : 0);
@@ -694,62 +787,47 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
     const bool l1[2] = {ex[0] && r1 && jx >= j0 - 1 && jx <= j0 + TJ, ex[1] && r1 && jx + 1 >= j0 - 1 && jx + 1 <= j0 + TJ};
     const bool ro = wr >= 2 && wr < 2 + hi_i;
     const bool own[2] = {ex[0] && ro && jx >= j0 && jx < j0 + hi_j, ex[1] && ro && jx + 1 >= j0 && jx + 1 < j0 + hi_j};
-    __syncthreads();   // (the tile constants)
 
     float2 base[4], ah[4], al[4];   // deviation of the pair at the launch's start, its increments
 #pragma unroll
     for (int k = 0; k < 4; k++) { base[k] = f2(0.f); ah[k] = f2(0.f); al[k] = f2(0.f); }
-    if (VEC && ex[0]) {   // (an even row length: the pair is inside or outside together)
-        float2 c2[4];
-        load_pair2(A, D, i, jx, kw, pp, phi, pli, ah, al, c2);
+    const int cell = D.base + i * D.ny + jx;
+    if (VEC) {   // (an even row length: the pair is inside or outside together)
+        if (ex[0]) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            base[k] = c2[k];
-            if (nbi >= 0) {
-                const float* o = nbi < 4 ? S.dn[nbi][k] : S.dnd[nbi - 4][k];
-                base[k] = add2(add2(base[k], f2(o[0])), f2(o[1]));
+            for (int k = 0; k < 4; k++) {
+                if (kw > 0) {
+                    ah[k] = *reinterpret_cast<const float2*>(phi + k * P + cell);
+                    al[k] = *reinterpret_cast<const float2*>(pli + k * P + cell);
+                }
+                base[k] = *reinterpret_cast<const float2*>(A.C + k * P + cell);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (!ex[q]) continue;   // outside the domain: zero deviation (finite fluxes, never applied)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (kw > 0) {
+                    set_lane(ah[k], q, phi[k * P + cell + q]);
+                    set_lane(al[k], q, pli[k * P + cell + q]);
+                }
+                set_lane(base[k], q, A.C[k * P + cell + q]);
             }
         }
     }
-#pragma unroll
-    for (int q = 0; q < 2 && !VEC; q++) {
-        if (!ex[q]) continue;   // outside the domain: zero deviation (finite fluxes, never applied)
-        const int cell = D.base + i * D.ny + jx + q;
-        float ch[4] = {0, 0, 0, 0}, cl[4] = {0, 0, 0, 0};
-        const bool edge = kw > 0 && on_edge_line(i, jx + q);
-        if (edge) edge_correction(A, D, i, jx + q, pp, ch, cl);
+    if (kw > 0) load_corrections(A, D, i0, j0, pp, S);
+    __syncthreads();   // (the tile constants and the corrections)
+    if (kw > 0) add_corrections(S, wr, wc, i, jx, ex, ah, al);
+    // deviation from this tile's frame: C (relative to the owner's frame) + the owner's frame offset
+    if (nbi >= 0) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const int idx = k * P + cell;
-            float h = 0.f, l = 0.f;
-            if (kw > 0) { h = phi[idx]; l = pli[idx]; }
-            if (edge) {   // the pending edge correction joins the increment pair
-                two_sum_acc(h, l, ch[k]);
-                l = __fadd_rn(l, cl[k]);
-            }
-            set_lane(ah[k], q, h);
-            set_lane(al[k], q, l);
-            // deviation from this tile's frame: C (relative to the owner's frame) + the owner's frame offset
-            float b = A.C[idx];
-            if (nbi >= 0) {
-                const float* o = nbi < 4 ? S.dn[nbi][k] : S.dnd[nbi - 4][k];
-                b = __fadd_rn(__fadd_rn(b, o[0]), o[1]);
-            }
-            set_lane(base[k], q, b);
-        }
-    }
-    // edge records of the tile's own boundary cells (each written only by the cell's owner thread)
-    const bool recW = ro && wr == 2 && i0 > 0, recE = ro && wr == 2 + hi_i - 1 && i + 1 < D.nx;
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        if (!own[q]) continue;
-        const int col = jx + q - j0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (recW) { S.recx[0][col][k][0] = 0.f; S.recx[0][col][k][1] = 0.f; }
-            if (recE) { S.recx[1][col][k][0] = 0.f; S.recx[1][col][k][1] = 0.f; }
-            if (jx + q == j0 && j0 > 0) { S.recy[0][wr - 2][k][0] = 0.f; S.recy[0][wr - 2][k][1] = 0.f; }
-            if (jx + q == j0 + hi_j - 1 && jx + q + 1 < D.ny) { S.recy[1][wr - 2][k][0] = 0.f; S.recy[1][wr - 2][k][1] = 0.f; }
+            const float* o = nbi < 4 ? S.dn[nbi][k] : S.dnd[nbi - 4][k];
+            const float2 b = add2(add2(base[k], f2(o[0])), f2(o[1]));
+            if (INNER) base[k] = b;
+            else base[k] = make_float2(ex[0] ? b.x : 0.f, ex[1] ? b.y : 0.f);
         }
     }
 
@@ -768,17 +846,20 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
         }
     };
     const float2 lx2 = f2(D.lxh), lxl2 = f2(D.lxl), ly2 = f2(D.lyh), lyl2 = f2(D.lyl);
-    const bool wS = jx == 0, wNx = jx == D.ny - 1, wNy = jx + 1 == D.ny - 1;   // y walls per lane
+    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == D.ny - 1, wNy = !INNER && jx + 1 == D.ny - 1;   // y walls per lane
     const float2 mS = make_float2(wS ? 0.f : 1.f, 1.f), mN = make_float2(wNx ? 0.f : 1.f, wNy ? 0.f : 1.f);
-    const int cs = max(wc - 1, 0), cn = min(wc + 1, WP - 1);   // (clamped: the lanes they serve are masked)
-    // one step's interface terms from buffer b added to the lanes `up`, the tile's edge records of the
-    // lanes `rec` accumulated
-    auto update = [&](int b, const bool up[2], const bool rec[2]) {
+    // (clamped neighbours: the lanes they serve are masked, or not read)
+    const int cs = max(wc - 1, 0), cn = min(wc + 1, WP - 1), rw = max(wr - 1, 0), re = min(wr + 1, WR2 - 1);
+    // one step's interface terms from buffer b added to the lanes `up`
+    auto update = [&](int b, const bool up[2]) {
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
+            th = mul2_alone(lh, x);
+            tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
+        };
+        auto lam_wall = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {   // (seen by no other cell)
             th = mul2(lh, x);
             tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
         };
-        auto record = [&](float* r, float th, float tl) { two_sum_acc(r[0], r[1], th); r[1] = __fadd_rn(r[1], tl); };
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 fp = flux(b, k, wr, wc), fm = flux(b, 4 + k, wr, wc);
@@ -794,47 +875,33 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
             };
             float2 th, tl;
             // x west
-            if (i > 0) {
-                lam(lx2, lxl2, add2(flux(b, k, wr - 1, wc), fm), th, tl);
+            if (INNER || i > 0) {
+                lam(lx2, lxl2, add2(flux(b, k, rw, wc), fm), th, tl);
                 acc(th, tl);
-                if (recW)
-                    for (int q = 0; q < 2; q++)
-                        if (rec[q]) record(S.recx[0][jx + q - j0][k], lane(th, q), lane(tl, q));
             } else {
                 two_sum_acc2(h2, l2, f2(S.wc[0][k][0]));
                 l2 = add2(l2, f2(S.wc[0][k][1]));
-                if (k == 1) { lam(lx2, lxl2, mul2(f2(2.f), fm), th, tl); acc(th, tl); }
+                if (k == 1) { lam_wall(lx2, lxl2, mul2(f2(2.f), fm), th, tl); acc(th, tl); }
             }
             // x east
-            if (i < D.nx - 1) {
-                lam(lx2, lxl2, add2(fp, flux(b, 4 + k, wr + 1, wc)), th, tl);
+            if (INNER || i < D.nx - 1) {
+                lam(lx2, lxl2, add2(fp, flux(b, 4 + k, re, wc)), th, tl);
                 dec(th, tl);
-                if (recE)
-                    for (int q = 0; q < 2; q++)
-                        if (rec[q]) record(S.recx[1][jx + q - j0][k], lane(th, q), lane(tl, q));
             } else {
                 two_sum_acc2(h2, l2, f2(S.wc[1][k][0]));
                 l2 = add2(l2, f2(S.wc[1][k][1]));
-                if (k == 1) { lam(lx2, lxl2, mul2(f2(-2.f), fp), th, tl); acc(th, tl); }
+                if (k == 1) { lam_wall(lx2, lxl2, mul2(f2(-2.f), fp), th, tl); acc(th, tl); }
             }
             // y south: lanes (jx-1 | jx) and (jx | jx+1)
-            {
-                lam(ly2, lyl2, add2(make_float2(flux(b, 8 + k, wr, cs).y, hp.x), hm), th, tl);
-                th = mul2(th, mS); tl = mul2(tl, mS);
-                acc(th, tl);
-                if (rec[0] && jx == j0 && j0 > 0) record(S.recy[0][wr - 2][k], th.x, tl.x);
-            }
+            lam(ly2, lyl2, add2(make_float2(flux(b, 8 + k, wr, cs).y, hp.x), hm), th, tl);
+            if (!INNER) { th = mul2(th, mS); tl = mul2(tl, mS); }
+            acc(th, tl);
             // y north: lanes (jx | jx+1) and (jx+1 | jx+2)
-            {
-                lam(ly2, lyl2, add2(hp, make_float2(hm.y, flux(b, 12 + k, wr, cn).x)), th, tl);
-                th = mul2(th, mN); tl = mul2(tl, mN);
-                dec(th, tl);
-                for (int q = 0; q < 2; q++)
-                    if (rec[q] && jx + q == j0 + hi_j - 1 && jx + q + 1 < D.ny)
-                        record(S.recy[1][wr - 2][k], lane(th, q), lane(tl, q));
-            }
+            lam(ly2, lyl2, add2(hp, make_float2(hm.y, flux(b, 12 + k, wr, cn).x)), th, tl);
+            if (!INNER) { th = mul2(th, mN); tl = mul2(tl, mN); }
+            dec(th, tl);
             // y walls
-            if (wS || wNx || wNy) {
+            if (!INNER && (wS || wNx || wNy)) {
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     const bool south = q == 0 && wS, north = q == 0 ? wNx : wNy;
@@ -851,59 +918,74 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
                     set_lane(h2, q, h); set_lane(l2, q, l);
                 }
             }
-            // only the lanes of the update region change
-            ah[k] = make_float2(up[0] ? h2.x : ah[k].x, up[1] ? h2.y : ah[k].y);
-            al[k] = make_float2(up[0] ? l2.x : al[k].x, up[1] ? l2.y : al[k].y);
+            if (INNER) {
+                ah[k] = h2;
+                al[k] = l2;
+            } else {   // only the lanes of the update region change
+                ah[k] = make_float2(up[0] ? h2.x : ah[k].x, up[1] ? h2.y : ah[k].y);
+                al[k] = make_float2(up[0] ? l2.x : al[k].x, up[1] ? l2.y : al[k].y);
+            }
         }
     };
 
+    const EdgeTask edge(D, i0, j0, hi_i, hi_j, A.ex[(A.step + ns - 1) % 3], A.ey[(A.step + ns - 1) % 3]);
+    float rh = 0.f, rl = 0.f;       // the edge task's terms, summed over the steps
+    auto record = [&](int b) {
+        if (!edge.valid) return;
+        float th, tl;
+        edge.term<LAM_POW2>(D, reinterpret_cast<const float*>(g_flux2 + b * 16 * WR2 * WP), th, tl);
+        two_sum_acc(rh, rl, th);
+        rl = __fadd_rn(rl, tl);
+    };
     fluxes(0);
     __syncthreads();
-    if (l1[0] || l1[1]) update(0, l1, own);
+    record(0);
+    if (INNER ? (ns == 2 || own[0]) : (l1[0] || l1[1])) update(0, l1);
     if (ns == 2) {
         fluxes(1);
         __syncthreads();
-        if (own[0] || own[1]) update(1, own, own);
+        record(1);
+        if (own[0] || own[1]) update(1, own);
     }
+    if (edge.valid) edge.store(S.lf, (float)ns, rh, rl);   // (1 or 2: exact scaling of the pairs)
 
-    // ---- the tile's increments and its edge records (full applied fluxes lam Fref ns + the sums) ----
-    const float sc = (float)ns;   // (1 or 2: exact scaling of the pairs)
+    // ---- the tile's increments ----
+    float* pho = A.Ph[(kw + ns) % 3];
+    float* plo = A.Pl[(kw + ns) % 3];
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        if (!own[q]) continue;
-        const int cell = D.base + i * D.ny + jx + q;
-        const int col = jx + q - j0;
+    for (int k = 0; k < 4; k++) {
+        if (VEC) {   // (both lanes own)
+            if (own[0]) {
+                *reinterpret_cast<float2*>(pho + k * P + cell) = ah[k];
+                *reinterpret_cast<float2*>(plo + k * P + cell) = al[k];
+            }
+        } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (VEC) {   // (both lanes own: written once, from lane x)
-                if (q == 0) {
-                    *reinterpret_cast<float2*>(pho + k * P + cell) = ah[k];
-                    *reinterpret_cast<float2*>(plo + k * P + cell) = al[k];
+            for (int q = 0; q < 2; q++)
+                if (own[q]) {
+                    pho[k * P + cell + q] = lane(ah[k], q);
+                    plo[k * P + cell + q] = lane(al[k], q);
                 }
-            } else {
-                pho[k * P + cell] = lane(ah[k], q);
-                plo[k * P + cell] = lane(al[k], q);
-            }
-            const float lxh = __fmul_rn(sc, S.lf[0][k][0]), lxl = __fmul_rn(sc, S.lf[0][k][1]);
-            const float lyh = __fmul_rn(sc, S.lf[1][k][0]), lyl = __fmul_rn(sc, S.lf[1][k][1]);
-            if (recW) {
-                float* rr = exo[D.ex_base + (i / TI - 1) * D.ny + jx + q].r[1][k];
-                ff_add(lxh, lxl, S.recx[0][col][k][0], S.recx[0][col][k][1], rr[0], rr[1]);
-            }
-            if (recE) {
-                float* rr = exo[D.ex_base + ((i + 1) / TI - 1) * D.ny + jx + q].r[0][k];
-                ff_add(lxh, lxl, S.recx[1][col][k][0], S.recx[1][col][k][1], rr[0], rr[1]);
-            }
-            if (jx + q == j0 && j0 > 0) {
-                float* rr = eyo[D.ey_base + (j0 / TJ - 1) * D.nx + i].r[1][k];
-                ff_add(lyh, lyl, S.recy[0][wr - 2][k][0], S.recy[0][wr - 2][k][1], rr[0], rr[1]);
-            }
-            if (jx + q == j0 + hi_j - 1 && jx + q + 1 < D.ny) {
-                float* rr = eyo[D.ey_base + ((jx + q + 1) / TJ - 1) * D.nx + i].r[0][k];
-                ff_add(lyh, lyl, S.recy[1][wr - 2][k][0], S.recy[1][wr - 2][k][1], rr[0], rr[1]);
-            }
         }
     }
+}
+
+template <bool KAHAN, bool LAM_POW2, bool VEC>
+__global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
+    __shared__ Smem22 S;
+    extern __shared__ __align__(16) float2 g_flux2[];   // [step][16][WR2][WP]
+    const TileD tile = A.tiles[blockIdx.x];
+    const Dom2 D = A.doms[tile.dom];
+    const int ns = min(2, D.steps - A.step);             // steps this domain takes in the launch
+    if (ns <= 0) return;
+    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
+    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
+    if (threadIdx.x < kTileC2Words)
+        reinterpret_cast<float*>(&S.wc)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[tb])[threadIdx.x];
+    if (i0 >= 2 && i0 + TI + 2 <= D.nx && j0 >= 2 && j0 + TJ + 2 <= D.ny)
+        step2d2_tile<KAHAN, LAM_POW2, VEC, true>(A, D, i0, j0, ns, S, g_flux2);
+    else
+        step2d2_tile<KAHAN, LAM_POW2, VEC, false>(A, D, i0, j0, ns, S, g_flux2);
 }
 
 // ---- one second-order time step of one tile ----

@@ -65,6 +65,16 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     return *reinterpret_cast<const float2*>(&d);
 }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+// a * b per lane, never fused into a sum that follows: a product whose only use is a packed sum is
+// fused with it by the assembler, even as mul.rn (the same value unless the product is subnormal, where
+// a fused term would differ from the one that the neighbouring cell or the record of a tile edge sees).
+// A fused multiply-add of zero rounds like the product and costs the same.
+__device__ __forceinline__ float2 mul2_alone(float2 a, float2 b) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d)
+        : "l"(*reinterpret_cast<const unsigned long long*>(&a)), "l"(*reinterpret_cast<const unsigned long long*>(&b)), "l"(0ull));
+    return *reinterpret_cast<const float2*>(&d);
+}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(fast_rcp(a.x), fast_rcp(a.y)); }
 __device__ __forceinline__ float2 rsqrt2(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
