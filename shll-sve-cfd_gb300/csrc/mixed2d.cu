@@ -1003,35 +1003,30 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
 // their increment pairs, and the tile's edge records (as in the first-order kernel).
 constexpr int kStepO2Smem = 2 * 16 * WR2 * WP * (int)sizeof(float2);   // split fluxes, face values
 
-struct SmemO2 {             // the tile's step constants (a copy of its TileC2)
-    float wc[4][4][2];
+struct SmemO2 {
+    float wc[4][4][2];           // the tile's step constants (a copy of its TileC2)
     float lf[2][4][2];
     float dn[4][4][2];
     float dnd[4][4][2];
     Coef2D cf;
+    float2 rowc[2][TJ + 4][4];   // edge corrections (see Smem22)
+    float2 colc[2][WR2][4];
 };
-static_assert(sizeof(SmemO2) == sizeof(TileC2), "the tile constants are copied word for word");
+static_assert(sizeof(TileC2) == offsetof(SmemO2, rowc), "the tile constants are copied word for word");
 
-template <bool KAHAN, bool LAM_POW2, int LIM, bool VEC>
-__global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
-    __shared__ SmemO2 S;
-    extern __shared__ __align__(16) float2 g_o2[];   // [32][WR2][WP]: fp fm hp hm, then Lx Rx Ly Ry
-    const TileD tile = A.tiles[blockIdx.x];
-    const Dom2 D = A.doms[tile.dom];
-    if (A.step >= D.steps) return;
+// INNER: the whole window lies inside the domain (no walls, no cut tile)
+template <bool KAHAN, bool LAM_POW2, int LIM, bool VEC, bool INNER>
+__device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, const int i0, const int j0, SmemO2& S,
+                                               float2* g_o2) {
     const int tid = threadIdx.x;
     const int kw = A.step - A.s0;                         // step within the fold window
-    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
-    const int hi_i = min(TI, D.nx - i0), hi_j = min(TJ, D.ny - j0);
+    const int hi_i = INNER ? TI : min(TI, D.nx - i0), hi_j = INNER ? TJ : min(TJ, D.ny - j0);
     const int P = A.plane;
-    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
     const float* phi = A.Ph[kw % 3];                      // increments so far (kw = 0: none)
     const float* pli = A.Pl[kw % 3];
     float* pho = A.Ph[(kw + 1) % 3];
     float* plo = A.Pl[(kw + 1) % 3];
     const int pp = (A.step + 2) % 3;                      // edge buffers of the previous step
-    if (tid < kTileC2Words)
-        reinterpret_cast<float*>(&S)[tid] = reinterpret_cast<const float*>(&A.tc[tb])[tid];
     auto fl = [&](int q, int r, int c) -> float2& { return g_o2[(q * WR2 + r) * WP + c]; };
 
     // ---- this thread's window pair: row wr (cell row i), pair column wc (cells jx, jx + 1) ----
@@ -1044,10 +1039,10 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
     bool ex[2];
 #pragma unroll
     for (int q = 0; q < 2; q++)
-        ex[q] = pt && (di == 0 || dj == 0) && i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny;
+        ex[q] = pt && (di == 0 || dj == 0) && (INNER || (i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny));
     const bool ro = wr >= 2 && wr < 2 + hi_i;
     const bool own[2] = {ex[0] && ro && jx >= j0 && jx < j0 + hi_j, ex[1] && ro && jx + 1 >= j0 && jx + 1 < j0 + hi_j};
-    __syncthreads();   // (the tile constants)
+    const int cell = D.base + i * D.ny + jx;
 
     // ---- phase 1: deviations and split fluxes ----
     float2 ah[4], al[4];   // the pair's increments so far (own pairs)
@@ -1055,38 +1050,42 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
         float2 d[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) { d[k] = f2(0.f); ah[k] = f2(0.f); al[k] = f2(0.f); }
-        if (VEC && ex[0]) {   // (an even row length: the pair is inside or outside together)
-            float2 c2[4];
-            load_pair2(A, D, i, jx, kw, pp, phi, pli, ah, al, c2);
+        if (VEC) {   // (an even row length: the pair is inside or outside together)
+            if (ex[0]) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                float2 b = c2[k];
-                if (nbi >= 0) b = add2(add2(b, f2(S.dn[nbi][k][0])), f2(S.dn[nbi][k][1]));
-                d[k] = add2(b, add2(ah[k], al[k]));
+                for (int k = 0; k < 4; k++) {
+                    if (kw > 0) {
+                        ah[k] = *reinterpret_cast<const float2*>(phi + k * P + cell);
+                        al[k] = *reinterpret_cast<const float2*>(pli + k * P + cell);
+                    }
+                    d[k] = *reinterpret_cast<const float2*>(A.C + k * P + cell);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (!ex[q]) continue;   // outside the domain or a corner: zero deviation (finite, never applied)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (kw > 0) {
+                        set_lane(ah[k], q, phi[k * P + cell + q]);
+                        set_lane(al[k], q, pli[k * P + cell + q]);
+                    }
+                    set_lane(d[k], q, A.C[k * P + cell + q]);
+                }
             }
         }
+        if (kw > 0) load_corrections(A, D, i0, j0, pp, S);
+        __syncthreads();   // (the tile constants and the corrections)
+        if (kw > 0) add_corrections(S, wr, wc, i, jx, ex, ah, al);
 #pragma unroll
-        for (int q = 0; q < 2 && !VEC; q++) {
-            if (!ex[q]) continue;   // outside the domain or a corner: zero deviation (finite, never applied)
-            const int cell = D.base + i * D.ny + jx + q;
-            float ch[4] = {0, 0, 0, 0}, cl[4] = {0, 0, 0, 0};
-            const bool edge = kw > 0 && on_edge_line(i, jx + q);
-            if (edge) edge_correction(A, D, i, jx + q, pp, ch, cl);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int idx = k * P + cell;
-                float h = 0.f, l = 0.f;
-                if (kw > 0) { h = phi[idx]; l = pli[idx]; }
-                if (edge) {   // the pending edge correction joins the increment pair
-                    two_sum_acc(h, l, ch[k]);
-                    l = __fadd_rn(l, cl[k]);
-                }
-                set_lane(ah[k], q, h);
-                set_lane(al[k], q, l);
-                float b = A.C[idx];
-                if (nbi >= 0) b = __fadd_rn(__fadd_rn(b, S.dn[nbi][k][0]), S.dn[nbi][k][1]);
-                set_lane(d[k], q, __fadd_rn(b, __fadd_rn(h, l)));
+        for (int k = 0; k < 4; k++) {
+            float2 b = d[k];
+            if (nbi >= 0) {
+                b = add2(add2(b, f2(S.dn[nbi][k][0])), f2(S.dn[nbi][k][1]));
+                b = make_float2(ex[0] ? b.x : 0.f, ex[1] ? b.y : 0.f);
             }
+            d[k] = add2(b, add2(ah[k], al[k]));
         }
         float2 fp[4], fm[4], hp[4], hm[4];
         dflux2x2(S.cf, d, fp, fm, hp, hm);
@@ -1104,7 +1103,7 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
     const float alpha = D.alpha;
     if (pt && wr >= 1 && wr <= TI + 2 && wc >= 1 && wc <= TJ / 2) {
         // x: slopes along i, zero on the edge cells i = 0, nx - 1 (and outside the domain)
-        const float hx = (i <= 0 || i >= D.nx - 1) ? 0.f : 0.5f;
+        const float hx = !INNER && (i <= 0 || i >= D.nx - 1) ? 0.f : 0.5f;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 pm = fl(k, wr - 1, wc), pc = fl(k, wr, wc), pq = fl(k, wr + 1, wc);
@@ -1117,8 +1116,8 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
         // y: slopes along j (lane x needs the south pair's lane y, lane y the north pair's lane x;
         // the clamped neighbours only serve lanes that no interface reads), zero on j = 0, ny - 1
         const int cs = max(wc - 1, 0), cn = min(wc + 1, WP - 1);
-        const float2 hy = make_float2((jx <= 0 || jx >= D.ny - 1) ? 0.f : 0.5f,
-                                      (jx + 1 <= 0 || jx + 1 >= D.ny - 1) ? 0.f : 0.5f);
+        const float2 hy = make_float2(!INNER && (jx <= 0 || jx >= D.ny - 1) ? 0.f : 0.5f,
+                                      !INNER && (jx + 1 <= 0 || jx + 1 >= D.ny - 1) ? 0.f : 0.5f);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 pc = fl(8 + k, wr, wc);
@@ -1130,26 +1129,25 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
         }
     }
     __syncthreads();
-    if (!(own[0] || own[1])) return;
 
-    // ---- phase 3: interfaces and increments of the own pair ----
-    const bool has_y = own[1];
+    // ---- phase 3: the tile's edge records, the interfaces and increments of the own pairs ----
+    const EdgeTask edge(D, i0, j0, hi_i, hi_j, A.ex[A.step % 3], A.ey[A.step % 3]);
+    if (edge.valid) {
+        float th, tl;   // (the face values lie as the split fluxes do, 16 planes further)
+        edge.term<LAM_POW2>(D, reinterpret_cast<const float*>(g_o2 + 16 * WR2 * WP), th, tl);
+        edge.store(S.lf, 1.f, th, tl);
+    }
+    if (!(own[0] || own[1])) return;
     const float2 lx2 = f2(D.lxh), lxl2 = f2(D.lxl), ly2 = f2(D.lyh), lyl2 = f2(D.lyl);
-    const bool wW = i == 0, wE = i == D.nx - 1;                       // x walls (whole pair)
-    const bool wS = jx == 0, wNx = jx == D.ny - 1, wNy = jx + 1 == D.ny - 1;   // y walls per lane
-    const bool recW = wr == 2 && i0 > 0, recE = wr == 2 + hi_i - 1 && i + 1 < D.nx;
-    const int jn = j0 + hi_j - 1;   // the tile's north edge column
-    const bool recN = jn + 1 < D.ny && (jx == jn || jx + 1 == jn);
-    const int qn = jx == jn ? 0 : 1;
-    Edge* exo = A.ex[A.step % 3];
-    Edge* eyo = A.ey[A.step % 3];
+    const bool wW = !INNER && i == 0, wE = !INNER && i == D.nx - 1;   // x walls (whole pair)
+    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == D.ny - 1, wNy = !INNER && jx + 1 == D.ny - 1;   // y walls per lane
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const float2 Lx = fl(16 + k, wr, wc), Rx = fl(20 + k, wr, wc);
         const float2 Ly = fl(24 + k, wr, wc), Ry = fl(28 + k, wr, wc);
         float2 h = ah[k], l = al[k];
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
-            th = mul2(lh, x);
+            th = mul2_alone(lh, x);
             tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
         };
         float2 th, tl;
@@ -1157,45 +1155,43 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
         lam(lx2, lxl2, add2(wW ? Lx : fl(16 + k, wr - 1, wc), Rx), th, tl);
         two_sum_acc2(h, l, th);
         if (!LAM_POW2) l = add2(l, tl);
-        if (recW) {   // the tile's west edge: record the full flux this tile applied
-            Edge* e = exo + D.ex_base + (i / TI - 1) * D.ny + jx;
-            ff_add(S.lf[0][k][0], S.lf[0][k][1], th.x, tl.x, e[0].r[1][k][0], e[0].r[1][k][1]);
-            if (has_y) ff_add(S.lf[0][k][0], S.lf[0][k][1], th.y, tl.y, e[1].r[1][k][0], e[1].r[1][k][1]);
-        }
         // x east: F_{i+1/2} = Lx_i + Rx_{i+1}
         lam(lx2, lxl2, add2(Lx, wE ? Rx : fl(20 + k, wr + 1, wc)), th, tl);
         two_diff_acc2(h, l, th);
         if (!LAM_POW2) l = sub2(l, tl);
-        if (recE) {
-            Edge* e = exo + D.ex_base + ((i + 1) / TI - 1) * D.ny + jx;
-            ff_add(S.lf[0][k][0], S.lf[0][k][1], th.x, tl.x, e[0].r[0][k][0], e[0].r[0][k][1]);
-            if (has_y) ff_add(S.lf[0][k][0], S.lf[0][k][1], th.y, tl.y, e[1].r[0][k][0], e[1].r[0][k][1]);
-        }
         // y south: lanes (jx-1 | jx) and (jx | jx+1); lane x at the south wall: its own Ly + Ry
         lam(ly2, lyl2, add2(make_float2(wS ? Ly.x : fl(24 + k, wr, wc - 1).y, Ly.x), Ry), th, tl);
         two_sum_acc2(h, l, th);
         if (!LAM_POW2) l = add2(l, tl);
-        if (jx == j0 && j0 > 0) {   // the tile's south edge (lane x)
-            float* rr = eyo[D.ey_base + (j0 / TJ - 1) * D.nx + i].r[1][k];
-            ff_add(S.lf[1][k][0], S.lf[1][k][1], th.x, tl.x, rr[0], rr[1]);
-        }
         // y north: lanes (jx | jx+1) and (jx+1 | jx+2); at the north wall the lane's own Ly + Ry
         lam(ly2, lyl2, add2(Ly, make_float2(wNx ? Ry.x : Ry.y, wNy ? Ry.y : fl(28 + k, wr, min(wc + 1, WP - 1)).x)), th, tl);
         two_diff_acc2(h, l, th);
         if (!LAM_POW2) l = sub2(l, tl);
-        if (recN) {
-            float* rr = eyo[D.ey_base + ((jn + 1) / TJ - 1) * D.nx + i].r[0][k];
-            ff_add(S.lf[1][k][0], S.lf[1][k][1], lane(th, qn), lane(tl, qn), rr[0], rr[1]);
-        }
-        const int cell = D.base + i * D.ny + jx;
         if (VEC) {   // (both lanes own)
             *reinterpret_cast<float2*>(pho + k * P + cell) = h;
             *reinterpret_cast<float2*>(plo + k * P + cell) = l;
         } else {
             if (own[0]) { pho[k * P + cell] = h.x; plo[k * P + cell] = l.x; }
-            if (has_y) { pho[k * P + cell + 1] = h.y; plo[k * P + cell + 1] = l.y; }
+            if (own[1]) { pho[k * P + cell + 1] = h.y; plo[k * P + cell + 1] = l.y; }
         }
     }
+}
+
+template <bool KAHAN, bool LAM_POW2, int LIM, bool VEC>
+__global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
+    __shared__ SmemO2 S;
+    extern __shared__ __align__(16) float2 g_o2[];   // [32][WR2][WP]: fp fm hp hm, then Lx Rx Ly Ry
+    const TileD tile = A.tiles[blockIdx.x];
+    const Dom2 D = A.doms[tile.dom];
+    if (A.step >= D.steps) return;
+    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
+    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
+    if (threadIdx.x < kTileC2Words)
+        reinterpret_cast<float*>(&S)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[tb])[threadIdx.x];
+    if (i0 >= 2 && i0 + TI + 2 <= D.nx && j0 >= 2 && j0 + TJ + 2 <= D.ny)
+        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, true>(A, D, i0, j0, S, g_o2);
+    else
+        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, false>(A, D, i0, j0, S, g_o2);
 }
 
 }  // namespace
