@@ -31,7 +31,10 @@ struct shll_ctx {
     void* P = nullptr;
     void* F[4] = {nullptr, nullptr, nullptr, nullptr};  // fp, fm, hp, hm (staged; lazily allocated)
     bool fluxes_valid = false;
-    unsigned* prog = nullptr;      // progress counters of 1D runs (allocated by the first one)
+    double* planes = nullptr;      // staging of primitive planes handed over or back (plain paths)
+    bool own_planes = false;       // an allocation of its own (large problems, by the first use)
+    void* slab = nullptr;          // one allocation: U, P, flags, progress counters, small staging planes
+    unsigned* prog = nullptr;      // progress counters of 1D runs
     // device checkpoint of the plain state
     void* ckU = nullptr;
     void* ckP = nullptr;
@@ -229,6 +232,8 @@ static PlainArgs plain_args(shll_ctx* c) {
     a.R = c->R; a.GAMMA = c->GAMMA; a.CV = c->CV; a.DT_ON_DX = c->DT_ON_DX; a.DT_ON_DY = c->DT_ON_DY;
     a.mc_alpha = c->p.mc_alpha;
     a.flag = c->d_flag;
+    a.worst = c->d_flag + 1;
+    a.planes = c->planes;
     a.stream = c->stream;
     return a;
 }
@@ -270,12 +275,28 @@ extern "C" int shll_create(const shll_params* p, shll_ctx** out) {
     }
     c->own_stream = true;
     const size_t rb = c->real_bits / 8, n = (size_t)c->n;
-    bool ok = cudaMalloc(&c->d_flag, sizeof(int)) == cudaSuccess;
-    ok = ok && cudaMemset(c->d_flag, 0, sizeof(int)) == cudaSuccess;
+    bool ok = true;
     if (c->plain) {
-        ok = ok && cudaMalloc(&c->U[0], c->nv * n * rb) == cudaSuccess;
-        ok = ok && cudaMalloc(&c->U[1], c->nv * n * rb) == cudaSuccess;
-        ok = ok && cudaMalloc(&c->P, (c->nv + 1) * n * rb) == cudaSuccess;
+        // one allocation (each costs tens of microseconds, as does its release): state, primitives, error
+        // flags (with the refused cell and the flags of a state being loaded), progress counters, and the
+        // staging planes of problems up to 64 MB of them
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t ub = up(c->nv * n * rb), pb = up((c->nv + 1) * n * rb), fb = 256;
+        const size_t gb = c->p.dim == 1 ? up(sizeof(unsigned) * kPlainProgStride * kPlainProgChunks) : 0;
+        size_t sb = up(c->nv * n * sizeof(double));
+        if (sb > (64u << 20)) sb = 0;
+        unsigned char* m = nullptr;
+        ok = cudaMalloc(&m, 2 * ub + pb + fb + gb + sb) == cudaSuccess;
+        if (ok) {
+            c->slab = m;
+            c->U[0] = m;
+            c->U[1] = m + ub;
+            c->P = m + 2 * ub;
+            c->d_flag = reinterpret_cast<int*>(m + 2 * ub + pb);
+            if (gb) c->prog = reinterpret_cast<unsigned*>(m + 2 * ub + pb + fb);
+            if (sb) c->planes = reinterpret_cast<double*>(m + 2 * ub + pb + fb + gb);
+            ok = cudaMemset(c->d_flag, 0, 3 * sizeof(int)) == cudaSuccess;
+        }
     } else {
         c->mixed = mixed_create(&c->p, c->DT_ON_DX, c->DT_ON_DY, c->CV, c->stream, c->err, sizeof(c->err));
         ok = ok && c->mixed != nullptr;
@@ -292,10 +313,9 @@ extern "C" int shll_create(const shll_params* p, shll_ctx** out) {
 extern "C" void shll_destroy(shll_ctx* c) {
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    cudaFree(c->U[0]); cudaFree(c->U[1]); cudaFree(c->P); cudaFree(c->ckU); cudaFree(c->ckP);
+    cudaFree(c->slab); cudaFree(c->ckU); cudaFree(c->ckP);
     for (int k = 0; k < 4; k++) cudaFree(c->F[k]);
-    cudaFree(c->d_flag);
-    cudaFree(c->prog);
+    if (c->own_planes) cudaFree(c->planes);
     if (c->mixed) mixed_destroy(c->mixed);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -355,7 +375,7 @@ static int load_primitives(shll_ctx* c, const double* prim, bool derive = true) 
     const size_t n = (size_t)c->n, nv = c->nv;
     c->steps_taken = 0;
     c->fluxes_valid = false;
-    CUDA_TRY(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->stream));
+    if (c->plain) CUDA_TRY(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->stream));
     if (!c->plain) {
         int rc = mixed_load(c->mixed, prim, c->err, sizeof(c->err));
         if (rc != SHLL_OK) return rc;
@@ -405,6 +425,19 @@ extern "C" int shll_initial_primitives(const shll_params* p, double* rho, double
     return SHLL_OK;
 }
 
+// nv planes of doubles on the device (plain paths)
+static int ensure_planes(shll_ctx* c) {
+    if (c->planes) return SHLL_OK;
+    if (cudaMalloc(&c->planes, sizeof(double) * c->nv * (size_t)c->n) != cudaSuccess) {
+        cudaGetLastError();
+        c->planes = nullptr;
+        set_err(c, "cudaMalloc of the primitive planes failed");
+        return SHLL_ERR_NOMEM;
+    }
+    c->own_planes = true;
+    return SHLL_OK;
+}
+
 extern "C" int shll_set_primitives(shll_ctx* c, const double* rho, const double* u, const double* v, const double* T) {
     if (!c || !rho || !u || !T || (c->p.dim == 2 && !v)) return SHLL_ERR_ARG;
     if (!c->plain) {  // copied as given and converted (and checked) on the device
@@ -416,24 +449,37 @@ extern "C" int shll_set_primitives(shll_ctx* c, const double* rho, const double*
         c->initialized = true;
         return check_flag(c);
     }
+    // copied as given (at full link speed from pinned memory), then checked and converted on the device:
+    // one synchronisation, no copy on the host
     const size_t n = (size_t)c->n;
-    std::vector<double> prim(c->nv * n);
-    memcpy(prim.data(), rho, n * sizeof(double));
-    memcpy(prim.data() + n, u, n * sizeof(double));
-    if (c->p.dim == 2) {
-        memcpy(prim.data() + 2 * n, v, n * sizeof(double));
-        memcpy(prim.data() + 3 * n, T, n * sizeof(double));
-    } else {
-        memcpy(prim.data() + 2 * n, T, n * sizeof(double));
+    int rc = ensure_planes(c);
+    if (rc != SHLL_OK) return rc;
+    const double* planes[4] = {rho, u, c->p.dim == 2 ? v : T, T};
+    for (int k = 0; k < c->nv; k++)
+        CUDA_TRY(c, cudaMemcpyAsync(c->planes + k * n, planes[k], n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(c->d_flag + 1, 0xff, sizeof(int), c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(c->d_flag + 2, 0, sizeof(int), c->stream));
+    PlainArgs a = plain_args(c);
+    a.Uout = c->U[0];
+    a.flag = c->d_flag + 2;
+    CUDA_TRY(c, plain_stage(c, a, STAGE_LOAD));
+    int got[2] = {-1, 0};
+    CUDA_TRY(c, cudaMemcpyAsync(got, c->d_flag + 1, sizeof(got), cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (got[0] >= 0) {
+        set_err(c, "cell %zu: density and temperature must be positive", n - 1 - (size_t)got[0]);
+        return SHLL_ERR_ARG;
     }
-    for (size_t i = 0; i < n; i++) {
-        double r = prim[i], t = prim[(c->nv - 1) * n + i];
-        if (!(r > 0) || !(t > 0)) {
-            set_err(c, "cell %zu: density and temperature must be positive", i);
-            return SHLL_ERR_ARG;
-        }
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_flag, c->d_flag + 2, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
+    c->steps_taken = 0;
+    c->fluxes_valid = false;
+    c->cur = 0;
+    c->initialized = true;
+    if (got[1] & SHLL_FLAG_NONPOSITIVE) {
+        set_err(c, "non-positive or NaN density/temperature reached");
+        return SHLL_ERR_NUMERIC;
     }
-    return load_primitives(c, prim.data());
+    return SHLL_OK;
 }
 
 static int stage_call(shll_ctx* c, int which) {
@@ -474,10 +520,6 @@ extern "C" int shll_step(shll_ctx* c, long nsteps) {
     }
     // 1D: several steps per launch (plain_resident.cuh), except that a single step has nothing to share
     if (c->p.dim == 1 && nsteps > 1) {
-        if (!c->prog && cudaMalloc(&c->prog, sizeof(unsigned) * kPlainProgStride * kPlainProgChunks) != cudaSuccess) {
-            cudaGetLastError();   // (then one launch per sweep, which needs none)
-            c->prog = nullptr;
-        }
         PlainArgs a = plain_args(c);
         a.Uin = c->U[c->cur];
         a.Uout = c->U[c->cur ^ 1];
@@ -592,7 +634,21 @@ extern "C" int shll_get_primitives(shll_ctx* c, double* rho, double* u, double* 
     if (!c->plain) return mixed_get_primitives(c->mixed, rho, u, v, T, c->err, sizeof(c->err));
     double* d2[3] = {rho, u, T};
     double* d3[4] = {rho, u, v, T};
-    return fetch_planes(c, c->P, 0, c->nv, c->p.dim == 2 ? d3 : d2);
+    double* const* out = c->p.dim == 2 ? d3 : d2;
+    const double* src = static_cast<const double*>(c->P);   // FP64: the planes as they are
+    if (c->real_bits == 32) {
+        int rc = ensure_planes(c);
+        if (rc != SHLL_OK) return rc;
+        PlainArgs a = plain_args(c);
+        a.planes = c->planes;
+        CUDA_TRY(c, plain_stage(c, a, STAGE_DUMP));
+        src = c->planes;
+    }
+    for (int k = 0; k < c->nv; k++)
+        if (out[k])
+            CUDA_TRY(c, cudaMemcpyAsync(out[k], src + (size_t)k * c->n, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    return SHLL_OK;
 }
 
 extern "C" int shll_get_conserved(shll_ctx* c, double* planes) {

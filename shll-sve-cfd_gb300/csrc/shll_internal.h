@@ -23,7 +23,8 @@ void shll_count_launches(long n);
 // the chunk that shll_debug_stall_chunk keeps from publishing its progress (-1: none)
 int shll_stall_chunk();
 
-enum { STAGE_U_FROM_P = 0, STAGE_P_FROM_U = 1, STAGE_F_FROM_P = 2, STAGE_UPDATE = 3 };
+enum { STAGE_U_FROM_P = 0, STAGE_P_FROM_U = 1, STAGE_F_FROM_P = 2, STAGE_UPDATE = 3,
+       STAGE_LOAD = 4, STAGE_DUMP = 5 };   // primitives from / to planes of doubles on the device
 
 // Arguments of the plain (reference-arithmetic) kernels.  The constants are the reference's
 // REAL-typed values widened to double (exact), converted back inside the launchers.
@@ -35,7 +36,9 @@ struct PlainArgs {
     void* P;      // nv primitive planes followed by the sound-speed plane
     void* fp; void* fm; void* hp; void* hm;
     double R, GAMMA, CV, DT_ON_DX, DT_ON_DY, mc_alpha;
-    int* flag;
+    int* flag;      // error flags; STAGE_LOAD: the flags of the new state
+    int* worst;     // STAGE_LOAD: n - 1 - (lowest cell with a non-positive density or temperature), else -1
+    double* planes; // STAGE_LOAD / STAGE_DUMP: nv planes of doubles
     cudaStream_t stream;
     bool chained;   // a step that follows another of the same run directly (2D: programmatic launch)
 };

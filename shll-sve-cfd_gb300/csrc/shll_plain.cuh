@@ -708,6 +708,50 @@ __global__ void k_p_from_u(const REAL* __restrict__ U, REAL* __restrict__ P, lon
     if (bad) atomicOr(flag, SHLL_FLAG_NONPOSITIVE);
 }
 
+// Primitives handed over as planes of doubles: refused as a whole (worst, nothing else written) when a
+// density or temperature is not positive, ...
+template <typename REAL>
+__global__ void k_check_planes(const double* __restrict__ in, long n, int nv, int* __restrict__ worst) {
+    for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x)
+        if (!positive(in[c]) || !positive(in[(nv - 1) * n + c])) {
+            atomicMax(worst, (int)(n - 1 - c));
+            return;   // (a thread's later cells have higher indices)
+        }
+}
+// ... else taken over as main() does (base_shll.c:202-205): P rounded to REAL, U from P, P from U
+template <typename REAL>
+__global__ void k_load_planes(const double* __restrict__ in, REAL* __restrict__ P, REAL* __restrict__ U, long n, int dim,
+                              const __grid_constant__ Gas<REAL> g, const int* __restrict__ worst, int* __restrict__ flag) {
+    if (*worst >= 0) return;
+    int bad = 0;
+    for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
+        if (dim == 1) {
+            const REAL p0 = (REAL)in[c], q1 = (REAL)in[n + c], q2 = (REAL)in[2 * n + c];
+            const REAL u1 = p0 * q1, u2 = (REAL)(D(p0) * (D(q2 * g.CV) + 0.5 * D(q1) * D(q1)));
+            REAL p1, p2, a;
+            prim1(g, p0, u1, u2, p1, p2, a);
+            U[c] = p0; U[n + c] = u1; U[2 * n + c] = u2;
+            P[c] = p0; P[n + c] = p1; P[2 * n + c] = p2; P[3 * n + c] = a;
+            bad |= !positive(p0) || !positive(p2);
+        } else {
+            const REAL p0 = (REAL)in[c], q1 = (REAL)in[n + c], q2 = (REAL)in[2 * n + c], q3 = (REAL)in[3 * n + c];
+            const REAL u1 = p0 * q1, u2 = p0 * q2;
+            const REAL u3 = (REAL)(D(p0) * (D(q3 * g.CV) + 0.5 * D(q1 * q1 + q2 * q2)));
+            REAL p1, p2, p3, a;
+            prim2(g, p0, u1, u2, u3, p1, p2, p3, a);
+            U[c] = p0; U[n + c] = u1; U[2 * n + c] = u2; U[3 * n + c] = u3;
+            P[c] = p0; P[n + c] = p1; P[2 * n + c] = p2; P[3 * n + c] = p3; P[4 * n + c] = a;
+            bad |= !positive(p0) || !positive(p3);
+        }
+    }
+    if (bad) atomicOr(flag, SHLL_FLAG_NONPOSITIVE);
+}
+template <typename REAL>
+__global__ void k_dump_planes(const REAL* __restrict__ P, double* __restrict__ out, long words) {
+    for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < words; c += (long)gridDim.x * blockDim.x)
+        out[c] = D(P[c]);
+}
+
 // Compute_F_from_P from the stored P (and its a plane) and U, as the reference reads both.
 template <typename REAL>
 __global__ void k_f_from_p(const REAL* __restrict__ U, const REAL* __restrict__ P, REAL* __restrict__ fp,
@@ -847,6 +891,14 @@ static cudaError_t stage_t(const PlainArgs& a, int which) {
             k_update_staged<REAL><<<blocks, threads, 0, a.stream>>>(
                 U, static_cast<const REAL*>(a.fp), static_cast<const REAL*>(a.fm), static_cast<const REAL*>(a.hp),
                 static_cast<const REAL*>(a.hm), a.nx, a.dim == 2 ? a.ny : 1, a.dim, a.order, g);
+            break;
+        case STAGE_LOAD:
+            k_check_planes<REAL><<<blocks, threads, 0, a.stream>>>(a.planes, n, a.dim == 2 ? 4 : 3, a.worst);
+            k_load_planes<REAL><<<blocks, threads, 0, a.stream>>>(a.planes, P, U, n, a.dim, g, a.worst, a.flag);
+            shll_count_launches(1);
+            break;
+        case STAGE_DUMP:
+            k_dump_planes<REAL><<<blocks, threads, 0, a.stream>>>(P, a.planes, n * (a.dim == 2 ? 4 : 3));
             break;
         default: return cudaErrorInvalidValue;
     }
