@@ -533,12 +533,18 @@ constexpr size_t smem2(int TI, int H) {
 // One fused 2D time step on a TI x TJ tile.  Shared memory holds fp, fm, hp, hm (4 components
 // each) for the tile plus an ORDER-wide halo, then (order 2) the x and y slopes.
 // Body of one 2D tile with origin (i0, j0) of an nx x ny domain whose component k lives at
-// U[k*stride + i*ny + j].
-template <typename REAL, int ORDER>
-__device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* __restrict__ Uout, int nx, int ny,
+// U[k*stride + i*ny + j].  STAGED: Update_U_from_F, the split fluxes read from the planes of
+// Compute_F_from_P instead of evaluated (Uin == Uout: a cell reads only its own state).
+template <typename REAL, int ORDER, bool STAGED = false>
+__device__ __forceinline__ void step2_tile(const REAL* Uin, REAL* Uout, int nx, int ny,
                                            long stride, const Gas<REAL>& g, int* __restrict__ flag, int i0, int j0,
-                                           const int TI) {
+                                           const int TI, const REAL* const* planes = nullptr) {
     constexpr int H = ORDER, WJ = TJ + 2 * H;
+    constexpr REAL kInvScale = STAGED ? (REAL)1 : (REAL)1 / kFluxScale<REAL>;
+    const Factor<REAL>& fx = STAGED ? g.lx : g.sx;
+    const Factor<REAL>& fy = STAGED ? g.ly : g.sy;
+    const Factor<REAL>& hfx = STAGED ? g.hlx : g.hsx;
+    const Factor<REAL>& hfy = STAGED ? g.hly : g.hsy;
     const int CELLS = (TI + 2 * H) * WJ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     REAL* sf = reinterpret_cast<REAL*>(smem_raw);      // [16][CELLS]: fp0..3 fm0..3 hp0..3 hm0..3
@@ -558,9 +564,19 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
         const int i = i0 - H + li, j = j0 - H + lj;
         if (li < TI + 2 * H && (d0 == 0 || li < TI + H) && i >= 0 && i < nx && j >= 0 && j < ny) {
             const long c = (long)i * ny + j;
+            if constexpr (STAGED) {
+                if (h < 0) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) u[k] = Uin[k * n + c];
-            bad = cell2(g, u, d0, d1, sf + li * WJ + lj, CELLS);
+                    for (int k = 0; k < 4; k++) u[k] = Uin[k * n + c];
+                }
+#pragma unroll
+                for (int q = 0; q < 16; q++)
+                    if (q / 8 >= d0 && q / 8 <= d1) sf[q * CELLS + li * WJ + lj] = planes[q / 4][(q % 4) * n + c];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) u[k] = Uin[k * n + c];
+                bad = cell2(g, u, d0, d1, sf + li * WJ + lj, CELLS);
+            }
         }
     }
     __syncthreads();
@@ -574,8 +590,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             for (int k = 0; k < 4; k++) {
                 REAL dp = 0, dm = 0;
                 if (i > 0 && i < nx - 1 && j < ny) {
-                    dp = slope(g, F(0, k, li - 1, ljj), F(0, k, li, ljj), F(0, k, li + 1, ljj));
-                    dm = slope(g, F(1, k, li - 1, ljj), F(1, k, li, ljj), F(1, k, li + 1, ljj));
+                    dp = slope(g, F(0, k, li - 1, ljj), F(0, k, li, ljj), F(0, k, li + 1, ljj), kInvScale);
+                    dm = slope(g, F(1, k, li - 1, ljj), F(1, k, li, ljj), F(1, k, li + 1, ljj), kInvScale);
                 }
                 sd[k * NXS + t] = dp; sd[(4 + k) * NXS + t] = dm;
             }
@@ -588,8 +604,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             for (int k = 0; k < 4; k++) {
                 REAL dp = 0, dm = 0;
                 if (j > 0 && j < ny - 1 && i < nx) {
-                    dp = slope(g, F(2, k, li, lj - 1), F(2, k, li, lj), F(2, k, li, lj + 1));
-                    dm = slope(g, F(3, k, li, lj - 1), F(3, k, li, lj), F(3, k, li, lj + 1));
+                    dp = slope(g, F(2, k, li, lj - 1), F(2, k, li, lj), F(2, k, li, lj + 1), kInvScale);
+                    dm = slope(g, F(3, k, li, lj - 1), F(3, k, li, lj), F(3, k, li, lj + 1), kInvScale);
                 }
                 sd[8 * NXS + k * NYS + t] = dp; sd[8 * NXS + (4 + k) * NYS + t] = dm;
             }
@@ -615,8 +631,8 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = sy * hm; Tt = F(3, k, li, lj + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = sy * hp; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); }
-            v = sub_scaled(v, g.sx, fp - fm + Rr - L);
-            v = sub_scaled(v, g.sy, hp - hm + Tt - B);
+            v = sub_scaled(v, fx, fp - fm + Rr - L);
+            v = sub_scaled(v, fy, hp - hm + Tt - B);
         } else {
             // outflow walls, slopes zero on edge cells (2nd_order_base_shll.c:210-458)
             auto DX_ = [&](int q, int r) -> REAL { return sd[(q * 4 + k) * NXS + r * TJ + tx]; };
@@ -631,10 +647,10 @@ __device__ __forceinline__ void step2_tile(const REAL* __restrict__ Uin, REAL* _
             if (j == 0) { B = hp; Tt = F(3, k, li, lj + 1); Bdf = 0; Tdf = DY_(1, cc + 1); }
             else if (j == ny - 1) { B = F(2, k, li, lj - 1); Tt = hm; Bdf = DY_(0, cc - 1); Tdf = 0; }
             else { B = F(2, k, li, lj - 1); Tt = F(3, k, li, lj + 1); Bdf = DY_(0, cc - 1); Tdf = DY_(1, cc + 1); }
-            v = sub_scaled(v, g.sx, fp - fm + Rr - L);
-            v = sub_half_scaled(v, g.hsx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
-            v = sub_scaled(v, g.sy, hp - hm + Tt - B);
-            v = sub_half_scaled(v, g.hsy, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
+            v = sub_scaled(v, fx, fp - fm + Rr - L);
+            v = sub_half_scaled(v, hfx, DX_(0, r) + DX_(1, r) - Rdf - Ldf);
+            v = sub_scaled(v, fy, hp - hm + Tt - B);
+            v = sub_half_scaled(v, hfy, DY_(0, cc) + DY_(1, cc) - Tdf - Bdf);
         }
         Uout[k * n + c] = v;
     }
@@ -649,6 +665,13 @@ __global__ void __launch_bounds__(kTileThreads) k_step2(const REAL* __restrict__
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     step2_tile<REAL, ORDER>(Uin, Uout, nx, ny, (long)nx * ny, g, flag, blockIdx.y * TI, blockIdx.x * TJ, TI);
+}
+
+static int device_sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    return sms;
 }
 
 // Tile height of a domain.  FP64: the one with the least work on the busiest SM, counting a halo cell
@@ -773,62 +796,43 @@ __global__ void k_f_from_p(const REAL* __restrict__ U, const REAL* __restrict__ 
     }
 }
 
-// Update_U_from_F from stored split-flux planes (in place: each cell reads only its own U).
+// Update_U_from_F from stored split-flux planes (in place: each cell reads only its own U).  2D: the
+// tile kernel's slopes and update (a cell's slopes evaluated once and not for each of the three cells
+// that use them: 512 x 480 cells, FP64, second order, 73.6 -> 59.5 us).
+template <typename REAL, int ORDER>
+__global__ void __launch_bounds__(kTileThreads) k_update2_staged(REAL* U, const REAL* fp, const REAL* fm, const REAL* hp,
+                                                                 const REAL* hm, int nx, int ny,
+                                                                 const __grid_constant__ Gas<REAL> g, int TI) {
+    const REAL* const planes[4] = {fp, fm, hp, hm};
+    step2_tile<REAL, ORDER, true>(U, U, nx, ny, (long)nx * ny, g, nullptr, blockIdx.y * TI, blockIdx.x * TJ, TI, planes);
+}
 template <typename REAL>
-__global__ void k_update_staged(REAL* __restrict__ U, const REAL* __restrict__ fp, const REAL* __restrict__ fm,
-                                const REAL* __restrict__ hp, const REAL* __restrict__ hm, int nx, int ny, int dim,
-                                int order, Gas<REAL> g) {
-    const long n = (long)nx * ny;
-    const int nv = dim == 2 ? 4 : 3, sx_ = ny;  // x stride (1D: ny = 1)
-    for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(c / ny), j = (int)(c % ny);
-        for (int k = 0; k < nv; k++) {
-            const REAL* Fp = fp + k * n; const REAL* Fm = fm + k * n;
-            REAL u = U[k * n + c];
+__global__ void k_update1_staged(REAL* __restrict__ U, const REAL* __restrict__ fp, const REAL* __restrict__ fm, int n,
+                                 int order, const __grid_constant__ Gas<REAL> g) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        for (int k = 0; k < 3; k++) {
+            const REAL* Fp = fp + (long)k * n; const REAL* Fm = fm + (long)k * n;
+            REAL u = U[(long)k * n + i];
             if (order == 1) {
                 const REAL sx = (k == 1) ? (REAL)1 : (REAL)-1;
                 REAL L, Rr;
-                if (i == 0) { L = sx * Fm[c]; Rr = Fm[c + sx_]; }
-                else if (i == nx - 1) { L = Fp[c - sx_]; Rr = sx * Fp[c]; }
-                else { L = Fp[c - sx_]; Rr = Fm[c + sx_]; }
-                u = sub_scaled(u, g.lx, Fp[c] - Fm[c] + Rr - L);
-                if (dim == 2) {
-                    const REAL* Hp = hp + k * n; const REAL* Hm = hm + k * n;
-                    const REAL sy = (k == 2) ? (REAL)1 : (REAL)-1;
-                    REAL B, Tt;
-                    if (j == 0) { B = sy * Hm[c]; Tt = Hm[c + 1]; }
-                    else if (j == ny - 1) { B = Hp[c - 1]; Tt = sy * Hp[c]; }
-                    else { B = Hp[c - 1]; Tt = Hm[c + 1]; }
-                    u = sub_scaled(u, g.ly, Hp[c] - Hm[c] + Tt - B);
-                }
+                if (i == 0) { L = sx * Fm[i]; Rr = Fm[i + 1]; }
+                else if (i == n - 1) { L = Fp[i - 1]; Rr = sx * Fp[i]; }
+                else { L = Fp[i - 1]; Rr = Fm[i + 1]; }
+                u = sub_scaled(u, g.lx, Fp[i] - Fm[i] + Rr - L);
             } else {
-                auto sl = [&](const REAL* f, long cc, int ii, int st, int nn) -> REAL {
-                    if (ii <= 0 || ii >= nn - 1) return (REAL)0;
-                    return slope(g, f[cc - st], f[cc], f[cc + st], (REAL)1);
+                auto sl = [&](const REAL* f, int c) -> REAL {
+                    if (c <= 0 || c >= n - 1) return (REAL)0;
+                    return slope(g, f[c - 1], f[c], f[c + 1], (REAL)1);
                 };
                 REAL L, Rr, Ldf, Rdf;
-                if (i == 0) { L = Fp[c]; Rr = Fm[c + sx_]; Ldf = 0; Rdf = sl(Fm, c + sx_, i + 1, sx_, nx); }
-                else if (i == nx - 1) { L = Fp[c - sx_]; Rr = Fm[c]; Ldf = sl(Fp, c - sx_, i - 1, sx_, nx); Rdf = 0; }
-                else {
-                    L = Fp[c - sx_]; Rr = Fm[c + sx_];
-                    Ldf = sl(Fp, c - sx_, i - 1, sx_, nx); Rdf = sl(Fm, c + sx_, i + 1, sx_, nx);
-                }
-                u = sub_scaled(u, g.lx, Fp[c] - Fm[c] + Rr - L);
-                u = sub_half_scaled(u, g.hlx, sl(Fp, c, i, sx_, nx) + sl(Fm, c, i, sx_, nx) - Rdf - Ldf);
-                if (dim == 2) {
-                    const REAL* Hp = hp + k * n; const REAL* Hm = hm + k * n;
-                    REAL B, Tt, Bdf, Tdf;
-                    if (j == 0) { B = Hp[c]; Tt = Hm[c + 1]; Bdf = 0; Tdf = sl(Hm, c + 1, j + 1, 1, ny); }
-                    else if (j == ny - 1) { B = Hp[c - 1]; Tt = Hm[c]; Bdf = sl(Hp, c - 1, j - 1, 1, ny); Tdf = 0; }
-                    else {
-                        B = Hp[c - 1]; Tt = Hm[c + 1];
-                        Bdf = sl(Hp, c - 1, j - 1, 1, ny); Tdf = sl(Hm, c + 1, j + 1, 1, ny);
-                    }
-                    u = sub_scaled(u, g.ly, Hp[c] - Hm[c] + Tt - B);
-                    u = sub_half_scaled(u, g.hly, sl(Hp, c, j, 1, ny) + sl(Hm, c, j, 1, ny) - Tdf - Bdf);
-                }
+                if (i == 0) { L = Fp[i]; Rr = Fm[i + 1]; Ldf = 0; Rdf = sl(Fm, i + 1); }
+                else if (i == n - 1) { L = Fp[i - 1]; Rr = Fm[i]; Ldf = sl(Fp, i - 1); Rdf = 0; }
+                else { L = Fp[i - 1]; Rr = Fm[i + 1]; Ldf = sl(Fp, i - 1); Rdf = sl(Fm, i + 1); }
+                u = sub_scaled(u, g.lx, Fp[i] - Fm[i] + Rr - L);
+                u = sub_half_scaled(u, g.hlx, sl(Fp, i) + sl(Fm, i) - Rdf - Ldf);
             }
-            U[k * n + c] = u;
+            U[(long)k * n + i] = u;
         }
     }
 }
@@ -847,10 +851,8 @@ static cudaError_t step_t(const PlainArgs& a) {
         if (a.order == 1) k_step1<REAL, 1><<<grid, T1, 0, a.stream>>>(Uin, Uout, a.nx, g, a.flag);
         else k_step1<REAL, 2><<<grid, T1, 0, a.stream>>>(Uin, Uout, a.nx, g, a.flag);
     } else {
-        int dev = 0, sms = 152;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int TI = tile_rows(a.nx, a.ny, a.order, sms, sizeof(REAL) == 8);
+        cudaError_t e = cudaSuccess;
+        const int TI = tile_rows(a.nx, a.ny, a.order, device_sm_count(), sizeof(REAL) == 8);
         auto* kern = a.order == 1 ? k_step2<REAL, 1> : k_step2<REAL, 2>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)((a.ny + TJ - 1) / TJ), (unsigned)((a.nx + TI - 1) / TI));
@@ -887,11 +889,21 @@ static cudaError_t stage_t(const PlainArgs& a, int which) {
                                                              static_cast<REAL*>(a.hp), static_cast<REAL*>(a.hm), n,
                                                              a.dim, g);
             break;
-        case STAGE_UPDATE:
-            k_update_staged<REAL><<<blocks, threads, 0, a.stream>>>(
-                U, static_cast<const REAL*>(a.fp), static_cast<const REAL*>(a.fm), static_cast<const REAL*>(a.hp),
-                static_cast<const REAL*>(a.hm), a.nx, a.dim == 2 ? a.ny : 1, a.dim, a.order, g);
+        case STAGE_UPDATE: {
+            const REAL *fp = static_cast<const REAL*>(a.fp), *fm = static_cast<const REAL*>(a.fm);
+            if (a.dim == 1) {
+                k_update1_staged<REAL><<<blocks, threads, 0, a.stream>>>(U, fp, fm, a.nx, a.order, g);
+                break;
+            }
+            const int TI = tile_rows(a.nx, a.ny, a.order, device_sm_count(), sizeof(REAL) == 8);
+            auto* kern = a.order == 1 ? k_update2_staged<REAL, 1> : k_update2_staged<REAL, 2>;
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2<REAL>(20, a.order));
+            if (e != cudaSuccess) return e;
+            kern<<<dim3((unsigned)((a.ny + TJ - 1) / TJ), (unsigned)((a.nx + TI - 1) / TI)), tile_threads(TI, a.order),
+                   smem2<REAL>(TI, a.order), a.stream>>>(U, fp, fm, static_cast<const REAL*>(a.hp),
+                                                         static_cast<const REAL*>(a.hm), a.nx, a.ny, g, TI);
             break;
+        }
         case STAGE_LOAD:
             k_check_planes<REAL><<<blocks, threads, 0, a.stream>>>(a.planes, n, a.dim == 2 ? 4 : 3, a.worst);
             k_load_planes<REAL><<<blocks, threads, 0, a.stream>>>(a.planes, P, U, n, a.dim, g, a.worst, a.flag);
