@@ -72,7 +72,15 @@ struct Chunk {
     int a, b;        // owned cells [a, b)
     int anc;         // anchor cell of the chunk's frame
     int id, idL, idR;  // this chunk's and its neighbours' ids (-1 if none), index of bsum
+    // Resident runs may give a chunk to several blocks (parts): this block's cells [sa, sb) of [a, b).
+    // Then id is the part's, idL / idR are the adjacent part of the neighbouring chunk when this part is
+    // the first / last of its chunk (else -1: the cells beyond are a sibling's, in the same frame), and
+    // [w0, w1] are the ids whose previous sweep this part waits for.
+    int sa, sb, w0, w1;
 };
+inline Chunk whole_chunk(int tube, int a, int b, int anc, int id, int idL, int idR) {
+    return {tube, a, b, anc, id, idL, idR, a, b, idL >= 0 ? idL : id, idR >= 0 ? idR : id};
+}
 
 struct Frame1 {
     double U[3];      // anchor state
@@ -182,6 +190,13 @@ __device__ __forceinline__ bool pair_mode(const SweepArgs& A, const Chunk& ch, i
     return v != 0;
 }
 
+// the same for a part of a resident run: any part of the chunk and its neighbours (those it waits for)
+__device__ __forceinline__ bool pair_mode_parts(const SweepArgs& A, const Chunk& ch, int sweep) {
+    const int* f = ((sweep - 1) & 1) ? A.mode[1] : A.mode[0];
+    const int q = ch.w0 + (int)threadIdx.x;
+    return __syncthreads_or(q <= ch.w1 && __ldcg(f + q) != 0) != 0;
+}
+
 // correction owed to the first owned cell of the chunk with id `right` by its left neighbour
 // `left` for the sweep whose sums are in bs: lam*sum(F_left) - lam*sum(F_right) at their interface
 __device__ __forceinline__ double boundary_correction(const BSum* bs, int left, int right, int k) {
@@ -236,8 +251,8 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     const int steps = min(tp.B, tp.steps - sweep * tp.B);
     if (steps <= 0) return;
     const int H = R_ * steps;
-    const int ws = max(0, ch.a - H), we = min(n, ch.b + H), L = we - ws;
-    const int pa = ch.a - ws, pb = ch.b - ws;  // first owned / one past the last owned, window coords
+    const int ws = max(0, ch.sa - H), we = min(n, ch.sb + H), L = we - ws;
+    const int pa = ch.sa - ws, pb = ch.sb - ws;  // first owned / one past the last owned, window coords
     const int inb = (tp.par + sweep) & 1, outb = inb ^ 1;
     // position in the fold window: the first sweep reads the stored state and sets the frame,
     // the last one writes the state back; the sweeps between exchange deviation pairs
@@ -275,7 +290,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     const double lam = tp.lam;
     const float lamh = (float)lam, laml = (float)(lam - (double)lamh);
 
-    if (L > MW || tp.B > MW / 16 || tp.B < 1) {  // host guarantees this never happens; refuse rather than overrun
+    if (L > 2 * (int)blockDim.x || tp.B > MW / 16 || tp.B < 1) {  // host guarantees this never happens; refuse rather than overrun
         if (tid == 0) atomicOr(A.flag, SHLL_FLAG_BADARG);
         return;
     }
@@ -349,7 +364,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                     U[k] = ldx<RES>(static_cast<const double*>(hin) + idx);
                 }
             }
-            make_frame(fr, U, tp, ORDER == 1 && (ch.idL < 0 || ch.idR < 0));
+            make_frame(fr, U, tp, ORDER == 1 && (ch.a == 0 || ch.b == n));
             if (KAHAN)  // the stored pair itself, so that the anchor cell's deviation is exactly 0
                 for (int k = 0; k < 3; k++) { fr.Uh[k] = Uanc_h[k]; fr.Ul[k] = Uanc_l[k]; }
         }
@@ -381,7 +396,8 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                 if (!wstart) {
                     // deviation pair relative to the owner's frame -> relative to this frame
                     h = uh[q][k]; l = ul[q][k];
-                    if (w < pa || w >= pb) {
+                    // (a sibling part's cells are in the same frame)
+                    if ((w < pa && ch.idL >= 0) || (w >= pb && ch.idR >= 0)) {
                         const int sd = w < pa ? 0 : 1;
                         ff_add(h, l, S.dnb[sd][k][0], S.dnb[sd][k][1], h, l);
                     }
@@ -441,7 +457,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     const bool rin0 = hasL && w0 == pa, rin1 = hasL && w0 + 1 == pa;
     const bool rout0 = hasR && w0 == pb - 1, rout1 = hasR && w0 + 1 == pb - 1;
     const bool any_rec = rin0 || rin1 || rout0 || rout1;
-    const int jl = max(w0 - 2, 0), jr = min(w0 + 2, MW - 2);  // neighbour pairs (clamped)
+    const int jl = max(w0 - 2, 0), jr = min(w0 + 2, 2 * (int)blockDim.x - 2);  // neighbour pairs (clamped)
 
     if constexpr (FF) {
         // The same step in double-FP32 arithmetic: each cell's state U = U* + (dh + dl) as a pair,
@@ -830,7 +846,6 @@ __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, bool CLU>
 __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
     __shared__ Smem1 S;
-    __shared__ int s_ok;
     const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
     const TubeP tp = A.tubes[ch.tube];
     const int nsw = (tp.steps + tp.B - 1) / tp.B;
@@ -841,28 +856,22 @@ __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
             // every block of the cluster (every chunk of the tube) has completed the previous sweep
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         } else if (sw > 0) {
-            if (threadIdx.x == 0) {
-                // both counters polled at once (a chunk without a neighbour on one side reads its
-                // own counter there, which is ahead)
-                const unsigned* pl = prog + (long)(ch.idL >= 0 ? ch.idL : ch.id) * kProgStride;
-                const unsigned* pr = prog + (long)(ch.idR >= 0 ? ch.idR : ch.id) * kProgStride;
-                bool ok = false;
-                for (long it = 0; it < kSpinLimit && !ok; it++) {
-                    const unsigned vl = ld_acquire_gpu(pl), vr = ld_acquire_gpu(pr);
-                    ok = vl >= (unsigned)sw && vr >= (unsigned)sw;
-                    if (!ok) {
-                        // another block gave up: so does this one (now rather than after its own
-                        // limit; every 64th poll, as all blocks read this word)
-                        if ((it & 63) == 63 && (ld_acquire_gpu(reinterpret_cast<const unsigned*>(A.flag)) & SHLL_FLAG_TIMEOUT))
-                            break;
-                        __nanosleep(32);
-                    }
+            // one thread per counter of the parts this one waits for: the neighbouring chunks' and, as
+            // they share an anchor, its siblings
+            const int q = ch.w0 + (int)threadIdx.x;
+            bool ok = q > ch.w1 || q == ch.id;
+            for (long it = 0; it < kSpinLimit && !ok; it++) {
+                ok = ld_acquire_gpu(prog + (long)q * kProgStride) >= (unsigned)sw;
+                if (!ok) {
+                    // another block gave up: so does this one (now rather than after its own
+                    // limit; every 64th poll, as all blocks read this word)
+                    if ((it & 63) == 63 && (ld_acquire_gpu(reinterpret_cast<const unsigned*>(A.flag)) & SHLL_FLAG_TIMEOUT))
+                        break;
+                    __nanosleep(32);
                 }
-                if (!ok) atomicOr(A.flag, SHLL_FLAG_TIMEOUT);
-                s_ok = ok;
             }
-            __syncthreads();
-            if (!s_ok) return;
+            if (!ok) atomicOr(A.flag, SHLL_FLAG_TIMEOUT);
+            if (!__syncthreads_and(ok)) return;
         }
         // sweeps of B steps inside a fold window share the geometry of the one before
         const bool reuse = sw % F != 0 && tp.steps - sw * tp.B >= tp.B;
@@ -871,7 +880,7 @@ __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
         // they were written before the neighbours' release; block-uniform)
         if constexpr (FM == 2)
             sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, true>(A, sw, ch, tp, S, dh, dl, reuse, keep);
-        else if (FM == 1 && A.mode[0] && pair_mode(A, ch, sw))
+        else if (FM == 1 && A.mode[0] && pair_mode_parts(A, ch, sw))
             sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, FM == 1>(A, sw, ch, tp, S, dh, dl, reuse, keep);
         else
             sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true>(A, sw, ch, tp, S, dh, dl, reuse, keep);
@@ -1029,7 +1038,7 @@ static_assert(kPairSmem <= kSoloSmem, "the pair-flux buffers fit in the padding 
 // resident form of a run (k_tube1d): a cooperative launch of one block per chunk, each alone on
 // its SM (the same shared-memory padding as single-wave sweeps)
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM>
-static cudaError_t launch_res(int grid, cudaStream_t s, const SweepArgs& A, unsigned* prog, bool check_only) {
+static cudaError_t launch_res(int grid, int threads, cudaStream_t s, const SweepArgs& A, unsigned* prog, bool check_only) {
     static unsigned long long attr_set = 0;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1042,13 +1051,13 @@ static cudaError_t launch_res(int grid, cudaStream_t s, const SweepArgs& A, unsi
     if (check_only) {  // every block must be resident at once
         int per_sm = 0;
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM>,
-                                                                      MT, kSoloSmem);
+                                                                      threads, kSoloSmem);
         if (e != cudaSuccess) return e;
         return (long)per_sm * device_sms() >= grid ? cudaSuccess : cudaErrorCooperativeLaunchTooLarge;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(MT);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = kSoloSmem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -1113,34 +1122,34 @@ static cudaError_t launch_cluster(int variant, bool kahan, int grid, int csize, 
 
 // all_pairs: the pair flux everywhere (second order then needs the pair-flux kernel; first order
 // chooses per chunk and sweep either way)
-static cudaError_t launch_resident(int variant, bool kahan, int grid, cudaStream_t s, const SweepArgs& A,
+static cudaError_t launch_resident(int variant, bool kahan, int grid, int threads, cudaStream_t s, const SweepArgs& A,
                                    unsigned* prog, bool check_only, bool all_pairs) {
     const int v = variant * 2 + (kahan ? 1 : 0);
     if (variant >= 2 && all_pairs) {
         switch (v) {
-            case 4: return launch_res<2, false, true, 0, 2>(grid, s, A, prog, check_only);
-            case 5: return launch_res<2, true, true, 0, 2>(grid, s, A, prog, check_only);
-            case 6: return launch_res<2, false, false, 0, 2>(grid, s, A, prog, check_only);
-            case 7: return launch_res<2, true, false, 0, 2>(grid, s, A, prog, check_only);
-            case 8: return launch_res<2, false, true, 1, 2>(grid, s, A, prog, check_only);
-            case 9: return launch_res<2, true, true, 1, 2>(grid, s, A, prog, check_only);
-            case 10: return launch_res<2, false, false, 1, 2>(grid, s, A, prog, check_only);
-            default: return launch_res<2, true, false, 1, 2>(grid, s, A, prog, check_only);
+            case 4: return launch_res<2, false, true, 0, 2>(grid, threads, s, A, prog, check_only);
+            case 5: return launch_res<2, true, true, 0, 2>(grid, threads, s, A, prog, check_only);
+            case 6: return launch_res<2, false, false, 0, 2>(grid, threads, s, A, prog, check_only);
+            case 7: return launch_res<2, true, false, 0, 2>(grid, threads, s, A, prog, check_only);
+            case 8: return launch_res<2, false, true, 1, 2>(grid, threads, s, A, prog, check_only);
+            case 9: return launch_res<2, true, true, 1, 2>(grid, threads, s, A, prog, check_only);
+            case 10: return launch_res<2, false, false, 1, 2>(grid, threads, s, A, prog, check_only);
+            default: return launch_res<2, true, false, 1, 2>(grid, threads, s, A, prog, check_only);
         }
     }
     switch (v) {
-        case 0: return launch_res<1, false, true, 0, 1>(grid, s, A, prog, check_only);
-        case 1: return launch_res<1, true, true, 0, 1>(grid, s, A, prog, check_only);
-        case 2: return launch_res<1, false, false, 0, 1>(grid, s, A, prog, check_only);
-        case 3: return launch_res<1, true, false, 0, 1>(grid, s, A, prog, check_only);
-        case 4: return launch_res<2, false, true, 0, 0>(grid, s, A, prog, check_only);
-        case 5: return launch_res<2, true, true, 0, 0>(grid, s, A, prog, check_only);
-        case 6: return launch_res<2, false, false, 0, 0>(grid, s, A, prog, check_only);
-        case 7: return launch_res<2, true, false, 0, 0>(grid, s, A, prog, check_only);
-        case 8: return launch_res<2, false, true, 1, 0>(grid, s, A, prog, check_only);
-        case 9: return launch_res<2, true, true, 1, 0>(grid, s, A, prog, check_only);
-        case 10: return launch_res<2, false, false, 1, 0>(grid, s, A, prog, check_only);
-        default: return launch_res<2, true, false, 1, 0>(grid, s, A, prog, check_only);
+        case 0: return launch_res<1, false, true, 0, 1>(grid, threads, s, A, prog, check_only);
+        case 1: return launch_res<1, true, true, 0, 1>(grid, threads, s, A, prog, check_only);
+        case 2: return launch_res<1, false, false, 0, 1>(grid, threads, s, A, prog, check_only);
+        case 3: return launch_res<1, true, false, 0, 1>(grid, threads, s, A, prog, check_only);
+        case 4: return launch_res<2, false, true, 0, 0>(grid, threads, s, A, prog, check_only);
+        case 5: return launch_res<2, true, true, 0, 0>(grid, threads, s, A, prog, check_only);
+        case 6: return launch_res<2, false, false, 0, 0>(grid, threads, s, A, prog, check_only);
+        case 7: return launch_res<2, true, false, 0, 0>(grid, threads, s, A, prog, check_only);
+        case 8: return launch_res<2, false, true, 1, 0>(grid, threads, s, A, prog, check_only);
+        case 9: return launch_res<2, true, true, 1, 0>(grid, threads, s, A, prog, check_only);
+        case 10: return launch_res<2, false, false, 1, 0>(grid, threads, s, A, prog, check_only);
+        default: return launch_res<2, true, false, 1, 0>(grid, threads, s, A, prog, check_only);
     }
 }
 
@@ -1277,10 +1286,13 @@ static void build_chunks(MixedState* m) {
         for (int c = 0; c < k; c++) anc[c] = c == 0 ? 0 : (c == k - 1 ? n - 1 : (edges[c] + edges[c + 1]) / 2);
         const int id0 = (int)m->chunks.size();
         for (int c = 0; c < k; c++)
-            m->chunks.push_back({t, edges[c], edges[c + 1], anc[c], id0 + c, c > 0 ? id0 + c - 1 : -1,
-                                 c + 1 < k ? id0 + c + 1 : -1});
+            m->chunks.push_back(whole_chunk(t, edges[c], edges[c + 1], anc[c], id0 + c, c > 0 ? id0 + c - 1 : -1,
+                                            c + 1 < k ? id0 + c + 1 : -1));
     }
 }
+
+// entries of the per-chunk tables: the chunks, or the parts of a resident run (at most one per SM)
+static size_t chunk_slots(const MixedState* m) { return std::max(m->chunks.size(), (size_t)device_sms()); }
 
 // fold windows of several sweeps need every halo cell to come from the adjacent chunk
 static void fix_fold_sweeps(MixedState* m) {
@@ -1296,8 +1308,8 @@ static cudaError_t alloc_mode_flags(MixedState* m) {
     m->has_first = false;
     for (const TubeP& tp : m->tubes) m->has_first = m->has_first || tp.order == 1;
     for (int b = 0; b < 2; b++) {
-        cudaError_t e = cudaMalloc(&m->mode[b], sizeof(int) * m->chunks.size());
-        if (e == cudaSuccess) e = cudaMemset(m->mode[b], 0, sizeof(int) * m->chunks.size());
+        cudaError_t e = cudaMalloc(&m->mode[b], sizeof(int) * chunk_slots(m));
+        if (e == cudaSuccess) e = cudaMemset(m->mode[b], 0, sizeof(int) * chunk_slots(m));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1316,8 +1328,8 @@ static int alloc_mixed(MixedState* m, char* err, size_t len) {
         }
     }
     for (int b = 0; b < 2; b++) {
-        if (cudaMalloc(&m->bsum[b], sizeof(BSum) * m->chunks.size()) != cudaSuccess ||
-            cudaMemset(m->bsum[b], 0, sizeof(BSum) * m->chunks.size()) != cudaSuccess) {
+        if (cudaMalloc(&m->bsum[b], sizeof(BSum) * chunk_slots(m)) != cudaSuccess ||
+            cudaMemset(m->bsum[b], 0, sizeof(BSum) * chunk_slots(m)) != cudaSuccess) {
             snprintf(err, len, "cudaMalloc of boundary sums failed");
             return SHLL_ERR_NOMEM;
         }
@@ -1331,7 +1343,7 @@ static int alloc_mixed(MixedState* m, char* err, size_t len) {
                 snprintf(err, len, "cudaMalloc of deviation planes failed");
                 return SHLL_ERR_NOMEM;
             }
-        if (cudaMalloc(&m->frames, sizeof(Frame1) * m->chunks.size()) != cudaSuccess) {
+        if (cudaMalloc(&m->frames, sizeof(Frame1) * chunk_slots(m)) != cudaSuccess) {
             snprintf(err, len, "cudaMalloc of the frame table failed");
             return SHLL_ERR_NOMEM;
         }
@@ -1454,7 +1466,7 @@ MixedState* mixed_create_batch(const shll_params* items, int count, cudaStream_t
     build_chunks(m);
     fix_fold_sweeps(m);
     int rc = alloc_mixed(m, err, len);
-    if (rc == SHLL_OK && cudaMalloc(&m->d_chunks, sizeof(Chunk) * m->chunks.size()) != cudaSuccess) rc = SHLL_ERR_NOMEM;
+    if (rc == SHLL_OK && cudaMalloc(&m->d_chunks, sizeof(Chunk) * chunk_slots(m)) != cudaSuccess) rc = SHLL_ERR_NOMEM;
     if (rc != SHLL_OK) {
         mixed_destroy(m);
         return nullptr;
@@ -1788,6 +1800,16 @@ int shll_stall_chunk() { return g_stall.load(); }
 static std::atomic<int> g_pair_flux{1};
 extern "C" void shll_set_pair_flux(int on) { g_pair_flux = on == 2 ? 2 : (on ? 1 : 0); }
 
+// threads of a resident block: two cells each over the widest window
+static int resident_threads(MixedState* m, const std::vector<Chunk>& order) {
+    int cells = 0;
+    for (const Chunk& c : order) {
+        const TubeP& tp = m->tubes[c.tube];
+        cells = std::max(cells, c.sb - c.sa + 2 * tp.order * tp.B);
+    }
+    return std::min(MT, std::max(64, (cells / 2 + 1 + 31) / 32 * 32));
+}
+
 // issues the launches of one run on m->stream: the sweeps of every variant group (or, resident,
 // one launch for all sweeps of the run's single variant group), then the fix-up
 // cluster > 0: the cluster form of a resident run, clusters of that many chunks (one tube each)
@@ -1840,7 +1862,8 @@ static cudaError_t issue_run(MixedState* m, const std::vector<Chunk>& order, lon
         A.chunk0 = 0;
         cudaError_t e = cudaMemsetAsync(m->prog, 0, sizeof(unsigned) * kProgStride * order.size(), m->stream);
         if (e == cudaSuccess)
-            e = launch_resident(groups[0].variant, m->kahan, (int)order.size(), m->stream, A, m->prog, false,
+            e = launch_resident(groups[0].variant, m->kahan, (int)order.size(), resident_threads(m, order), m->stream, A,
+                                m->prog, false,
                                 pairs && pf == 2);
         if (e != cudaSuccess) return e;
         n = 1;
@@ -1912,29 +1935,66 @@ static int cluster_run(MixedState* m, const std::vector<Chunk>& order) {
     return k;
 }
 
-static bool resident_run(MixedState* m, const std::vector<Chunk>& order) {
+// Parts: with few chunks, each is given to several blocks on SMs of their own, which compute windows of
+// part of its cells in the chunk's frame: the same bits at a shorter step.  A block of 8 warps takes about
+// 1200 clocks a step (its 512 cells' packed FP32 instructions, two warps to a scheduler, and the barrier),
+// a window of up to 128 cells in 2 warps little more than the step's dependent chain.  As many parts as
+// bring the window down to 128 cells, as the SMs hold, and as leave every part the halo width.
+static int resident_parts(MixedState* m, const std::vector<Chunk>& order) {
+    int parts = device_sms() / (int)order.size();
+    int want = 1;
+    for (const Chunk& c : order) {
+        const TubeP& tp = m->tubes[c.tube];
+        const int H = tp.order * tp.B, owned = c.b - c.a, to = std::max(H, 128 - 2 * H);
+        parts = std::min(parts, owned / H);
+        want = std::max(want, (owned + to - 1) / to);
+    }
+    return std::max(1, std::min(parts, want));
+}
+// the parts of every chunk, in id order (part q of chunk c has id c * parts + q)
+static std::vector<Chunk> split_chunks(const std::vector<Chunk>& order, int parts) {
+    std::vector<Chunk> out;
+    for (const Chunk& c : order)
+        for (int q = 0; q < parts; q++) {
+            Chunk s = c;
+            s.id = c.id * parts + q;
+            s.idL = q == 0 && c.idL >= 0 ? c.idL * parts + parts - 1 : -1;
+            s.idR = q == parts - 1 && c.idR >= 0 ? c.idR * parts : -1;
+            s.sa = c.a + (int)((long)(c.b - c.a) * q / parts);
+            s.sb = c.a + (int)((long)(c.b - c.a) * (q + 1) / parts);
+            s.w0 = (c.idL >= 0 ? c.idL : c.id) * parts;
+            s.w1 = (c.idR >= 0 ? c.idR : c.id) * parts + parts - 1;
+            out.push_back(s);
+        }
+    return out;
+}
+// (order: on return the run's blocks, whole chunks or parts)
+static bool resident_run(MixedState* m, std::vector<Chunk>& order) {
     if (!g_resident.load() || order.empty() || (long)order.size() > device_sms()) return false;
     const int v = tube_variant(m->tubes[order[0].tube]);
     for (const Chunk& c : order) {
         const TubeP& tp = m->tubes[c.tube];
         if (tube_variant(tp) != v || c.b - c.a < tp.order * tp.B) return false;
     }
-    if (m->prog_n < order.size()) {
+    const int parts = resident_parts(m, order);
+    std::vector<Chunk> blocks = parts > 1 ? split_chunks(order, parts) : order;
+    if (m->prog_n < blocks.size()) {
         cudaFree(m->prog);
         m->prog = nullptr;
         m->prog_n = 0;
-        if (cudaMalloc(&m->prog, sizeof(unsigned) * kProgStride * order.size()) != cudaSuccess) {
+        if (cudaMalloc(&m->prog, sizeof(unsigned) * kProgStride * chunk_slots(m)) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
-        m->prog_n = order.size();
+        m->prog_n = chunk_slots(m);
     }
     SweepArgs none{};
-    if (launch_resident(v, m->kahan, (int)order.size(), m->stream, none, m->prog, true, g_pair_flux.load() == 2) !=
-        cudaSuccess) {
+    if (launch_resident(v, m->kahan, (int)blocks.size(), resident_threads(m, blocks), m->stream, none, m->prog, true,
+                        g_pair_flux.load() == 2) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
+    order = std::move(blocks);
     return true;
 }
 
@@ -1959,6 +2019,8 @@ static int run_tubes(MixedState* m, const std::vector<long>& steps, char* err, s
         if (vx != vy) return vx < vy;
         return sweeps_of(m->tubes[x.tube]) > sweeps_of(m->tubes[y.tube]);
     });
+    const int cluster = cluster_run(m, order);
+    const bool resident = !cluster && resident_run(m, order);
     if (cudaMemcpyAsync(m->d_tubes, m->tubes.data(), sizeof(TubeP) * m->nitems, cudaMemcpyHostToDevice, m->stream) != cudaSuccess ||
         cudaMemcpyAsync(m->d_chunks, order.data(), sizeof(Chunk) * order.size(), cudaMemcpyHostToDevice, m->stream) != cudaSuccess) {
         snprintf(err, len, "descriptor upload failed");
@@ -1970,8 +2032,6 @@ static int run_tubes(MixedState* m, const std::vector<long>& steps, char* err, s
     cudaError_t e = allow_solo_padding();
     if (e != cudaSuccess) { snprintf(err, len, "kernel attribute: %s", cudaGetErrorString(e)); return SHLL_ERR_CUDA; }
     MixedState::GraphEntry* hit = nullptr;
-    const int cluster = cluster_run(m, order);
-    const bool resident = !cluster && resident_run(m, order);
     // (a resident or cluster run is one launch: nothing to gain from a graph)
     const bool replay = g_graph_replay.load() != 0 && !m->tuning && !resident && !cluster;
     if (replay)
@@ -2029,7 +2089,7 @@ static int rebuild_chunks(MixedState* m, char* err, size_t len) {
     for (auto& g : m->graphs) cudaGraphExecDestroy(g.exec);
     m->graphs.clear();
     m->seen.clear();
-    const size_t nch = m->chunks.size();
+    const size_t nch = chunk_slots(m);
     cudaFree(m->d_chunks); m->d_chunks = nullptr;
     cudaFree(m->frames); m->frames = nullptr;
     for (int b = 0; b < 2; b++) { cudaFree(m->bsum[b]); m->bsum[b] = nullptr; }
@@ -2438,7 +2498,7 @@ extern "C" int shll_tube_run_static(const shll_params* p, double* d_cons, long n
     for (int c = 0; c < k; c++) {
         const int a = (int)((long)n * c / k), b = (int)((long)n * (c + 1) / k);
         const int anc = c == 0 ? 0 : (c == k - 1 ? n - 1 : (a + b) / 2);
-        chunks[c] = {0, a, b, anc, c, c > 0 ? c - 1 : -1, c + 1 < k ? c + 1 : -1};
+        chunks[c] = whole_chunk(0, a, b, anc, c, c > 0 ? c - 1 : -1, c + 1 < k ? c + 1 : -1);
     }
     TubeP* d_tube = reinterpret_cast<TubeP*>(sc + kStaticTubeOff);
     Chunk* d_chunks = reinterpret_cast<Chunk*>(sc + kStaticChunkOff);
