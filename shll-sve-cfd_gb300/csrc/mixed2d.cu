@@ -71,7 +71,13 @@ struct __align__(16) Dom2 {
 };
 static_assert(offsetof(Dom2, lxh) == 32 && offsetof(Dom2, tiles_i) == 48, "step fields in 16-byte groups");
 
-struct __align__(16) TileD { int dom, ti, tj; };
+// (with the geometry of its domain, so that a step's loads need no second descriptor first; the tile's
+// index in the tables is its place in the list)
+struct __align__(16) TileD {
+    int dom, ti, tj, base;
+    int nx, ny, ex_base, ey_base;
+};
+static_assert(sizeof(TileD) == 32, "two vector loads");
 
 // one edge interface: the full flux lam*F applied by the west/south tile (side 0) and by the
 // east/north tile (side 1), four components each, as FP32 pairs (value, remainder)
@@ -650,37 +656,57 @@ struct Smem22 {
 };
 static_assert(sizeof(TileC2) == offsetof(Smem22, rowc), "the tile constants are copied word for word");
 
-// one component of the correction owed to cell (i, j) (edge_correction), as an FP32 pair
-__device__ __forceinline__ float2 edge_correction1(const Args2& A, const Dom2& D, int i, int j, int pp, int k) {
-    float ch = 0.f, cl = 0.f;
-    auto add = [&](const Edge* e) {
-        const float2 w = *reinterpret_cast<const float2*>(&e->r[0][k][0]), o = *reinterpret_cast<const float2*>(&e->r[1][k][0]);
-        two_sum_acc(ch, cl, w.x);
-        two_sum_acc(ch, cl, -o.x);
-        cl = __fadd_rn(cl, __fadd_rn(w.y, -o.y));
-    };
-    if (i > 0 && i % TI == 0) add(&A.ex[pp][D.ex_base + (i / TI - 1) * D.ny + j]);
-    if (j > 0 && j % TJ == 0) add(&A.ey[pp][D.ey_base + (j / TJ - 1) * D.nx + i]);
-    return make_float2(ch, cl);
-}
-
-// The corrections of the window's cells on tile edge lines (those rows and columns of the window, which
-// starts at row i0 - 2 and column j0 - 2), one thread per cell and component: a pair of cells that
-// gathered them for itself made every warp run that code for the few lanes on a line.
+// The corrections (edge_correction) of the window's cells on tile edge lines (those rows and columns of the
+// window, which starts at row i0 - 2 and column j0 - 2), one thread per cell and component: a pair of cells
+// that gathered them for itself made every warp run that code for the few lanes on a line.  The 448
+// tasks are one or two per thread, all their loads in flight at once.
 template <class SM>
-__device__ __forceinline__ void load_corrections(const Args2& A, const Dom2& D, int i0, int j0, int pp, SM& S) {
+__device__ __forceinline__ void load_corrections(const Args2& A, const TileD& G, int i0, int j0, int pp, SM& S) {
     constexpr int NR = 2 * (TJ + 4) * 4, NC = 2 * WR2 * 4;
-    for (int t = threadIdx.x; t < NR + NC; t += NT2) {
-        const int k = t & 3;
+    static_assert(NR + NC <= 2 * NT2, "at most two tasks per thread");
+    const int k = threadIdx.x & 3;
+    float2 w[2][2], o[2][2];     // [task][x edge, y edge]: the west/south and the own tile's flux
+    float2* dst[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int t = threadIdx.x + q * NT2;
+        int i, j;
         if (t < NR) {
             const int c = (t >> 2) % (TJ + 4), line = (t >> 2) / (TJ + 4);
-            const int i = i0 + line * TI, j = j0 - 2 + c;
-            if (i > 0 && i < D.nx && j >= 0 && j < D.ny) S.rowc[line][c][k] = edge_correction1(A, D, i, j, pp, k);
+            i = i0 + line * TI;
+            j = j0 - 2 + c;
+            dst[q] = &S.rowc[line][c][k];
         } else {
-            const int q = (t - NR) >> 2, r = q % WR2, line = q / WR2;
-            const int i = i0 - 2 + r, j = j0 + line * TJ;
-            if (j > 0 && j < D.ny && i >= 0 && i < D.nx) S.colc[line][r][k] = edge_correction1(A, D, i, j, pp, k);
+            const int r = ((t - NR) >> 2) % WR2, line = ((t - NR) >> 2) / WR2;
+            i = i0 - 2 + r;
+            j = j0 + line * TJ;
+            dst[q] = &S.colc[line][r][k];
         }
+        if (t >= NR + NC || i < 0 || i >= G.nx || j < 0 || j >= G.ny) dst[q] = nullptr;
+#pragma unroll
+        for (int e = 0; e < 2; e++) w[q][e] = o[q][e] = f2(0.f);
+        if (dst[q] && i > 0 && i % TI == 0) {
+            const Edge* e = &A.ex[pp][G.ex_base + (i / TI - 1) * G.ny + j];
+            w[q][0] = *reinterpret_cast<const float2*>(&e->r[0][k][0]);
+            o[q][0] = *reinterpret_cast<const float2*>(&e->r[1][k][0]);
+        }
+        if (dst[q] && j > 0 && j % TJ == 0) {
+            const Edge* e = &A.ey[pp][G.ey_base + (j / TJ - 1) * G.nx + i];
+            w[q][1] = *reinterpret_cast<const float2*>(&e->r[0][k][0]);
+            o[q][1] = *reinterpret_cast<const float2*>(&e->r[1][k][0]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        if (!dst[q]) continue;
+        float ch = 0.f, cl = 0.f;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {   // (the edge that is none adds zeros)
+            two_sum_acc(ch, cl, w[q][e].x);
+            two_sum_acc(ch, cl, -o[q][e].x);
+            cl = __fadd_rn(cl, __fadd_rn(w[q][e].y, -o[q][e].y));
+        }
+        *dst[q] = make_float2(ch, cl);
     }
 }
 // adds them to the increment pairs of the pair at window row wr, pair column wc (cells (i, jx), (i, jx + 1))
@@ -715,7 +741,7 @@ struct EdgeTask {
     bool valid;
     int xa, xb, dir, k;
     float* out;       // the record's pair of this tile's side
-    __device__ __forceinline__ EdgeTask(const Dom2& D, int i0, int j0, int hi_i, int hi_j, Edge* exo, Edge* eyo) {
+    __device__ __forceinline__ EdgeTask(const TileD& G, int i0, int j0, int hi_i, int hi_j, Edge* exo, Edge* eyo) {
         const int t = threadIdx.x;
         k = t & 3;
         auto at = [](int q, int r, int c) { return (q * WR2 + r) * 2 * WP + c; };
@@ -723,18 +749,18 @@ struct EdgeTask {
             const int col = (t >> 2) % TJ, east = (t >> 2) / TJ, c = 2 + col;
             const int i = east ? i0 + hi_i : i0;      // the cell east of the interface
             dir = 0;
-            valid = col < hi_j && (east ? i < D.nx : i > 0);
+            valid = col < hi_j && (east ? i < G.nx : i > 0);
             xa = at(k, i - i0 + 1, c);                // fp of the western cell
             xb = at(4 + k, i - i0 + 2, c);            // fm of the eastern cell
-            out = valid ? exo[D.ex_base + (i / TI - 1) * D.ny + j0 + col].r[east ? 0 : 1][k] : nullptr;
+            out = valid ? exo[G.ex_base + (i / TI - 1) * G.ny + j0 + col].r[east ? 0 : 1][k] : nullptr;
         } else {
             const int q = (t - 2 * TJ * 4) >> 2, row = q % TI, north = q / TI;
             const int j = north ? j0 + hi_j : j0;
             dir = 1;
-            valid = row < hi_i && (north ? j < D.ny : j > 0);
+            valid = row < hi_i && (north ? j < G.ny : j > 0);
             xa = at(8 + k, row + 2, j - j0 + 1);
             xb = at(12 + k, row + 2, j - j0 + 2);
-            out = valid ? eyo[D.ey_base + (j / TJ - 1) * D.nx + i0 + row].r[north ? 0 : 1][k] : nullptr;
+            out = valid ? eyo[G.ey_base + (j / TJ - 1) * G.nx + i0 + row].r[north ? 0 : 1][k] : nullptr;
         }
     }
     // the term applied at the interface, lam (x_a + x_b), as an FP32 pair
@@ -757,11 +783,11 @@ static_assert(2 * TJ * 4 + 2 * TI * 4 == NT2, "one edge task per thread");
 // INNER: the whole window lies inside the domain (no walls, no cut tile): no bounds, masks or selects;
 // the values that the outermost window cells take after the first step are read by no own cell.
 template <bool KAHAN, bool LAM_POW2, bool VEC, bool INNER>
-__device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, const int i0, const int j0, const int ns,
+__device__ __forceinline__ void step2d2_tile(const Args2& A, const TileD& G, const int i0, const int j0,
                                              Smem22& S, float2* g_flux2) {
     const int tid = threadIdx.x;
     const int kw = A.step - A.s0;                         // step within the fold window
-    const int hi_i = INNER ? TI : min(TI, D.nx - i0), hi_j = INNER ? TJ : min(TJ, D.ny - j0);
+    const int hi_i = INNER ? TI : min(TI, G.nx - i0), hi_j = INNER ? TJ : min(TJ, G.ny - j0);
     const int P = A.plane;
     const float* phi = A.Ph[kw % 3];                      // increments so far (kw = 0: none)
     const float* pli = A.Pl[kw % 3];
@@ -774,7 +800,7 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
     const int i = i0 - 2 + wr, jx = j0 - 2 + 2 * wc;
     bool ex[2];
 #pragma unroll
-    for (int q = 0; q < 2; q++) ex[q] = INNER || (pt && i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny);
+    for (int q = 0; q < 2; q++) ex[q] = INNER || (pt && i >= 0 && i < G.nx && jx + q >= 0 && jx + q < G.ny);
     // owner tile of the pair relative to this one (rows i0-2, i0-1 west, i0+16.. east; pair 0 south,
     // pair 17 north); -1: this tile
     const int di = wr < 2 ? -1 : (wr >= 2 + TI ? 1 : 0), dj = wc == 0 ? -1 : (wc == WP - 1 ? 1 : 0);
@@ -791,7 +817,7 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
     float2 base[4], ah[4], al[4];   // deviation of the pair at the launch's start, its increments
 #pragma unroll
     for (int k = 0; k < 4; k++) { base[k] = f2(0.f); ah[k] = f2(0.f); al[k] = f2(0.f); }
-    const int cell = D.base + i * D.ny + jx;
+    const int cell = G.base + i * G.ny + jx;
     if (VEC) {   // (an even row length: the pair is inside or outside together)
         if (ex[0]) {
 #pragma unroll
@@ -817,7 +843,10 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
             }
         }
     }
-    if (kw > 0) load_corrections(A, D, i0, j0, pp, S);
+    const Dom2& D = A.doms[G.dom];
+    const int ns = min(2, D.steps - A.step);              // steps this domain takes in the launch
+    if (kw > 0) load_corrections(A, G, i0, j0, pp, S);
+    if (ns <= 0) return;
     __syncthreads();   // (the tile constants and the corrections)
     if (kw > 0) add_corrections(S, wr, wc, i, jx, ex, ah, al);
     // deviation from this tile's frame: C (relative to the owner's frame) + the owner's frame offset
@@ -846,7 +875,7 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
         }
     };
     const float2 lx2 = f2(D.lxh), lxl2 = f2(D.lxl), ly2 = f2(D.lyh), lyl2 = f2(D.lyl);
-    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == D.ny - 1, wNy = !INNER && jx + 1 == D.ny - 1;   // y walls per lane
+    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == G.ny - 1, wNy = !INNER && jx + 1 == G.ny - 1;   // y walls per lane
     const float2 mS = make_float2(wS ? 0.f : 1.f, 1.f), mN = make_float2(wNx ? 0.f : 1.f, wNy ? 0.f : 1.f);
     // (clamped neighbours: the lanes they serve are masked, or not read)
     const int cs = max(wc - 1, 0), cn = min(wc + 1, WP - 1), rw = max(wr - 1, 0), re = min(wr + 1, WR2 - 1);
@@ -884,7 +913,7 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
                 if (k == 1) { lam_wall(lx2, lxl2, mul2(f2(2.f), fm), th, tl); acc(th, tl); }
             }
             // x east
-            if (INNER || i < D.nx - 1) {
+            if (INNER || i < G.nx - 1) {
                 lam(lx2, lxl2, add2(fp, flux(b, 4 + k, re, wc)), th, tl);
                 dec(th, tl);
             } else {
@@ -928,7 +957,7 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const Dom2& D, cons
         }
     };
 
-    const EdgeTask edge(D, i0, j0, hi_i, hi_j, A.ex[(A.step + ns - 1) % 3], A.ey[(A.step + ns - 1) % 3]);
+    const EdgeTask edge(G, i0, j0, hi_i, hi_j, A.ex[(A.step + ns - 1) % 3], A.ey[(A.step + ns - 1) % 3]);
     float rh = 0.f, rl = 0.f;       // the edge task's terms, summed over the steps
     auto record = [&](int b) {
         if (!edge.valid) return;
@@ -974,18 +1003,14 @@ template <bool KAHAN, bool LAM_POW2, bool VEC>
 __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
     __shared__ Smem22 S;
     extern __shared__ __align__(16) float2 g_flux2[];   // [step][16][WR2][WP]
-    const TileD tile = A.tiles[blockIdx.x];
-    const Dom2 D = A.doms[tile.dom];
-    const int ns = min(2, D.steps - A.step);             // steps this domain takes in the launch
-    if (ns <= 0) return;
-    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
-    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
+    const TileD G = A.tiles[blockIdx.x];
     if (threadIdx.x < kTileC2Words)
-        reinterpret_cast<float*>(&S.wc)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[tb])[threadIdx.x];
-    if (i0 >= 2 && i0 + TI + 2 <= D.nx && j0 >= 2 && j0 + TJ + 2 <= D.ny)
-        step2d2_tile<KAHAN, LAM_POW2, VEC, true>(A, D, i0, j0, ns, S, g_flux2);
+        reinterpret_cast<float*>(&S.wc)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[blockIdx.x])[threadIdx.x];
+    const int i0 = G.ti * TI, j0 = G.tj * TJ;
+    if (i0 >= 2 && i0 + TI + 2 <= G.nx && j0 >= 2 && j0 + TJ + 2 <= G.ny)
+        step2d2_tile<KAHAN, LAM_POW2, VEC, true>(A, G, i0, j0, S, g_flux2);
     else
-        step2d2_tile<KAHAN, LAM_POW2, VEC, false>(A, D, i0, j0, ns, S, g_flux2);
+        step2d2_tile<KAHAN, LAM_POW2, VEC, false>(A, G, i0, j0, S, g_flux2);
 }
 
 // ---- one second-order time step of one tile ----
@@ -1016,11 +1041,11 @@ static_assert(sizeof(TileC2) == offsetof(SmemO2, rowc), "the tile constants are 
 
 // INNER: the whole window lies inside the domain (no walls, no cut tile)
 template <bool KAHAN, bool LAM_POW2, int LIM, bool VEC, bool INNER>
-__device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, const int i0, const int j0, SmemO2& S,
+__device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, const int i0, const int j0, SmemO2& S,
                                                float2* g_o2) {
     const int tid = threadIdx.x;
     const int kw = A.step - A.s0;                         // step within the fold window
-    const int hi_i = INNER ? TI : min(TI, D.nx - i0), hi_j = INNER ? TJ : min(TJ, D.ny - j0);
+    const int hi_i = INNER ? TI : min(TI, G.nx - i0), hi_j = INNER ? TJ : min(TJ, G.ny - j0);
     const int P = A.plane;
     const float* phi = A.Ph[kw % 3];                      // increments so far (kw = 0: none)
     const float* pli = A.Pl[kw % 3];
@@ -1039,12 +1064,13 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
     bool ex[2];
 #pragma unroll
     for (int q = 0; q < 2; q++)
-        ex[q] = pt && (di == 0 || dj == 0) && (INNER || (i >= 0 && i < D.nx && jx + q >= 0 && jx + q < D.ny));
+        ex[q] = pt && (di == 0 || dj == 0) && (INNER || (i >= 0 && i < G.nx && jx + q >= 0 && jx + q < G.ny));
     const bool ro = wr >= 2 && wr < 2 + hi_i;
     const bool own[2] = {ex[0] && ro && jx >= j0 && jx < j0 + hi_j, ex[1] && ro && jx + 1 >= j0 && jx + 1 < j0 + hi_j};
-    const int cell = D.base + i * D.ny + jx;
+    const int cell = G.base + i * G.ny + jx;
 
     // ---- phase 1: deviations and split fluxes ----
+    const Dom2& D = A.doms[G.dom];
     float2 ah[4], al[4];   // the pair's increments so far (own pairs)
     {
         float2 d[4];
@@ -1075,7 +1101,8 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
                 }
             }
         }
-        if (kw > 0) load_corrections(A, D, i0, j0, pp, S);
+        if (kw > 0) load_corrections(A, G, i0, j0, pp, S);
+        if (A.step >= D.steps) return;
         __syncthreads();   // (the tile constants and the corrections)
         if (kw > 0) add_corrections(S, wr, wc, i, jx, ex, ah, al);
 #pragma unroll
@@ -1103,7 +1130,7 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
     const float alpha = D.alpha;
     if (pt && wr >= 1 && wr <= TI + 2 && wc >= 1 && wc <= TJ / 2) {
         // x: slopes along i, zero on the edge cells i = 0, nx - 1 (and outside the domain)
-        const float hx = !INNER && (i <= 0 || i >= D.nx - 1) ? 0.f : 0.5f;
+        const float hx = !INNER && (i <= 0 || i >= G.nx - 1) ? 0.f : 0.5f;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 pm = fl(k, wr - 1, wc), pc = fl(k, wr, wc), pq = fl(k, wr + 1, wc);
@@ -1116,8 +1143,8 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
         // y: slopes along j (lane x needs the south pair's lane y, lane y the north pair's lane x;
         // the clamped neighbours only serve lanes that no interface reads), zero on j = 0, ny - 1
         const int cs = max(wc - 1, 0), cn = min(wc + 1, WP - 1);
-        const float2 hy = make_float2(!INNER && (jx <= 0 || jx >= D.ny - 1) ? 0.f : 0.5f,
-                                      !INNER && (jx + 1 <= 0 || jx + 1 >= D.ny - 1) ? 0.f : 0.5f);
+        const float2 hy = make_float2(!INNER && (jx <= 0 || jx >= G.ny - 1) ? 0.f : 0.5f,
+                                      !INNER && (jx + 1 <= 0 || jx + 1 >= G.ny - 1) ? 0.f : 0.5f);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 pc = fl(8 + k, wr, wc);
@@ -1131,7 +1158,7 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
     __syncthreads();
 
     // ---- phase 3: the tile's edge records, the interfaces and increments of the own pairs ----
-    const EdgeTask edge(D, i0, j0, hi_i, hi_j, A.ex[A.step % 3], A.ey[A.step % 3]);
+    const EdgeTask edge(G, i0, j0, hi_i, hi_j, A.ex[A.step % 3], A.ey[A.step % 3]);
     if (edge.valid) {
         float th, tl;   // (the face values lie as the split fluxes do, 16 planes further)
         edge.term<LAM_POW2>(D, reinterpret_cast<const float*>(g_o2 + 16 * WR2 * WP), th, tl);
@@ -1139,8 +1166,8 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const Dom2& D, co
     }
     if (!(own[0] || own[1])) return;
     const float2 lx2 = f2(D.lxh), lxl2 = f2(D.lxl), ly2 = f2(D.lyh), lyl2 = f2(D.lyl);
-    const bool wW = !INNER && i == 0, wE = !INNER && i == D.nx - 1;   // x walls (whole pair)
-    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == D.ny - 1, wNy = !INNER && jx + 1 == D.ny - 1;   // y walls per lane
+    const bool wW = !INNER && i == 0, wE = !INNER && i == G.nx - 1;   // x walls (whole pair)
+    const bool wS = !INNER && jx == 0, wNx = !INNER && jx == G.ny - 1, wNy = !INNER && jx + 1 == G.ny - 1;   // y walls per lane
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const float2 Lx = fl(16 + k, wr, wc), Rx = fl(20 + k, wr, wc);
@@ -1181,17 +1208,14 @@ template <bool KAHAN, bool LAM_POW2, int LIM, bool VEC>
 __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
     __shared__ SmemO2 S;
     extern __shared__ __align__(16) float2 g_o2[];   // [32][WR2][WP]: fp fm hp hm, then Lx Rx Ly Ry
-    const TileD tile = A.tiles[blockIdx.x];
-    const Dom2 D = A.doms[tile.dom];
-    if (A.step >= D.steps) return;
-    const int i0 = tile.ti * TI, j0 = tile.tj * TJ;
-    const int tb = D.tile_base + tile.ti * D.tiles_j + tile.tj;
+    const TileD G = A.tiles[blockIdx.x];
     if (threadIdx.x < kTileC2Words)
-        reinterpret_cast<float*>(&S)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[tb])[threadIdx.x];
-    if (i0 >= 2 && i0 + TI + 2 <= D.nx && j0 >= 2 && j0 + TJ + 2 <= D.ny)
-        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, true>(A, D, i0, j0, S, g_o2);
+        reinterpret_cast<float*>(&S)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[blockIdx.x])[threadIdx.x];
+    const int i0 = G.ti * TI, j0 = G.tj * TJ;
+    if (i0 >= 2 && i0 + TI + 2 <= G.nx && j0 >= 2 && j0 + TJ + 2 <= G.ny)
+        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, true>(A, G, i0, j0, S, g_o2);
     else
-        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, false>(A, D, i0, j0, S, g_o2);
+        step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, false>(A, G, i0, j0, S, g_o2);
 }
 
 }  // namespace
@@ -1291,7 +1315,7 @@ MixedState* mixed2d_attach(MixedState* m, char* err, size_t len) {
         D.alpha = (float)p.mc_alpha;
         d->doms.push_back(D);
         for (int a = 0; a < D.tiles_i; a++)
-            for (int b = 0; b < D.tiles_j; b++) d->tiles.push_back({t, a, b});
+            for (int b = 0; b < D.tiles_j; b++) d->tiles.push_back({t, a, b, D.base, D.nx, D.ny, D.ex_base, D.ey_base});
         off += (long)p.nx * p.ny;
         otile += (long)D.tiles_i * D.tiles_j;
         oex += (long)(D.tiles_i - 1) * p.ny;
