@@ -424,6 +424,14 @@ struct Smem2 {
     Coef2D cf;
 };
 
+// Steps inside a fold window are chained by programmatic dependent launch: the next step's blocks are
+// launched, and past the loads of their descriptors and tile constants (which only a fold changes), when
+// this step completes.
+__device__ __forceinline__ void after_previous_step() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // VEC: every domain of the batch has an even row length; the pairs are loaded and stored with
 // 8-byte accesses (load_pair2)
 template <bool KAHAN, bool LAM_POW2, bool VEC>
@@ -431,6 +439,7 @@ __global__ void __launch_bounds__(NTP, 3) k_step2d(Args2 A) {
     __shared__ Smem2 S;
     const TileD tile = A.tiles[blockIdx.x];
     const Dom2 D = A.doms[tile.dom];
+    after_previous_step();
     if (A.step >= D.steps) return;
     const int tid = threadIdx.x;
     const int kw = A.step - A.s0;                       // step within the fold window
@@ -1006,6 +1015,7 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d2(Args2 A) {
     const TileD G = A.tiles[blockIdx.x];
     if (threadIdx.x < kTileC2Words)
         reinterpret_cast<float*>(&S.wc)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[blockIdx.x])[threadIdx.x];
+    after_previous_step();
     const int i0 = G.ti * TI, j0 = G.tj * TJ;
     if (i0 >= 2 && i0 + TI + 2 <= G.nx && j0 >= 2 && j0 + TJ + 2 <= G.ny)
         step2d2_tile<KAHAN, LAM_POW2, VEC, true>(A, G, i0, j0, S, g_flux2);
@@ -1126,7 +1136,10 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, c
     }
     __syncthreads();
 
-    // ---- phase 2: face values ----
+    // ---- phase 2: face values (to shared memory for the neighbours, and kept for the pair itself) ----
+    float2 Lxs[4], Rxs[4], Lys[4], Rys[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) Lxs[k] = Rxs[k] = Lys[k] = Rys[k] = f2(0.f);
     const float alpha = D.alpha;
     if (pt && wr >= 1 && wr <= TI + 2 && wc >= 1 && wc <= TJ / 2) {
         // x: slopes along i, zero on the edge cells i = 0, nx - 1 (and outside the domain)
@@ -1134,9 +1147,9 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, c
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float2 pm = fl(k, wr - 1, wc), pc = fl(k, wr, wc), pq = fl(k, wr + 1, wc);
-            fl(16 + k, wr, wc) = fma2(f2(hx), slope2<LIM>(sub2(pc, pm), sub2(pq, pc), alpha), pc);
+            fl(16 + k, wr, wc) = Lxs[k] = fma2(f2(hx), slope2<LIM>(sub2(pc, pm), sub2(pq, pc), alpha), pc);
             const float2 mm = fl(4 + k, wr - 1, wc), mc = fl(4 + k, wr, wc), mq = fl(4 + k, wr + 1, wc);
-            fl(20 + k, wr, wc) = fma2(f2(-hx), slope2<LIM>(sub2(mc, mm), sub2(mq, mc), alpha), mc);
+            fl(20 + k, wr, wc) = Rxs[k] = fma2(f2(-hx), slope2<LIM>(sub2(mc, mm), sub2(mq, mc), alpha), mc);
         }
     }
     if (pt && wr >= 2 && wr < 2 + TI) {
@@ -1149,10 +1162,10 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, c
         for (int k = 0; k < 4; k++) {
             const float2 pc = fl(8 + k, wr, wc);
             const float2 pb = make_float2(fl(8 + k, wr, cs).y, pc.x), pn = make_float2(pc.y, fl(8 + k, wr, cn).x);
-            fl(24 + k, wr, wc) = fma2(hy, slope2<LIM>(sub2(pc, pb), sub2(pn, pc), alpha), pc);
+            fl(24 + k, wr, wc) = Lys[k] = fma2(hy, slope2<LIM>(sub2(pc, pb), sub2(pn, pc), alpha), pc);
             const float2 mc = fl(12 + k, wr, wc);
             const float2 mb = make_float2(fl(12 + k, wr, cs).y, mc.x), mn = make_float2(mc.y, fl(12 + k, wr, cn).x);
-            fl(28 + k, wr, wc) = fma2(neg2(hy), slope2<LIM>(sub2(mc, mb), sub2(mn, mc), alpha), mc);
+            fl(28 + k, wr, wc) = Rys[k] = fma2(neg2(hy), slope2<LIM>(sub2(mc, mb), sub2(mn, mc), alpha), mc);
         }
     }
     __syncthreads();
@@ -1170,8 +1183,7 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, c
     const bool wS = !INNER && jx == 0, wNx = !INNER && jx == G.ny - 1, wNy = !INNER && jx + 1 == G.ny - 1;   // y walls per lane
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const float2 Lx = fl(16 + k, wr, wc), Rx = fl(20 + k, wr, wc);
-        const float2 Ly = fl(24 + k, wr, wc), Ry = fl(28 + k, wr, wc);
+        const float2 Lx = Lxs[k], Rx = Rxs[k], Ly = Lys[k], Ry = Rys[k];
         float2 h = ah[k], l = al[k];
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
             th = mul2_alone(lh, x);
@@ -1211,6 +1223,7 @@ __global__ void __launch_bounds__(NT2, 2) k_step2d_o2(Args2 A) {
     const TileD G = A.tiles[blockIdx.x];
     if (threadIdx.x < kTileC2Words)
         reinterpret_cast<float*>(&S)[threadIdx.x] = reinterpret_cast<const float*>(&A.tc[blockIdx.x])[threadIdx.x];
+    after_previous_step();
     const int i0 = G.ti * TI, j0 = G.tj * TJ;
     if (i0 >= 2 && i0 + TI + 2 <= G.nx && j0 >= 2 && j0 + TJ + 2 <= G.ny)
         step2d_o2_tile<KAHAN, LAM_POW2, LIM, VEC, true>(A, G, i0, j0, S, g_o2);
@@ -1393,44 +1406,58 @@ int mixed2d_planes(MixedState* m, int item, MixedPlanes* out) {
     return SHLL_OK;
 }
 
+// a step kernel's launch; chained: it follows another step of the same fold window
+static void launch_chained(void (*kern)(Args2), int grid, int threads, size_t smem, cudaStream_t s, const Args2& A, bool chained) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, A);
+}
 // the second-order step kernel of the batch's variant
 template <bool VEC>
-static void launch_o2v(bool kahan, bool pow2, int lim, int ntiles, cudaStream_t s, const Args2& A) {
+static void launch_o2v(bool kahan, bool pow2, int lim, int ntiles, cudaStream_t s, const Args2& A, bool chained) {
     switch ((kahan ? 4 : 0) + (pow2 ? 2 : 0) + lim) {
-        case 0: k_step2d_o2<false, false, 0, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 1: k_step2d_o2<false, false, 1, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 2: k_step2d_o2<false, true, 0, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 3: k_step2d_o2<false, true, 1, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 4: k_step2d_o2<true, false, 0, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 5: k_step2d_o2<true, false, 1, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        case 6: k_step2d_o2<true, true, 0, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
-        default: k_step2d_o2<true, true, 1, VEC><<<ntiles, NT2, kStepO2Smem, s>>>(A); break;
+        case 0: launch_chained(k_step2d_o2<false, false, 0, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 1: launch_chained(k_step2d_o2<false, false, 1, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 2: launch_chained(k_step2d_o2<false, true, 0, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 3: launch_chained(k_step2d_o2<false, true, 1, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 4: launch_chained(k_step2d_o2<true, false, 0, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 5: launch_chained(k_step2d_o2<true, false, 1, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        case 6: launch_chained(k_step2d_o2<true, true, 0, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
+        default: launch_chained(k_step2d_o2<true, true, 1, VEC>, ntiles, NT2, kStepO2Smem, s, A, chained); break;
     }
 }
-static void launch_o2(bool vec, bool kahan, bool pow2, int lim, int ntiles, cudaStream_t s, const Args2& A) {
-    if (vec) launch_o2v<true>(kahan, pow2, lim, ntiles, s, A);
-    else launch_o2v<false>(kahan, pow2, lim, ntiles, s, A);
+static void launch_o2(bool vec, bool kahan, bool pow2, int lim, int ntiles, cudaStream_t s, const Args2& A, bool chained) {
+    if (vec) launch_o2v<true>(kahan, pow2, lim, ntiles, s, A, chained);
+    else launch_o2v<false>(kahan, pow2, lim, ntiles, s, A, chained);
 }
 // the two-step kernel of the batch's variant
 template <bool VEC>
-static void launch_step2(bool kahan, bool pow2, int ntiles, cudaStream_t s, const Args2& A) {
+static void launch_step2(bool kahan, bool pow2, int ntiles, cudaStream_t s, const Args2& A, bool chained) {
     if (kahan) {
-        if (pow2) k_step2d2<true, true, VEC><<<ntiles, NT2, kStep2Smem, s>>>(A);
-        else k_step2d2<true, false, VEC><<<ntiles, NT2, kStep2Smem, s>>>(A);
+        if (pow2) launch_chained(k_step2d2<true, true, VEC>, ntiles, NT2, kStep2Smem, s, A, chained);
+        else launch_chained(k_step2d2<true, false, VEC>, ntiles, NT2, kStep2Smem, s, A, chained);
     } else {
-        if (pow2) k_step2d2<false, true, VEC><<<ntiles, NT2, kStep2Smem, s>>>(A);
-        else k_step2d2<false, false, VEC><<<ntiles, NT2, kStep2Smem, s>>>(A);
+        if (pow2) launch_chained(k_step2d2<false, true, VEC>, ntiles, NT2, kStep2Smem, s, A, chained);
+        else launch_chained(k_step2d2<false, false, VEC>, ntiles, NT2, kStep2Smem, s, A, chained);
     }
 }
 // the first-order one-step kernel of the batch's variant
 template <bool VEC>
-static void launch_step1(bool kahan, bool pow2, int ntiles, cudaStream_t s, const Args2& A) {
+static void launch_step1(bool kahan, bool pow2, int ntiles, cudaStream_t s, const Args2& A, bool chained) {
     if (kahan) {
-        if (pow2) k_step2d<true, true, VEC><<<ntiles, NTP, 0, s>>>(A);
-        else k_step2d<true, false, VEC><<<ntiles, NTP, 0, s>>>(A);
+        if (pow2) launch_chained(k_step2d<true, true, VEC>, ntiles, NTP, 0, s, A, chained);
+        else launch_chained(k_step2d<true, false, VEC>, ntiles, NTP, 0, s, A, chained);
     } else {
-        if (pow2) k_step2d<false, true, VEC><<<ntiles, NTP, 0, s>>>(A);
-        else k_step2d<false, false, VEC><<<ntiles, NTP, 0, s>>>(A);
+        if (pow2) launch_chained(k_step2d<false, true, VEC>, ntiles, NTP, 0, s, A, chained);
+        else launch_chained(k_step2d<false, false, VEC>, ntiles, NTP, 0, s, A, chained);
     }
 }
 
@@ -1476,15 +1503,16 @@ static long issue_run2d(Mixed2D* d, MixedState* m, long maxsteps, cudaStream_t s
         // two steps per launch inside a fold window, one for an odd remainder
         const long wend = std::min<long>(s0 + d->fold, maxsteps);
         const int k = d->kstep == 2 && wend - st >= 2 ? 2 : 1;
+        const bool chained = st > s0;
         if (d->order == 2) {
-            launch_o2(d->vec, kahan, pow2, d->lim, ntiles, s, A);
+            launch_o2(d->vec, kahan, pow2, d->lim, ntiles, s, A, chained);
         } else if (k == 2) {
-            if (d->vec) launch_step2<true>(kahan, pow2, ntiles, s, A);
-            else launch_step2<false>(kahan, pow2, ntiles, s, A);
+            if (d->vec) launch_step2<true>(kahan, pow2, ntiles, s, A, chained);
+            else launch_step2<false>(kahan, pow2, ntiles, s, A, chained);
         } else if (d->vec) {
-            launch_step1<true>(kahan, pow2, ntiles, s, A);
+            launch_step1<true>(kahan, pow2, ntiles, s, A, chained);
         } else {
-            launch_step1<false>(kahan, pow2, ntiles, s, A);
+            launch_step1<false>(kahan, pow2, ntiles, s, A, chained);
         }
         launches++;
         st += k;
