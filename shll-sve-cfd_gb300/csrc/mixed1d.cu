@@ -1219,6 +1219,10 @@ struct MixedState {
         long launches;
     };
     std::vector<GraphEntry> graphs;
+    // streams of the variant groups after the first (1D), created by the first run that has several
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> side_done;
+    cudaEvent_t fork = nullptr;
     std::vector<std::pair<std::vector<long>, std::vector<int>>> seen;  // runs launched once so far
     bool tuning = false;               // autotuner trials: launch directly, no capture
     long cell_updates = 0;
@@ -1493,6 +1497,9 @@ void mixed_destroy(MixedState* m) {
     cudaFree(m->d_bad);
     cudaFree(m->d_bad_items);
     for (auto& g : m->graphs) cudaGraphExecDestroy(g.exec);
+    for (cudaStream_t s : m->side) cudaStreamDestroy(s);
+    for (cudaEvent_t e : m->side_done) cudaEventDestroy(e);
+    if (m->fork) cudaEventDestroy(m->fork);
     cudaFree(m->d_tubes);
     cudaFree(m->d_chunks);
     cudaFree(m->bsum[0]);
@@ -1800,6 +1807,30 @@ int shll_stall_chunk() { return g_stall.load(); }
 static std::atomic<int> g_pair_flux{1};
 extern "C" void shll_set_pair_flux(int on) { g_pair_flux = on == 2 ? 2 : (on ? 1 : 0); }
 
+// side streams and events for `count` variant groups beside the first; false (one stream then) if none
+// can be had
+static bool ensure_side_streams(MixedState* m, int count) {
+    if (count <= 0) return false;
+    if (!m->fork && cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        m->fork = nullptr;
+        return false;
+    }
+    while ((int)m->side.size() < count) {
+        cudaStream_t s = nullptr;
+        cudaEvent_t e = nullptr;
+        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            if (s) cudaStreamDestroy(s);
+            return false;
+        }
+        m->side.push_back(s);
+        m->side_done.push_back(e);
+    }
+    return true;
+}
+
 // threads of a resident block: two cells each over the widest window
 static int resident_threads(MixedState* m, const std::vector<Chunk>& order) {
     int cells = 0;
@@ -1869,26 +1900,46 @@ static cudaError_t issue_run(MixedState* m, const std::vector<Chunk>& order, lon
         n = 1;
         nsweeps = 0;
     }
+    // Variant groups do not depend on each other: each has its own stream between the start-of-run
+    // kernel and the fix-up, so that one group's last, partly filled wave of blocks (and, late in a run,
+    // sweeps of less than one wave) shares the SMs with another group's sweeps.
+    const int ng = nsweeps > 0 && ensure_side_streams(m, (int)groups.size() - 1) ? (int)groups.size() : 1;
+    auto stream_of = [&](int q) { return q == 0 || ng == 1 ? m->stream : m->side[q - 1]; };
+    if (ng > 1) {
+        cudaError_t e = cudaEventRecord(m->fork, m->stream);
+        for (int q = 1; q < ng && e == cudaSuccess; q++) e = cudaStreamWaitEvent(m->side[q - 1], m->fork, 0);
+        if (e != cudaSuccess) return e;
+    }
+    std::vector<long> issued(groups.size(), 0);   // sweep launches in the group's stream so far
     for (long k = 0; k < nsweeps; k++) {
         A.sweep = (int)k;
-        for (const Group& g : groups) {
+        for (size_t q = 0; q < groups.size(); q++) {
+            const Group& g = groups[q];
             const int cnt = g.active[k + 1];
             if (cnt == 0) continue;
             A.chunk0 = g.first;
+            long& in = issued[ng > 1 ? q : 0];
             // the FP32 form (not needed when every chunk takes the pair flux), then the same
             // chunks' pair-flux form (first order, or every order when asked for everywhere)
             cudaError_t e = cudaSuccess;
             if (!(pairs && pf == 2)) {
-                e = launch_sweep(g.variant, m->kahan, cnt, m->stream, A, n > 0);
+                e = launch_sweep(g.variant, m->kahan, cnt, stream_of((int)q), A, in > 0);
                 if (e != cudaSuccess) return e;
                 n++;
+                in++;
             }
             if (pairs && (g.variant <= 1 || pf == 2)) {
-                e = launch_sweep_ff(g.variant, m->kahan, cnt, m->stream, A, n > 0);
+                e = launch_sweep_ff(g.variant, m->kahan, cnt, stream_of((int)q), A, in > 0);
                 if (e != cudaSuccess) return e;
                 n++;
+                in++;
             }
         }
+    }
+    for (int q = 1; q < ng; q++) {
+        cudaError_t e = cudaEventRecord(m->side_done[q - 1], m->side[q - 1]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(m->stream, m->side_done[q - 1], 0);
+        if (e != cudaSuccess) return e;
     }
     A.chunk0 = 0;
     const int nch = (int)order.size();
