@@ -182,15 +182,17 @@ struct ResPlan {
 };
 
 // Chunks, window and steps per sweep.  One chunk per SM where the windows fit; then the window of
-// least estimated time per step: the larger of the step's chain (`chain` clocks) and the block's
-// instruction time (`work` clocks per warp: FP64 about 42 + 10 instructions of 19 clocks for order 1,
-// 70 + 12 for order 2; float about 260 / 400 instructions over four schedulers), plus the exchange
-// (about 4500 clocks) over the S steps it serves.  A narrower window means less redundant work per
-// step, a wider one fewer exchanges.
+// least estimated time per step: the step's chain (`chain` clocks) plus a share per warp (`share`), or,
+// where it is more, the block's instruction time (`work` clocks per warp: FP64 about 42 + 10 instructions
+// of 19 clocks for order 1, 70 + 12 for order 2), plus the exchange (about 4500 clocks) over the S steps
+// it serves.  A narrower window means less redundant work per step, a wider one fewer exchanges.
+// Measured, us a step with 32 / 64 / 96 / 128 / 256 / 512 threads at 1024 cells: FP64 first order 1.70 /
+// 1.64 / 1.62 / 1.66 / 2.10 / 3.11, float 0.53 / 0.47 / 0.45 / 0.44 / 0.45 / 0.51.
 template <typename REAL, int ORDER>
 static ResPlan res_plan(int n, long steps, int sms) {
     const bool wide = sizeof(REAL) == 8;
-    const double chain = wide ? (ORDER == 1 ? 2200 : 3000) : (ORDER == 1 ? 700 : 900);
+    const double chain = wide ? (ORDER == 1 ? 3000 : 5200) : (ORDER == 1 ? 800 : 1450);
+    const double share = wide ? (ORDER == 1 ? 300 : 450) : (ORDER == 1 ? 30 : 45);
     const double work = wide ? (ORDER == 1 ? 1000 : 1560) : (ORDER == 1 ? 70 : 110);
     ResPlan best = {0, 0, 0, false};
     double best_t = 1e30;
@@ -200,7 +202,7 @@ static ResPlan res_plan(int n, long steps, int sms) {
         const int S = (int)std::min<long>((T - owned) / (2 * ORDER), steps);
         if (S < 1) continue;
         const double warps = (owned + ORDER * (S + 1)) / 32.0 + 0.5;
-        const double t = std::max(chain, warps * work) + 4500.0 / S;
+        const double t = std::max(chain + (warps + std::max(0, T / 32 - 4) * 0.5) * share, warps * work) + (wide ? 3000.0 : 4500.0) / S;
         if (t < best_t) { best_t = t; best = {k, T, S, true}; }
     }
     // more cells than one window per SM holds (or windows with hardly any margin): several blocks per
