@@ -39,15 +39,21 @@ struct ResArgs {
     int stall;         // test hook: this chunk never publishes its progress (-1: none)
 };
 
+// LANES: threads per cell, 1, or 4 (FP64): lane q of a cell's group holds component q (lane 3 doubles
+// component 0 and stores nothing)
 template <typename REAL, int ORDER>
-constexpr size_t res_smem(int threads) {
-    return (size_t)(ORDER == 1 ? 12 : 18) * threads * sizeof(REAL);
+constexpr size_t res_smem(int cells) {
+    return (size_t)(ORDER == 1 ? 12 : 18) * cells * sizeof(REAL);
 }
 
-template <typename REAL, int ORDER>
+template <typename REAL, int ORDER, int LANES>
 __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, Gas<REAL> g) {
     extern __shared__ __align__(16) unsigned char res_raw[];
-    const int T = blockDim.x, tid = threadIdx.x, n = A.n;
+    constexpr int NQ = LANES == 1 ? 3 : 1;               // components of this thread
+    const int T = blockDim.x / LANES, tid = threadIdx.x / LANES, n = A.n;   // window cells, this thread's
+    const int lane = LANES == 1 ? 0 : threadIdx.x & 3;
+    const int q0 = lane == 3 ? 0 : lane;                 // first component
+    const bool writes = LANES == 1 || lane < 3;
     REAL* flux = reinterpret_cast<REAL*>(res_raw);     // [2][fp, fm][3][T], by step parity
     REAL* slp = flux + 12 * T;                         // order 2: [dp, dm][3][T]
     const long k = gridDim.x, c = blockIdx.x;
@@ -58,7 +64,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
     // the chunks that own the window's cells (cell x belongs to chunk ((x + 1) k - 1) / n)
     const int first = max(a - H, 0), last = min(b + H, n) - 1;
     const int c0 = (int)(((first + 1) * k - 1) / n), nc = (int)(((last + 1) * k - 1) / n) - c0 + 1;
-    REAL u[3] = {1, 0, 1};
+    REAL u[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) u[q] = q0 + q == 1 ? (REAL)0 : (REAL)1;
     int bad = 0, par = 0;
     for (long sweep = 0; sweep * A.S < A.steps; sweep++) {
         const int s_now = (int)min((long)A.S, A.steps - sweep * A.S);
@@ -68,7 +76,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
             // every chunk of the window has completed the previous sweep: its cells can be read, and
             // it no longer reads the buffer that this sweep writes
             bool ok = true;
-            for (int q = tid; q < nc; q += T) {
+            for (int q = threadIdx.x; q < nc; q += blockDim.x) {
                 const unsigned* p = A.prog + (long)(c0 + q) * kPlainProgStride;
                 bool got = c0 + q == c;
                 for (long it = 0; it < kResSpin && !got; it++) {
@@ -87,87 +95,97 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
         // cells valid before step s: [a - ORDER (s_now - s), b + ORDER (s_now - s)) within the tube
         if (i >= max(a - ORDER * s_now, 0) && i < min(b + ORDER * s_now, n) && (sweep == 0 || !own)) {
 #pragma unroll
-            for (int q = 0; q < 3; q++) u[q] = __ldcg(Uin + (long)q * n + i);
+            for (int q = 0; q < NQ; q++) u[q] = __ldcg(Uin + (long)(q0 + q) * n + i);
         }
         for (int s = 0; s < s_now; s++, par ^= 1) {
             const int lo = a - ORDER * (s_now - s), hi = b + ORDER * (s_now - s);
             const bool valid = i >= max(lo, 0) && i < min(hi, n);
             const bool next = i >= max(lo + ORDER, 0) && i < min(hi - ORDER, n);
             REAL* F = flux + par * 6 * T;
-            REAL fp[3], fm[3];
-            if (valid) {
-                bad |= cell1(g, u, fp, fm);
+            REAL fp[NQ], fm[NQ];
+            if constexpr (LANES == 1) {
+                if (valid) bad |= cell1(g, u, fp, fm);
+            } else {
+                // (whole warps, as the lanes of a group exchange their values)
+                if (__any_sync(0xffffffffu, valid)) {
+                    const int b = cell1_lanes(g, u[0], fp[0], fm[0]);
+                    bad |= valid && b;
+                }
+            }
+            if (valid && writes) {
 #pragma unroll
-                for (int q = 0; q < 3; q++) { F[q * T + tid] = fp[q]; F[(3 + q) * T + tid] = fm[q]; }
+                for (int q = 0; q < NQ; q++) { F[(q0 + q) * T + tid] = fp[q]; F[(3 + q0 + q) * T + tid] = fm[q]; }
             }
             __syncthreads();
             if constexpr (ORDER == 1) {
                 if (next) {
-                    REAL x[3], v[3];
+                    REAL x[NQ], v[NQ];
                     bool special = false;
 #pragma unroll
-                    for (int q = 0; q < 3; q++) {
+                    for (int q = 0; q < NQ; q++) {
                         // reflective walls (base_shll.c:93-110)
-                        const REAL sg = (q == 1) ? (REAL)1 : (REAL)-1;
-                        const REAL L = i == 0 ? sg * fm[q] : F[q * T + tid - 1];
-                        const REAL Rr = i == n - 1 && i != 0 ? sg * fp[q] : F[(3 + q) * T + tid + 1];
+                        const REAL sg = (q0 + q == 1) ? (REAL)1 : (REAL)-1;
+                        const REAL L = i == 0 ? sg * fm[q] : F[(q0 + q) * T + tid - 1];
+                        const REAL Rr = i == n - 1 && i != 0 ? sg * fp[q] : F[(3 + q0 + q) * T + tid + 1];
                         x[q] = fp[q] - fm[q] + Rr - L;
                         v[q] = sub_scaled_plain(u[q], g.sx, x[q], &special);
                     }
 #pragma unroll
-                    for (int q = 0; q < 3; q++) u[q] = special ? sub_scaled(u[q], g.sx, x[q]) : v[q];
+                    for (int q = 0; q < NQ; q++) u[q] = special ? sub_scaled(u[q], g.sx, x[q]) : v[q];
                 }
             } else {
-                REAL dp[3] = {0, 0, 0}, dm[3] = {0, 0, 0};
+                REAL dp[NQ], dm[NQ];
+#pragma unroll
+                for (int q = 0; q < NQ; q++) dp[q] = dm[q] = 0;
                 if (valid && i >= max(lo + 1, 0) && i < min(hi - 1, n)) {
                     if (i > 0 && i < n - 1) {
                         bool special = false;
 #pragma unroll
-                        for (int q = 0; q < 3; q++) {
-                            dp[q] = slope_plain(g, F[q * T + tid - 1], fp[q], F[q * T + tid + 1], &special);
-                            dm[q] = slope_plain(g, F[(3 + q) * T + tid - 1], fm[q], F[(3 + q) * T + tid + 1], &special);
+                        for (int q = 0; q < NQ; q++) {
+                            dp[q] = slope_plain(g, F[(q0 + q) * T + tid - 1], fp[q], F[(q0 + q) * T + tid + 1], &special);
+                            dm[q] = slope_plain(g, F[(3 + q0 + q) * T + tid - 1], fm[q], F[(3 + q0 + q) * T + tid + 1], &special);
                         }
                         if (special) {
 #pragma unroll
-                            for (int q = 0; q < 3; q++) {
-                                dp[q] = slope(g, F[q * T + tid - 1], fp[q], F[q * T + tid + 1]);
-                                dm[q] = slope(g, F[(3 + q) * T + tid - 1], fm[q], F[(3 + q) * T + tid + 1]);
+                            for (int q = 0; q < NQ; q++) {
+                                dp[q] = slope(g, F[(q0 + q) * T + tid - 1], fp[q], F[(q0 + q) * T + tid + 1]);
+                                dm[q] = slope(g, F[(3 + q0 + q) * T + tid - 1], fm[q], F[(3 + q0 + q) * T + tid + 1]);
                             }
                         }
                     }
 #pragma unroll
-                    for (int q = 0; q < 3; q++) { slp[q * T + tid] = dp[q]; slp[(3 + q) * T + tid] = dm[q]; }
+                    for (int q = 0; q < NQ; q++) if (writes) { slp[(q0 + q) * T + tid] = dp[q]; slp[(3 + q0 + q) * T + tid] = dm[q]; }
                 }
                 __syncthreads();
                 if (next) {   // outflow walls (2nd_order_base_shll.c:210-262)
-                    REAL x[3], y[3], v[3];
+                    REAL x[NQ], y[NQ], v[NQ];
                     bool special = false;
 #pragma unroll
-                    for (int q = 0; q < 3; q++) {
+                    for (int q = 0; q < NQ; q++) {
                         const bool wl = i == 0, wr = i == n - 1 && i != 0;
-                        const REAL L = wl ? fp[q] : F[q * T + tid - 1], Ldf = wl ? (REAL)0 : slp[q * T + tid - 1];
-                        const REAL Rr = wr ? fm[q] : F[(3 + q) * T + tid + 1];
-                        const REAL Rdf = wr ? (REAL)0 : slp[(3 + q) * T + tid + 1];
+                        const REAL L = wl ? fp[q] : F[(q0 + q) * T + tid - 1], Ldf = wl ? (REAL)0 : slp[(q0 + q) * T + tid - 1];
+                        const REAL Rr = wr ? fm[q] : F[(3 + q0 + q) * T + tid + 1];
+                        const REAL Rdf = wr ? (REAL)0 : slp[(3 + q0 + q) * T + tid + 1];
                         x[q] = fp[q] - fm[q] + Rr - L;
                         y[q] = dp[q] + dm[q] - Rdf - Ldf;
                         v[q] = sub_half_scaled_plain(sub_scaled_plain(u[q], g.sx, x[q], &special), g.hsx, y[q], &special);
                     }
 #pragma unroll
-                    for (int q = 0; q < 3; q++)
+                    for (int q = 0; q < NQ; q++)
                         u[q] = special ? sub_half_scaled(sub_scaled(u[q], g.sx, x[q]), g.hsx, y[q]) : v[q];
                 }
             }
         }
         // the next sweep's windows reach H cells into this chunk; after the last sweep, all of it
         const bool done = (sweep + 1) * A.S >= A.steps;
-        if (own && (done || i < a + H || i >= b - H)) {
+        if (own && writes && (done || i < a + H || i >= b - H)) {
 #pragma unroll
-            for (int q = 0; q < 3; q++) Uout[(long)q * n + i] = u[q];
+            for (int q = 0; q < NQ; q++) Uout[(long)(q0 + q) * n + i] = u[q];
         }
         if (!done) {
             __syncthreads();
             // (the barrier orders the block's stores before the release)
-            if (tid == 0 && c != A.stall)
+            if (threadIdx.x == 0 && c != A.stall)
                 asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(A.prog + c * kPlainProgStride),
                              "r"((unsigned)(sweep + 1)) : "memory");
         }
@@ -177,7 +195,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_resident1(ResArgs<REAL> A, G
 
 // ---------------- host ----------------
 struct ResPlan {
-    int chunks, threads, S;
+    int chunks, threads, S, lanes;
     bool resident;
 };
 
@@ -194,7 +212,7 @@ static ResPlan res_plan(int n, long steps, int sms) {
     const double chain = wide ? (ORDER == 1 ? 3000 : 5200) : (ORDER == 1 ? 800 : 1450);
     const double share = wide ? (ORDER == 1 ? 300 : 450) : (ORDER == 1 ? 30 : 45);
     const double work = wide ? (ORDER == 1 ? 1000 : 1560) : (ORDER == 1 ? 70 : 110);
-    ResPlan best = {0, 0, 0, false};
+    ResPlan best = {0, 0, 0, 1, false};
     double best_t = 1e30;
     const int k = std::min(sms, n);
     const int owned = (n + k - 1) / k;
@@ -202,29 +220,46 @@ static ResPlan res_plan(int n, long steps, int sms) {
         const int S = (int)std::min<long>((T - owned) / (2 * ORDER), steps);
         if (S < 1) continue;
         const double warps = (owned + ORDER * (S + 1)) / 32.0 + 0.5;
-        const double t = std::max(chain + (warps + std::max(0, T / 32 - 4) * 0.5) * share, warps * work) + (wide ? 3000.0 : 4500.0) / S;
-        if (t < best_t) { best_t = t; best = {k, T, S, true}; }
+        const double t = std::max(chain + (warps + std::max(0, T / 32 - 4) * 0.5) * share, warps * work) +
+                         (wide ? 3000.0 : 4500.0) / S;
+        if (t < best_t) { best_t = t; best = {k, T, S, 1, true}; }
+    }
+    // FP64 with four lanes per cell: a shorter chain, more FP64 instructions in all (1024 cells: first order
+    // 1.62 -> 1.26 us a step, second 2.80 -> 1.82; from 8192 cells on one lane per cell is faster, first order
+    // 1.67 against 2.08)
+    if (wide) {
+        for (int T = 128; T <= 256; T += 64) {
+            const int S = (int)std::min<long>((T / 4 - owned) / (2 * ORDER), steps);
+            if (S < 1) continue;
+            const double warps = 4 * (owned + ORDER * (S + 1)) / 32.0;
+            const double t = (ORDER == 1 ? 2200 : 3400) + std::max(0.0, warps - 3.0) * (ORDER == 1 ? 300 : 450) +
+                             std::max(0, T / 32 - 4) * 60.0 + 3000.0 / S;
+            if (t < best_t) { best_t = t; best = {k, T, S, 4, true}; }
+        }
     }
     // more cells than one window per SM holds (or windows with hardly any margin): several blocks per
     // SM, one launch per sweep of 8 steps
-    if (best.chunks == 0 || best.S < 4) {
+    if (best.chunks == 0 || (best.S < 4 && best.lanes == 1)) {
         const int T = 256, S = (int)std::min<long>(8, steps), per = T - 2 * ORDER * S;
-        best = {(n + per - 1) / per, T, S, false};
+        best = {(n + per - 1) / per, T, S, 1, false};
     }
     return best;
 }
 
 template <typename REAL, int ORDER>
 static cudaError_t run1_t(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps) {
-    auto* kern = k_resident1<REAL, ORDER>;
     int dev = 0, sms = 1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_smem<REAL, ORDER>(kResThreads));
     if (e != cudaSuccess) return e;
     ResPlan p = res_plan<REAL, ORDER>(a.nx, steps, std::min(sms, kPlainProgChunks));
-    const size_t smem = res_smem<REAL, ORDER>(p.threads);
+    auto* kern = k_resident1<REAL, ORDER, 1>;
+    if constexpr (sizeof(REAL) == 8) {
+        if (p.lanes == 4) kern = k_resident1<REAL, ORDER, 4>;
+    }
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)res_smem<REAL, ORDER>(kResThreads));
+    if (e != cudaSuccess) return e;
+    const size_t smem = res_smem<REAL, ORDER>(p.threads / p.lanes);
     const Gas<REAL> g = make_gas<REAL>(a);
     ResArgs<REAL> A;
     A.U[0] = static_cast<REAL*>(const_cast<void*>(a.Uin));

@@ -261,6 +261,43 @@ __device__ __forceinline__ int cell1(const Gas<double>& g, const double u[3], do
     for (int k = 0; k < 3; k++) { fp[k] = c.f[k]; fm[k] = c.f[3 + k]; }
     return c.bad;
 }
+// The same by a group of four lanes, FP64: lane k < 3 of the group evaluates component k alone (lane 3
+// doubles lane 0), so that one lane issues 17 FP64 instructions and not 32 (25 and not 40 without fused
+// operations): a scheduler starts one FP64 warp instruction in about 70 clocks whatever its
+// dependences, which is what a step of a small tube waits for.  u: this lane's component.
+__device__ __forceinline__ int cell1_lanes(const Gas<double>& g, double u, double& fp, double& fm) {
+    const int k = threadIdx.x & 3;
+    const double u0 = __shfl_sync(0xffffffffu, u, 0, 4), u1 = __shfl_sync(0xffffffffu, u, 1, 4),
+                 u2 = __shfl_sync(0xffffffffu, u, 2, 4);
+    const exact_math::Divisor rho = exact_math::divisor(u0);
+    const double q = exact_math::divide_plain(k == 2 ? u2 : u1, rho);
+    const double q1 = __shfl_sync(0xffffffffu, q, 1, 4), e = __shfl_sync(0xffffffffu, q, 2, 4);
+    const double p1 = is_zero(u1) ? u1 : q1;
+    const double t = __fma_rn(-0.5, __dmul_rn(p1, p1), e);
+    const double p2 = exact_math::divide_plain(t, g.cv);
+    exact_math::Divisor snd;
+    const double a = exact_math::square_root_plain(g.gR * p2, &snd);
+    const double M = divide_or_zero(p1, snd);
+    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * (1.0 - M * M);   // twice the reference's
+    const double P = times_R(g, u0) * p2;
+    // F = u1, u1 p1 + P, p1 (u2 + P)
+    double F;
+#if SHLL_PLAIN_FMA
+    F = __fma_rn(k == 2 ? 1.0 : u1, k == 2 ? u2 : p1, P);
+#else
+    F = (k == 2 ? u2 : u1 * p1) + P;
+#endif
+    const double F2 = p1 * F;
+    F = k == 1 ? F : k == 2 ? F2 : u1;
+    const double v = k == 1 ? u1 : k == 2 ? u2 : u0;
+    fp = F * Z1 + v * Z2;
+    fm = -F * Z3 - v * Z2;
+    if (g.plain && in_range(u0, 923, 200) && in_range(u2, 923, 200) && momentum_plain(u1) && in_range(t, 900, 250)) return 0;
+    const auto c = cell1_general(g, u0, u1, u2);
+    fp = k == 1 ? c.f[1] : k == 2 ? c.f[2] : c.f[0];
+    fm = k == 1 ? c.f[4] : k == 2 ? c.f[5] : c.f[3];
+    return c.bad;
+}
 __device__ __forceinline__ int cell1(const Gas<float>& g, const float u[3], float fp[3], float fm[3]) {
     const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
     const float p1 = exact_math::divide_plain(u[1], u[0], y), e = exact_math::divide_plain(u[2], u[0], y);
