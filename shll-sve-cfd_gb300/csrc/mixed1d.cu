@@ -39,6 +39,7 @@
 #include <mutex>
 #include <vector>
 
+#include "exact_math.cuh"
 #include "mixed.h"
 #include "mixed_common.cuh"
 #include "shll_internal.h"
@@ -1580,15 +1581,17 @@ __global__ void k_prim_from_u(MixedPlanes s, double* __restrict__ out) {
             U[k] = KAHAN ? (double)static_cast<const float*>(s.hi)[idx] + (double)s.lo[idx]
                          : static_cast<const double*>(s.hi)[idx];
         }
-        const double u0 = U[0], p1 = U[1] / u0;
+        // (quotients on the integer pipes: correctly rounded, as the host's)
+        const exact_math::Divisor d0 = exact_math::divisor(U[0]), dc = exact_math::divisor(s.CV);
+        const double u0 = U[0], p1 = exact_math::divide(U[1], d0);
         out[i] = u0;
         out[n + i] = p1;
         if (s.nv == 3) {
-            out[2 * n + i] = ((U[2] / u0) - 0.5 * p1 * p1) / s.CV;
+            out[2 * n + i] = exact_math::divide(exact_math::divide(U[2], d0) - 0.5 * p1 * p1, dc);
         } else {
-            const double p2 = U[2] / u0;
+            const double p2 = exact_math::divide(U[2], d0);
             out[2 * n + i] = p2;
-            out[3 * n + i] = ((U[3] / u0) - 0.5 * (p1 * p1 + p2 * p2)) / s.CV;
+            out[3 * n + i] = exact_math::divide(exact_math::divide(U[3], d0) - 0.5 * (p1 * p1 + p2 * p2), dc);
         }
     }
 }

@@ -34,6 +34,7 @@
 #include <mutex>
 #include <vector>
 
+#include "exact_math.cuh"
 #include "mixed.h"
 #include "mixed_common.cuh"
 #include "shll_internal.h"
@@ -119,37 +120,72 @@ struct TileC2 {
 constexpr int kTileC2Words = (int)(sizeof(TileC2) / 4);
 static_assert(sizeof(TileC2) % 4 == 0, "word copy");
 
-__device__ void make_frame2(Frame2& f, const double U[4], const Dom2& d) {
-    const double rho = U[0], m = U[1], nn = U[2], E = U[3];
-    const double u = m / rho, v = nn / rho, e = E / rho;
-    const double T = (e - 0.5 * (u * u + v * v)) / d.CV;
-    const double a = sqrt(d.gamma * d.R * T);
-    const double P = rho * d.R * T;
-    const double Fx[4] = {m, m * u + P, m * v, u * (E + P)};
-    const double Fy[4] = {nn, nn * u, nn * v + P, v * (E + P)};
-    const double Mx = u / a, My = v / a;
-    const double Z1x = 0.5 * (Mx + 1.0), Z2x = 0.5 * a * (1.0 - Mx * Mx), Z3x = 0.5 * (Mx - 1.0);
-    const double Z1y = 0.5 * (My + 1.0), Z2y = 0.5 * a * (1.0 - My * My), Z3y = 0.5 * (My - 1.0);
-    for (int k = 0; k < 4; k++) {
-        f.U[k] = U[k]; f.Fx[k] = Fx[k]; f.Fy[k] = Fy[k];
-        f.cx.F[k] = (float)Fx[k]; f.cy.F[k] = (float)Fy[k];
-        f.cx.Uf[k] = f.cy.Uf[k] = (float)U[k];
+// A tile's frame: the FP64 values by one thread (divisions and the square root on the integer pipes, the
+// same bits as the FP64 pipe's), their FP32 coefficients by the first threads of the block together.
+// fr: in shared memory; v: scratch.  Ends with a block barrier.
+constexpr int kFrame2Values = 27;   // U 0-3, Fx 4-7, Fy 8-11, u v e T a P gR R 1/CV 12-20, M Z1 Z2 of x 21-23, of y 24-26
+constexpr int kCoefWords = (int)(sizeof(AnchorCoef) / 4);
+static_assert(kCoefWords == 21, "the order of AnchorCoef's fields");
+__device__ const signed char kCoefOf[2][kCoefWords] = {
+    {0, 12, 13, 14, 15, 16, 21, 17, 22, 23, 18, 19, 20, 4, 5, 6, 7, 0, 1, 2, 3},
+    {0, 12, 13, 14, 15, 16, 24, 17, 25, 26, 18, 19, 20, 8, 9, 10, 11, 0, 1, 2, 3}};
+__device__ void make_frame2(Frame2& f, double* x, const double U[4], const Dom2& d) {
+    using exact_math::divide;
+    if (threadIdx.x == 0) {
+        const double rho = U[0], m = U[1], nn = U[2], E = U[3];
+        const exact_math::Divisor dr = exact_math::divisor(rho);
+        const double u = divide(m, dr), v = divide(nn, dr), e = divide(E, dr);
+        const double T = divide(e - 0.5 * (u * u + v * v), exact_math::divisor(d.CV));
+        const double a = exact_math::square_root(d.gamma * d.R * T);
+        const double P = rho * d.R * T;
+        const double Fx[4] = {m, m * u + P, m * v, u * (E + P)};
+        const double Fy[4] = {nn, nn * u, nn * v + P, v * (E + P)};
+        const exact_math::Divisor da = exact_math::divisor(a);
+        const double Mx = divide(u, da), My = divide(v, da);
+        const double Z1x = 0.5 * (Mx + 1.0), Z2x = 0.5 * a * (1.0 - Mx * Mx), Z3x = 0.5 * (Mx - 1.0);
+        const double Z1y = 0.5 * (My + 1.0), Z2y = 0.5 * a * (1.0 - My * My), Z3y = 0.5 * (My - 1.0);
+        for (int k = 0; k < 4; k++) {
+            f.U[k] = x[k] = U[k]; f.Fx[k] = x[4 + k] = Fx[k]; f.Fy[k] = x[8 + k] = Fy[k];
+        }
+        f.fpS1 = Fx[1] * Z1x + m * Z2x;
+        f.fmS1 = -Fx[1] * Z3x - m * Z2x;
+        f.hpS2 = Fy[2] * Z1y + nn * Z2y;
+        f.hmS2 = -Fy[2] * Z3y - nn * Z2y;
+        x[12] = u; x[13] = v; x[14] = e; x[15] = T; x[16] = a; x[17] = P;
+        x[18] = d.gamma * d.R; x[19] = d.R; x[20] = divide(1.0, exact_math::divisor(d.CV));
+        x[21] = Mx; x[22] = Z1x; x[23] = Z2x;
+        x[24] = My; x[25] = Z1y; x[26] = Z2y;
     }
-    f.fpS1 = Fx[1] * Z1x + m * Z2x;
-    f.fmS1 = -Fx[1] * Z3x - m * Z2x;
-    f.hpS2 = Fy[2] * Z1y + nn * Z2y;
-    f.hmS2 = -Fy[2] * Z3y - nn * Z2y;
-    AnchorCoef* c[2] = {&f.cx, &f.cy};
-    for (int q = 0; q < 2; q++) {
-        c[q]->rho = (float)rho; c[q]->u = (float)u; c[q]->v = (float)v; c[q]->e = (float)e;
-        c[q]->T = (float)T; c[q]->a = (float)a; c[q]->P = (float)P;
-        c[q]->gR = (float)(d.gamma * d.R); c[q]->R = (float)d.R; c[q]->cvinv = (float)(1.0 / d.CV);
+    __syncthreads();
+    if (threadIdx.x < 2 * kCoefWords) {
+        const int dir = threadIdx.x / kCoefWords, w = threadIdx.x % kCoefWords;
+        reinterpret_cast<float*>(dir ? &f.cy : &f.cx)[w] = (float)x[kCoefOf[dir][w]];
     }
-    f.cx.M = (float)Mx; f.cx.Z1 = (float)Z1x; f.cx.Z2 = (float)Z2x;
-    f.cy.M = (float)My; f.cy.Z1 = (float)Z1y; f.cy.Z2 = (float)Z2y;
+    __syncthreads();
 }
 
-
+// float <-> double without the FP64 pipe's conversions (19 clocks per warp instruction per SM): the same
+// values; subnormal and non-finite operands or results take the conversion instruction
+__device__ __forceinline__ double to_double(float x) {
+    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+    if (e - 1u < 254u)
+        return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+    return (b << 1) == 0u ? __hiloint2double((int)b, 0) : (double)x;
+}
+__device__ __forceinline__ float to_float(double x) {   // round to nearest even
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = (hi >> 20) & 0x7ffu;
+    if (e - 897u < 253u) {
+        const unsigned r = __funnelshift_l(lo, hi & 0x7fffffffu, 3) - (896u << 23), rest = lo & 0x1fffffffu;
+        const unsigned up = rest > 0x10000000u || (rest == 0x10000000u && (r & 1u)) ? 1u : 0u;
+        return __uint_as_float((hi & 0x80000000u) | (r + up));
+    }
+    return ((hi << 1) | lo) == 0u ? __uint_as_float(hi) : (float)x;
+}
+__device__ __forceinline__ bool positive_finite(double x) {
+    const long long b = __double_as_longlong(x);
+    return b > 0 && b < 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool finite(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
 
 // dflux2 for two cells at once (same deviation identities, lane by lane; the minus fluxes from
 // dfp + dfm = dF)
@@ -299,9 +335,12 @@ __device__ __forceinline__ void load_pair2(const Args2& A, const Dom2& D, int i,
 }
 
 // ---- fold: B += P (+ the last edge corrections), new frames, C = B - U* ----
+// Was bound by the FP64 pipe; per cell and component three FP64 additions are left (five for the cells on
+// edge lines), the conversions, checks and the frame's divisions run on the integer pipes, and three blocks
+// share an SM while one thread of each computes a frame: a fold of 4096 x 4096 cells 3.4 -> 1.5 ms.
 template <bool KAHAN>
-__global__ void __launch_bounds__(NT) k_fold2d(Args2 A) {
-    __shared__ double sU[4];
+__global__ void __launch_bounds__(NT, 3) k_fold2d(Args2 A) {
+    __shared__ double sU[4], sx[kFrame2Values];
     __shared__ Frame2 fr;
     const TileD tile = A.tiles[blockIdx.x];
     const Dom2 D = A.doms[tile.dom];
@@ -319,7 +358,8 @@ __global__ void __launch_bounds__(NT) k_fold2d(Args2 A) {
     int bad = 0;
     if (own) {
         float ch[4] = {0, 0, 0, 0}, cl[4] = {0, 0, 0, 0};
-        if (wd > 0 && on_edge_line(i, j)) edge_correction(A, D, i, j, (A.s0 + wd - 1) % 3, ch, cl);
+        const bool edge = wd > 0 && on_edge_line(i, j);
+        if (edge) edge_correction(A, D, i, j, (A.s0 + wd - 1) % 3, ch, cl);
         const float* ph = A.Ph[wd % 3];
         const float* pl = A.Pl[wd % 3];
         for (int k = 0; k < 4; k++) {
@@ -335,29 +375,29 @@ __global__ void __launch_bounds__(NT) k_fold2d(Args2 A) {
                     static_cast<float*>(A.B)[idx] = h;
                     A.Blo[idx] = l;
                 }
-                U[k] = (double)h + (double)l;
+                U[k] = to_double(h) + to_double(l);
             } else {
                 double v = static_cast<double*>(A.B)[idx];
                 if (wd > 0) {
-                    v = v + ((double)ph[idx] + (double)pl[idx]) + ((double)ch[k] + (double)cl[k]);
+                    v = v + (to_double(ph[idx]) + to_double(pl[idx]));
+                    if (edge) v = v + (to_double(ch[k]) + to_double(cl[k]));
                     static_cast<double*>(A.B)[idx] = v;
                 }
                 U[k] = v;
             }
         }
         // breakdown: non-positive density or energy, or a non-finite state
-        bad = !(U[0] > 0.0) || !(U[3] > 0.0) || !isfinite(U[0] + U[1] + U[2] + U[3]);
+        bad = !positive_finite(U[0]) || !positive_finite(U[3]) || !finite(U[1]) || !finite(U[2]);
         if (li == hi_i / 2 && lj == hi_j / 2)
             for (int k = 0; k < 4; k++) sU[k] = U[k];
     }
     __syncthreads();
-    if (tid == 0) {
-        make_frame2(fr, sU, D);
-        A.frames[D.tile_base + tile.ti * D.tiles_j + tile.tj] = fr;
-    }
-    __syncthreads();
+    make_frame2(fr, sx, sU, D);
+    if (tid < (int)(sizeof(Frame2) / 4))
+        reinterpret_cast<unsigned*>(&A.frames[D.tile_base + tile.ti * D.tiles_j + tile.tj])[tid] =
+            reinterpret_cast<const unsigned*>(&fr)[tid];
     if (own)
-        for (int k = 0; k < 4; k++) A.C[k * P + cell] = (float)(U[k] - fr.U[k]);
+        for (int k = 0; k < 4; k++) A.C[k * P + cell] = to_float(U[k] - fr.U[k]);
     if (bad) {
         atomicOr(A.flag, SHLL_FLAG_NONPOSITIVE);
         atomicOr(&A.item_flags[tile.dom], SHLL_FLAG_NONPOSITIVE);
