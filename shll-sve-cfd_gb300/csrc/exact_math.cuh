@@ -243,7 +243,8 @@ EM_FN float square_root_plain(float x, float* y) {
 
 // (float)((D(e) - k) / D(c)) with k = kh + kl the exact subtrahend (D(k) a double of at most 48
 // bits) and rc an approximation of 1 / c
-EM_FN float temperature_ref(float e, float kh, float kl, float c, float rc) {
+// (*ok cleared: the value may be the other neighbour, temperature_slow decides)
+EM_FN float temperature_plain(float e, float kh, float kl, float c, float rc, bool* ok) {
     float sl;
     const float sh = two_sum(e, -kh, sl);
     sl = em_add(sl, -kl);
@@ -252,19 +253,30 @@ EM_FN float temperature_ref(float e, float kh, float kl, float c, float rc) {
     const float R = em_add(qh, ql);
     const float rem = em_add(ql, -em_add(R, -qh));
     // (no large cancellation, which would magnify the rounding of sl)
-    if (rounds_to(R, rem) && fabsf(kh) < 16.0f * fabsf(sh)) return R;
-    return temperature_slow(e, kh, kl, c);
+    *ok = *ok && rounds_to(R, rem) && fabsf(kh) < 16.0f * fabsf(sh);
+    return R;
+}
+EM_FN float temperature_ref(float e, float kh, float kl, float c, float rc) {
+    bool ok = true;
+    const float R = temperature_plain(e, kh, kl, c, rc, &ok);
+    return ok ? R : temperature_slow(e, kh, kl, c);
 }
 
 // (float)(0.5 * D(a) * (1.0 - D(t)))
-EM_FN float z2_ref(float a, float t) {
+EM_FN float z2_plain(float a, float t, bool* ok) {
     float wl;
     const float wh = two_sum(1.0f, -t, wl);
     const float ph = em_mul(a, wh);
     const float pl = em_fma(a, wl, em_fma(a, wh, -ph));
     const float R = em_add(ph, pl);
     const float rem = em_add(pl, -em_add(R, -ph));
-    return rounds_to(R, rem) ? em_mul(0.5f, R) : z2_slow(a, t);
+    *ok = *ok && rounds_to(R, rem);
+    return em_mul(0.5f, R);
+}
+EM_FN float z2_ref(float a, float t) {
+    bool ok = true;
+    const float z = z2_plain(a, t, &ok);
+    return ok ? z : z2_slow(a, t);
 }
 
 // (float)(D(u) - D(c) * D(s)) for a float c (the product is exact in double)

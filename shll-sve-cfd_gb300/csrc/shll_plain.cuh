@@ -301,17 +301,23 @@ __device__ __forceinline__ int cell1_lanes(const Gas<double>& g, double u, doubl
 __device__ __forceinline__ int cell1(const Gas<float>& g, const float u[3], float fp[3], float fm[3]) {
     const float y = exact_math::reciprocal_plain(u[0], exact_math::em_rcp(u[0]));
     const float p1 = exact_math::divide_plain(u[1], u[0], y), e = exact_math::divide_plain(u[2], u[0], y);
-    const float p2 = temp1(g, e, p1), x = g.gR * p2;
+    // A rounding that the FP32 forms leave open takes the general functions, too: one branch at the end
+    // and none in the chain (1024 cells: 0.44 -> 0.40 us a step, second order 0.77 -> 0.73; the same in
+    // Cell2<float> gains nothing: 512 x 480 cells, second order, 14.0 us both, 301 x 277 7.6 -> 7.8).
+    bool ok = true;
+    const float kh = __fmul_rn(p1, p1);
+    const float p2 = exact_math::temperature_plain(e, 0.5f * kh, 0.5f * __fmaf_rn(p1, p1, -kh), g.CV, g.rCV, &ok);
+    const float x = g.gR * p2;
     float ya;
     const float a = exact_math::square_root_plain(x, &ya);
     const float M = exact_math::divide_plain(p1, a, exact_math::reciprocal_plain(a, ya));
-    const float Z1 = half_sum(M, 1.f), Z3 = half_sum(M, -1.f), Z2 = z2(a, M);
+    const float Z1 = half_sum(M, 1.f), Z3 = half_sum(M, -1.f), Z2 = exact_math::z2_plain(a, M * M, &ok);
     const float P = times_R(g, u[0]) * p2;
     const float F[3] = {u[1], u[1] * p1 + P, p1 * (u[2] + P)};
 #pragma unroll
     for (int k = 0; k < 3; k++) { fp[k] = F[k] * Z1 + u[k] * Z2; fm[k] = -F[k] * Z3 - u[k] * Z2; }
     // (a divisor of all-ones significand is the exception of the residual step)
-    if (g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[2], 87, 80) && momentum_plain(u[1]) &&
+    if (ok && g.plain && in_range(u[0], 97, 60) && !all_ones(u[0]) && in_range(u[2], 87, 80) && momentum_plain(u[1]) &&
         in_range(x, 87, 80) && !all_ones(a))
         return 0;
     const auto c = cell1_general(g, u[0], u[1], u[2]);
