@@ -440,11 +440,19 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
         if (w >= L) return false;
         return ORDER == 2 ? (w < L - 1 || i == n - 1) : (i < n - 1 && w < L - 1);
     };
-    // lam per lane and side, 0 where the interface is not applied (the mask folded into lam)
+    // lam per lane and side, 0 where the interface is not applied (the mask folded into lam).  The
+    // interface between the two cells is one value: lane x's right one and, where lane y holds a cell,
+    // lane y's left one (lamin, lamlin: lane x's left one alone)
+    const float lamin = in_ok(w0) ? lamh : 0.f, lamlin = in_ok(w0) ? laml : 0.f;
     const float2 lin2 = make_float2(in_ok(w0) ? lamh : 0.f, in_ok(w0 + 1) ? lamh : 0.f);
     const float2 lout2 = make_float2(out_ok(w0) ? lamh : 0.f, out_ok(w0 + 1) ? lamh : 0.f);
     const float2 llin2 = make_float2(in_ok(w0) ? laml : 0.f, in_ok(w0 + 1) ? laml : 0.f);
     const float2 llout2 = make_float2(out_ok(w0) ? laml : 0.f, out_ok(w0 + 1) ? laml : 0.f);
+    const bool two = ORDER == 1 || w0 + 1 < L;   // (first order: the mask of lane x's right interface says so)
+    // One value instead of two saves FP32 issue time, which bounds sweeps of several blocks per SM (2^20
+    // cells: first order 6.02 -> 5.86 us a step, second 9.21 -> 8.76), but selecting it for lane y
+    // lengthens the chain, which bounds a resident sweep (65536 cells, second order: 0.855 -> 0.896 us)
+    constexpr bool kPackIn = RES && ORDER == 2;
     // first-order reflective walls: lane q is cell 0 or n-1 (a few threads)
     bool wallq[2];
 #pragma unroll
@@ -503,9 +511,10 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
             for (int k = 0; k < 3; k++) {
                 const FF2 pL = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jl]), *at(sfpl, b, k, jl)};  // fp_{w0-2}, fp_{w0-1}
                 const FF2 mR = {*reinterpret_cast<const float2*>(&S.sfm[b][k][jr]), *at(sfml, b, k, jr)};  // fm_{w0+2}, fm_{w0+3}
-                FF2 IN, OUT;
+                FFS IN;   // lane x's left interface (lane y's is OUT's lane x)
+                FF2 OUT;
                 if constexpr (ORDER == 1) {
-                    IN = ffadd_u({make_float2(pL.h.y, fp[k].h.x), make_float2(pL.l.y, fp[k].l.x)}, fm[k]);
+                    IN = ffadd_u(FFS{pL.h.y, pL.l.y}, FFS{fm[k].h.x, fm[k].l.x});
                     OUT = ffadd_u(fp[k], {make_float2(fm[k].h.y, mR.h.x), make_float2(fm[k].l.y, mR.l.x)});
                 } else {  // the FP32 step's reconstruction (see below), in pairs
                     const FF2 pR = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jr]), *at(sfpl, b, k, jr)};  // fp_{w0+2}
@@ -530,17 +539,19 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                     const FF2 Ro = ffadd(fm[k], {mul2(nhm, sm.h), mul2(nhm, sm.l)});
                     const float2 fe = make_float2(hpl, nhmr);
                     const FF2 Le = ffadd({make_float2(fplh, fmrh), make_float2(fpll, fmrl)}, {mul2(fe, se.h), mul2(fe, se.l)});
-                    IN = ffadd_u({make_float2(Le.h.x, Lo.h.x), make_float2(Le.l.x, Lo.l.x)}, Ro);
+                    IN = ffadd_u(FFS{Le.h.x, Le.l.x}, FFS{Ro.h.x, Ro.l.x});
                     OUT = ffadd_u(Lo, {make_float2(Ro.h.y, Le.h.y), make_float2(Ro.l.y, Le.l.y)});
                 }
-                FF2 tin, tout;
+                FFS ti;
+                FF2 tout;
                 if (LAM_POW2) {  // lam a power of two (or 0 where masked): exact scaling
-                    tin = {mul2(lin2, IN.h), mul2(lin2, IN.l)};
+                    ti = {__fmul_rn(lamin, IN.h), __fmul_rn(lamin, IN.l)};
                     tout = {mul2(lout2, OUT.h), mul2(lout2, OUT.l)};
                 } else {
-                    tin = ffmul_u(IN, {lin2, llin2});
+                    ti = ffmul_u(IN, FFS{lamin, lamlin});
                     tout = ffmul_u(OUT, {lout2, llout2});
                 }
+                const FF2 tin = {make_float2(ti.h, two ? tout.h.x : 0.f), make_float2(ti.l, two ? tout.l.x : 0.f)};
                 FF2 v = ffadd({dh[k], dl[k]}, ffsub(tin, tout));
                 if (any_wall && k == 1) {  // (the wall's own interface is masked out of tin / tout)
 #pragma unroll
@@ -587,15 +598,16 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
             *reinterpret_cast<float2*>(&S.sfm[b][k][w0]) = fm[k];
         }
         __syncthreads();
-        // ---- interfaces w0-1/2 (IN.x), w0+1/2 (IN.y = OUT.x), w0+3/2 (OUT.y) ----
+        // ---- interfaces w0-1/2 (IN), w0+1/2 (OUT.x), w0+3/2 (OUT.y) ----
         float2 ihk[3], ohk[3], ilk[3], olk[3];  // applied terms (for the boundary records)
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const float2 pL = *reinterpret_cast<const float2*>(&S.sfp[b][k][jl]);  // fp_{w0-2}, fp_{w0-1}
             const float2 mR = *reinterpret_cast<const float2*>(&S.sfm[b][k][jr]);  // fm_{w0+2}, fm_{w0+3}
+            // Lane y's left interface is OUT's lane x: only lane x's is summed (kPackIn: both)
             float2 IN, OUT;
             if (ORDER == 1) {
-                IN = add2(make_float2(pL.y, fp[k].x), fm[k]);
+                IN = f2(__fadd_rn(pL.y, fm[k].x));
                 OUT = add2(fp[k], make_float2(fm[k].y, mR.x));
             } else {
                 const float2 pR = *reinterpret_cast<const float2*>(&S.sfp[b][k][jr]);  // fp_{w0+2}
@@ -614,14 +626,24 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                 const float Ll = __fmaf_rn(hpl, slope_s<LIM>(dpl, dpo.x, tp.alpha), fpl);       // j = w0-1
                 const float2 Ro = fma2(nhm, slope2<LIM>(dmo, dmr, tp.alpha), fm[k]);          // j = w0, w0+1
                 const float Rr = __fmaf_rn(nhmr, slope_s<LIM>(dmr.y, dmrr, tp.alpha), fmr);     // j = w0+2
-                IN = add2(make_float2(Ll, Lo.x), Ro);
+                if constexpr (kPackIn) IN = add2(make_float2(Ll, Lo.x), Ro);
+                else IN = f2(__fadd_rn(Ll, Ro.x));
                 OUT = add2(Lo, make_float2(Ro.y, Rr));
             }
-            const float2 ih = mul2(lin2, IN), oh = mul2(lout2, OUT);
-            float2 il = f2(0.f), ol = f2(0.f);
-            if (!LAM_POW2) {
-                il = add2(fma2(lin2, IN, neg2(ih)), mul2(llin2, IN));
-                ol = add2(fma2(lout2, OUT, neg2(oh)), mul2(llout2, OUT));
+            float2 ih, oh, il = f2(0.f), ol = f2(0.f);
+            if constexpr (kPackIn) {
+                ih = mul2(lin2, IN); oh = mul2(lout2, OUT);
+                if (!LAM_POW2) {
+                    il = add2(fma2(lin2, IN, neg2(ih)), mul2(llin2, IN));
+                    ol = add2(fma2(lout2, OUT, neg2(oh)), mul2(llout2, OUT));
+                }
+            } else {
+                oh = mul2(lout2, OUT);
+                ih = make_float2(__fmul_rn(lamin, IN.x), two ? oh.x : 0.f);
+                if (!LAM_POW2) {
+                    ol = add2(fma2(lout2, OUT, neg2(oh)), mul2(llout2, OUT));
+                    il = make_float2(__fmaf_rn(lamlin, IN.x, __fmaf_rn(lamin, IN.x, -ih.x)), two ? ol.x : 0.f);
+                }
             }
             two_sum_acc2(dh[k], dl[k], ih);
             two_diff_acc2(dh[k], dl[k], oh);
@@ -758,9 +780,12 @@ __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
 // The pair-flux form of a first-order sweep, launched after the FP32 form for the same chunks
 // (each block runs its chunk only when the chunk's pair-flux decision calls for it).  Its own
 // kernel so that the longer double-FP32 step does not raise the register count, and so lower the
-// occupancy, of the FP32 sweeps.
+// occupancy, of the FP32 sweeps.  It is bound by FP32 issue and the barrier of each step: three blocks
+// per SM fit without spills in first order (2^20 cells with the pair flux everywhere: 17.8 -> 16.7 us a
+// step, with the shared interface sums and packed subtracts of the step), but not in second, where it
+// runs only when asked for everywhere.
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
-__global__ void __launch_bounds__(MT, 2) k_sweep1d_ff(SweepArgs A) {
+__global__ void __launch_bounds__(MT, ORDER == 1 ? 3 : 2) k_sweep1d_ff(SweepArgs A) {
     __shared__ Smem1 S;
     const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
     const TubeP tp = A.tubes[ch.tube];

@@ -248,7 +248,6 @@ struct FF2 {
     float2 h, l;
 };
 __device__ __forceinline__ FF2 ffv(float h, float l) { return {f2(h), f2(l)}; }
-__device__ __forceinline__ FF2 ffneg(FF2 a) { return {neg2(a.h), neg2(a.l)}; }
 // a * s for a power of two s (exact)
 __device__ __forceinline__ FF2 ffscale(FF2 a, float s) { return {mul2(a.h, f2(s)), mul2(a.l, f2(s))}; }
 // renormalisation of p + e with |e| small against |p|
@@ -268,7 +267,28 @@ __device__ __forceinline__ FF2 ffadd(FF2 a, FF2 b) {
     const FF2 t = ffadd_u(a, b);
     return ffnorm(t.h, t.l);
 }
-__device__ __forceinline__ FF2 ffsub(FF2 a, FF2 b) { return ffadd(a, ffneg(b)); }
+// ffadd(a, -b), written with packed subtracts: a packed operand's negation is not folded, it costs an
+// instruction per lane
+__device__ __forceinline__ FF2 ffsub(FF2 a, FF2 b) {
+    const float2 s = sub2(a.h, b.h);
+    const float2 bp = sub2(s, a.h);
+    const float2 e = sub2(sub2(a.h, sub2(s, bp)), add2(b.h, bp));
+    return ffnorm(s, add2(e, sub2(a.l, b.l)));
+}
+// one lane (a scalar instruction takes half the issue time of a packed one)
+struct FFS {
+    float h, l;
+};
+__device__ __forceinline__ FFS ffadd_u(FFS a, FFS b) {
+    const float s = __fadd_rn(a.h, b.h);
+    const float bp = __fadd_rn(s, -a.h);
+    const float e = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(s, -bp)), __fadd_rn(b.h, -bp));
+    return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
+}
+__device__ __forceinline__ FFS ffmul_u(FFS a, FFS b) {
+    const float p = __fmul_rn(a.h, b.h);
+    return {p, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.h, b.h, -p)))};
+}
 // product left unnormalised, (p, e) with |e| <= about 2^-22 |p|; for products that feed a sum or
 // another product, which renormalise
 __device__ __forceinline__ FF2 ffmul_u(FF2 a, FF2 b) {
