@@ -2,7 +2,7 @@
 """Benchmark of the SHLL Euler hot path on one GB300 (or N independent replicas under torchrun).
 
 Metric: cell-updates/s of the FP32-flux / FP64-accumulate solver (SHLL_PREC_MIXED_F64), next to
-the plain FP64 path (one launch per time step), with the L1 error against FP64 and the fraction of
+the plain FP64 path (1D tubes several time steps per launch, else one launch per step), with the L1 error against FP64 and the fraction of
 the HBM roofline (algorithmic bytes per cell-update: 48 in 1D = 3 FP64 conserved values read and
 written once, 64 in 2D).
 
@@ -465,8 +465,9 @@ def measure(shll, torch, stream, workload, cells, order, args, steps, W, dist, w
     # CUDA-event time, i.e. per launch of the run's kernels over their average launch duration
     hbm, peak_kind = peaks()
     bytes_per_cu = 64.0 if prob.dim == 2 else 48.0
+    plane = "k_step2" if not precision.startswith("mixed") else "k_step2d" if any(k.startswith("1/") for k in prob.tuning() or {}) else "k_step2d2"
     kernel = {"sod1d": "k_tube1d" if launches <= 3 * steps else "k_sweep1d", "batch1d": "k_sweep1d",
-              "circle2d": "k_step2d", "batch2d": "k_step2d",
+              "circle2d": plane, "batch2d": plane,
               "omp2d": "k_step2d_o2" if precision.startswith("mixed") else "k_step2"}[workload]
     achieved = bytes_per_cu * prob.cu * steps / t_total / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
@@ -698,7 +699,7 @@ def pair_flux_run(shll, torch, stream, prob, f64_out, t_run, runs=3):
 
 
 def fp64_comparison(shll, torch, stream, prob, args, cells, order, mixed_out, t_run):
-    """Plain FP64 path (one launch per step) on the same workload (or a seeded subsample for the
+    """Plain FP64 path on the same workload (or a seeded subsample for the
     batches): throughput, L1 of the mixed result against it, CPU baseline."""
     out = {}
     if prob.batch:
@@ -781,7 +782,8 @@ def fp64_comparison(shll, torch, stream, prob, args, cells, order, mixed_out, t_
     ctx.close()
     l1 = np.mean(np.abs(mixed_out - f64_out), axis=1)
     names = ["rho", "u", "v", "T"] if prob.dim == 2 else ["rho", "u", "T"]
-    out["fp64_plain"] = {"value": prob.cu / t64, "unit": "cell-updates/s", "schedule": "one launch per step",
+    out["fp64_plain"] = {"value": prob.cu / t64, "unit": "cell-updates/s",
+                         "schedule": "several steps per launch" if p64.dim == 1 else "one launch per step",
                          "precision": prec64}
     out["speedup_vs_fp64_plain"] = (prob.cu / t_run) / (prob.cu / t64)
     out["l1_vs_fp64"] = dict(zip(names, [float(x) for x in l1]))

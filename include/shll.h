@@ -126,9 +126,9 @@ int shll_init_state(shll_ctx* ctx);
  * Allocate_and_Init_Memory writes them into its globals). */
 int shll_initial_primitives(const shll_params* p, double* rho, double* u, double* v, double* T);
 /* Replaces the primitives (host arrays of nx*ny doubles; v ignored in 1D) and recomputes U and
- * P as shll_init_state does; SHLL_ERR_ARG if a density or temperature is not positive.  In the
- * mixed modes the arrays are copied as given (at full link speed from pinned host memory) and
- * converted on the device; shll_get_primitives likewise converts on the device. */
+ * P as shll_init_state does; SHLL_ERR_ARG if a density or temperature is not positive.  The arrays
+ * are copied as given (at full link speed from pinned host memory), checked and converted on the
+ * device; shll_get_primitives likewise converts on the device. */
 int shll_set_primitives(shll_ctx* ctx, const double* rho, const double* u, const double* v,
                         const double* T);
 int shll_compute_U_from_P(shll_ctx* ctx);   /* base_shll.c:74-85 */
@@ -256,8 +256,8 @@ void shll_set_graph_replay(int on);
 
 /* Resident runs (no counterpart in the reference): a mixed-precision 1D run whose chunks fit on
  * the GPU at once (one block per multiprocessor: a tube of up to about 68000 cells at the default
- * sweep length) and share one scheme variant is one cooperative launch in which every chunk
- * waits, with a bounded wait, only for its two neighbours' previous sweep, and keeps its frame
+ * sweep length; fewer chunks are split into parts of a block each) and share one scheme variant is
+ * one cooperative launch in which every chunk waits, with a bounded wait, only for its two neighbours' previous sweep, and keeps its frame
  * and its cells' FP32 pairs on chip between the sweeps of a fold window.  Results are identical
  * to the one-launch-per-sweep schedule.  on = 0 selects that schedule for every run (default 1;
  * process-wide).  A wait that gives up makes the run return SHLL_ERR_TIMEOUT. */
@@ -284,10 +284,10 @@ void shll_set_pair_flux(int on);
  * (default 0, a measured alternative; process-wide). */
 void shll_set_cluster_runs(int on);
 
-/* Test hook (no counterpart in the reference): in resident runs the chunk with this index (chunks
- * are numbered along the tubes from 0) never publishes its progress, so its neighbours' bounded
- * waits run out and the run returns SHLL_ERR_TIMEOUT; -1 (the default) switches it off.
- * Process-wide. */
+/* Test hook (no counterpart in the reference): in resident runs (mixed ones and plain 1D ones) the
+ * chunk, or part of a chunk, with this index (numbered along the tubes from 0) never publishes its
+ * progress, so its neighbours' bounded waits run out and the run returns SHLL_ERR_TIMEOUT; -1 (the
+ * default) switches it off.  Process-wide. */
 void shll_debug_stall_chunk(int chunk);
 
 /* ---- the reference's own entry points on a process-wide default context ----

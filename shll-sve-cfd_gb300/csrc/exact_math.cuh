@@ -3,9 +3,9 @@
 //
 // GB300 executes FP64 arithmetic, comparisons and conversions at 1.68 lanes per clock per SM (one
 // warp instruction every 19 clocks per SM, 64 clocks of latency), 32-bit integer operations at about
-// 108.  A compiled FP64 division or square root is a sequence of 9-10 FP64 instructions (600 clocks
-// of latency); the integer forms here are about 60 integer operations (about 250 clocks), with the
-// same correctly rounded results bit for bit.  They are long division / digit-by-digit square root in
+// 108.  An FP64 division or square root on the FP64 pipe takes about 600 clocks (measured), as long as nine
+// dependent FP64 operations; the integer forms here are about 60 integer operations (about 250 clocks),
+// with the same correctly rounded results bit for bit.  They are long division / digit-by-digit square root in
 // a large radix (Knuth, TAOCP vol. 2, 4.3.1): a first partial result of 30 bits from a 32-bit
 // reciprocal (Newton's iteration on the FP32 seed), the exact 64-bit remainder, a second partial
 // result of 23 bits, and a final correction by the sign of the exact remainder.

@@ -205,7 +205,7 @@ struct ResPlan {
 // of 19 clocks for order 1, 70 + 12 for order 2), plus the exchange (about 4500 clocks) over the S steps
 // it serves.  A narrower window means less redundant work per step, a wider one fewer exchanges.
 // Measured, us a step with 32 / 64 / 96 / 128 / 256 / 512 threads at 1024 cells: FP64 first order 1.70 /
-// 1.64 / 1.62 / 1.66 / 2.10 / 3.11, float 0.53 / 0.47 / 0.45 / 0.44 / 0.45 / 0.51.
+// 1.64 / 1.62 / 1.66 / 2.10 / 3.11, float 0.53 / 0.47 / 0.45 / 0.44 / 0.45 / 0.51 (0.40 with the present cell1).
 template <typename REAL, int ORDER>
 static ResPlan res_plan(int n, long steps, int sms) {
     const bool wide = sizeof(REAL) == 8;

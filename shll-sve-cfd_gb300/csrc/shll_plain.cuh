@@ -91,9 +91,10 @@ __host__ Gas<REAL> make_gas(const PlainArgs& a) {
 // ---- the reference's expressions, FP64 ----
 // FP64 instructions are the scarce resource of these kernels (19 clocks per warp instruction per
 // SM), so divisions, square roots, comparisons and power-of-two scalings run on the integer pipes
-// (exact_math.cuh) with the same results; the float arithmetic does without FP64.  Measured: one
-// 2D step of 256 x 256 cells in FP64 40.3 -> 25.9 us, of 301 x 277 in float (second order) 29.5 ->
-// 13.4 us, one 1D step of 3001 cells (FP64, second order) 20.5 -> 16.4 us.
+// (exact_math.cuh) with the same results; the float arithmetic does without FP64.  Measured, by
+// itself: one 2D step of 256 x 256 cells in FP64 40.3 -> 25.9 us, of 301 x 277 in float (second order)
+// 29.5 -> 13.4 us, one 1D step of 3001 cells (FP64, second order) 20.5 -> 16.4 us; with the tile kernel
+// and the 1D runs of plain_resident.cuh these are 13.7, 7.6 and 2.4 us.
 __device__ __forceinline__ double half_of(double x) { return exact_math::scale_pow2(x, -1, 0.5); }
 __device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
 // 0.5 * (x + c) (the scaling is exact: one fused operation rounds like the sum)
