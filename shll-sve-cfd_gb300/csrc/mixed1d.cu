@@ -37,6 +37,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "exact_math.cuh"
@@ -241,7 +242,9 @@ __device__ __forceinline__ T ldx(const T* p) {
 // taken from dh/dl (this thread's registers after the previous sweep of the same geometry)
 // instead of memory; keep: the next sweep will do so, so only the cells that the neighbours read
 // as halo are stored.
-template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, bool RES, bool FF = false>
+// CELLS: cells per thread, two as the lanes of FP32x2 registers, or one (resident runs of small windows:
+// lane x alone, in scalar instructions, which take half the issue time).
+template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, bool RES, bool FF = false, int CELLS = 2>
 __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch, const TubeP& tp, Smem1& S,
                             float2 (&dh)[3], float2 (&dl)[3], const bool reuse, const bool keep) {
     constexpr int R_ = ORDER;  // stencil reach per step
@@ -291,16 +294,16 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     const double lam = tp.lam;
     const float lamh = (float)lam, laml = (float)(lam - (double)lamh);
 
-    if (L > 2 * (int)blockDim.x || tp.B > MW / 16 || tp.B < 1) {  // host guarantees this never happens; refuse rather than overrun
+    if (L > CELLS * (int)blockDim.x || tp.B > MW / 16 || tp.B < 1) {  // host guarantees this never happens; refuse rather than overrun
         if (tid == 0) atomicOr(A.flag, SHLL_FLAG_BADARG);
         return;
     }
     // the window's stored values, loaded first so that their latency overlaps the frame setup
-    const int w0 = 2 * tid;
+    const int w0 = CELLS * tid;
     double uin[2][3];           // FP64 state (window start)
     float uh[2][3], ul[2][3];   // FP32 value + compensation (KAHAN window start), or deviation pair
 #pragma unroll
-    for (int q = 0; q < 2; q++)
+    for (int q = 0; q < CELLS; q++)
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             uin[q][k] = 0.0; uh[q][k] = 0.f; ul[q][k] = 0.f;
@@ -388,7 +391,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
 
     // ---- the window as deviations from the frame ----
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < CELLS; q++) {
         const int w = w0 + q;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -411,7 +414,8 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
             set_lane(dl[k], q, l);
         }
     }
-    const Coef2 c2 = coef2(frp->c);
+    using V = std::conditional_t<CELLS == 2, float2, float>;
+    const auto c2 = coef2<V>(frp->c);
     const bool hasL = ch.idL >= 0, hasR = ch.idR >= 0;
     // loop-invariant roles of this thread's cells (i = tube cell of window cell w)
     auto edge = [&](int w) { const int i = ws + w; return i <= 0 || i >= n - 1; };
@@ -420,7 +424,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     const float2 hp = make_float2(edge(w0) ? 0.f : 0.5f, edge(w0 + 1) ? 0.f : 0.5f);
     const float2 nhm = neg2(hp);
     const float hpl = edge(w0 - 1) ? 0.f : 0.5f;    // cell w0 - 1 (sp only)
-    const float nhmr = edge(w0 + 2) ? -0.f : -0.5f; // cell w0 + 2 (sm only)
+    const float nhmr = edge(w0 + CELLS) ? -0.f : -0.5f; // cell w0 + CELLS (sm only)
     // Second order (outflow walls, base-c/2nd_order_base_shll.c:236-262): the wall flux is the
     // cell's own flux fp + fm, i.e. the regular interface formula with a ghost cell that copies
     // the wall cell (fp_{-1} = fp_0, fm_n = fm_{n-1}, zero slopes), so walls need no special
@@ -454,19 +458,20 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     // lengthens the chain, which bounds a resident sweep (65536 cells, second order: 0.855 -> 0.896 us)
     constexpr bool kPackIn = RES && ORDER == 2;
     // first-order reflective walls: lane q is cell 0 or n-1 (a few threads)
-    bool wallq[2];
+    bool wallq[2] = {false, false};
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < CELLS; q++) {
         const int w = w0 + q, i = ws + w;
         wallq[q] = ORDER == 1 && w < L && (i == 0 || i == n - 1);
     }
     const bool any_wall = wallq[0] || wallq[1];
     // chunk-boundary records: the terms applied at interface a-1/2 (cell a's left) and b-1/2
     // (cell b-1's right) are stored per step and summed at the end of the sweep
-    const bool rin0 = hasL && w0 == pa, rin1 = hasL && w0 + 1 == pa;
-    const bool rout0 = hasR && w0 == pb - 1, rout1 = hasR && w0 + 1 == pb - 1;
+    const bool rin0 = hasL && w0 == pa, rin1 = CELLS == 2 && hasL && w0 + 1 == pa;
+    const bool rout0 = hasR && w0 == pb - 1, rout1 = CELLS == 2 && hasR && w0 + 1 == pb - 1;
     const bool any_rec = rin0 || rin1 || rout0 || rout1;
-    const int jl = max(w0 - 2, 0), jr = min(w0 + 2, 2 * (int)blockDim.x - 2);  // neighbour pairs (clamped)
+    const int jl = max(w0 - 2, 0), jr = min(w0 + 2, CELLS * ((int)blockDim.x - 1));  // neighbour pairs (clamped)
+    const int il1 = max(w0 - 1, 0), ir1 = min(w0 + 1, (int)blockDim.x - 1);          // CELLS 1: neighbours (jl, jr: the next)
 
     if constexpr (FF) {
         // The same step in double-FP32 arithmetic: each cell's state U = U* + (dh + dl) as a pair,
@@ -484,7 +489,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
         for (int s = 0; s < steps; s++) {
             const int b = s & 1;
             FF2 fp[3], fm[3];
-            {
+            if constexpr (CELLS == 2) {
                 FF2 U[3];
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
@@ -494,7 +499,28 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                     U[k] = ffadd(ffv(frp->Uh[k], frp->Ul[k]), d);
                 }
                 flux1x2_ff(U, gg1, gm1, fp, fm);
+            } else {
+                static_assert(CELLS == 2 || ORDER == 1, "one cell per thread: first order");
+                FFS U[3], p[3], m[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const FFS d = ffnorm(dh[k].x, dl[k].x);
+                    dh[k].x = d.h;
+                    dl[k].x = d.l;
+                    U[k] = ffadd(FFS{frp->Uh[k], frp->Ul[k]}, d);
+                }
+                flux1x2_ff(U, FFS{tp.gg1p[0], tp.gg1p[1]}, FFS{tp.gm1p[0], tp.gm1p[1]}, p, m);
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    S.sfp[b][k][w0] = p[k].h;
+                    S.sfm[b][k][w0] = m[k].h;
+                    *reinterpret_cast<float*>(at(sfpl, b, k, w0)) = p[k].l;
+                    *reinterpret_cast<float*>(at(sfml, b, k, w0)) = m[k].l;
+                    fp[k] = ffv(p[k].h, p[k].l);
+                    fm[k] = ffv(m[k].h, m[k].l);
+                }
             }
+            if constexpr (CELLS == 2)
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 if (grx) {  // ghost fm_n of the right outflow wall (lane y holds no cell)
@@ -509,59 +535,72 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                const FF2 pL = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jl]), *at(sfpl, b, k, jl)};  // fp_{w0-2}, fp_{w0-1}
-                const FF2 mR = {*reinterpret_cast<const float2*>(&S.sfm[b][k][jr]), *at(sfml, b, k, jr)};  // fm_{w0+2}, fm_{w0+3}
-                FFS IN;   // lane x's left interface (lane y's is OUT's lane x)
-                FF2 OUT;
-                if constexpr (ORDER == 1) {
-                    IN = ffadd_u(FFS{pL.h.y, pL.l.y}, FFS{fm[k].h.x, fm[k].l.x});
-                    OUT = ffadd_u(fp[k], {make_float2(fm[k].h.y, mR.h.x), make_float2(fm[k].l.y, mR.l.x)});
-                } else {  // the FP32 step's reconstruction (see below), in pairs
-                    const FF2 pR = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jr]), *at(sfpl, b, k, jr)};  // fp_{w0+2}
-                    const FF2 mL = {*reinterpret_cast<const float2*>(&S.sfm[b][k][jl]), *at(sfml, b, k, jl)};  // fm_{w0-1}
-                    // fp_{w0-1} (ghost of the left wall: fp_0) and fm_{w0+2} (ghost of the right wall: fm_{n-1})
-                    const float fplh = gl ? fp[k].h.x : pL.h.y, fpll = gl ? fp[k].l.x : pL.l.y;
-                    const float fmrh = gry ? fm[k].h.y : mR.h.x, fmrl = gry ? fm[k].l.y : mR.l.x;
-                    // differences f_j - f_{j-1}
-                    const FF2 dpo = ffsub(fp[k], {make_float2(fplh, fp[k].h.x), make_float2(fpll, fp[k].l.x)});  // j = w0, w0+1
-                    const FF2 dpr = ffsub({make_float2(fp[k].h.y, pR.h.x), make_float2(fp[k].l.y, pR.l.x)}, fp[k]);  // j = w0+1, w0+2
-                    const FF2 dmo = ffsub(fm[k], {make_float2(mL.h.y, fm[k].h.x), make_float2(mL.l.y, fm[k].l.x)});
-                    const FF2 dmr = ffsub({make_float2(fm[k].h.y, fmrh), make_float2(fm[k].l.y, fmrl)}, fm[k]);
-                    // lane x: fp_{w0-1} - fp_{w0-2}; lane y: fm_{w0+3} - fm_{w0+2}
-                    const FF2 dedge = ffsub({make_float2(fplh, mR.h.y), make_float2(fpll, mR.l.y)},
-                                            {make_float2(pL.h.x, fmrh), make_float2(pL.l.x, fmrl)});
-                    const FF2 sp = ffslope<LIM>(dpo, dpr, tp.alpha), sm = ffslope<LIM>(dmo, dmr, tp.alpha);
-                    // lane x: the slope of fp at w0-1; lane y: the slope of fm at w0+2
-                    const FF2 se = ffslope<LIM>({make_float2(dedge.h.x, dmr.h.y), make_float2(dedge.l.x, dmr.l.y)},
-                                                {make_float2(dpo.h.x, dedge.h.y), make_float2(dpo.l.x, dedge.l.y)}, tp.alpha);
-                    // reconstructed L_j = fp_j + sp_j/2 and R_j = fm_j - sm_j/2 (factors 0 on edge cells: exact)
-                    const FF2 Lo = ffadd(fp[k], {mul2(hp, sp.h), mul2(hp, sp.l)});
-                    const FF2 Ro = ffadd(fm[k], {mul2(nhm, sm.h), mul2(nhm, sm.l)});
-                    const float2 fe = make_float2(hpl, nhmr);
-                    const FF2 Le = ffadd({make_float2(fplh, fmrh), make_float2(fpll, fmrl)}, {mul2(fe, se.h), mul2(fe, se.l)});
-                    IN = ffadd_u(FFS{Le.h.x, Le.l.x}, FFS{Ro.h.x, Ro.l.x});
-                    OUT = ffadd_u(Lo, {make_float2(Ro.h.y, Le.h.y), make_float2(Ro.l.y, Le.l.y)});
-                }
-                FFS ti;
-                FF2 tout;
-                if (LAM_POW2) {  // lam a power of two (or 0 where masked): exact scaling
-                    ti = {__fmul_rn(lamin, IN.h), __fmul_rn(lamin, IN.l)};
-                    tout = {mul2(lout2, OUT.h), mul2(lout2, OUT.l)};
+                FF2 tin, tout, v;
+                if constexpr (CELLS == 1) {
+                    const FFS IN = ffadd_u(FFS{S.sfp[b][k][il1], *reinterpret_cast<const float*>(at(sfpl, b, k, il1))},
+                                           FFS{fm[k].h.x, fm[k].l.x});
+                    const FFS OUT = ffadd_u(FFS{fp[k].h.x, fp[k].l.x},
+                                            FFS{S.sfm[b][k][ir1], *reinterpret_cast<const float*>(at(sfml, b, k, ir1))});
+                    const FFS ti = LAM_POW2 ? ffscale(IN, lamin) : ffmul_u(IN, FFS{lamin, lamlin});
+                    const FFS to = LAM_POW2 ? ffscale(OUT, lout2.x) : ffmul_u(OUT, FFS{lout2.x, llout2.x});
+                    const FFS x = ffadd(FFS{dh[k].x, dl[k].x}, ffsub(ti, to));
+                    tin = ffv(ti.h, ti.l);
+                    tout = ffv(to.h, to.l);
+                    v = ffv(x.h, x.l);
                 } else {
-                    ti = ffmul_u(IN, FFS{lamin, lamlin});
-                    tout = ffmul_u(OUT, {lout2, llout2});
+                    const FF2 pL = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jl]), *at(sfpl, b, k, jl)};  // fp_{w0-2}, fp_{w0-1}
+                    const FF2 mR = {*reinterpret_cast<const float2*>(&S.sfm[b][k][jr]), *at(sfml, b, k, jr)};  // fm_{w0+2}, fm_{w0+3}
+                    FFS IN;   // lane x's left interface (lane y's is OUT's lane x)
+                    FF2 OUT;
+                    if constexpr (ORDER == 1) {
+                        IN = ffadd_u(FFS{pL.h.y, pL.l.y}, FFS{fm[k].h.x, fm[k].l.x});
+                        OUT = ffadd_u(fp[k], FF2{make_float2(fm[k].h.y, mR.h.x), make_float2(fm[k].l.y, mR.l.x)});
+                    } else {  // the FP32 step's reconstruction (see below), in pairs
+                        const FF2 pR = {*reinterpret_cast<const float2*>(&S.sfp[b][k][jr]), *at(sfpl, b, k, jr)};  // fp_{w0+2}
+                        const FF2 mL = {*reinterpret_cast<const float2*>(&S.sfm[b][k][jl]), *at(sfml, b, k, jl)};  // fm_{w0-1}
+                        // fp_{w0-1} (ghost of the left wall: fp_0) and fm_{w0+2} (ghost of the right wall: fm_{n-1})
+                        const float fplh = gl ? fp[k].h.x : pL.h.y, fpll = gl ? fp[k].l.x : pL.l.y;
+                        const float fmrh = gry ? fm[k].h.y : mR.h.x, fmrl = gry ? fm[k].l.y : mR.l.x;
+                        // differences f_j - f_{j-1}
+                        const FF2 dpo = ffsub(fp[k], FF2{make_float2(fplh, fp[k].h.x), make_float2(fpll, fp[k].l.x)});  // j = w0, w0+1
+                        const FF2 dpr = ffsub(FF2{make_float2(fp[k].h.y, pR.h.x), make_float2(fp[k].l.y, pR.l.x)}, fp[k]);  // j = w0+1, w0+2
+                        const FF2 dmo = ffsub(fm[k], FF2{make_float2(mL.h.y, fm[k].h.x), make_float2(mL.l.y, fm[k].l.x)});
+                        const FF2 dmr = ffsub(FF2{make_float2(fm[k].h.y, fmrh), make_float2(fm[k].l.y, fmrl)}, fm[k]);
+                        // lane x: fp_{w0-1} - fp_{w0-2}; lane y: fm_{w0+3} - fm_{w0+2}
+                        const FF2 dedge = ffsub(FF2{make_float2(fplh, mR.h.y), make_float2(fpll, mR.l.y)},
+                                                FF2{make_float2(pL.h.x, fmrh), make_float2(pL.l.x, fmrl)});
+                        const FF2 sp = ffslope<LIM>(dpo, dpr, tp.alpha), sm = ffslope<LIM>(dmo, dmr, tp.alpha);
+                        // lane x: the slope of fp at w0-1; lane y: the slope of fm at w0+2
+                        const FF2 se = ffslope<LIM>(FF2{make_float2(dedge.h.x, dmr.h.y), make_float2(dedge.l.x, dmr.l.y)},
+                                                    {make_float2(dpo.h.x, dedge.h.y), make_float2(dpo.l.x, dedge.l.y)}, tp.alpha);
+                        // reconstructed L_j = fp_j + sp_j/2 and R_j = fm_j - sm_j/2 (factors 0 on edge cells: exact)
+                        const FF2 Lo = ffadd(fp[k], FF2{mul2(hp, sp.h), mul2(hp, sp.l)});
+                        const FF2 Ro = ffadd(fm[k], FF2{mul2(nhm, sm.h), mul2(nhm, sm.l)});
+                        const float2 fe = make_float2(hpl, nhmr);
+                        const FF2 Le = ffadd(FF2{make_float2(fplh, fmrh), make_float2(fpll, fmrl)}, FF2{mul2(fe, se.h), mul2(fe, se.l)});
+                        IN = ffadd_u(FFS{Le.h.x, Le.l.x}, FFS{Ro.h.x, Ro.l.x});
+                        OUT = ffadd_u(Lo, FF2{make_float2(Ro.h.y, Le.h.y), make_float2(Ro.l.y, Le.l.y)});
+                    }
+                    FFS ti;
+                    if (LAM_POW2) {  // lam a power of two (or 0 where masked): exact scaling
+                        ti = {__fmul_rn(lamin, IN.h), __fmul_rn(lamin, IN.l)};
+                        tout = {mul2(lout2, OUT.h), mul2(lout2, OUT.l)};
+                    } else {
+                        ti = ffmul_u(IN, FFS{lamin, lamlin});
+                        tout = ffmul_u(OUT, FF2{lout2, llout2});
+                    }
+                    tin = {make_float2(ti.h, two ? tout.h.x : 0.f), make_float2(ti.l, two ? tout.l.x : 0.f)};
+                    v = ffadd(FF2{dh[k], dl[k]}, ffsub(tin, tout));
                 }
-                const FF2 tin = {make_float2(ti.h, two ? tout.h.x : 0.f), make_float2(ti.l, two ? tout.l.x : 0.f)};
-                FF2 v = ffadd({dh[k], dl[k]}, ffsub(tin, tout));
                 if (any_wall && k == 1) {  // (the wall's own interface is masked out of tin / tout)
 #pragma unroll
-                    for (int q = 0; q < 2; q++) {
+                    for (int q = 0; q < CELLS; q++) {
                         if (!wallq[q]) continue;
                         const bool left = ws + w0 + q == 0;
                         const float sg = left ? 2.f : -2.f;  // + lam 2 fm1 at cell 0, - lam 2 fp1 at cell n-1
                         const FF2 wf = {f2(sg * lane(left ? fm[1].h : fp[1].h, q)), f2(sg * lane(left ? fm[1].l : fp[1].l, q))};
                         const FF2 t = LAM_POW2 ? ffscale(wf, lamh) : ffmul_u(wf, ffv(lamh, laml));
-                        const FF2 vq = ffadd({f2(lane(v.h, q)), f2(lane(v.l, q))}, t);
+                        const FF2 vq = ffadd(FF2{f2(lane(v.h, q)), f2(lane(v.l, q))}, t);
                         set_lane(v.h, q, vq.h.x);
                         set_lane(v.l, q, vq.l.x);
                     }
@@ -585,12 +624,25 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
         const int b = s & 1;
         // ---- split-flux deviations of both cells ----
         float2 fp[3], fm[3];
-        {
+        if constexpr (CELLS == 2) {
             float2 d[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) d[k] = add2(dh[k], dl[k]);
             dflux1x2(c2, d, fp, fm);
+        } else {
+            float d[3], p[3], m[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) d[k] = add2(dh[k].x, dl[k].x);
+            dflux1x2(c2, d, p, m);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                S.sfp[b][k][w0] = p[k];
+                S.sfm[b][k][w0] = m[k];
+                fp[k] = f2(p[k]);
+                fm[k] = f2(m[k]);
+            }
         }
+        if constexpr (CELLS == 2)
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             if (grx) fm[k].y = fm[k].x;  // ghost fm_n of the right wall (lane y holds no cell)
@@ -602,6 +654,36 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
         float2 ihk[3], ohk[3], ilk[3], olk[3];  // applied terms (for the boundary records)
 #pragma unroll
         for (int k = 0; k < 3; k++) {
+            if constexpr (CELLS == 1) {
+                const float p = fp[k].x, m = fm[k].x;
+                const float pl = gl ? p : S.sfp[b][k][il1], mr = grx ? m : S.sfm[b][k][ir1];   // fp_{w0-1}, fm_{w0+1}
+                float IN, OUT;
+                if (ORDER == 1) {
+                    IN = __fadd_rn(pl, m);
+                    OUT = __fadd_rn(p, mr);
+                } else {
+                    const float dpo = __fadd_rn(p, -pl), dmr = __fadd_rn(mr, -m);
+                    const float Lo = __fmaf_rn(hp.x, slope_s<LIM>(dpo, __fadd_rn(S.sfp[b][k][ir1], -p), tp.alpha), p);
+                    const float Ro = __fmaf_rn(nhm.x, slope_s<LIM>(__fadd_rn(m, -S.sfm[b][k][il1]), dmr, tp.alpha), m);
+                    const float Ll = __fmaf_rn(hpl, slope_s<LIM>(__fadd_rn(pl, -S.sfp[b][k][jl]), dpo, tp.alpha), pl);
+                    const float Rr = __fmaf_rn(nhmr, slope_s<LIM>(dmr, __fadd_rn(S.sfm[b][k][jr], -mr), tp.alpha), mr);
+                    IN = __fadd_rn(Ll, Ro);
+                    OUT = __fadd_rn(Lo, Rr);
+                }
+                const float ih = __fmul_rn(lamin, IN), oh = __fmul_rn(lout2.x, OUT);
+                float il = 0.f, ol = 0.f;
+                if (!LAM_POW2) {
+                    il = __fmaf_rn(lamlin, IN, __fmaf_rn(lamin, IN, -ih));
+                    ol = __fmaf_rn(llout2.x, OUT, __fmaf_rn(lout2.x, OUT, -oh));
+                }
+                float h = dh[k].x, l = dl[k].x;
+                two_sum_acc2(h, l, ih);
+                two_diff_acc2(h, l, oh);
+                if (!LAM_POW2) l = __fadd_rn(l, __fadd_rn(il, -ol));
+                dh[k].x = h; dl[k].x = l;
+                ihk[k] = f2(ih); ohk[k] = f2(oh); ilk[k] = f2(il); olk[k] = f2(ol);
+                continue;
+            }
             const float2 pL = *reinterpret_cast<const float2*>(&S.sfp[b][k][jl]);  // fp_{w0-2}, fp_{w0-1}
             const float2 mR = *reinterpret_cast<const float2*>(&S.sfm[b][k][jr]);  // fm_{w0+2}, fm_{w0+3}
             // Lane y's left interface is OUT's lane x: only lane x's is summed (kPackIn: both)
@@ -662,7 +744,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
         // ---- first-order reflective walls (the threads of cells 0 and n-1) ----
         if (ORDER == 1 && any_wall) {
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
+            for (int q = 0; q < CELLS; q++) {
                 if (!wallq[q]) continue;
                 const int i = ws + w0 + q;
                 const int bnd = i == 0 ? 0 : 1;
@@ -707,7 +789,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     float* dhout = outb ? A.dh[1] : A.dh[0];
     float* dlout = outb ? A.dl[1] : A.dl[0];
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < CELLS; q++) {
         const int w = w0 + q;
         if (w < pa || w >= pb) continue;
         float uf[3];
@@ -869,7 +951,7 @@ __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
 // CLU: the cluster form (k_cluster1d): the chunks of one tube are one thread-block cluster, and the
 // wait between sweeps is the cluster's hardware barrier (release / acquire at cluster scope) instead
 // of the neighbours' progress counters; the data still goes through L2.
-template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, bool CLU>
+template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, bool CLU, int CELLS = 2>
 __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
     __shared__ Smem1 S;
     const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
@@ -905,11 +987,11 @@ __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
         // (FM 1: the neighbours' flags of the previous sweep are visible after the wait above, as
         // they were written before the neighbours' release; block-uniform)
         if constexpr (FM == 2)
-            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, true>(A, sw, ch, tp, S, dh, dl, reuse, keep);
+            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, true, CELLS>(A, sw, ch, tp, S, dh, dl, reuse, keep);
         else if (FM == 1 && A.mode[0] && pair_mode_parts(A, ch, sw))
-            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, FM == 1>(A, sw, ch, tp, S, dh, dl, reuse, keep);
+            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, FM == 1, CELLS>(A, sw, ch, tp, S, dh, dl, reuse, keep);
         else
-            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true>(A, sw, ch, tp, S, dh, dl, reuse, keep);
+            sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, true, false, CELLS>(A, sw, ch, tp, S, dh, dl, reuse, keep);
         __syncthreads();
         // (the barrier orders the block's stores before thread 0's release at GPU scope)
         if (!CLU && threadIdx.x == 0 && ch.id != A.stall_id)
@@ -917,9 +999,10 @@ __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
     }
 }
 
-template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM>
-__global__ void __launch_bounds__(MT, 1) k_tube1d(SweepArgs A, unsigned* prog) {
-    tube_run<ORDER, KAHAN, LAM_POW2, LIM, FM, false>(A, prog);
+constexpr int kOneCellWindow = 320;   // most cells of a window that is computed with one cell per thread
+template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, int CELLS>
+__global__ void __launch_bounds__(CELLS == 1 ? kOneCellWindow : MT, 1) k_tube1d(SweepArgs A, unsigned* prog) {
+    tube_run<ORDER, KAHAN, LAM_POW2, LIM, FM, false, CELLS>(A, prog);
 }
 
 // The cluster form of a resident run (launched with one cluster per tube, all tubes of the launch
@@ -1063,20 +1146,24 @@ static_assert(kPairSmem <= kSoloSmem, "the pair-flux buffers fit in the padding 
 
 // resident form of a run (k_tube1d): a cooperative launch of one block per chunk, each alone on
 // its SM (the same shared-memory padding as single-wave sweeps)
-template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM>
-static cudaError_t launch_res(int grid, int threads, cudaStream_t s, const SweepArgs& A, unsigned* prog, bool check_only) {
+template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, int CELLS = 2>
+static cudaError_t launch_res(int grid, int threads, int cells, cudaStream_t s, const SweepArgs& A, unsigned* prog,
+                              bool check_only) {
+    if constexpr (FM != 2 && CELLS == 2) {
+        if (cells == 1) return launch_res<ORDER, KAHAN, LAM_POW2, LIM, FM, 1>(grid, threads, cells, s, A, prog, check_only);
+    }
     static unsigned long long attr_set = 0;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !(attr_set & (1ull << dev))) {
-        cudaError_t e = cudaFuncSetAttribute(k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM>,
+        cudaError_t e = cudaFuncSetAttribute(k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM, CELLS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloSmem);
         if (e != cudaSuccess) return e;
         attr_set |= 1ull << dev;
     }
     if (check_only) {  // every block must be resident at once
         int per_sm = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM>,
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM, CELLS>,
                                                                       threads, kSoloSmem);
         if (e != cudaSuccess) return e;
         return (long)per_sm * device_sms() >= grid ? cudaSuccess : cudaErrorCooperativeLaunchTooLarge;
@@ -1091,7 +1178,7 @@ static cudaError_t launch_res(int grid, int threads, cudaStream_t s, const Sweep
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM>, A, prog);
+    return cudaLaunchKernelEx(&cfg, k_tube1d<ORDER, KAHAN, LAM_POW2, LIM, FM, CELLS>, A, prog);
 }
 
 // cluster form: grid = the run's chunks, clusters of `csize` consecutive chunks (one tube each)
@@ -1148,34 +1235,34 @@ static cudaError_t launch_cluster(int variant, bool kahan, int grid, int csize, 
 
 // all_pairs: the pair flux everywhere (second order then needs the pair-flux kernel; first order
 // chooses per chunk and sweep either way)
-static cudaError_t launch_resident(int variant, bool kahan, int grid, int threads, cudaStream_t s, const SweepArgs& A,
-                                   unsigned* prog, bool check_only, bool all_pairs) {
+static cudaError_t launch_resident(int variant, bool kahan, int grid, int threads, int cells, cudaStream_t s,
+                                   const SweepArgs& A, unsigned* prog, bool check_only, bool all_pairs) {
     const int v = variant * 2 + (kahan ? 1 : 0);
     if (variant >= 2 && all_pairs) {
         switch (v) {
-            case 4: return launch_res<2, false, true, 0, 2>(grid, threads, s, A, prog, check_only);
-            case 5: return launch_res<2, true, true, 0, 2>(grid, threads, s, A, prog, check_only);
-            case 6: return launch_res<2, false, false, 0, 2>(grid, threads, s, A, prog, check_only);
-            case 7: return launch_res<2, true, false, 0, 2>(grid, threads, s, A, prog, check_only);
-            case 8: return launch_res<2, false, true, 1, 2>(grid, threads, s, A, prog, check_only);
-            case 9: return launch_res<2, true, true, 1, 2>(grid, threads, s, A, prog, check_only);
-            case 10: return launch_res<2, false, false, 1, 2>(grid, threads, s, A, prog, check_only);
-            default: return launch_res<2, true, false, 1, 2>(grid, threads, s, A, prog, check_only);
+            case 4: return launch_res<2, false, true, 0, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 5: return launch_res<2, true, true, 0, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 6: return launch_res<2, false, false, 0, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 7: return launch_res<2, true, false, 0, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 8: return launch_res<2, false, true, 1, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 9: return launch_res<2, true, true, 1, 2>(grid, threads, cells, s, A, prog, check_only);
+            case 10: return launch_res<2, false, false, 1, 2>(grid, threads, cells, s, A, prog, check_only);
+            default: return launch_res<2, true, false, 1, 2>(grid, threads, cells, s, A, prog, check_only);
         }
     }
     switch (v) {
-        case 0: return launch_res<1, false, true, 0, 1>(grid, threads, s, A, prog, check_only);
-        case 1: return launch_res<1, true, true, 0, 1>(grid, threads, s, A, prog, check_only);
-        case 2: return launch_res<1, false, false, 0, 1>(grid, threads, s, A, prog, check_only);
-        case 3: return launch_res<1, true, false, 0, 1>(grid, threads, s, A, prog, check_only);
-        case 4: return launch_res<2, false, true, 0, 0>(grid, threads, s, A, prog, check_only);
-        case 5: return launch_res<2, true, true, 0, 0>(grid, threads, s, A, prog, check_only);
-        case 6: return launch_res<2, false, false, 0, 0>(grid, threads, s, A, prog, check_only);
-        case 7: return launch_res<2, true, false, 0, 0>(grid, threads, s, A, prog, check_only);
-        case 8: return launch_res<2, false, true, 1, 0>(grid, threads, s, A, prog, check_only);
-        case 9: return launch_res<2, true, true, 1, 0>(grid, threads, s, A, prog, check_only);
-        case 10: return launch_res<2, false, false, 1, 0>(grid, threads, s, A, prog, check_only);
-        default: return launch_res<2, true, false, 1, 0>(grid, threads, s, A, prog, check_only);
+        case 0: return launch_res<1, false, true, 0, 1>(grid, threads, cells, s, A, prog, check_only);
+        case 1: return launch_res<1, true, true, 0, 1>(grid, threads, cells, s, A, prog, check_only);
+        case 2: return launch_res<1, false, false, 0, 1>(grid, threads, cells, s, A, prog, check_only);
+        case 3: return launch_res<1, true, false, 0, 1>(grid, threads, cells, s, A, prog, check_only);
+        case 4: return launch_res<2, false, true, 0, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 5: return launch_res<2, true, true, 0, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 6: return launch_res<2, false, false, 0, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 7: return launch_res<2, true, false, 0, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 8: return launch_res<2, false, true, 1, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 9: return launch_res<2, true, true, 1, 0>(grid, threads, cells, s, A, prog, check_only);
+        case 10: return launch_res<2, false, false, 1, 0>(grid, threads, cells, s, A, prog, check_only);
+        default: return launch_res<2, true, false, 1, 0>(grid, threads, cells, s, A, prog, check_only);
     }
 }
 
@@ -1859,14 +1946,25 @@ static bool ensure_side_streams(MixedState* m, int count) {
     return true;
 }
 
-// threads of a resident block: two cells each over the widest window
-static int resident_threads(MixedState* m, const std::vector<Chunk>& order) {
+// cells of a resident block's widest window
+static int resident_window(MixedState* m, const std::vector<Chunk>& order) {
     int cells = 0;
     for (const Chunk& c : order) {
         const TubeP& tp = m->tubes[c.tube];
         cells = std::max(cells, c.sb - c.sa + 2 * tp.order * tp.B);
     }
-    return std::min(MT, std::max(64, (cells / 2 + 1 + 31) / 32 * 32));
+    return cells;
+}
+// Cells per thread.  A scalar FP32 instruction takes half the issue time of a packed one, so in a window
+// of one or two warps to a scheduler one cell per thread shortens the step (us a step, first / second
+// order: 10007 cells 1.40 -> 1.15 / 0.66 -> 0.58, 2048 cells 1.40 -> 1.16 / 0.66 -> 0.47, 32768 cells,
+// windows of 270 / 285 cells, 1.63 -> 1.49 / 0.83 -> 0.70); a window of 512 cells is bound by issue, of
+// which two cells per thread need less (65536 cells: 1.64 against 1.73 / 0.855 against 0.862).  No window of
+// a default run lies between 288 and 480 cells.
+static int resident_cells(int window, bool all_pairs) { return window <= kOneCellWindow && !all_pairs ? 1 : 2; }
+// threads over the window
+static int resident_threads(int window, int cells) {
+    return std::min(cells == 1 ? kOneCellWindow : MT, std::max(64, (cells == 1 ? window + 31 : window / 2 + 1 + 31) / 32 * 32));
 }
 
 // issues the launches of one run on m->stream: the sweeps of every variant group (or, resident,
@@ -1921,9 +2019,11 @@ static cudaError_t issue_run(MixedState* m, const std::vector<Chunk>& order, lon
         A.chunk0 = 0;
         cudaError_t e = cudaMemsetAsync(m->prog, 0, sizeof(unsigned) * kProgStride * order.size(), m->stream);
         if (e == cudaSuccess)
-            e = launch_resident(groups[0].variant, m->kahan, (int)order.size(), resident_threads(m, order), m->stream, A,
-                                m->prog, false,
-                                pairs && pf == 2);
+        {
+            const int window = resident_window(m, order), cells = resident_cells(window, pairs && pf == 2);
+            e = launch_resident(groups[0].variant, m->kahan, (int)order.size(), resident_threads(window, cells), cells,
+                                m->stream, A, m->prog, false, pairs && pf == 2);
+        }
         if (e != cudaSuccess) return e;
         n = 1;
         nsweeps = 0;
@@ -2017,8 +2117,9 @@ static int cluster_run(MixedState* m, const std::vector<Chunk>& order) {
 // Parts: with few chunks, each is given to several blocks on SMs of their own, which compute windows of
 // part of its cells in the chunk's frame: the same bits at a shorter step.  A block of 8 warps takes about
 // 1200 clocks a step (its 512 cells' packed FP32 instructions, two warps to a scheduler, and the barrier),
-// a window of up to 128 cells in 2 warps little more than the step's dependent chain.  As many parts as
-// bring the window down to 128 cells, as the SMs hold, and as leave every part the halo width.
+// a window of up to 128 cells in 4 warps of one cell per thread little more than the step's dependent
+// chain.  As many parts as bring the window down to 128 cells, as the SMs hold, and as leave every part
+// the halo width.
 static int resident_parts(MixedState* m, const std::vector<Chunk>& order) {
     int parts = device_sms() / (int)order.size();
     int want = 1;
@@ -2068,8 +2169,10 @@ static bool resident_run(MixedState* m, std::vector<Chunk>& order) {
         m->prog_n = chunk_slots(m);
     }
     SweepArgs none{};
-    if (launch_resident(v, m->kahan, (int)blocks.size(), resident_threads(m, blocks), m->stream, none, m->prog, true,
-                        g_pair_flux.load() == 2) != cudaSuccess) {
+    const bool all_pairs = g_pair_flux.load() == 2;
+    const int window = resident_window(m, blocks), cells = resident_cells(window, all_pairs);
+    if (launch_resident(v, m->kahan, (int)blocks.size(), resident_threads(window, cells), cells, m->stream, none, m->prog,
+                        true, all_pairs) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -78,24 +78,41 @@ __device__ __forceinline__ float2 mul2_alone(float2 a, float2 b) {
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(fast_rcp(a.x), fast_rcp(a.y)); }
 __device__ __forceinline__ float2 rsqrt2(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+// the same operations on one cell, with the same names so that both forms share one text (V = float2 or
+// float below)
+__device__ __forceinline__ float neg2(float a) { return -a; }
+__device__ __forceinline__ float add2(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub2(float a, float b) { return __fadd_rn(a, -b); }
+__device__ __forceinline__ float mul2(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float rcp2(float a) { return fast_rcp(a); }
+__device__ __forceinline__ float rsqrt2(float a) { return rsqrtf(a); }
+template <class V>
+__device__ __forceinline__ V splat(float a);
+template <>
+__device__ __forceinline__ float2 splat<float2>(float a) { return f2(a); }
+template <>
+__device__ __forceinline__ float splat<float>(float a) { return a; }
 // lane q of a float2 (q a compile-time constant after unrolling)
 __device__ __forceinline__ float lane(float2 v, int q) { return q ? v.y : v.x; }
 __device__ __forceinline__ void set_lane(float2& v, int q, float x) { if (q) v.y = x; else v.x = x; }
 
 // h + l += v per lane (TwoSum)
-__device__ __forceinline__ void two_sum_acc2(float2& h, float2& l, float2 v) {
-    const float2 s = add2(h, v);
-    const float2 bp = sub2(s, h);
-    const float2 e = add2(sub2(h, sub2(s, bp)), sub2(v, bp));
+template <class V>
+__device__ __forceinline__ void two_sum_acc2(V& h, V& l, V v) {
+    const V s = add2(h, v);
+    const V bp = sub2(s, h);
+    const V e = add2(sub2(h, sub2(s, bp)), sub2(v, bp));
     h = s;
     l = add2(l, e);
 }
 // h + l -= v per lane: the same bits as two_sum_acc2(h, l, -v) (negation commutes with rounding
 // to nearest: (-v) - bp = -(v + bp))
-__device__ __forceinline__ void two_diff_acc2(float2& h, float2& l, float2 v) {
-    const float2 s = sub2(h, v);
-    const float2 bp = sub2(s, h);
-    const float2 e = sub2(sub2(h, sub2(s, bp)), add2(v, bp));
+template <class V>
+__device__ __forceinline__ void two_diff_acc2(V& h, V& l, V v) {
+    const V s = sub2(h, v);
+    const V bp = sub2(s, h);
+    const V e = sub2(sub2(h, sub2(s, bp)), add2(v, bp));
     h = s;
     l = add2(l, e);
 }
@@ -130,12 +147,15 @@ __device__ __forceinline__ float2 slope2(float2 a, float2 b, float alpha) {
 
 // anchor coefficients of a 1D frame, each duplicated into both lanes (negated where the
 // formulas subtract them)
-struct Coef2 {
-    float2 rho, u, nu, ne, T, a, na, M, nM, Z1, Z2, P, gR, R, cvinv, gm1;
-    float2 F[3], Uf[3];
+template <class V>
+struct CoefV {
+    V rho, u, nu, ne, T, a, na, M, nM, Z1, Z2, P, gR, R, cvinv, gm1;
+    V F[3], Uf[3];
 };
-__device__ __forceinline__ Coef2 coef2(const AnchorCoef& c) {
-    Coef2 k;
+template <class V>
+__device__ __forceinline__ CoefV<V> coef2(const AnchorCoef& c) {
+    CoefV<V> k;
+    const auto f2 = [](float a) { return splat<V>(a); };
     k.rho = f2(c.rho); k.u = f2(c.u); k.nu = f2(-c.u); k.ne = f2(-c.e); k.T = f2(c.T); k.a = f2(c.a); k.na = f2(-c.a);
     k.M = f2(c.M); k.nM = f2(-c.M); k.Z1 = f2(c.Z1); k.Z2 = f2(c.Z2); k.P = f2(c.P); k.gR = f2(c.gR);
     k.R = f2(c.R);
@@ -146,43 +166,43 @@ __device__ __forceinline__ Coef2 coef2(const AnchorCoef& c) {
 }
 
 // 1D split-flux deviations of two cells at once (the conserved deviations d = (drho, dm, dE) of
-// both cells as the lanes of FP32x2 registers)
-__device__ __forceinline__ void dflux1x2(const Coef2& c, const float2 d[3], float2 dfp[3], float2 dfm[3]) {
-    const float2 drho = d[0], dm = d[1], dE = d[2];
-    const float2 rho = add2(c.rho, drho);
-    const float2 r = rcp2(rho);
-    const float2 du = mul2(fma2(c.nu, drho, dm), r);
-    const float2 u = add2(c.u, du);
-    const float2 de = mul2(fma2(c.ne, drho, dE), r);
-    const float2 dT = mul2(fma2(f2(-0.5f), mul2(add2(u, c.u), du), de), c.cvinv);
-    const float2 T = add2(c.T, dT);
-    const float2 gRT = mul2(c.gR, T);
-    const float2 ainv = rsqrt2(gRT);
-    const float2 a = mul2(gRT, ainv);
-    const float2 da = mul2(mul2(c.gR, dT), rcp2(add2(a, c.a)));
-    const float2 dM = mul2(fma2(c.nM, da, du), ainv);
-    const float2 M = add2(c.M, dM);
-    const float2 dZ1 = mul2(f2(0.5f), dM);
-    const float2 Z1 = add2(c.Z1, dZ1);
+// both cells as the lanes of FP32x2 registers; V = float: of one cell)
+template <class V>
+__device__ __forceinline__ void dflux1x2(const CoefV<V>& c, const V d[3], V dfp[3], V dfm[3]) {
+    const V drho = d[0], dm = d[1], dE = d[2];
+    const V rho = add2(c.rho, drho);
+    const V r = rcp2(rho);
+    const V du = mul2(fma2(c.nu, drho, dm), r);
+    const V u = add2(c.u, du);
+    const V de = mul2(fma2(c.ne, drho, dE), r);
+    const V dT = mul2(fma2(splat<V>(-0.5f), mul2(add2(u, c.u), du), de), c.cvinv);
+    const V T = add2(c.T, dT);
+    const V gRT = mul2(c.gR, T);
+    const V ainv = rsqrt2(gRT);
+    const V da = mul2(mul2(c.gR, dT), rcp2(fma2(gRT, ainv, c.a)));   // (a = gRT ainv)
+    const V dM = mul2(fma2(c.nM, da, du), ainv);
+    const V M = add2(c.M, dM);
+    const V dZ1 = mul2(splat<V>(0.5f), dM);
+    const V Z1 = add2(c.Z1, dZ1);
     // (negations folded into the operations: -M = (-M*) - dM and -(a* s dM) = ((-a*) s) dM, the
     // same bits as negating the results)
-    const float2 omm = fma2(sub2(c.nM, dM), M, f2(1.0f));
-    const float2 dZ2 = mul2(f2(0.5f), fma2(da, omm, mul2(mul2(c.na, add2(M, c.M)), dM)));
-    const float2 Z2 = add2(c.Z2, dZ2);
+    const V omm = fma2(sub2(c.nM, dM), M, splat<V>(1.0f));
+    const V dZ2 = mul2(splat<V>(0.5f), fma2(da, omm, mul2(mul2(c.na, add2(M, c.M)), dM)));
+    const V Z2 = add2(c.Z2, dZ2);
     // P = (gamma-1)(E - m u / 2): dP = (gamma-1)(dE - (dm u + m* du) / 2).  At a contact (P and u
     // continuous) this cancels kinetic-energy-sized terms, where R (drho T + rho* dT) would cancel
     // internal-energy-sized ones
-    const float2 dP = mul2(c.gm1, fma2(f2(-0.5f), fma2(dm, u, mul2(c.Uf[1], du)), dE));
-    const float2 P = add2(c.P, dP);
-    const float2 E = add2(c.Uf[2], dE);
-    float2 dF[3];
+    const V x = fma2(splat<V>(-0.5f), fma2(dm, u, mul2(c.Uf[1], du)), dE);   // dP = gm1 x
+    const V P = fma2(c.gm1, x, c.P);
+    const V E = add2(c.Uf[2], dE);
+    V dF[3];
     dF[0] = dm;
-    dF[1] = add2(fma2(dm, u, mul2(c.Uf[1], du)), dP);
-    dF[2] = fma2(du, add2(E, P), mul2(c.u, add2(dE, dP)));
+    dF[1] = fma2(c.gm1, x, fma2(dm, u, mul2(c.Uf[1], du)));
+    dF[2] = fma2(du, add2(E, P), mul2(c.u, fma2(c.gm1, x, dE)));
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const float2 a1 = fma2(dF[k], Z1, mul2(c.F[k], dZ1));
-        const float2 a2 = fma2(d[k], Z2, mul2(c.Uf[k], dZ2));
+        const V a1 = fma2(dF[k], Z1, mul2(c.F[k], dZ1));
+        const V a2 = fma2(d[k], Z2, mul2(c.Uf[k], dZ2));
         dfp[k] = add2(a1, a2);
         // fp + fm = F (Z1 - Z3 = 1).  Besides saving the minus-flux products, the difference keeps
         // dfp + dfm = dF to one rounding, which the separately rounded form -(dF Z3 + F* dZ1 + d Z2)
@@ -244,78 +264,83 @@ __device__ __forceinline__ float d2f_bits(double x) {  // truncation to FP32 (sa
 // operand.  Used by the first-order sweeps of chunks in supersonic flow, where the reference scheme
 // amplifies per-step rounding errors (its split gives the u - a wave the negative numerical
 // viscosity a(1 - M)/2 once M > 1), so that FP32 rounding is not enough there.
-struct FF2 {
-    float2 h, l;
+template <class V>
+struct FFV {
+    V h, l;
 };
-__device__ __forceinline__ FF2 ffv(float h, float l) { return {f2(h), f2(l)}; }
+using FF2 = FFV<float2>;
+using FFS = FFV<float>;   // one cell or lane (a scalar instruction takes half the issue time of a packed one)
+template <class V = float2>
+__device__ __forceinline__ FFV<V> ffv(float h, float l) { return {splat<V>(h), splat<V>(l)}; }
 // a * s for a power of two s (exact)
-__device__ __forceinline__ FF2 ffscale(FF2 a, float s) { return {mul2(a.h, f2(s)), mul2(a.l, f2(s))}; }
+template <class V>
+__device__ __forceinline__ FFV<V> ffscale(FFV<V> a, float s) { return {mul2(a.h, splat<V>(s)), mul2(a.l, splat<V>(s))}; }
 // renormalisation of p + e with |e| small against |p|
-__device__ __forceinline__ FF2 ffnorm(float2 p, float2 e) {
-    const float2 h = add2(p, e);
+template <class V>
+__device__ __forceinline__ FFV<V> ffnorm(V p, V e) {
+    const V h = add2(p, e);
     return {h, sub2(e, sub2(h, p))};
+}
+// renormalisation of p + x y, the product unrounded
+template <class V>
+__device__ __forceinline__ FFV<V> ffnorm_mul(V p, V x, V y) {
+    const V h = fma2(x, y, p);
+    return {h, fma2(x, y, sub2(p, h))};
 }
 // sum without the final renormalisation: (s, e) with e = the rounding error of the high parts plus
 // the low parts; for sums that feed another sum or a product
-__device__ __forceinline__ FF2 ffadd_u(FF2 a, FF2 b) {
-    const float2 s = add2(a.h, b.h);
-    const float2 bp = sub2(s, a.h);
-    const float2 e = add2(sub2(a.h, sub2(s, bp)), sub2(b.h, bp));
+template <class V>
+__device__ __forceinline__ FFV<V> ffadd_u(FFV<V> a, FFV<V> b) {
+    const V s = add2(a.h, b.h);
+    const V bp = sub2(s, a.h);
+    const V e = add2(sub2(a.h, sub2(s, bp)), sub2(b.h, bp));
     return {s, add2(e, add2(a.l, b.l))};
 }
-__device__ __forceinline__ FF2 ffadd(FF2 a, FF2 b) {
-    const FF2 t = ffadd_u(a, b);
+template <class V>
+__device__ __forceinline__ FFV<V> ffadd(FFV<V> a, FFV<V> b) {
+    const FFV<V> t = ffadd_u(a, b);
     return ffnorm(t.h, t.l);
 }
 // ffadd(a, -b), written with packed subtracts: a packed operand's negation is not folded, it costs an
 // instruction per lane
-__device__ __forceinline__ FF2 ffsub(FF2 a, FF2 b) {
-    const float2 s = sub2(a.h, b.h);
-    const float2 bp = sub2(s, a.h);
-    const float2 e = sub2(sub2(a.h, sub2(s, bp)), add2(b.h, bp));
+template <class V>
+__device__ __forceinline__ FFV<V> ffsub(FFV<V> a, FFV<V> b) {
+    const V s = sub2(a.h, b.h);
+    const V bp = sub2(s, a.h);
+    const V e = sub2(sub2(a.h, sub2(s, bp)), add2(b.h, bp));
     return ffnorm(s, add2(e, sub2(a.l, b.l)));
-}
-// one lane (a scalar instruction takes half the issue time of a packed one)
-struct FFS {
-    float h, l;
-};
-__device__ __forceinline__ FFS ffadd_u(FFS a, FFS b) {
-    const float s = __fadd_rn(a.h, b.h);
-    const float bp = __fadd_rn(s, -a.h);
-    const float e = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(s, -bp)), __fadd_rn(b.h, -bp));
-    return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
-}
-__device__ __forceinline__ FFS ffmul_u(FFS a, FFS b) {
-    const float p = __fmul_rn(a.h, b.h);
-    return {p, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.h, b.h, -p)))};
 }
 // product left unnormalised, (p, e) with |e| <= about 2^-22 |p|; for products that feed a sum or
 // another product, which renormalise
-__device__ __forceinline__ FF2 ffmul_u(FF2 a, FF2 b) {
-    const float2 p = mul2(a.h, b.h);
-    float2 e = fma2(a.h, b.h, neg2(p));
+template <class V>
+__device__ __forceinline__ FFV<V> ffmul_u(FFV<V> a, FFV<V> b) {
+    const V p = mul2(a.h, b.h);
+    V e = fma2(a.h, b.h, neg2(p));
     e = fma2(a.h, b.l, e);
     return {p, fma2(a.l, b.h, e)};
 }
-__device__ __forceinline__ FF2 ffmul(FF2 a, FF2 b) {
-    const FF2 t = ffmul_u(a, b);
+template <class V>
+__device__ __forceinline__ FFV<V> ffmul(FFV<V> a, FFV<V> b) {
+    const FFV<V> t = ffmul_u(a, b);
     return ffnorm(t.h, t.l);
 }
 // 1/a: r0 = approximate FP32 reciprocal, e = 1 - a r0 (FMA residuals), r = r0 (1 + e + e^2)
-__device__ __forceinline__ FF2 ffrcp(FF2 a) {
-    const float2 r0 = rcp2(a.h);
-    float2 e = fma2(neg2(a.h), r0, f2(1.0f));
+template <class V>
+__device__ __forceinline__ FFV<V> ffrcp(FFV<V> a) {
+    const V r0 = rcp2(a.h);
+    V e = fma2(neg2(a.h), r0, splat<V>(1.0f));
     e = fma2(neg2(a.l), r0, e);
-    return ffnorm(r0, mul2(r0, fma2(e, e, e)));
+    return ffnorm_mul(r0, r0, fma2(e, e, e));
 }
 // sqrt(a), a > 0: FP32 estimate s0 from a Newton-refined reciprocal square root y, then
 // s = s0 + (a - s0^2) y / 2 (the residual a - s0^2 from an FMA)
-__device__ __forceinline__ FF2 ffsqrt(FF2 a) {
-    float2 y = rsqrt2(a.h);
-    y = mul2(y, fma2(mul2(f2(-0.5f), a.h), mul2(y, y), f2(1.5f)));
-    const float2 s0 = mul2(a.h, y);
-    const float2 e = add2(fma2(neg2(s0), s0, a.h), a.l);
-    return ffnorm(s0, mul2(mul2(f2(0.5f), e), y));
+template <class V>
+__device__ __forceinline__ FFV<V> ffsqrt(FFV<V> a) {
+    V y = rsqrt2(a.h);
+    y = mul2(y, fma2(mul2(splat<V>(-0.5f), a.h), mul2(y, y), splat<V>(1.5f)));
+    const V s0 = mul2(a.h, y);
+    const V e = add2(fma2(neg2(s0), s0, a.h), a.l);
+    return ffnorm_mul(s0, mul2(splat<V>(0.5f), e), y);
 }
 
 // The split fluxes of two cells (FP32x2 lanes) with conserved state U (pairs), evaluated directly
@@ -323,17 +348,18 @@ __device__ __forceinline__ FF2 ffsqrt(FF2 a) {
 // equals rho R T, and a^2 = gamma R T = gamma (gamma-1) (E - m u / 2) / rho).  Absolute errors are
 // about 2^-45 of the flux magnitudes, so no deviation form is needed.  gg1 = gamma (gamma-1),
 // gm1 = gamma - 1, as pairs.
-__device__ __forceinline__ void flux1x2_ff(const FF2 U[3], FF2 gg1, FF2 gm1, FF2 fp[3], FF2 fm[3]) {
-    const FF2 r = ffrcp(U[0]);
-    const FF2 u = ffmul(U[1], r);
-    const FF2 mu = ffmul_u(U[1], u);
-    const FF2 eint = ffsub(U[2], ffscale(mu, 0.5f));
-    const FF2 P = ffmul(gm1, eint);
-    const FF2 a = ffsqrt(ffmul(gg1, ffmul_u(eint, r)));
-    const FF2 M = ffmul(u, ffrcp(a));
-    const FF2 Z1 = ffscale(ffadd(M, ffv(1.0f, 0.0f)), 0.5f);
-    const FF2 Z2 = ffmul(ffscale(a, 0.5f), ffsub(ffv(1.0f, 0.0f), ffmul_u(M, M)));
-    FF2 F[3];
+template <class V>
+__device__ __forceinline__ void flux1x2_ff(const FFV<V> U[3], FFV<V> gg1, FFV<V> gm1, FFV<V> fp[3], FFV<V> fm[3]) {
+    const FFV<V> r = ffrcp(U[0]);
+    const FFV<V> u = ffmul(U[1], r);
+    const FFV<V> mu = ffmul_u(U[1], u);
+    const FFV<V> eint = ffsub(U[2], ffscale(mu, 0.5f));
+    const FFV<V> P = ffmul(gm1, eint);
+    const FFV<V> a = ffsqrt(ffmul(gg1, ffmul_u(eint, r)));
+    const FFV<V> M = ffmul(u, ffrcp(a));
+    const FFV<V> Z1 = ffscale(ffadd(M, ffv<V>(1.0f, 0.0f)), 0.5f);
+    const FFV<V> Z2 = ffmul(ffscale(a, 0.5f), ffsub(ffv<V>(1.0f, 0.0f), ffmul_u(M, M)));
+    FFV<V> F[3];
     F[0] = U[1];
     F[1] = ffadd(mu, P);
     F[2] = ffmul(u, ffadd_u(U[2], P));
