@@ -251,6 +251,13 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     Frame1& fr = S.fr;
 
     const int tid = threadIdx.x;
+    // Threads of the chunk's few scalars (rt 0-2 the correction, 0-5 wall terms and record sums, 6-11
+    // frame offsets).  Resident sweeps: the first of a middle warp, which has few or no halo cells to load
+    // and store in the chain between two sweeps (us a step: 65536 cells 1.63 -> 1.58 first, 0.856 ->
+    // 0.839 second order, 10007 cells first order 1.16 -> 1.13); not in the small windows of second order,
+    // whose every warp has halo cells (2048 cells: 0.483 against 0.492).
+    constexpr bool kMiddle = RES && (ORDER == 1 || CELLS == 2);
+    const unsigned rt = kMiddle ? (unsigned)(tid - (int)(blockDim.x / 64) * 32) : (unsigned)tid;
     const int n = tp.n;
     const int steps = min(tp.B, tp.steps - sweep * tp.B);
     if (steps <= 0) return;
@@ -269,11 +276,11 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     // k_sweep1d); L2-only loads, as this SM's L1 may hold the previous window's lines
     const bool early = !RES && !wstart && jw >= 2;
     unsigned fw = 0;
-    double va = 0.0, vb = 0.0;   // threads 0-5: a correction va - vb; 6-11: a frame offset va - vb
+    double va = 0.0, vb = 0.0;   // rt 0-5: a correction va - vb; 6-11: a frame offset va - vb
     if (early) {
         if (tid < kFrameWords) fw = __ldcg(reinterpret_cast<const unsigned*>(&A.frames[ch.id]) + tid);
-        if (tid >= 6 && tid < 12) {
-            const int side = (tid % 6) / 3, k = tid % 3;
+        if (rt >= 6 && rt < 12) {
+            const int side = (int)(rt % 6) / 3, k = (int)(rt % 3);
             const int nb = side == 0 ? ch.idL : ch.idR;
             if (nb >= 0) { va = __ldcg(&A.frames[nb].U[k]); vb = __ldcg(&A.frames[ch.id].U[k]); }
         }
@@ -329,13 +336,13 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     // store of a loaded value stalls the warp until that load returns (in-order issue), which
     // would serialise the L2 round trips
     if (!RES && !wstart && !early && tid < kFrameWords) fw = reinterpret_cast<const unsigned*>(&A.frames[ch.id])[tid];
-    // threads 0-2: the correction owed to cell a by the previous sweep, lam*sum(F_left - F_right)
+    // rt 0-2: the correction owed to cell a by the previous sweep, lam*sum(F_left - F_right)
     // at the interface a-1/2 (the left neighbour's record minus this chunk's), which the owner of
-    // cell a adds at the end of this sweep; threads 6-11: the neighbour-frame offsets
-    const bool cthread = tid < 3 || (tid >= 6 && tid < 12 && !wstart && (!RES || jw == 1));
+    // cell a adds at the end of this sweep; rt 6-11: the neighbour-frame offsets
+    const bool cthread = rt < 3 || (rt >= 6 && rt < 12 && !wstart && (!RES || jw == 1));
     if (cthread) {
-        const int side = (tid % 6) / 3, k = tid % 3;
-        if (tid < 3) {
+        const int side = (int)(rt % 6) / 3, k = (int)(rt % 3);
+        if (rt < 3) {
             if (sweep > 0 && ch.idL >= 0) {
                 const BSum* bs = ((sweep - 1) & 1) ? A.bsum[1] : A.bsum[0];
                 va = ldx<RES>(&bs[ch.idL].s[1][k]);
@@ -349,9 +356,9 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     if (!RES && !wstart && tid < kFrameWords) reinterpret_cast<unsigned*>(&fr)[tid] = fw;
     // as FP32 pairs, once per block; the resident kernel converts the correction only after the
     // steps, so that its loads do not hold up the first step
-    if (cthread && !(RES && tid < 3)) {
-        const int side = (tid % 6) / 3, k = tid % 3;
-        float* o = tid < 3 ? S.corrp[k] : S.dnb[side][k];
+    if (cthread && !(RES && rt < 3)) {
+        const int side = (int)(rt % 6) / 3, k = (int)(rt % 3);
+        float* o = rt < 3 ? S.corrp[k] : S.dnb[side][k];
         d2ff_bits(va - vb, o[0], o[1]);
     }
     if (wstart) {
@@ -378,12 +385,12 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
     if (!RES || jw < 2) __syncthreads();
     if (wstart && !wend && tid < kFrameWords)  // keep the frame for the rest of the window
         reinterpret_cast<unsigned*>(&A.frames[ch.id])[tid] = reinterpret_cast<const unsigned*>(&fr)[tid];
-    if (tid < 6 && ORDER == 1) {
+    if (rt < 6 && ORDER == 1) {
         // reflective walls: constant parts of the wall-cell increments (read after the first step's
         // barrier)
         // cell 0:   lam*F_{-1/2} - lam*Fref = (-lam F0, lam (2 fmS1 - F1), -lam F2) (+2 lam dfm1_0)
         // cell n-1: lam*Fref - lam*F_{n-1/2} = (lam F0, lam (F1 - 2 fpS1), lam F2) (-2 lam dfp1_{n-1})
-        const int bnd = tid / 3, k = tid % 3;
+        const int bnd = (int)(rt / 3), k = (int)(rt % 3);
         double w = bnd == 0 ? (k == 1 ? lam * (2.0 * frp->fmS1 - frp->F[1]) : -lam * frp->F[k])
                             : (k == 1 ? lam * (frp->F[1] - 2.0 * frp->fpS1) : lam * frp->F[k]);
         d2ff_bits(w, S.wall[bnd][k][0], S.wall[bnd][k][1]);
@@ -764,11 +771,11 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
             }
         }
     }
-    if (RES && tid < 3) d2ff_bits(va - vb, S.corrp[tid][0], S.corrp[tid][1]);   // (read after the barrier)
+    if (RES && rt < 3) d2ff_bits(va - vb, S.corrp[rt][0], S.corrp[rt][1]);   // (read after the barrier)
     // ---- boundary flux sums of this sweep (full flux: steps * lam * Fref + sum lam*Delta) ----
     __syncthreads();
-    if (tid < 6) {
-        const int side = tid / 3, k = tid % 3;
+    if (rt < 6) {
+        const int side = (int)(rt / 3), k = (int)(rt % 3);
         if (side == 0 ? hasL : hasR) {
             float h = 0.f, l = 0.f;
             for (int st = 0; st < steps; st++) {
