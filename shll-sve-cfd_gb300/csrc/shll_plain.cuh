@@ -239,6 +239,16 @@ __device__ __forceinline__ double divide_or_zero(double a, const exact_math::Div
     const double q = exact_math::divide_plain(a, d);
     return is_zero(a) ? a : q;
 }
+// x y + z, rounded once where products and sums may be fused.  Written out in cell1 and cell1_lanes: a
+// run's steps are taken by one or the other, as its length has it, and any split of a run into calls gives
+// the same bits only if both fuse the same products.
+__device__ __forceinline__ double product_sum(double x, double y, double z) {
+#if SHLL_PLAIN_FMA
+    return __fma_rn(x, y, z);
+#else
+    return x * y + z;
+#endif
+}
 
 __device__ __forceinline__ int cell1(const Gas<double>& g, const double u[3], double fp[3], double fm[3]) {
     const exact_math::Divisor rho = exact_math::divisor(u[0]);
@@ -250,11 +260,15 @@ __device__ __forceinline__ int cell1(const Gas<double>& g, const double u[3], do
     exact_math::Divisor snd;
     const double a = exact_math::square_root_plain(g.gR * p2, &snd);
     const double M = divide_or_zero(p1, snd);
-    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * (1.0 - M * M);   // twice the reference's
-    const double P = times_R(g, u[0]) * p2;
-    const double F[3] = {u[1], u[1] * p1 + P, p1 * (u[2] + P)};
+    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * product_sum(-M, M, 1.0);   // twice the reference's
+    const double rR = times_R(g, u[0]), P = rR * p2;
+    const double F[3] = {u[1], product_sum(u[1], p1, P), p1 * product_sum(rR, p2, u[2])};
 #pragma unroll
-    for (int k = 0; k < 3; k++) { fp[k] = F[k] * Z1 + u[k] * Z2; fm[k] = -F[k] * Z3 - u[k] * Z2; }
+    for (int k = 0; k < 3; k++) {
+        const double w = u[k] * Z2;
+        fp[k] = product_sum(F[k], Z1, w);
+        fm[k] = product_sum(-F[k], Z3, -w);
+    }
     if (g.plain && in_range(u[0], 923, 200) && in_range(u[2], 923, 200) && momentum_plain(u[1]) && in_range(t, 900, 250))
         return 0;
     const auto c = cell1_general(g, u[0], u[1], u[2]);
@@ -279,20 +293,15 @@ __device__ __forceinline__ int cell1_lanes(const Gas<double>& g, double u, doubl
     exact_math::Divisor snd;
     const double a = exact_math::square_root_plain(g.gR * p2, &snd);
     const double M = divide_or_zero(p1, snd);
-    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * (1.0 - M * M);   // twice the reference's
-    const double P = times_R(g, u0) * p2;
+    const double Z1 = M + 1.0, Z3 = M - 1.0, Z2 = a * product_sum(-M, M, 1.0);   // twice the reference's
+    const double rR = times_R(g, u0), P = rR * p2;
     // F = u1, u1 p1 + P, p1 (u2 + P)
-    double F;
-#if SHLL_PLAIN_FMA
-    F = __fma_rn(k == 2 ? 1.0 : u1, k == 2 ? u2 : p1, P);
-#else
-    F = (k == 2 ? u2 : u1 * p1) + P;
-#endif
+    double F = product_sum(k == 2 ? rR : u1, k == 2 ? p2 : p1, k == 2 ? u2 : P);
     const double F2 = p1 * F;
     F = k == 1 ? F : k == 2 ? F2 : u1;
-    const double v = k == 1 ? u1 : k == 2 ? u2 : u0;
-    fp = F * Z1 + v * Z2;
-    fm = -F * Z3 - v * Z2;
+    const double w = (k == 1 ? u1 : k == 2 ? u2 : u0) * Z2;
+    fp = product_sum(F, Z1, w);
+    fm = product_sum(-F, Z3, -w);
     if (g.plain && in_range(u0, 923, 200) && in_range(u2, 923, 200) && momentum_plain(u1) && in_range(t, 900, 250)) return 0;
     const auto c = cell1_general(g, u0, u1, u2);
     fp = k == 1 ? c.f[1] : k == 2 ? c.f[2] : c.f[0];
