@@ -147,7 +147,8 @@ long shll_steps_taken(const shll_ctx* ctx);
 /* ---- checkpoint / resume on the device ----
  * The reference keeps no checkpoint (results.dat is its only output).  shll_checkpoint copies
  * the state and the step counter into device memory owned by the context; shll_restore puts
- * them back, so a run can be repeated from the same state or split at any step. */
+ * them back, so a run can be repeated from the same state or split at any step.  Restoring also
+ * clears the error flags raised after the checkpoint. */
 int shll_checkpoint(shll_ctx* ctx);
 int shll_restore(shll_ctx* ctx);
 /* Number of CUDA kernels this library has launched in the process so far. */

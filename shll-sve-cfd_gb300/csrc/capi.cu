@@ -602,6 +602,8 @@ extern "C" int shll_restore(shll_ctx* c) {
     c->cur = c->ck_cur;
     CUDA_TRY(c, cudaMemcpyAsync(c->U[c->cur], c->ckU, c->nv * n * rb, cudaMemcpyDeviceToDevice, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(c->P, c->ckP, (c->nv + 1) * n * rb, cudaMemcpyDeviceToDevice, c->stream));
+    // error flags raised after the checkpoint no longer apply (a run would take an expired wait's for its own)
+    CUDA_TRY(c, cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->stream));
     c->steps_taken = c->ck_steps;
     c->fluxes_valid = false;
     return SHLL_OK;
