@@ -176,7 +176,8 @@ EM_FN double minmod_plain(double l, double r, bool* special) {
     const uint64_t lb = em_dbits(l), rb = em_dbits(r);
     const uint64_t la = lb << 1, ra = rb << 1;
     const int el = (int)(la >> 53), er = (int)(ra >> 53);
-    *special = *special || (el + er < 1000 && la != 0 && ra != 0) || el == 2047 || er == 2047;
+    // (1080: a subnormal's exponent, 0 here, stands for up to 52 less; and l and r may be scaled by 2 each)
+    *special = *special || (el + er < 1080 && la != 0 && ra != 0) || el == 2047 || er == 2047;
     const bool negative = (int32_t)((lb ^ rb) >> 32) < 0 && la != 0 && ra != 0;
     const uint64_t m = la < ra ? lb : rb;
     return em_bitsd(negative ? 0 : m);
