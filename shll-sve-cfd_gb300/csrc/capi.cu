@@ -16,6 +16,10 @@
 #include "plain_batch.h"
 #include "shll_internal.h"
 
+// Largest staging planes that a float context holds beside its state: up to here the launches between the
+// copies of load_by_planes would cost 7 % of a transfer and more (524288 cells in 2D; see there).
+constexpr size_t kSmallPlanes = 16u << 20;
+
 struct shll_ctx {
     shll_params p;
     int n = 0, nv = 0, real_bits = 64;
@@ -31,9 +35,8 @@ struct shll_ctx {
     void* P = nullptr;
     void* F[4] = {nullptr, nullptr, nullptr, nullptr};  // fp, fm, hp, hm (staged; lazily allocated)
     bool fluxes_valid = false;
-    double* planes = nullptr;      // staging of primitive planes handed over or back (plain paths)
-    bool own_planes = false;       // an allocation of its own (large problems, by the first use)
-    void* slab = nullptr;          // one allocation: U, P, flags, progress counters, small staging planes
+    double* planes = nullptr;      // staging of a small float problem's primitive planes
+    void* slab = nullptr;          // one allocation: U, P, flags, progress counters, those planes
     unsigned* prog = nullptr;      // progress counters of 1D runs
     // device checkpoint of the plain state
     void* ckU = nullptr;
@@ -233,7 +236,7 @@ static PlainArgs plain_args(shll_ctx* c) {
     a.mc_alpha = c->p.mc_alpha;
     a.flag = c->d_flag;
     a.worst = c->d_flag + 1;
-    a.planes = c->planes;
+    a.planes = c->real_bits == 64 ? static_cast<double*>(c->U[c->cur ^ 1]) : c->planes;
     a.stream = c->stream;
     return a;
 }
@@ -278,13 +281,15 @@ extern "C" int shll_create(const shll_params* p, shll_ctx** out) {
     bool ok = true;
     if (c->plain) {
         // one allocation (each costs tens of microseconds, as does its release): state, primitives, error
-        // flags (with the refused cell and the flags of a state being loaded), progress counters, and the
-        // staging planes of problems up to 64 MB of them
+        // flags (with the refused cell and the flags of a state being loaded) and progress counters.
+        // Primitives handed over or back are staged in the state buffer that is not in use, so that a
+        // context holds no more than its state; only small float problems (kSmallPlanes) have planes of
+        // their own.
         auto up = [](size_t b) { return (b + 255) / 256 * 256; };
         const size_t ub = up(c->nv * n * rb), pb = up((c->nv + 1) * n * rb), fb = 256;
         const size_t gb = c->p.dim == 1 ? up(sizeof(unsigned) * kPlainProgStride * kPlainProgChunks) : 0;
-        size_t sb = up(c->nv * n * sizeof(double));
-        if (sb > (64u << 20)) sb = 0;
+        size_t sb = c->real_bits == 32 ? up(c->nv * n * sizeof(double)) : 0;
+        if (sb > kSmallPlanes) sb = 0;
         unsigned char* m = nullptr;
         ok = cudaMalloc(&m, 2 * ub + pb + fb + gb + sb) == cudaSuccess;
         if (ok) {
@@ -315,7 +320,6 @@ extern "C" void shll_destroy(shll_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     cudaFree(c->slab); cudaFree(c->ckU); cudaFree(c->ckP);
     for (int k = 0; k < 4; k++) cudaFree(c->F[k]);
-    if (c->own_planes) cudaFree(c->planes);
     if (c->mixed) mixed_destroy(c->mixed);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -425,19 +429,6 @@ extern "C" int shll_initial_primitives(const shll_params* p, double* rho, double
     return SHLL_OK;
 }
 
-// nv planes of doubles on the device (plain paths)
-static int ensure_planes(shll_ctx* c) {
-    if (c->planes) return SHLL_OK;
-    if (cudaMalloc(&c->planes, sizeof(double) * c->nv * (size_t)c->n) != cudaSuccess) {
-        cudaGetLastError();
-        c->planes = nullptr;
-        set_err(c, "cudaMalloc of the primitive planes failed");
-        return SHLL_ERR_NOMEM;
-    }
-    c->own_planes = true;
-    return SHLL_OK;
-}
-
 extern "C" int shll_set_primitives(shll_ctx* c, const double* rho, const double* u, const double* v, const double* T) {
     if (!c || !rho || !u || !T || (c->p.dim == 2 && !v)) return SHLL_ERR_ARG;
     if (!c->plain) {  // copied as given and converted (and checked) on the device
@@ -450,19 +441,20 @@ extern "C" int shll_set_primitives(shll_ctx* c, const double* rho, const double*
         return check_flag(c);
     }
     // copied as given (at full link speed from pinned memory), then checked and converted on the device:
-    // one synchronisation, no copy on the host
+    // one synchronisation, no copy on the host.  A refused state leaves the one that is there.
     const size_t n = (size_t)c->n;
-    int rc = ensure_planes(c);
-    if (rc != SHLL_OK) return rc;
     const double* planes[4] = {rho, u, c->p.dim == 2 ? v : T, T};
-    for (int k = 0; k < c->nv; k++)
-        CUDA_TRY(c, cudaMemcpyAsync(c->planes + k * n, planes[k], n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaMemsetAsync(c->d_flag + 1, 0xff, sizeof(int), c->stream));
     CUDA_TRY(c, cudaMemsetAsync(c->d_flag + 2, 0, sizeof(int), c->stream));
     PlainArgs a = plain_args(c);
-    a.Uout = c->U[0];
     a.flag = c->d_flag + 2;
-    CUDA_TRY(c, plain_stage(c, a, STAGE_LOAD));
+    if (a.planes) {
+        for (int k = 0; k < c->nv; k++)
+            CUDA_TRY(c, cudaMemcpyAsync(a.planes + k * n, planes[k], n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        CUDA_TRY(c, plain_stage(c, a, STAGE_LOAD));
+    } else {
+        CUDA_TRY(c, plain_exact::load_by_planes(a, planes, c->U[c->cur ^ 1]));
+    }
     int got[2] = {-1, 0};
     CUDA_TRY(c, cudaMemcpyAsync(got, c->d_flag + 1, sizeof(got), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -473,7 +465,6 @@ extern "C" int shll_set_primitives(shll_ctx* c, const double* rho, const double*
     CUDA_TRY(c, cudaMemcpyAsync(c->d_flag, c->d_flag + 2, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
     c->steps_taken = 0;
     c->fluxes_valid = false;
-    c->cur = 0;
     c->initialized = true;
     if (got[1] & SHLL_FLAG_NONPOSITIVE) {
         set_err(c, "non-positive or NaN density/temperature reached");
@@ -639,12 +630,13 @@ extern "C" int shll_get_primitives(shll_ctx* c, double* rho, double* u, double* 
     double* const* out = c->p.dim == 2 ? d3 : d2;
     const double* src = static_cast<const double*>(c->P);   // FP64: the planes as they are
     if (c->real_bits == 32) {
-        int rc = ensure_planes(c);
-        if (rc != SHLL_OK) return rc;
-        PlainArgs a = plain_args(c);
-        a.planes = c->planes;
+        const PlainArgs a = plain_args(c);
+        if (!a.planes) {
+            CUDA_TRY(c, plain_exact::dump_by_planes(a, out, c->U[c->cur ^ 1]));
+            return SHLL_OK;
+        }
         CUDA_TRY(c, plain_stage(c, a, STAGE_DUMP));
-        src = c->planes;
+        src = a.planes;
     }
     for (int k = 0; k < c->nv; k++)
         if (out[k])

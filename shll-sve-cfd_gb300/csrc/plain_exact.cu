@@ -10,6 +10,12 @@ cudaError_t step(const PlainArgs& a) { return a.real_bits == 32 ? step_t<float>(
 cudaError_t run(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps) {
     return a.real_bits == 32 ? run_t<float>(a, steps, prog, stall, swaps) : run_t<double>(a, steps, prog, stall, swaps);
 }
+cudaError_t load_by_planes(const PlainArgs& a, const double* const* in, void* work) {
+    return load_by_planes_t<float>(a, in, work);
+}
+cudaError_t dump_by_planes(const PlainArgs& a, double* const* out, void* work) {
+    return dump_by_planes_t<float>(a, out, work);
+}
 cudaError_t stage(const PlainArgs& a, int which) {
     return a.real_bits == 32 ? stage_t<float>(a, which) : stage_t<double>(a, which);
 }

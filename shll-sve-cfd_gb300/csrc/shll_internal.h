@@ -38,7 +38,7 @@ struct PlainArgs {
     double R, GAMMA, CV, DT_ON_DX, DT_ON_DY, mc_alpha;
     int* flag;      // error flags; STAGE_LOAD: the flags of the new state
     int* worst;     // STAGE_LOAD: n - 1 - (lowest cell with a non-positive density or temperature), else -1
-    double* planes; // STAGE_LOAD / STAGE_DUMP: nv planes of doubles
+    double* planes; // STAGE_LOAD / STAGE_DUMP: nv planes of doubles (null: load_by_planes, dump_by_planes)
     cudaStream_t stream;
     bool chained;   // a step that follows another of the same run directly (2D: programmatic launch)
 };
@@ -56,4 +56,8 @@ namespace plain_exact {
 cudaError_t step(const PlainArgs& a);
 cudaError_t run(const PlainArgs& a, long steps, unsigned* prog, int stall, int* swaps);
 cudaError_t stage(const PlainArgs& a, int which);
+// float arithmetic: STAGE_LOAD from planes on the host and STAGE_DUMP to such (null: left out), through `work`
+// of a state buffer's size, one or two planes at a time.  dump_by_planes waits for the copies.
+cudaError_t load_by_planes(const PlainArgs& a, const double* const* in, void* work);
+cudaError_t dump_by_planes(const PlainArgs& a, double* const* out, void* work);
 }
