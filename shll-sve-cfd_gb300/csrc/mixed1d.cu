@@ -719,18 +719,20 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
                 else IN = f2(__fadd_rn(Ll, Ro.x));
                 OUT = add2(Lo, make_float2(Ro.y, Rr));
             }
+            // (the remainders' fusion is written out, the same for one cell and two, left and right: both cells
+            // at an interface apply the same term)
             float2 ih, oh, il = f2(0.f), ol = f2(0.f);
             if constexpr (kPackIn) {
                 ih = mul2(lin2, IN); oh = mul2(lout2, OUT);
                 if (!LAM_POW2) {
-                    il = add2(fma2(lin2, IN, neg2(ih)), mul2(llin2, IN));
-                    ol = add2(fma2(lout2, OUT, neg2(oh)), mul2(llout2, OUT));
+                    il = fma2(llin2, IN, fma2(lin2, IN, neg2(ih)));
+                    ol = fma2(llout2, OUT, fma2(lout2, OUT, neg2(oh)));
                 }
             } else {
                 oh = mul2(lout2, OUT);
                 ih = make_float2(__fmul_rn(lamin, IN.x), two ? oh.x : 0.f);
                 if (!LAM_POW2) {
-                    ol = add2(fma2(lout2, OUT, neg2(oh)), mul2(llout2, OUT));
+                    ol = fma2(llout2, OUT, fma2(lout2, OUT, neg2(oh)));
                     il = make_float2(__fmaf_rn(lamlin, IN.x, __fmaf_rn(lamin, IN.x, -ih.x)), two ? ol.x : 0.f);
                 }
             }

@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(NTP, 3) k_step2d(Args2 A) {
         float2 ah = Ph[k], al = Pl[k];
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
             th = mul2(lh, x);
-            tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
+            tl = LAM_POW2 ? f2(0.f) : fma2(ll, x, fma2(lh, x, neg2(th)));
         };
         auto acc = [&](float2 th, float2 tl) {   // (ah, al) += (th, tl)
             two_sum_acc2(ah, al, th);
@@ -817,7 +817,7 @@ struct EdgeTask {
     __device__ __forceinline__ void term(const Dom2& D, const float* f, float& th, float& tl) const {
         const float x = __fadd_rn(f[xa], f[xb]), lh = dir ? D.lyh : D.lxh, ll = dir ? D.lyl : D.lxl;
         th = __fmul_rn(lh, x);
-        // (fused as the assembler fuses the packed form that the cells apply)
+        // (as the cells' packed form)
         tl = LAM_POW2 ? 0.f : __fmaf_rn(ll, x, __fmaf_rn(lh, x, -th));
     }
     // the full flux applied: steps times lam Fref, plus the terms
@@ -932,11 +932,11 @@ __device__ __forceinline__ void step2d2_tile(const Args2& A, const TileD& G, con
     auto update = [&](int b, const bool up[2]) {
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
             th = mul2_alone(lh, x);
-            tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
+            tl = LAM_POW2 ? f2(0.f) : fma2(ll, x, fma2(lh, x, neg2(th)));
         };
         auto lam_wall = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {   // (seen by no other cell)
             th = mul2(lh, x);
-            tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
+            tl = LAM_POW2 ? f2(0.f) : fma2(ll, x, fma2(lh, x, neg2(th)));
         };
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -1227,7 +1227,7 @@ __device__ __forceinline__ void step2d_o2_tile(const Args2& A, const TileD& G, c
         float2 h = ah[k], l = al[k];
         auto lam = [&](float2 lh, float2 ll, float2 x, float2& th, float2& tl) {
             th = mul2_alone(lh, x);
-            tl = LAM_POW2 ? f2(0.f) : add2(fma2(lh, x, neg2(th)), mul2(ll, x));
+            tl = LAM_POW2 ? f2(0.f) : fma2(ll, x, fma2(lh, x, neg2(th)));
         };
         float2 th, tl;
         // x west: F_{i-1/2} = Lx_{i-1} + Rx_i (wall: the cell's own Lx + Rx)
