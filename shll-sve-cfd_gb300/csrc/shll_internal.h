@@ -37,7 +37,7 @@ struct PlainArgs {
     void* fp; void* fm; void* hp; void* hm;
     double R, GAMMA, CV, DT_ON_DX, DT_ON_DY, mc_alpha;
     int* flag;      // error flags; STAGE_LOAD: the flags of the new state
-    int* worst;     // STAGE_LOAD: n - 1 - (lowest cell with a non-positive density or temperature), else -1
+    int* worst;     // STAGE_LOAD: n - (lowest cell with a non-positive density or temperature), else 0
     double* planes; // STAGE_LOAD / STAGE_DUMP: nv planes of doubles (null: load_by_planes, dump_by_planes)
     cudaStream_t stream;
     bool chained;   // a step that follows another of the same run directly (2D: programmatic launch)

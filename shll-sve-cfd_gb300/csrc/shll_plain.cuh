@@ -800,7 +800,7 @@ template <typename REAL>
 __global__ void k_check_planes(const double* __restrict__ in, long n, int nv, int* __restrict__ worst) {
     for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x)
         if (!positive(in[c]) || !positive(in[(nv - 1) * n + c])) {
-            atomicMax(worst, (int)(n - 1 - c));
+            atomicMax(worst, (int)(n - c));
             return;   // (a thread's later cells have higher indices)
         }
 }
@@ -811,7 +811,7 @@ template <typename REAL, typename ENDS>
 __global__ void k_load_planes(const ENDS* ends, long reach, const double* __restrict__ mid, REAL* P, REAL* __restrict__ U,
                               long n, int dim, const __grid_constant__ Gas<REAL> g, const int* __restrict__ worst,
                               int* __restrict__ flag) {
-    if (*worst >= 0) return;
+    if (*worst > 0) return;
     int bad = 0;
     for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
         const REAL p0 = (REAL)ends[c], q1 = (REAL)mid[c], qT = (REAL)ends[reach + c];
@@ -838,7 +838,7 @@ __global__ void k_load_planes(const ENDS* ends, long reach, const double* __rest
 // one plane taken over as REAL, unless worst says that the state is refused
 template <typename REAL, typename IN>
 __global__ void k_take_plane(const IN* __restrict__ in, REAL* __restrict__ out, long n, const int* __restrict__ worst) {
-    if (worst && *worst >= 0) return;
+    if (worst && *worst > 0) return;
     for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) out[c] = (REAL)in[c];
 }
 template <typename REAL>

@@ -2,6 +2,8 @@
 (base_shll.c:202-205) or, refused, leave it; handed back they are the state's; and neither needs device memory
 beside the state.  Sizes below and above the largest with staging planes of their own (float), and an odd
 number of steps before, which leaves the state in the other buffer."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -81,6 +83,30 @@ def test_refused_state_leaves_the_one_that_is_there(shll, oracle, prec, dim, nx,
     ctx.init_state()
     ctx.run()
     assert np.array_equal(out, ctx.primitives())
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", ["f64_exact", "f32_exact"])
+@pytest.mark.parametrize("dim,nx,ny", [(1, 40, 1), (1, 9000, 1), (2, 30, 20), (2, 120, 90)])
+def test_planes_apart_and_adjoining(shll, oracle, prec, dim, nx, ny):
+    """Planes in one buffer (a single copy), in separate ones, and some left out when handed back."""
+    prim = primitives(oracle, prec, dim, nx, ny)
+    ctx = make(shll, prec, dim, nx, ny)
+    hand_over(ctx, prim)
+    whole = ctx.primitives()
+    apart = [p.copy() for p in prim]
+    if dim == 1:
+        ctx.set_primitives(apart[0], apart[1], apart[2])
+    else:
+        ctx.set_primitives(apart[0], apart[1], apart[3], v=apart[2])
+    assert np.array_equal(ctx.primitives(), whole)
+    for left_out in range(-1, dim + 2):
+        out = [np.full(nx * ny, -7.0) for _ in prim]
+        ptr = [None if k == left_out else o.ctypes.data_as(ctypes.POINTER(ctypes.c_double)) for k, o in enumerate(out)]
+        args = ptr if dim == 2 else [ptr[0], ptr[1], None, ptr[2]]
+        assert shll.lib().shll_get_primitives(ctx.h, *args) == shll.OK
+        for k, o in enumerate(out):
+            assert np.all(o == -7.0) if k == left_out else np.array_equal(o, whole[k])
     ctx.close()
 
 
