@@ -69,20 +69,32 @@ struct TubeP {
     float gg1p[2], gm1p[2];  // gamma (gamma-1) and gamma-1 = R/CV as FP32 pairs (pair flux)
 };
 
+// One block's chunk as it is kept and uploaded with every run (28 bytes; with each field an int, 44 bytes, a
+// run of one step of 10^6 second-order cells took 129 us instead of 119).  Ids run along
+// the tubes; a chunk's neighbours are the ids next to it.
 struct Chunk {
     int tube;
     int a, b;        // owned cells [a, b)
     int anc;         // anchor cell of the chunk's frame
-    int id, idL, idR;  // this chunk's and its neighbours' ids (-1 if none), index of bsum
-    // Resident runs may give a chunk to several blocks (parts): this block's cells [sa, sb) of [a, b).
-    // Then id is the part's, idL / idR are the adjacent part of the neighbouring chunk when this part is
-    // the first / last of its chunk (else -1: the cells beyond are a sibling's, in the same frame), and
-    // [w0, w1] are the ids whose previous sweep this part waits for.
-    int sa, sb, w0, w1;
+    int id;          // index of bsum
+    // Resident runs may give a chunk to several blocks (parts): this block's cells are [a + sa, a + sb).  Then id
+    // is the part's.  id - dl and id + dr are the first and last part whose previous sweep this one waits
+    // for: all of the chunk's own and of its neighbours'.
+    short sa, sb, dl, dr;
 };
-inline Chunk whole_chunk(int tube, int a, int b, int anc, int id, int idL, int idR) {
-    return {tube, a, b, anc, id, idL, idR, a, b, idL >= 0 ? idL : id, idR >= 0 ? idR : id};
+inline Chunk whole_chunk(int tube, int a, int b, int anc, int id, bool left, bool right) {
+    return {tube, a, b, anc, id, 0, (short)(b - a), (short)left, (short)right};
 }
+// The same in a kernel: [sa, sb) in cells of the tube, [w0, w1] the ids waited for, and idL / idR the neighbouring
+// chunk's adjacent part when this part is the first / last of its chunk (else -1: a wall, or the cells beyond
+// are a sibling's, in the same frame).
+struct Part {
+    int tube, a, b, anc, id, idL, idR, sa, sb, w0, w1;
+    __device__ __forceinline__ explicit Part(const Chunk& c)
+        : tube(c.tube), a(c.a), b(c.b), anc(c.anc), id(c.id), idL(c.sa == 0 && c.dl > 0 ? c.id - 1 : -1),
+          idR(c.sb == c.b - c.a && c.dr > 0 ? c.id + 1 : -1), sa(c.a + c.sa), sb(c.a + c.sb), w0(c.id - c.dl), w1(c.id + c.dr) {}
+};
+static_assert(sizeof(Chunk) == 28, "packed");
 
 struct Frame1 {
     double U[3];      // anchor state
@@ -184,7 +196,7 @@ constexpr int kPairSmem = 2 * 2 * 3 * MW * (int)sizeof(float);
 
 // the pair-flux decision for a chunk's sweep `sweep` (flags of the previous sweep, or of the
 // state at the start of the run for sweep 0); L2 loads, as the flags are written by other blocks
-__device__ __forceinline__ bool pair_mode(const SweepArgs& A, const Chunk& ch, int sweep) {
+__device__ __forceinline__ bool pair_mode(const SweepArgs& A, const Part& ch, int sweep) {
     const int* f = ((sweep - 1) & 1) ? A.mode[1] : A.mode[0];
     int v = __ldcg(f + ch.id);
     if (ch.idL >= 0) v |= __ldcg(f + ch.idL);
@@ -193,7 +205,7 @@ __device__ __forceinline__ bool pair_mode(const SweepArgs& A, const Chunk& ch, i
 }
 
 // the same for a part of a resident run: any part of the chunk and its neighbours (those it waits for)
-__device__ __forceinline__ bool pair_mode_parts(const SweepArgs& A, const Chunk& ch, int sweep) {
+__device__ __forceinline__ bool pair_mode_parts(const SweepArgs& A, const Part& ch, int sweep) {
     const int* f = ((sweep - 1) & 1) ? A.mode[1] : A.mode[0];
     const int q = ch.w0 + (int)threadIdx.x;
     return __syncthreads_or(q <= ch.w1 && __ldcg(f + q) != 0) != 0;
@@ -245,7 +257,7 @@ __device__ __forceinline__ T ldx(const T* p) {
 // CELLS: cells per thread, two as the lanes of FP32x2 registers, or one (resident runs of small windows:
 // lane x alone, in scalar instructions, which take half the issue time).
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, bool RES, bool FF = false, int CELLS = 2>
-__device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch, const TubeP& tp, Smem1& S,
+__device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch, const TubeP& tp, Smem1& S,
                             float2 (&dh)[3], float2 (&dl)[3], const bool reuse, const bool keep) {
     constexpr int R_ = ORDER;  // stencil reach per step
     Frame1& fr = S.fr;
@@ -861,7 +873,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Chunk& ch
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
 __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
     __shared__ Smem1 S;
-    const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
+    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     float2 dh[3], dl[3];
     // (waits for the previous sweep inside)
@@ -878,7 +890,7 @@ __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
 __global__ void __launch_bounds__(MT, ORDER == 1 ? 3 : 2) k_sweep1d_ff(SweepArgs A) {
     __shared__ Smem1 S;
-    const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
+    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     float2 dh[3], dl[3];
     sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, false, true>(A, A.sweep, ch, tp, S, dh, dl, false, false);
@@ -894,7 +906,7 @@ constexpr int kJumpReach = 16;
 template <bool KAHAN>
 __global__ void __launch_bounds__(256) k_mode1d(SweepArgs A) {
     __shared__ float wmax[8], wmin[8];
-    const Chunk ch = A.chunks[blockIdx.x];
+    const Part ch(A.chunks[blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     int fast = tp.order == 2 && A.pair_m2 < 0.f;   // second order: only where asked for everywhere
     float pmax = 0.f, pmin = 3.0e38f;
@@ -963,7 +975,7 @@ __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, bool CLU, int CELLS = 2>
 __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
     __shared__ Smem1 S;
-    const Chunk ch = A.chunks[A.chunk0 + blockIdx.x];
+    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     const int nsw = (tp.steps + tp.B - 1) / tp.B;
     const int F = tp.fold_sweeps;
@@ -1281,7 +1293,7 @@ template <bool KAHAN>
 __global__ void k_fixup1d(SweepArgs A, int nchunks) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
-    const Chunk ch = A.chunks[c];
+    const Part ch(A.chunks[c]);
     const TubeP tp = A.tubes[ch.tube];
     if (ch.idL < 0 || tp.steps <= 0) return;
     const int sweeps = (tp.steps + tp.B - 1) / tp.B;
@@ -1412,8 +1424,7 @@ static void build_chunks(MixedState* m) {
         for (int c = 0; c < k; c++) anc[c] = c == 0 ? 0 : (c == k - 1 ? n - 1 : (edges[c] + edges[c + 1]) / 2);
         const int id0 = (int)m->chunks.size();
         for (int c = 0; c < k; c++)
-            m->chunks.push_back(whole_chunk(t, edges[c], edges[c + 1], anc[c], id0 + c, c > 0 ? id0 + c - 1 : -1,
-                                            c + 1 < k ? id0 + c + 1 : -1));
+            m->chunks.push_back(whole_chunk(t, edges[c], edges[c + 1], anc[c], id0 + c, c > 0, c + 1 < k));
     }
 }
 
@@ -2147,12 +2158,10 @@ static std::vector<Chunk> split_chunks(const std::vector<Chunk>& order, int part
         for (int q = 0; q < parts; q++) {
             Chunk s = c;
             s.id = c.id * parts + q;
-            s.idL = q == 0 && c.idL >= 0 ? c.idL * parts + parts - 1 : -1;
-            s.idR = q == parts - 1 && c.idR >= 0 ? c.idR * parts : -1;
-            s.sa = c.a + (int)((long)(c.b - c.a) * q / parts);
-            s.sb = c.a + (int)((long)(c.b - c.a) * (q + 1) / parts);
-            s.w0 = (c.idL >= 0 ? c.idL : c.id) * parts;
-            s.w1 = (c.idR >= 0 ? c.idR : c.id) * parts + parts - 1;
+            s.sa = (short)((long)(c.b - c.a) * q / parts);
+            s.sb = (short)((long)(c.b - c.a) * (q + 1) / parts);
+            s.dl = (short)(q + (c.dl > 0 ? parts : 0));
+            s.dr = (short)(parts - 1 - q + (c.dr > 0 ? parts : 0));
             out.push_back(s);
         }
     return out;
@@ -2689,7 +2698,7 @@ extern "C" int shll_tube_run_static(const shll_params* p, double* d_cons, long n
     for (int c = 0; c < k; c++) {
         const int a = (int)((long)n * c / k), b = (int)((long)n * (c + 1) / k);
         const int anc = c == 0 ? 0 : (c == k - 1 ? n - 1 : (a + b) / 2);
-        chunks[c] = whole_chunk(0, a, b, anc, c, c > 0 ? c - 1 : -1, c + 1 < k ? c + 1 : -1);
+        chunks[c] = whole_chunk(0, a, b, anc, c, c > 0, c + 1 < k);
     }
     TubeP* d_tube = reinterpret_cast<TubeP*>(sc + kStaticTubeOff);
     Chunk* d_chunks = reinterpret_cast<Chunk*>(sc + kStaticChunkOff);
