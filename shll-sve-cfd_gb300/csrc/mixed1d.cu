@@ -70,7 +70,7 @@ struct TubeP {
 };
 
 // One block's chunk as it is kept and uploaded with every run (28 bytes; with each field an int, 44 bytes, a
-// run of one step of 10^6 second-order cells took 129 us instead of 119).  Ids run along
+// run of one step of 10^6 second-order cells took 129 us instead of 116).  Ids run along
 // the tubes; a chunk's neighbours are the ids next to it.
 struct Chunk {
     int tube;
@@ -85,14 +85,18 @@ struct Chunk {
 inline Chunk whole_chunk(int tube, int a, int b, int anc, int id, bool left, bool right) {
     return {tube, a, b, anc, id, 0, (short)(b - a), (short)left, (short)right};
 }
-// The same in a kernel: [sa, sb) in cells of the tube, [w0, w1] the ids waited for, and idL / idR the neighbouring
-// chunk's adjacent part when this part is the first / last of its chunk (else -1: a wall, or the cells beyond
-// are a sibling's, in the same frame).
+// The same in a kernel: [sa, sb) in cells of the tube, [w0, w1] the ids waited for, and whether this part is the
+// first / last of its chunk and has a neighbouring chunk there, whose adjacent part is id - 1 / id + 1 (else a
+// wall, or the cells beyond are a sibling's, in the same frame).  (The ids kept instead spill one word
+// more in second-order sweeps.)  RES: of a resident run; every other launch has whole chunks only.
 struct Part {
-    int tube, a, b, anc, id, idL, idR, sa, sb, w0, w1;
-    __device__ __forceinline__ explicit Part(const Chunk& c)
-        : tube(c.tube), a(c.a), b(c.b), anc(c.anc), id(c.id), idL(c.sa == 0 && c.dl > 0 ? c.id - 1 : -1),
-          idR(c.sb == c.b - c.a && c.dr > 0 ? c.id + 1 : -1), sa(c.a + c.sa), sb(c.a + c.sb), w0(c.id - c.dl), w1(c.id + c.dr) {}
+    int tube, a, b, anc, id, left, right, sa, sb, w0, w1;
+    template <bool RES>
+    static __device__ __forceinline__ Part of(const Chunk& c) {
+        const bool left = c.dl > 0 && (!RES || c.sa == 0), right = c.dr > 0 && (!RES || c.sb == c.b - c.a);
+        return {c.tube, c.a, c.b, c.anc, c.id, left, right,
+                RES ? c.a + c.sa : c.a, RES ? c.a + c.sb : c.b, c.id - c.dl, c.id + c.dr};
+    }
 };
 static_assert(sizeof(Chunk) == 28, "packed");
 
@@ -199,8 +203,8 @@ constexpr int kPairSmem = 2 * 2 * 3 * MW * (int)sizeof(float);
 __device__ __forceinline__ bool pair_mode(const SweepArgs& A, const Part& ch, int sweep) {
     const int* f = ((sweep - 1) & 1) ? A.mode[1] : A.mode[0];
     int v = __ldcg(f + ch.id);
-    if (ch.idL >= 0) v |= __ldcg(f + ch.idL);
-    if (ch.idR >= 0) v |= __ldcg(f + ch.idR);
+    if (ch.left) v |= __ldcg(f + ch.id - 1);
+    if (ch.right) v |= __ldcg(f + ch.id + 1);
     return v != 0;
 }
 
@@ -293,7 +297,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch,
         if (tid < kFrameWords) fw = __ldcg(reinterpret_cast<const unsigned*>(&A.frames[ch.id]) + tid);
         if (rt >= 6 && rt < 12) {
             const int side = (int)(rt % 6) / 3, k = (int)(rt % 3);
-            const int nb = side == 0 ? ch.idL : ch.idR;
+            const int nb = side == 0 ? (ch.left ? ch.id - 1 : -1) : (ch.right ? ch.id + 1 : -1);
             if (nb >= 0) { va = __ldcg(&A.frames[nb].U[k]); vb = __ldcg(&A.frames[ch.id].U[k]); }
         }
     }
@@ -355,13 +359,13 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch,
     if (cthread) {
         const int side = (int)(rt % 6) / 3, k = (int)(rt % 3);
         if (rt < 3) {
-            if (sweep > 0 && ch.idL >= 0) {
+            if (sweep > 0 && ch.left) {
                 const BSum* bs = ((sweep - 1) & 1) ? A.bsum[1] : A.bsum[0];
-                va = ldx<RES>(&bs[ch.idL].s[1][k]);
+                va = ldx<RES>(&bs[ch.id - 1].s[1][k]);
                 vb = ldx<RES>(&bs[ch.id].s[0][k]);
             }
         } else if (!early) {
-            const int nb = side == 0 ? ch.idL : ch.idR;
+            const int nb = side == 0 ? (ch.left ? ch.id - 1 : -1) : (ch.right ? ch.id + 1 : -1);
             if (nb >= 0) { va = ldx<RES>(&A.frames[nb].U[k]); vb = ldx<RES>(&A.frames[ch.id].U[k]); }
         }
     }
@@ -420,7 +424,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch,
                     // deviation pair relative to the owner's frame -> relative to this frame
                     h = uh[q][k]; l = ul[q][k];
                     // (a sibling part's cells are in the same frame)
-                    if ((w < pa && ch.idL >= 0) || (w >= pb && ch.idR >= 0)) {
+                    if ((w < pa && ch.left) || (w >= pb && ch.right)) {
                         const int sd = w < pa ? 0 : 1;
                         ff_add(h, l, S.dnb[sd][k][0], S.dnb[sd][k][1], h, l);
                     }
@@ -435,7 +439,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch,
     }
     using V = std::conditional_t<CELLS == 2, float2, float>;
     const auto c2 = coef2<V>(frp->c);
-    const bool hasL = ch.idL >= 0, hasR = ch.idR >= 0;
+    const bool hasL = ch.left, hasR = ch.right;
     // loop-invariant roles of this thread's cells (i = tube cell of window cell w)
     auto edge = [&](int w) { const int i = ws + w; return i <= 0 || i >= n - 1; };
     // half-slope factors: 0.5, or 0 on edge cells (the reference's zero slopes there) and on the
@@ -873,7 +877,7 @@ __device__ void sweep_chunk(const SweepArgs& A, const int sweep, const Part& ch,
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
 __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
     __shared__ Smem1 S;
-    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
+    const Part ch = Part::of<false>(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     float2 dh[3], dl[3];
     // (waits for the previous sweep inside)
@@ -890,7 +894,7 @@ __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
 __global__ void __launch_bounds__(MT, ORDER == 1 ? 3 : 2) k_sweep1d_ff(SweepArgs A) {
     __shared__ Smem1 S;
-    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
+    const Part ch = Part::of<false>(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     float2 dh[3], dl[3];
     sweep_chunk<ORDER, KAHAN, LAM_POW2, LIM, false, true>(A, A.sweep, ch, tp, S, dh, dl, false, false);
@@ -906,7 +910,7 @@ constexpr int kJumpReach = 16;
 template <bool KAHAN>
 __global__ void __launch_bounds__(256) k_mode1d(SweepArgs A) {
     __shared__ float wmax[8], wmin[8];
-    const Part ch(A.chunks[blockIdx.x]);
+    const Part ch = Part::of<true>(A.chunks[blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     int fast = tp.order == 2 && A.pair_m2 < 0.f;   // second order: only where asked for everywhere
     float pmax = 0.f, pmin = 3.0e38f;
@@ -975,7 +979,7 @@ __device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int FM, bool CLU, int CELLS = 2>
 __device__ __forceinline__ void tube_run(const SweepArgs& A, unsigned* prog) {
     __shared__ Smem1 S;
-    const Part ch(A.chunks[A.chunk0 + blockIdx.x]);
+    const Part ch = Part::of<!CLU>(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
     const int nsw = (tp.steps + tp.B - 1) / tp.B;
     const int F = tp.fold_sweeps;
@@ -1293,15 +1297,15 @@ template <bool KAHAN>
 __global__ void k_fixup1d(SweepArgs A, int nchunks) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
-    const Part ch(A.chunks[c]);
+    const Part ch = Part::of<true>(A.chunks[c]);
     const TubeP tp = A.tubes[ch.tube];
-    if (ch.idL < 0 || tp.steps <= 0) return;
+    if (!ch.left || tp.steps <= 0) return;
     const int sweeps = (tp.steps + tp.B - 1) / tp.B;
     const BSum* bs = ((sweeps - 1) & 1) ? A.bsum[1] : A.bsum[0];
     const int buf = (tp.par + sweeps) & 1;
     for (int k = 0; k < 3; k++) {
         const long idx = k * A.plane + tp.base + ch.a;
-        const double corr = boundary_correction(bs, ch.idL, ch.id, k);
+        const double corr = boundary_correction(bs, ch.id - 1, ch.id, k);
         if (KAHAN) {
             float* h = static_cast<float*>(buf ? A.hi[1] : A.hi[0]);
             float* l = buf ? A.lo[1] : A.lo[0];
