@@ -887,12 +887,13 @@ __global__ void __launch_bounds__(MT, 3) k_sweep1d(SweepArgs A) {
 // The pair-flux form of a first-order sweep, launched after the FP32 form for the same chunks
 // (each block runs its chunk only when the chunk's pair-flux decision calls for it).  Its own
 // kernel so that the longer double-FP32 step does not raise the register count, and so lower the
-// occupancy, of the FP32 sweeps.  It is bound by FP32 issue and the barrier of each step: three blocks
-// per SM fit without spills in first order (2^20 cells with the pair flux everywhere: 17.8 -> 16.7 us a
-// step, with the shared interface sums and packed subtracts of the step), but not in second, where it
-// runs only when asked for everywhere.
-template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
-__global__ void __launch_bounds__(MT, ORDER == 1 ? 3 : 2) k_sweep1d_ff(SweepArgs A) {
+// occupancy, of the FP32 sweeps.  It is bound by FP32 issue and the barrier of each step.  BLOCKS per SM: three
+// fit without spills in first order (2^20 cells with the pair flux everywhere: 17.8 -> 16.7 us a step, with the
+// shared interface sums and packed subtracts of the step), but not in second, where it runs only when
+// asked for everywhere.  A block alone takes longer with the registers of three, and where the blocks whose
+// chunk asks for the pair flux do not fill the SMs, that is what a sweep waits for: kThreeBlocks below.
+template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM, int BLOCKS = 2>
+__global__ void __launch_bounds__(MT, BLOCKS) k_sweep1d_ff(SweepArgs A) {
     __shared__ Smem1 S;
     const Part ch = Part::of<false>(A.chunks[A.chunk0 + blockIdx.x]);
     const TubeP tp = A.tubes[ch.tube];
@@ -1104,6 +1105,8 @@ static cudaError_t allow_solo_padding() {
         (const void*)k_sweep1d<2, false, false, 1>, (const void*)k_sweep1d<2, true, false, 1>,
         (const void*)k_sweep1d_ff<1, false, true, 0>, (const void*)k_sweep1d_ff<1, true, true, 0>,
         (const void*)k_sweep1d_ff<1, false, false, 0>, (const void*)k_sweep1d_ff<1, true, false, 0>,
+        (const void*)k_sweep1d_ff<1, false, true, 0, 3>, (const void*)k_sweep1d_ff<1, true, true, 0, 3>,
+        (const void*)k_sweep1d_ff<1, false, false, 0, 3>, (const void*)k_sweep1d_ff<1, true, false, 0, 3>,
         (const void*)k_sweep1d_ff<2, false, true, 0>, (const void*)k_sweep1d_ff<2, true, true, 0>,
         (const void*)k_sweep1d_ff<2, false, false, 0>, (const void*)k_sweep1d_ff<2, true, false, 0>,
         (const void*)k_sweep1d_ff<2, false, true, 1>, (const void*)k_sweep1d_ff<2, true, true, 1>,
@@ -1137,6 +1140,11 @@ static cudaError_t launch_sweep(int variant, bool kahan, int grid, cudaStream_t 
 
 // the pair-flux sweep of a first-order variant group (variants 0, 1); its dynamic shared memory
 // holds the remainders of the split fluxes (within the padding when the grid is a single wave)
+// Chunks per SM from which first-order pair-flux sweeps have three blocks per SM.  Us a step with two / three,
+// tubes of 5000 cells on 152 SMs, half of the chunks in the pair flux (density ratio 8): 165 chunks 3.28 / 4.26, 300
+// 4.07 / 5.06, 600 4.30 / 5.29, 1100 6.09 / 6.62, 1430 7.57 / 7.26, 3300 15.3 / 14.5; with little of it (ratio 2):
+// 165 1.66 / 1.36, 300 1.67 / 1.71, 1100 3.93 / 3.85, 3300 10.1 / 9.8.
+constexpr int kThreeBlocks = 8;
 template <int ORDER, bool KAHAN, bool LAM_POW2, int LIM>
 static cudaError_t launch_one_ff(int grid, cudaStream_t s, const SweepArgs& A, bool pdl) {
     cudaLaunchConfig_t cfg = {};
@@ -1149,7 +1157,11 @@ static cudaError_t launch_one_ff(int grid, cudaStream_t s, const SweepArgs& A, b
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_sweep1d_ff<ORDER, KAHAN, LAM_POW2, LIM>, A);
+    auto* kern = k_sweep1d_ff<ORDER, KAHAN, LAM_POW2, LIM>;
+    if constexpr (ORDER == 1) {
+        if (grid >= kThreeBlocks * device_sms()) kern = k_sweep1d_ff<ORDER, KAHAN, LAM_POW2, LIM, 3>;
+    }
+    return cudaLaunchKernelEx(&cfg, kern, A);
 }
 static cudaError_t launch_sweep_ff(int variant, bool kahan, int grid, cudaStream_t s, const SweepArgs& A, bool pdl) {
     switch (variant * 2 + (kahan ? 1 : 0)) {
