@@ -720,11 +720,12 @@ static dim3 tile_grid(int nx, int ny, int TI) {
 __device__ __forceinline__ int tile_i0(int TI) { return (int)(blockIdx.y + blockIdx.z * gridDim.y) * TI; }
 
 // Consecutive steps are chained by programmatic dependent launch: the next step's blocks are resident
-// and past their launch when this grid completes (griddepcontrol.wait).
+// and past their launch when this grid completes (griddepcontrol.wait).  Uin is written while this grid already
+// runs, so it must not be declared read-only (const __restrict__): such loads may take the non-coherent
+// path, and may be moved above the wait.
 template <typename REAL, int ORDER>
-__global__ void __launch_bounds__(kTileThreads) k_step2(const REAL* __restrict__ Uin, REAL* __restrict__ Uout, int nx,
-                                                        int ny, const __grid_constant__ Gas<REAL> g,
-                                                        int* __restrict__ flag, int TI) {
+__global__ void __launch_bounds__(kTileThreads) k_step2(const REAL* Uin, REAL* Uout, int nx, int ny,
+                                                        const __grid_constant__ Gas<REAL> g, int* flag, int TI) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     step2_tile<REAL, ORDER>(Uin, Uout, nx, ny, (long)nx * ny, g, flag, tile_i0(TI), blockIdx.x * TJ, TI);
