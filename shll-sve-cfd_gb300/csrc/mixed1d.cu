@@ -2155,17 +2155,25 @@ static int cluster_run(MixedState* m, const std::vector<Chunk>& order) {
 // 1200 clocks a step (its 512 cells' packed FP32 instructions, two warps to a scheduler, and the barrier),
 // a window of up to 128 cells in 4 warps of one cell per thread little more than the step's dependent
 // chain.  As many parts as bring the window down to 128 cells, as the SMs hold, and as leave every part
-// the halo width.
+// the halo width.  Not for runs of a few steps, whose time is the descriptors' upload, the launch and the frames,
+// of which more blocks take more: a call of one step of 5000 cells, second order, 34.3 us with parts and 30.9
+// without, of four 34.3 and 31.5.  From six steps on parts are as fast or faster (eight steps of 5000 cells, first
+// order, 49.7 against 55.7; 1500 cells, second order, 31.3 against 33.5), second order with more than 32 blocks from
+// about nine (10000 cells, six steps 36.1 against 33.9, eight 36.4 against 35.1; sixteen of 5000 cells 36.5 against 43.6).
+constexpr int kPartSteps = 6, kPartStepsMany = 9;
 static int resident_parts(MixedState* m, const std::vector<Chunk>& order) {
     int parts = device_sms() / (int)order.size();
-    int want = 1;
+    int want = 1, steps = 0;
+    for (const Chunk& c : order) steps = std::max(steps, m->tubes[c.tube].steps);
     for (const Chunk& c : order) {
         const TubeP& tp = m->tubes[c.tube];
         const int H = tp.order * tp.B, owned = c.b - c.a, to = std::max(H, 128 - 2 * H);
         parts = std::min(parts, owned / H);
         want = std::max(want, (owned + to - 1) / to);
     }
-    return std::max(1, std::min(parts, want));
+    parts = std::max(1, std::min(parts, want));
+    const bool many = m->tubes[order[0].tube].order == 2 && parts * (int)order.size() > 32;
+    return steps < (many ? kPartStepsMany : kPartSteps) ? 1 : parts;
 }
 // the parts of every chunk, in id order (part q of chunk c has id c * parts + q)
 static std::vector<Chunk> split_chunks(const std::vector<Chunk>& order, int parts) {
