@@ -258,8 +258,9 @@ void shll_set_graph_replay(int on);
 /* Resident runs (no counterpart in the reference): a mixed-precision 1D run whose chunks fit on
  * the GPU at once (one block per multiprocessor: a tube of up to about 68000 cells at the default
  * sweep length; fewer chunks are split into parts of a block each) and share one scheme variant is
- * one cooperative launch in which every chunk waits, with a bounded wait, only for its two neighbours' previous sweep, and keeps its frame
- * and its cells' FP32 pairs on chip between the sweeps of a fold window.  Results are identical
+ * one cooperative launch in which every block waits, with a bounded wait, only for the previous sweep
+ * of its two neighbouring chunks and of its own chunk's other parts, and keeps its frame and its cells'
+ * FP32 pairs on chip between the sweeps of a fold window.  Results are identical
  * to the one-launch-per-sweep schedule.  on = 0 selects that schedule for every run (default 1;
  * process-wide).  A wait that gives up makes the run return SHLL_ERR_TIMEOUT. */
 void shll_set_resident(int on);

@@ -47,7 +47,6 @@ EM_FN float em_mul(float a, float b) { EM_PICK(__fmul_rn(a, b), a * b); }
 EM_FN float em_fma(float a, float b, float c) { EM_PICK(__fmaf_rn(a, b, c), fmaf(a, b, c)); }
 EM_FN double em_add(double a, double b) { EM_PICK(__dadd_rn(a, b), a + b); }
 EM_FN double em_mul(double a, double b) { EM_PICK(__dmul_rn(a, b), a * b); }
-EM_FN double em_fma(double a, double b, double c) { EM_PICK(__fma_rn(a, b, c), fma(a, b, c)); }
 
 constexpr uint64_t kOne52 = 1ull << 52;
 
@@ -191,7 +190,8 @@ EM_FN double minmod_general(double l, double r, double inv_scale) {
 // ---- the published arithmetic's double expressions of float values, in FP32 -----------------
 // The reference's float solver widens some expressions to double (its 0.5 and 1.0 literals, sqrt) and
 // rounds the result back to float.  Each value below is first evaluated in FP32 as an unevaluated sum
-// R + rem that is exact to about 2^-21 of half a unit in R's last place (half_ulp); when rem is
+// R + rem that is exact to 2^-18 of half a unit in R's last place (half_ulp; 2^-21 where no
+// cancellation magnifies the rounding of a low part, up to 2^4 is let through); when rem is
 // clear of the half-way points the rounded double expression can only be R, otherwise (a chance of
 // about 2^-17) the double expression itself decides.
 
@@ -210,7 +210,7 @@ static EM_SLOW float sub_product_slow(float u, float c, float s) {
     return (float)em_add((double)u, -em_mul((double)c, (double)s));
 }
 
-// true when R + rem (exact to 2^-18 half units) certainly rounds to R, R in the middle of the range
+// true when R + rem (exact as above) certainly rounds to R, R in the middle of the range
 EM_FN bool rounds_to(float R, float rem) {
     const uint32_t b = em_fbits(R), e = b & 0x7f800000u;
     const float half_ulp = em_bitsf(e - (24u << 23));

@@ -944,9 +944,9 @@ __global__ void __launch_bounds__(256) k_mode1d(SweepArgs A) {
     }
 }
 
-// polls of the neighbours' progress counters before a resident block gives up (under a second,
-// at about half a microsecond per poll; a sweep of a co-resident neighbour takes tens of
-// microseconds)
+// polls of a progress counter (a neighbouring chunk's part or a sibling's, one thread per counter) before a
+// resident block gives up (under a second, at about half a microsecond per poll; a sweep of a
+// co-resident block takes tens of microseconds)
 constexpr long kSpinLimit = 1L << 20;
 // progress counters one 128-byte line apart: a poll then touches only the counter's own line, so
 // the pollers of one chunk do not delay the release stores of the others
@@ -1995,8 +1995,10 @@ static int resident_window(MixedState* m, const std::vector<Chunk>& order) {
 // of one or two warps to a scheduler one cell per thread shortens the step (us a step, first / second
 // order: 10007 cells 1.40 -> 1.15 / 0.66 -> 0.58, 2048 cells 1.40 -> 1.16 / 0.66 -> 0.47, 32768 cells,
 // windows of 270 / 285 cells, 1.63 -> 1.49 / 0.83 -> 0.70); a window of 512 cells is bound by issue, of
-// which two cells per thread need less (65536 cells: 1.64 against 1.73 / 0.855 against 0.862).  No window of
-// a default run lies between 288 and 480 cells.
+// which two cells per thread need less (65536 cells: 1.64 against 1.73 / 0.855 against 0.862).  No window of a
+// single tube's default run lies between 288 and 480 cells; those of a batch do: 70 tubes of 490 to 574 cells
+// (windows of 277 to 319) 1.58 -> 1.46, of 452 to 510 cells, second order (290 to 319), 0.79 -> 0.70.  Windows of
+// 320 to 480 cells with one cell per thread were not measured (two: 1.58 to 1.59 / 0.80).
 static int resident_cells(int window, bool all_pairs) { return window <= kOneCellWindow && !all_pairs ? 1 : 2; }
 // threads over the window
 static int resident_threads(int window, int cells) {

@@ -2,7 +2,7 @@
 // -fmad=false): SHLL_PREC_F64_EXACT batch items are bit-identical to the FP64 reference build,
 // as the single-problem exact path is (plain_exact.cu).
 #define SHLL_PLAIN_NS plain_batch_exact_ns
-#define SHLL_PLAIN_FMA 0   // products and sums may be fused
+#define SHLL_PLAIN_FMA 0   // every product is rounded before it is added
 #include "plain_batch_kernels.cuh"
 
 cudaError_t plain_batch_exact_launch(int dim, int order, int nb, cudaStream_t s, const void* items, const void* blks,

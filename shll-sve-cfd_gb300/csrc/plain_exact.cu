@@ -2,7 +2,7 @@
 // rounded separately (this file is compiled with -fmad=false), IEEE division and square root:
 // bit-identical to the reference's gcc builds (which contain no fused multiply-add on x86-64).
 #define SHLL_PLAIN_NS plain_exact
-#define SHLL_PLAIN_FMA 0   // products and sums may be fused
+#define SHLL_PLAIN_FMA 0   // every product is rounded before it is added
 #include "plain_resident.cuh"
 
 namespace plain_exact {

@@ -744,6 +744,9 @@ static int device_sm_count() {
 // 22.5).  Float steps are bound by latency, which several small tiles on an SM hide from each
 // other: 6 rows (256 x 256, first order: 4.3 us against 5.0 with 14), second order 8 rows (301 x 277:
 // 7.6 us against 8.7 with 10) unless one tile per SM will do (256 x 256: 6.2 us against 7.2 with 8).
+// On large domains the redundant halo rows count for more: 6 / 8 / 12 rows, first order, 700 x 700 12.2 / 11.8 /
+// 11.7 us, 1024 x 1024 23.2 / 22.3 / 21.5, 2048 x 2048 87.9 / 84.0 / 80.5; second order 8 / 16 rows 23.0 / 22.3, 44.9 /
+// 42.3, 175 / 161.  The rule does not follow that yet.
 static int tile_rows(int nx, int ny, int H, int sms, bool wide) {
     int best = kBatchTI;
     long best_tiles = 0;
